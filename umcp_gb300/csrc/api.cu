@@ -480,6 +480,7 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
     block_rows += group_block_rows(prm->precision, G->ncp, G->npt, G->nfaces);
     arena.stage(G->cp, cp);
     arena.stage(G->basis, basis);
+    if (prm->precision == UMCP_FP64) arena.stage(G->table, fixed::basis_table(basis, G->ncp, G->npt, ncpp));
     if (prm->precision == UMCP_FP32_CENTRED) {  // the precision form's kernels read only the FP32 copies
       arena.stage(G->g0f, std::vector<float>(g0.begin(), g0.end()));
       arena.stage(G->rr0f, std::vector<float>(rr0.begin(), rr0.end()));
@@ -598,7 +599,7 @@ size_t umcp::interleave_slots(const std::vector<int> &counts, std::vector<int> *
 
 int umcp::group_blocks(int precision, bool tc, int ncp, int npt, int nfaces) {
   if (tc) return face_blocks_tc(nfaces);
-  return precision == UMCP_FP64 ? face_blocks<double>(nfaces, ncp, npt) : face_blocks<float>(nfaces, ncp, npt);
+  return precision == UMCP_FP64 ? face_blocks64(nfaces) : face_blocks(nfaces, ncp, npt);
 }
 
 int umcp::group_block_rows(int precision, int ncp, int npt, int nfaces) {
@@ -648,29 +649,32 @@ static GeoArgs geo_args(umcp_mesh *m, const double *d_r) {
   return G;
 }
 
-// Face launches of an evaluation at d_r. With restraints on, the area and
-// volume sums run first (the face pass's finish adds their energy) and their
-// gradient is added into the partial slots after it. The irregular groups run
-// on the ctx's side stream beside the regular group; every block of every
-// launch counts toward the finish (FinishArgs::nblk), so whichever block is
-// the last of all sums the block partials.
-template <typename T>
-static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs *fin_in) {
+// Where one evaluation's face launches read positions and write partials,
+// block sums and the status word: the mesh's own buffers, or a caller's.
+struct FaceBuffers {
+  const double *r;
+  F32Pos f32;
+  void *partial;
+  double *blockpart;
+  int *status;
+};
+
+// The face launches of every group. Plain path: one launch. Precision form:
+// one per group, the irregular ones on the ctx's side stream beside the regular
+// one when fork is set. Every block counts toward the finish
+// (FinishArgs::nblk), so whichever block is the last of all sums the block
+// partials.
+static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const FinishArgs &fin, bool fork) {
   cudaStream_t s = m->ctx->stream;
-  FinishArgs none{};
-  FinishArgs fin_geo{};
-  const FinishArgs *fin = fin_in;
-  const bool geo = m->rs.on && fin_in;
-  GeoArgs GA{};
-  if (geo) {
-    GA = geo_args(m, d_r);
-    cudaError_t e = launch_geo_sums(GA, m->precision == UMCP_FP64, s);
-    if (e != cudaSuccess) return e;
-    fin_geo = *fin_in;
-    fin_geo.gterm = m->gterm.as<double>();
-    fin = &fin_geo;
+  if (m->precision == UMCP_FP64) {
+    FaceSet64 F{};
+    for (auto &G : m->groups)
+      F.g[F.ngroups++] = FaceGroup64{G->cp.as<uint32_t>(), G->g0.as<double>(), G->rr0.as<double>(), G->comp.as<double>(),
+                                     G->weight.as<double>(), G->dest.as<int>(), G->table.as<int>(), G->dudv, G->nfaces,
+                                     G->ncp, G->nblocks, G->block_base};
+    return launch_faces64(F, m->P, B.r, (double *)B.partial, B.blockpart, fin, s);
   }
-  const bool fork = m->groups.size() > 1;
+  fork = fork && m->groups.size() > 1;
   if (fork) {
     cudaError_t e = cudaEventRecord(m->ctx->fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(m->ctx->side, m->ctx->fork, 0);
@@ -683,9 +687,6 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
     L.nfaces = G->nfaces;
     L.block_base = G->block_base;
     L.cp = G->cp.as<uint32_t>();
-    L.g0 = G->g0.as<double>();
-    L.rr0 = G->rr0.as<double>();
-    L.comp = G->comp.as<double>();
     L.g0f = G->g0f.as<float>();
     L.rr0f = G->rr0f.as<float>();
     L.compf = G->compf.as<float>();
@@ -693,19 +694,11 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
     L.weight = G->weight.as<double>();
     L.dudv = G->dudv;
     L.irregular = G->irregular;
-    cudaError_t e;
-    if constexpr (sizeof(T) == 4) {
-      if (G->tc)
-        e = launch_faces_tc(L, G->dest.as<int>(), m->P, d_r, m->rhi.as<float>(), m->rlo.as<float>(),
-                            m->dsp.as<float>(), m->partial.as<float>(), m->blockpart.as<double>(), m->status.as<int>(), G->nblocks,
-                            fin ? *fin : none, on);
-      else
-        e = launch_faces<T>(L, G->dest.as<int>(), G->ncp, G->npt, m->P, d_r, m->f32pos(), m->partial.as<T>(), m->blockpart.as<double>(), m->status.as<int>(), G->nblocks,
-                            fin ? *fin : none, on);
-    } else {
-      e = launch_faces<T>(L, G->dest.as<int>(), G->ncp, G->npt, m->P, d_r, m->f32pos(), m->partial.as<T>(), m->blockpart.as<double>(), m->status.as<int>(), G->nblocks,
-                          fin ? *fin : none, on);
-    }
+    const cudaError_t e =
+        G->tc ? launch_faces_tc(L, G->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, (float *)B.partial,
+                                B.blockpart, B.status, G->nblocks, fin, on)
+              : launch_faces(L, G->dest.as<int>(), G->ncp, G->npt, m->P, B.r, B.f32, (float *)B.partial, B.blockpart,
+                             B.status, G->nblocks, fin, on);
     if (e != cudaSuccess) return e;
   }
   if (fork) {
@@ -713,6 +706,27 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
     if (e == cudaSuccess) e = cudaStreamWaitEvent(s, m->ctx->join, 0);
     if (e != cudaSuccess) return e;
   }
+  return cudaSuccess;
+}
+
+// Face launches of an evaluation at d_r. With restraints on, the area and
+// volume sums run first (the face pass's finish adds their energy) and their
+// gradient is added into the partial slots after it.
+template <typename T>
+static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs *fin_in) {
+  cudaStream_t s = m->ctx->stream;
+  FinishArgs fin = fin_in ? *fin_in : FinishArgs{};
+  const bool geo = m->rs.on && fin_in;
+  GeoArgs GA{};
+  if (geo) {
+    GA = geo_args(m, d_r);
+    cudaError_t e = launch_geo_sums(GA, m->precision == UMCP_FP64, s);
+    if (e != cudaSuccess) return e;
+    fin.gterm = m->gterm.as<double>();
+  }
+  const FaceBuffers B{d_r, m->f32pos(), m->partial.p, m->blockpart.as<double>(), m->status.as<int>()};
+  const cudaError_t e = queue_groups(m, B, fin, true);
+  if (e != cudaSuccess) return e;
   if (geo) return launch_geo_grad<T>(GA, m->partial.as<T>(), s);
   return cudaSuccess;
 }
@@ -820,7 +834,7 @@ extern "C" umcp_status umcp_mesh_info_get(const umcp_mesh *m, umcp_mesh_info *in
   long long h2d = (long long)(m->off.bytes + (3 * (size_t)m->nv + 3) * sizeof(double));
   for (auto &G : m->groups)
     for (const DevBuf *x : {&G->cp, &G->g0, &G->rr0, &G->comp, &G->basis, &G->weight, &G->dest, &G->g0f, &G->rr0f,
-                            &G->compf, &G->basis_w})
+                            &G->compf, &G->basis_w, &G->table})
       h2d += (long long)x->bytes;
   info->h2d_bytes = h2d;
   info->mass_form = !m->mrows ? 0 : m->mass_dense ? 1 : 2;
@@ -849,6 +863,7 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
     const size_t ncpp = (size_t)(B.ncp + 3) / 4 * 4;
     b += nf * B.ncp * 4 + (size_t)B.npt * 5 * ncpp * 8 + B.weight.size() * 8 + nf * B.ncp * 4 +
          (size_t)B.npt * B.ncp * 8;
+    if (!f32) b += (size_t)fixed::table_ints(B.ncp, B.npt) * 4;
     const size_t es = f32 ? 4 : 8;  // g0, reference angles and composition in the form's own type
     b += 2 * nf * B.npt * es + nf * 3 * es;
     nblocks += group_block_rows(precision, B.ncp, B.npt, (int)nf);
@@ -1291,40 +1306,17 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
     f32.r0 = m->r0.as<double>();
     f32.dsp = (float *)(base + off_dsp);
   }
-  float *rhi = f32.hi, *rlo = f32.lo;
   cudaStream_t s = m->ctx->stream;
   // The array keeps the previous call's contents: the status word and the
   // finished-block counter must start at zero.
   UMCP_CUDA(cudaMemsetAsync(base + off_flags, 0, 256, s));
   if (fp32) UMCP_CUDA(launch_split_positions(3 * m->nv, d_r, f32, s));
   FinishArgs fin{m->nblocks, d_E, nullptr, d_g ? d_g + 3 * m->nv : nullptr, nullptr, nullptr, 0.0, status, done};
-  for (size_t gi = 0; gi < m->groups.size(); ++gi) {
-    auto &G = m->groups[gi];
-    dev::FaceLaunch L;
-    L.nfaces = G->nfaces;
-    L.block_base = G->block_base;
-    L.cp = G->cp.as<uint32_t>();
-    L.g0 = G->g0.as<double>();
-    L.rr0 = G->rr0.as<double>();
-    L.comp = G->comp.as<double>();
-    L.g0f = G->g0f.as<float>();
-    L.rr0f = G->rr0f.as<float>();
-    L.compf = G->compf.as<float>();
-    L.basis = G->basis.as<double>();
-    L.weight = G->weight.as<double>();
-    L.dudv = G->dudv;
-    L.irregular = G->irregular;
-    const FinishArgs &f = fin;  // every block of every launch counts toward the finish
-    cudaError_t e = (fp32 && G->tc) ? launch_faces_tc(L, G->dest.as<int>(), m->P, d_r, rhi, rlo, f32.dsp,
-                                                       (float *)(base + off_partial), blockpart, status, G->nblocks, f, s)
-                    : fp32 ? launch_faces<float>(L, G->dest.as<int>(), G->ncp, G->npt, m->P, d_r, f32,
-                                               (float *)(base + off_partial), blockpart, status, G->nblocks, f, s)
-                         : launch_faces<double>(L, G->dest.as<int>(), G->ncp, G->npt, m->P, d_r, f32,
-                                                (double *)(base + off_partial), blockpart, status, G->nblocks, f, s);
-    if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("face pass: ") + cudaGetErrorString(e));
-  }
+  const FaceBuffers B{d_r, f32, base + off_partial, blockpart, status};
+  cudaError_t e = queue_groups(m, B, fin, false);
+  if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("face pass: ") + cudaGetErrorString(e));
   if (d_g) {
-    cudaError_t e = fp32 ? launch_gather<float>(m->nv, (float *)(base + off_partial), m->off.as<int>(), d_g, s)
+    e = fp32 ? launch_gather<float>(m->nv, (float *)(base + off_partial), m->off.as<int>(), d_g, s)
                          : launch_gather<double>(m->nv, (double *)(base + off_partial), m->off.as<int>(), d_g, s);
     if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("gather: ") + cudaGetErrorString(e));
   }

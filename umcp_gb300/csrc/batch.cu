@@ -60,6 +60,7 @@ struct umcp_batch {
   int npt[kTypes] = {0, 0, 0};
   double dudv[kTypes] = {0, 0, 0};
   DevBuf basis[kTypes], weight[kTypes];
+  DevBuf table[kTypes];  // FP64: the fixed-point rows instead of basis (fixed64.h)
   int face_grid[kTypes] = {0, 0, 0};
   int vgrid = 0;
   // device tables
@@ -180,7 +181,7 @@ static umcp_status rebuild(umcp_batch *b) {
   // Irregular faces (a few dozen per closed vesicle) go in tiles of at most
   // four faces per half-warp of their kernel, so that they spread over the
   // grid instead of queueing on one block per job.
-  const int hw = b->precision == UMCP_FP64 ? dev::FaceCfg<double>::half_warps : dev::FaceCfg<float>::half_warps;
+  const int hw = b->precision == UMCP_FP64 ? kHalfWarps64 : kHalfWarps32;
   for (int t = 0; t < kTypes; ++t) {
     b->counts[kCountTileBase + t] = (int)tiles.size();
     const int tft = t == 0 ? tf : (b->irr_tile > 0 ? b->irr_tile : std::min(tf, 4 * hw));
@@ -300,11 +301,14 @@ static umcp_status resplit(umcp_batch *b) {
   return UMCP_OK;
 }
 
-template <typename T>
-static cudaError_t queue_faces_t(umcp_batch *b) {
+static cudaError_t queue_faces(umcp_batch *b) {
   cudaStream_t s = b->ctx->stream;
   auto launch = [&](int t, cudaStream_t on) {
-    return launch_batch_faces<T>(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
+    if (b->precision == UMCP_FP64)
+      return launch_batch_faces64(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
+                                  b->table[t].as<int>(), b->weight[t].as<double>(), kTypeNcp[t], b->dudv[t],
+                                  b->d_tile_sums.as<double>(), b->face_grid[t], on);
+    return launch_batch_faces(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
                                  b->basis[t].as<double>(), b->weight[t].as<double>(), kTypeNcp[t], b->npt[t],
                                  b->dudv[t], t > 0, b->d_tile_sums.as<double>(), b->face_grid[t],
                                  b->d_next_tile.as<int>(), on);
@@ -323,10 +327,6 @@ static cudaError_t queue_faces_t(umcp_batch *b) {
     if (b->have_type[t] && (e = launch(t, b->side)) != cudaSuccess) return e;
   if ((e = cudaEventRecord(b->join, b->side)) != cudaSuccess) return e;
   return cudaStreamWaitEvent(s, b->join, 0);
-}
-
-static cudaError_t queue_faces(umcp_batch *b) {
-  return b->precision == UMCP_FP64 ? queue_faces_t<double>(b) : queue_faces_t<float>(b);
 }
 
 static cudaError_t queue_step(umcp_batch *b) {
@@ -478,7 +478,7 @@ static umcp_status autotune(umcp_batch *b, long long faces) {
     }
   }
   const bool f64 = b->precision == UMCP_FP64;
-  const int hw = f64 ? dev::FaceCfg<double>::half_warps : dev::FaceCfg<float>::half_warps;
+  const int hw = f64 ? kHalfWarps64 : kHalfWarps32;
   int sms = 0;
   UMCP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->ctx->device));
   const int max_bps = std::max(1, b->max_grid[0] / std::max(sms, 1));
@@ -493,7 +493,7 @@ static umcp_status autotune(umcp_batch *b, long long faces) {
     L.face_ms = time_face_launches(b, e0, e1, &st);
     if (st == UMCP_OK && (best.tile_faces == 0 || L.face_ms < best.face_ms)) best = L;
   };
-  const int unit = f64 ? dev::FaceCfg<double>::half_warps : 32;
+  const int unit = f64 ? kHalfWarps64 : 32;
   for (int mult : {1, 2, 4, 8, 16, 32, 64}) {
     if ((f64 && mult > 32) || (!f64 && mult < 4)) continue;
     trial(Layout{unit * mult, 4 * hw, max_bps, 0});
@@ -542,8 +542,7 @@ extern "C" umcp_status umcp_batch_create(umcp_ctx *ctx, int precision, const umc
   UMCP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   for (int t = 0; t < kTypes; ++t) {
     const int npt = t == 0 ? 15 : 16;
-    int g = precision == UMCP_FP64 ? batch_face_blocks<double>(kTypeNcp[t], npt)
-                                   : batch_face_blocks<float>(kTypeNcp[t], npt);
+    int g = precision == UMCP_FP64 ? batch_face_blocks64(kTypeNcp[t]) : batch_face_blocks(kTypeNcp[t], npt);
     b->max_grid[t] = std::max(g, 1);
     if (b->opt_blocks_per_sm > 0) g = std::min(g, b->opt_blocks_per_sm * sms);
     b->face_grid[t] = std::max(g, 1);
@@ -594,9 +593,11 @@ extern "C" umcp_status umcp_batch_add(umcp_batch *b, umcp_mesh *m, const umcp_in
     const Group &G = *Gp;
     const int t = type_of(G);
     if (b->have_type[t]) continue;
-    UMCP_CUDA(b->basis[t].alloc(G.basis.bytes));
+    DevBuf &rows = b->precision == UMCP_FP64 ? b->table[t] : b->basis[t];
+    const DevBuf &from = b->precision == UMCP_FP64 ? G.table : G.basis;
+    UMCP_CUDA(rows.alloc(from.bytes));
     UMCP_CUDA(b->weight[t].alloc(G.weight.bytes));
-    UMCP_CUDA(cudaMemcpyAsync(b->basis[t].p, G.basis.p, G.basis.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
+    UMCP_CUDA(cudaMemcpyAsync(rows.p, from.p, from.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
     UMCP_CUDA(cudaMemcpyAsync(b->weight[t].p, G.weight.p, G.weight.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
     b->npt[t] = G.npt;
     b->dudv[t] = G.dudv;

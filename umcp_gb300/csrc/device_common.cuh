@@ -1,0 +1,80 @@
+// Device helpers shared by the kernels' translation units.
+#pragma once
+#include <cuda_runtime.h>
+#include <stdint.h>
+
+#include "launch.h"
+
+namespace umcp {
+namespace dev {
+
+// Programmatic dependent launch: a kernel launched with programmatic stream
+// serialization may start while the kernel before it on the stream finishes;
+// it waits here, before its first read of that kernel's results (a no-op
+// when it was launched without the attribute).
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// A job takes the step when it has neither stopped nor reached its limit.
+__device__ __forceinline__ bool job_active(const BatchFaceJob &J) { return !*J.status && J.cnt[1] < J.limit; }
+
+// Sum of q over the warp in a fixed (xor-tree) order.
+__device__ __forceinline__ double warp_sum(double q) {
+#pragma unroll
+  for (int off = 16; off >= 1; off >>= 1) q += __shfl_xor_sync(0xFFFFFFFFu, q, off);
+  return q;
+}
+
+// Fixed-order sum of the block partials, done by one block of NT threads: each
+// warp takes a quantity at a time, its lanes every 32nd row, then an xor tree.
+// (With a thread per row and a shared-memory tree over the block, every FP64
+// add of the tree cost a warp instruction for a few active lanes.) Writes E,
+// its parts and dE/dalpha; in a run also records E, flags non-finite or
+// diverging energies (src/hd.C:1280-1305) and advances the run index. The
+// box-scale sums are formed only where the caller takes them.
+template <int NT>
+__device__ void finish_sums(const FinishArgs &F, const double *__restrict__ blockpart) {
+  __shared__ double tot[6];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nq = F.galpha ? 6 : 3;
+  for (int q = warp; q < nq; q += NT / 32) {
+    double a = 0;
+    for (int b = lane; b < F.nblk; b += 32) a += __ldcg(&blockpart[6 * (size_t)b + q]);
+    a = warp_sum(a);
+    if (lane == 0) tot[q] = a;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double e = tot[0] + tot[1] + tot[2];
+    if (F.gterm) e += F.gterm[kGeoE];  // the global restraints, summed before the face pass
+    if (F.E) F.E[0] = e;
+    if (F.parts) { F.parts[0] = tot[0]; F.parts[1] = tot[1]; F.parts[2] = tot[2]; }
+    if (F.galpha)
+      for (int c = 0; c < 3; ++c) F.galpha[c] += tot[3 + c] + (F.gterm ? F.gterm[kGeoDAlpha + c] : 0.0);
+    if (!isfinite(e)) atomicOr(F.status, kStatusNonFinite);
+    if (F.energies) {
+      const uint64_t idx = F.cnt[1];
+      F.energies[idx] = e;
+      if (F.threshold > 0 && idx > 0 && e - F.energies[idx - 1] > F.threshold) atomicOr(F.status, kStatusDiverged);
+      F.cnt[1] = idx + 1;
+    }
+  }
+}
+
+// The end of a face launch's block that has written its row of block partials:
+// it counts on F.done, and the block that completes the pass's count sums the
+// rows (the order of that sum does not depend on which block it is).
+template <int NT>
+__device__ __forceinline__ void count_and_finish(const FinishArgs &F, const double *__restrict__ blockpart) {
+  if (!F.done) return;
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = (atomicAdd(F.done, 1u) == (unsigned)F.nblk - 1u);
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  finish_sums<NT>(F, blockpart);
+  if (threadIdx.x == 0) *F.done = 0u;
+}
+
+}  // namespace dev
+}  // namespace umcp

@@ -41,15 +41,12 @@ struct SurfaceParams {
   int nv;
 };
 
-// Per-mesh view for a face launch.
+// Per-mesh view for a face launch of the precision form.
 struct FaceLaunch {
   int nfaces;              // faces in this launch
   int block_base;          // first block-partial row of this launch
   const uint32_t *cp;      // [nfaces][ncp] packed control points
-  const double *g0;        // [nfaces][npt] (plain path)
-  const double *rr0;       // [nfaces][npt]
-  const double *comp;      // [nfaces][3]: P2, Hbar, Pres
-  const float *g0f, *rr0f, *compf;  // the same in FP32 (precision form)
+  const float *g0f, *rr0f, *compf;  // [nfaces][npt], [nfaces][npt], [nfaces][3]: P2, Hbar, Pres
   const double *basis;     // [npt][5][ncp rounded up to 4] rows u,v,uu,uv,vv (staged to shared)
   const double *weight;    // [npt]
   double dudv;

@@ -84,18 +84,33 @@ struct F32Pos {
 
 // Persistent grid of the face pass for one patch type (fixed per device and
 // face count, so the order of every sum is fixed).
-template <typename T>
 int face_blocks(int nfaces, int ncp, int npt);
 
-// Face pass for one patch type (ncp 12/npt 15 regular; ncp 11 or 13, npt 16
-// irregular). T selects the arithmetic: double (plain path) or float
-// (face-centred precision form). partial[dest[f*ncp+x]] receives the
+// The FP64 face pass (face64.cu): every patch type of a mesh in one launch. A
+// group's blocks write the block-partial rows [block_base, block_base + nblocks),
+// the groups' rows following one another from 0.
+struct FaceGroup64 {
+  const uint32_t *cp;
+  const double *g0, *rr0, *comp, *weight;
+  const int *dest, *table;  // gradient-partial slots; the patch type's fixed-point rows (fixed64.h)
+  double dudv;
+  int nfaces, ncp, nblocks, block_base;
+};
+struct FaceSet64 {
+  FaceGroup64 g[3];
+  int ngroups;
+};
+int face_blocks64(int nfaces);
+cudaError_t launch_faces64(const FaceSet64 &F, const dev::SurfaceParams &P, const double *r, double *partial,
+                           double *blockpart, const FinishArgs &fin, cudaStream_t s);
+
+// Face pass of the precision form for one patch type (ncp 12/npt 15 regular;
+// ncp 11 or 13, npt 16 irregular). partial[dest[f*ncp+x]] receives the
 // alpha-scaled gradient of control point x of face f; blockpart[L.block_base
 // + b] receives block b's sums {E_area, E_curvature, E_angle, dE/dalpha_xyz}.
-// f: the FP32 positions and displacements (read by the float instantiation only).
-template <typename T>
+// f: the FP32 positions and displacements.
 cudaError_t launch_faces(const dev::FaceLaunch &L, const int *dest, int ncp, int npt, const dev::SurfaceParams &P,
-                         const double *r, const F32Pos &f, T *partial, double *blockpart, int *status, int grid,
+                         const double *r, const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
                          const FinishArgs &fin, cudaStream_t s);
 
 // The regular faces of the precision form on the tensor cores (face_tc_kernel):
@@ -112,11 +127,6 @@ cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cuda
 
 // *dst |= *src on the device (one thread).
 cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s);
-
-// Fixed-order sum of F.nblk block partials: E, parts (3), galpha (+= 3). With
-// energies/cnt given (a run): energies[cnt[1]] = E, divergence and non-finite
-// flags (src/hd.C:1280-1305), cnt[1] += 1.
-cudaError_t launch_finish(const FinishArgs &F, const double *blockpart, cudaStream_t s);
 
 // Per vertex: g[3v+c] += sum of its partial slots off[2v] + 32 k, k < off[2v+1]
 // (32 vertices interleaved per group, see interleave_slots).
@@ -183,12 +193,15 @@ constexpr int kVertexTile = 256;  // vertices per vertex tile (one thread each)
 // from counts[3 + group] in tiles); tile_sums[3 * global tile] receives each
 // tile's energy terms. Persistent grid; tiles of stopped or finished jobs are
 // skipped.
-template <typename T>
-// next_tile: a device int the regular FP32 launch hands tiles out from (zeroed
-// by the launch wrapper, on s, before the kernel).
+// next_tile: {tiles handed out, blocks done} of the regular launch, which leaves
+// both zero.
 cudaError_t launch_batch_faces(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
                                const double *basis, const double *weight, int ncp, int npt, double dudv,
                                int irregular, double *tile_sums, int grid, int *next_tile, cudaStream_t s);
+// The same in FP64 (table: the patch type's fixed-point rows, fixed64.h).
+cudaError_t launch_batch_faces64(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
+                                 const int *table, const double *weight, int ncp, double dudv, double *tile_sums,
+                                 int grid, cudaStream_t s);
 // Per job: tile sums in listed order (tile_idx[tile_off[j] .. tile_off[j+1])),
 // energy record, flags, steps done; live[j] and prog[j] = {done, status}.
 cudaError_t launch_batch_reduce(const BatchJob *jobs, const int *counts, int max_jobs, const int *tile_off,
@@ -209,8 +222,11 @@ cudaError_t launch_batch_unpack(const BatchJob *jobs, const BatchTile *vtiles, c
 cudaError_t launch_batch_pack(const BatchJob *jobs, const BatchTile *vtiles, const int *counts, const long long *off,
                               double *pack, double *E, int grid, cudaStream_t s);
 // Device-filling grid of a batch face launch for a patch type.
-template <typename T>
 int batch_face_blocks(int ncp, int npt);
+int batch_face_blocks64(int ncp);
+// Faces in flight per block of the half-warp kernels, FP64 and FP32: the units
+// of a batch's tile sizes.
+constexpr int kHalfWarps64 = 4, kHalfWarps32 = 8;
 
 // out[3i+c] (+)= scale/alpha_c^2 * (scalev ? scalev[c*nrow+i] : 1) * sum_k val[k] in[3 col[k]+c].
 // accumulate=0 overwrites out. alphas: device pointer to 3 doubles (or NULL = 1).

@@ -5,10 +5,10 @@
 #include <math.h>
 #include <stdint.h>
 
-#include <mutex>
-
+#include "device_common.cuh"
 #include "kernels.cuh"
 #include "launch.h"
+#include "launch_host.h"
 #include "philox.h"
 
 namespace umcp {
@@ -61,12 +61,6 @@ struct FaceSmem<float, NCP, NPT> {
 };
 
 // Error-free sum: s + e == a + b exactly (Knuth's two-sum).
-// Programmatic dependent launch: a kernel launched with programmatic stream
-// serialization may start while the kernel before it on the stream finishes;
-// it waits here, before its first read of that kernel's results (a no-op
-// when it was launched without the attribute).
-__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 __device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
   s = a + b;
   float bb = s - a;
@@ -94,45 +88,6 @@ struct HalfWarpSums<float> {
   }
   __device__ __forceinline__ double get(int q) const { return (double)s[q] - (double)c[q]; }
 };
-
-// Fixed-order sum of the block partials, done by one block: thread t sums
-// rows t, t+NT, ..., then a shared-memory tree. Writes E, its parts and
-// dE/dalpha; in a run also records E, flags non-finite or diverging energies
-// (src/hd.C:1280-1305) and advances the run index.
-template <int NT>
-__device__ void finish_sums(const FinishArgs &F, const double *__restrict__ blockpart, double (*red)[NT]) {
-  double a[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < F.nblk; b += NT)
-#pragma unroll
-    for (int q = 0; q < 6; ++q) a[q] += __ldcg(&blockpart[6 * (size_t)b + q]);
-#pragma unroll
-  for (int q = 0; q < 6; ++q) red[q][threadIdx.x] = a[q];
-  __syncthreads();
-  for (int width = NT / 2; width > 0; width >>= 1) {
-    if ((int)threadIdx.x < width)
-#pragma unroll
-      for (int q = 0; q < 6; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + width];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    double e = red[0][0] + red[1][0] + red[2][0];
-    double ga[3] = {red[3][0], red[4][0], red[5][0]};
-    if (F.gterm) {  // the global restraints, summed before the face pass
-      e += F.gterm[kGeoE];
-      for (int c = 0; c < 3; ++c) ga[c] += F.gterm[kGeoDAlpha + c];
-    }
-    if (F.E) F.E[0] = e;
-    if (F.parts) { F.parts[0] = red[0][0]; F.parts[1] = red[1][0]; F.parts[2] = red[2][0]; }
-    if (F.galpha) { F.galpha[0] += ga[0]; F.galpha[1] += ga[1]; F.galpha[2] += ga[2]; }
-    if (!isfinite(e)) atomicOr(F.status, kStatusNonFinite);
-    if (F.energies) {
-      const uint64_t idx = F.cnt[1];
-      F.energies[idx] = e;
-      if (F.threshold > 0 && idx > 0 && e - F.energies[idx - 1] > F.threshold) atomicOr(F.status, kStatusDiverged);
-      F.cnt[1] = idx + 1;
-    }
-  }
-}
 
 template <typename T>
 __device__ __forceinline__ T point_data(const double *d64, const float *d32, size_t i) {
@@ -489,7 +444,7 @@ __global__ void __launch_bounds__(FaceCfg<T>::threads, FaceCfg<T>::min_blocks)
   const T dudv = (T)L.dudv;
   const bool reg_alpha = L.irregular && P.k_reg != 0.0;
   const Moduli<T> mod(P);
-  const FaceSrc src{L.cp, L.g0, L.rr0, L.comp, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
+  const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
   HalfWarpSums<T> acc;
 
   const int stride = gridDim.x * HW;
@@ -521,21 +476,7 @@ __global__ void __launch_bounds__(FaceCfg<T>::threads, FaceCfg<T>::min_blocks)
     for (int h = 0; h < HW; ++h) s += sm.red[h][threadIdx.x];
     blockpart[6 * (size_t)(L.block_base + blockIdx.x) + threadIdx.x] = s;
   }
-  if (fin.done) {
-    // The last block of the mesh's last face launch to finish sums all block
-    // partials (the order of that sum does not depend on which block it is).
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(fin.done, 1u) == (unsigned)fin.nblk - 1u);
-    __syncthreads();
-    if (last) {
-      __threadfence();
-      static_assert(sizeof(sm.Tc) >= sizeof(double) * 6 * NT, "finish scratch must fit in the transpose buffer");
-      finish_sums<NT>(fin, blockpart, reinterpret_cast<double(*)[NT]>(sm.scratch()));
-      if (threadIdx.x == 0) *fin.done = 0u;
-    }
-  }
+  count_and_finish<NT>(fin, blockpart);
 }
 
 // ---------------------------------------------------------------- tensor-core face pass
@@ -1074,7 +1015,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
   const float am1[3] = {(float)(r[3 * P.nv] - 1.0), (float)(r[3 * P.nv + 1] - 1.0), (float)(r[3 * P.nv + 2] - 1.0)};
   const Moduli<float> mod(P);
-  const FaceSrc src{L.cp, L.g0, L.rr0, L.comp, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
+  const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
   HalfWarpSums<float> acc;
   uint32_t phase = 0;
   bool ok = true;
@@ -1087,18 +1028,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
   if (!ok && threadIdx.x == 0) atomicOr(status, kStatusTimeout);
   tc::teardown(sm, phase, !ok);
   tc::block_sums(sm, acc, blockpart + 6 * (size_t)(L.block_base + blockIdx.x));
-  if (fin.done) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(fin.done, 1u) == (unsigned)fin.nblk - 1u);
-    __syncthreads();
-    if (last) {
-      __threadfence();
-      finish_sums<tc::kThreads>(fin, blockpart, reinterpret_cast<double(*)[tc::kThreads]>(&sm.A2[0][0]));
-      if (threadIdx.x == 0) *fin.done = 0u;
-    }
-  }
+  count_and_finish<tc::kThreads>(fin, blockpart);
 }
 
 // The precision form's FP32 copies of one position coordinate x = r[i]:
@@ -1124,13 +1054,6 @@ __global__ void split_positions_kernel(int n, const double *__restrict__ r, floa
 __global__ void status_merge_kernel(const int *__restrict__ src, int *__restrict__ dst) {
   const int v = *src;
   if (v) *dst |= v;
-}
-
-// Stand-alone form of the block-partial sum (used when the face launches do
-// not finish themselves).
-__global__ void finish_kernel(FinishArgs F, const double *__restrict__ blockpart) {
-  __shared__ double red[6][256];
-  finish_sums<256>(F, blockpart, red);
 }
 
 // Sum of a vertex's gradient partials in slot order: FP64 in the plain path,
@@ -1392,9 +1315,6 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
 // noise stream, step counter and step limit, so a mesh's trajectory does not
 // depend on what else is in the batch. Tile and job counts are read from
 // device memory, so a captured step stays valid when the membership changes.
-
-// A job takes the step when it has neither stopped nor reached its limit.
-__device__ __forceinline__ bool job_active(const BatchFaceJob &J) { return !*J.status && J.cnt[1] < J.limit; }
 
 template <typename T, int NCP, int NPT>
 __global__ void __launch_bounds__(FaceCfg<T>::threads, FaceCfg<T>::min_blocks)
@@ -1760,13 +1680,6 @@ struct SharedSums {
   }
 };
 
-// Sum of q over the warp in a fixed (xor-tree) order.
-__device__ __forceinline__ double warp_sum(double q) {
-#pragma unroll
-  for (int off = 16; off >= 1; off >>= 1) q += __shfl_xor_sync(0xFFFFFFFFu, q, off);
-  return q;
-}
-
 // Single mesh, regular faces, precision form: persistent grid, warp w of the
 // grid takes faces 32 w .. 32 w + 31, then 32 (w + warps in the grid) ...
 // Writes one block partial of the energy terms and dE/dalpha; the last block
@@ -1787,7 +1700,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
   const float am1[3] = {(float)(r[3 * P.nv] - 1.0), (float)(r[3 * P.nv + 1] - 1.0), (float)(r[3 * P.nv + 2] - 1.0)};
   const Moduli<float> mod(P);
-  const FaceSrc src{L.cp, L.g0, L.rr0, L.comp, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
+  const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
   const bool vec = tpf_vec(src);
   const float dudv = (float)L.dudv;
   const bool kg_reg = P.kg != 0.0 || P.k_reg != 0.0;  // else the pointwise step leaves those terms out
@@ -1819,19 +1732,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
     for (int w = 0; w < kWarps; ++w) s += sm.red[w][threadIdx.x];
     blockpart[6 * (size_t)(L.block_base + blockIdx.x) + threadIdx.x] = s;
   }
-  if (fin.done) {
-    __shared__ bool last;
-    __threadfence();
-    __syncthreads();
-    if (threadIdx.x == 0) last = (atomicAdd(fin.done, 1u) == (unsigned)fin.nblk - 1u);
-    __syncthreads();
-    if (last) {
-      __threadfence();
-      static_assert(kSumBytes >= sizeof(double) * 6 * kThreads, "finish scratch must fit in the sums' space");
-      finish_sums<kThreads>(fin, blockpart, reinterpret_cast<double(*)[kThreads]>(tpf_dyn));
-      if (threadIdx.x == 0) *fin.done = 0u;
-    }
-  }
+  count_and_finish<kThreads>(fin, blockpart);
 }
 
 // Batched regular faces, precision form: a block takes a tile (faces of one
@@ -2774,46 +2675,6 @@ __global__ void to_f32x4_kernel(int n, const double *__restrict__ in, float4 *__
 
 }  // namespace dev
 
-static int grid_for(int n, int per_block) {
-  int g = (n + per_block - 1) / per_block;
-  return g < 1 ? 1 : g;
-}
-
-// A value fixed per device and computed once on it (thread-safe: meshes may
-// be made on several threads). cudaFuncSetAttribute applies to the current
-// device only, and the persistent grids follow each device's SM count, so
-// neither may be shared between the devices of one process.
-constexpr int kMaxDevices = 64;
-// Launch with programmatic stream serialization: the kernel may be scheduled
-// while the kernel before it on the stream drains, and waits for it in
-// grid_dependency_wait (which it calls before reading that kernel's results).
-template <typename... P, typename... A>
-static cudaError_t launch_after(void (*kernel)(P...), int grid, int block, size_t smem, cudaStream_t s, A... args) {
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3((unsigned)block);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
-}
-
-struct PerDevice {
-  std::once_flag once[kMaxDevices];
-  int value[kMaxDevices] = {};
-};
-template <class F>
-static int per_device(PerDevice &pd, F make) {
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= kMaxDevices) return make();
-  std::call_once(pd.once[dev], [&] { pd.value[dev] = make(); });
-  return pd.value[dev];
-}
 // The dynamic shared memory limit above 48 KB that the tensor-core kernel
 // opts into, once per device; returns the cudaError_t of the opt-in.
 static cudaError_t tc_opt_in() {
@@ -2823,16 +2684,6 @@ static cudaError_t tc_opt_in() {
                                      (int)dev::tc::kSmemBytes);
   });
 }
-static int sm_count() {
-  static PerDevice pd;
-  return per_device(pd, [] {
-    int dev = 0, n = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-    return n > 0 ? n : 1;
-  });
-}
-
 template <typename T, int NCP, int NPT>
 static int face_grid_size(int nfaces) {
   // Persistent grid: as many blocks as fit on the device at once (a fixed
@@ -2861,50 +2712,32 @@ static int face_grid_size_tpf(int nfaces) {
   return need < cached ? need : cached;
 }
 
-template <typename T>
 int face_blocks(int nfaces, int ncp, int npt) {
   if (nfaces <= 0) return 0;
-  if (sizeof(T) == 4 && ncp == 12 && npt == 15) return face_grid_size_tpf(nfaces);
-  if (ncp == 12 && npt == 15) return face_grid_size<T, 12, 15>(nfaces);
-  if (ncp == 11 && npt == 16) return face_grid_size<T, 11, 16>(nfaces);
-  if (ncp == 13 && npt == 16) return face_grid_size<T, 13, 16>(nfaces);
+  if (ncp == 12 && npt == 15) return face_grid_size_tpf(nfaces);
+  if (ncp == 11 && npt == 16) return face_grid_size<float, 11, 16>(nfaces);
+  if (ncp == 13 && npt == 16) return face_grid_size<float, 13, 16>(nfaces);
   return 0;
 }
-template int face_blocks<double>(int, int, int);
-template int face_blocks<float>(int, int, int);
 
-template <typename T>
 cudaError_t launch_faces(const dev::FaceLaunch &L, const int *dest, int ncp, int npt, const dev::SurfaceParams &P,
-                         const double *r, const F32Pos &f, T *partial, double *blockpart, int *status, int grid,
+                         const double *r, const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
                          const FinishArgs &fin, cudaStream_t s) {
   if (L.nfaces <= 0) return cudaSuccess;
-  constexpr int NT = dev::FaceCfg<T>::threads;
+  constexpr int NT = dev::FaceCfg<float>::threads;
   const float *rhi = f.hi, *rlo = f.lo, *dsp = f.dsp;
-  if constexpr (sizeof(T) == 4) {
-    if (!rhi || !rlo || !dsp) return cudaErrorInvalidValue;
-    if (ncp == 12 && npt == 15)
-      return launch_after(dev::face_tpf_kernel, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, rhi,
-                          rlo, dsp, partial, blockpart, status, fin);
-  }
+  if (!rhi || !rlo || !dsp) return cudaErrorInvalidValue;
   if (ncp == 12 && npt == 15)
-    return launch_after(dev::face_kernel<T, 12, 15>, grid, NT, 0, s, L, dest, P, r, rhi, rlo, dsp, partial, blockpart,
-                        status, fin);
-  else if (ncp == 11 && npt == 16)
-    dev::face_kernel<T, 11, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status,
-                                                           fin);
+    return launch_after(dev::face_tpf_kernel, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, rhi,
+                        rlo, dsp, partial, blockpart, status, fin);
+  if (ncp == 11 && npt == 16)
+    dev::face_kernel<float, 11, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status, fin);
   else if (ncp == 13 && npt == 16)
-    dev::face_kernel<T, 13, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status,
-                                                           fin);
+    dev::face_kernel<float, 13, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status, fin);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
-template cudaError_t launch_faces<double>(const dev::FaceLaunch &, const int *, int, int, const dev::SurfaceParams &,
-                                          const double *, const F32Pos &, double *, double *, int *, int,
-                                          const FinishArgs &, cudaStream_t);
-template cudaError_t launch_faces<float>(const dev::FaceLaunch &, const int *, int, int, const dev::SurfaceParams &,
-                                         const double *, const F32Pos &, float *, double *, int *, int,
-                                         const FinishArgs &, cudaStream_t);
 
 cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
@@ -2915,11 +2748,6 @@ cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cuda
 
 cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s) {
   dev::status_merge_kernel<<<1, 1, 0, s>>>(src, dst);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_finish(const FinishArgs &F, const double *blockpart, cudaStream_t s) {
-  dev::finish_kernel<<<1, 256, 0, s>>>(F, blockpart);
   return cudaGetLastError();
 }
 
@@ -2990,9 +2818,8 @@ cudaError_t launch_spmv(int nrow, const int *row_ptr, const int *col, const doub
 
 namespace umcp {
 
-template <typename T>
 int batch_face_blocks(int ncp, int npt) {
-  if (sizeof(T) == 4 && ncp == 12 && npt == 15) {  // the batched thread-per-face kernel's own occupancy
+  if (ncp == 12 && npt == 15) {  // the batched thread-per-face kernel's own occupancy
     static PerDevice pd;
     return per_device(pd, [] {
       int per_sm = 0;
@@ -3000,42 +2827,28 @@ int batch_face_blocks(int ncp, int npt) {
       return sm_count() * (per_sm > 0 ? per_sm : 1);
     });
   }
-  return face_blocks<T>(1 << 30, ncp, npt);  // device-filling persistent grid
+  return face_blocks(1 << 30, ncp, npt);  // device-filling persistent grid
 }
-template int batch_face_blocks<double>(int, int);
-template int batch_face_blocks<float>(int, int);
 
-template <typename T>
 cudaError_t launch_batch_faces(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
                                const double *basis, const double *weight, int ncp, int npt, double dudv,
                                int irregular, double *tile_sums, int grid, int *next_tile, cudaStream_t s) {
-  constexpr int NT = dev::FaceCfg<T>::threads;
-  if constexpr (sizeof(T) == 4) {
-    if (ncp == 12 && npt == 15) {
-      if (!next_tile) return cudaErrorInvalidValue;
-      return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, jobs, group, tiles, counts,
-                          basis, weight, dudv, tile_sums, next_tile);
-    }
+  constexpr int NT = dev::FaceCfg<float>::threads;
+  if (ncp == 12 && npt == 15) {
+    if (!next_tile) return cudaErrorInvalidValue;
+    return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, jobs, group, tiles, counts, basis,
+                        weight, dudv, tile_sums, next_tile);
   }
-  if (ncp == 12 && npt == 15)
-    dev::batch_face_kernel<T, 12, 15><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv, irregular,
-                                                          tile_sums);
-  else if (ncp == 11 && npt == 16)
-    dev::batch_face_kernel<T, 11, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv, irregular,
-                                                          tile_sums);
+  if (ncp == 11 && npt == 16)
+    dev::batch_face_kernel<float, 11, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv,
+                                                              irregular, tile_sums);
   else if (ncp == 13 && npt == 16)
-    dev::batch_face_kernel<T, 13, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv, irregular,
-                                                          tile_sums);
+    dev::batch_face_kernel<float, 13, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv,
+                                                              irregular, tile_sums);
   else
     return cudaErrorInvalidValue;
   return cudaGetLastError();
 }
-template cudaError_t launch_batch_faces<double>(const BatchJob *, int, const BatchTile *, const int *,
-                                                const double *, const double *, int, int, double, int, double *, int,
-                                                int *, cudaStream_t);
-template cudaError_t launch_batch_faces<float>(const BatchJob *, int, const BatchTile *, const int *, const double *,
-                                               const double *, int, int, double, int, double *, int, int *,
-                                               cudaStream_t);
 
 cudaError_t launch_batch_reduce(const BatchJob *jobs, const int *counts, int max_jobs, const int *tile_off,
                                 const int *tile_idx, const double *tile_sums, int *live, unsigned long long *prog,
