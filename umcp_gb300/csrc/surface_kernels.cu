@@ -1056,38 +1056,51 @@ __global__ void status_merge_kernel(const int *__restrict__ src, int *__restrict
   if (v) *dst |= v;
 }
 
-// Sum of a vertex's gradient partials in slot order: FP64 in the plain path,
-// FP32 with Kahan compensation in the precision form.
-// Sum of vertex v's gradient partials: its slots are loc[2 v] + 32 k for
-// k < loc[2 v + 1] (32 vertices interleaved, so the 32 lanes of a warp read
-// consecutive slots), summed in k order (FP64, or Kahan FP32).
+// Sum of coordinate c of vertex v's gradient partials: its slots are
+// loc[2 v] + 32 k for k < loc[2 v + 1] (32 vertices interleaved, so the lanes of
+// a warp read consecutive slots), summed in k order (FP64, or FP32 with Kahan
+// compensation: hi - lo). Eight slots' loads are issued before they are added;
+// every partial is read once (evict-first).
+template <typename T, class F>
+__device__ __forceinline__ void each_partial(const T *__restrict__ partial, int base, int n, int c, F add) {
+  const T *q = partial + 3 * (size_t)base + c;
+  int k = 0;
+  for (; k + 8 <= n; k += 8) {
+    T x[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) x[i] = __ldcs(q + 96 * (size_t)(k + i));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) add(x[i]);
+  }
+  for (; k < n; ++k) add(__ldcs(q + 96 * (size_t)k));
+}
+struct GradSum {
+  float hi, lo;
+};
+__device__ __forceinline__ GradSum coordinate_sum(const float *__restrict__ partial, int base, int n, int c) {
+  GradSum s{0.f, 0.f};
+  each_partial(partial, base, n, c, [&](float x) {
+    const float y = x - s.lo, t = s.hi + y;
+    s.lo = (t - s.hi) - y;
+    s.hi = t;
+  });
+  return s;
+}
+__device__ __forceinline__ double coordinate_gradient(const float *__restrict__ partial, int base, int n, int c) {
+  const GradSum s = coordinate_sum(partial, base, n, c);
+  return (double)s.hi - (double)s.lo;
+}
+__device__ __forceinline__ double coordinate_gradient(const double *__restrict__ partial, int base, int n, int c) {
+  double a = 0;
+  each_partial(partial, base, n, c, [&](double x) { a += x; });
+  return a;
+}
 template <typename T>
 __device__ __forceinline__ void vertex_gradient(const T *__restrict__ partial, const int *__restrict__ loc, int v,
                                                 double gg[3]) {
   const int base = loc[2 * (size_t)v], n = loc[2 * (size_t)v + 1];
-  if constexpr (sizeof(T) == 8) {
-    double a0 = 0, a1 = 0, a2 = 0;
-    for (int k = 0; k < n; ++k) {
-      const size_t s = (size_t)base + 32 * (size_t)k;
-      a0 += partial[3 * s];
-      a1 += partial[3 * s + 1];
-      a2 += partial[3 * s + 2];
-    }
-    gg[0] = a0; gg[1] = a1; gg[2] = a2;
-  } else {
-    float s3[3] = {0, 0, 0}, c3[3] = {0, 0, 0};
-    for (int k = 0; k < n; ++k) {
-      const size_t s = (size_t)base + 32 * (size_t)k;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float y = partial[3 * s + c] - c3[c], t = s3[c] + y;
-        c3[c] = (t - s3[c]) - y;
-        s3[c] = t;
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) gg[c] = (double)s3[c] - (double)c3[c];
-  }
+  for (int c = 0; c < 3; ++c) gg[c] = coordinate_gradient(partial, base, n, c);
 }
 
 // The same sum in the precision form, its compensated total rounded to FP32.
@@ -1126,90 +1139,84 @@ __device__ __forceinline__ void vertex_gradient_f32(const float *__restrict__ pa
   for (int c = 0; c < 3; ++c) g[c] = s3[c] - c3[c];
 }
 
+// g += the gathered gradient, one thread per coordinate: on meshes of a few
+// thousand vertices a thread per vertex left most of the GPU idle while its 72
+// adds (64 cycles each in FP64) ran one after another.
 template <typename T>
 __global__ void gather_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off,
                               double *__restrict__ g) {
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    double gg[3];
-    vertex_gradient(partial, off, v, gg);
-    g[3 * (size_t)v] += gg[0];
-    g[3 * (size_t)v + 1] += gg[1];
-    g[3 * (size_t)v + 2] += gg[2];
+  grid_dependency_wait();  // the partials come from the face launches
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
+    const int v = i / 3, c = i - 3 * v;
+    const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
+    g[i] += coordinate_gradient(partial, at.x, at.y, c);
   }
 }
 
-// Three unit normals per vertex from two Philox draws (Box-Muller). The
-// plain path transforms in FP64 (bit-for-bit the oracle's draws up to libm
-// rounding); the precision form in FP32 from 24-bit uniforms.
-__device__ __forceinline__ void normals3_f32(uint64_t seed, uint32_t stream, uint64_t step, int v, float n[3]) {
-  philox_out o = philox4x32_10((uint32_t)v, (uint32_t)step, (uint32_t)(step >> 32), stream, (uint32_t)seed,
-                               (uint32_t)(seed >> 32));
+// Component c of a vertex's three unit normals (Box-Muller on Philox draws). The
+// plain path transforms two draws in FP64 (the oracle's draws up to libm
+// rounding), the precision form one draw in FP32 from 24-bit uniforms.
+// Components 0 and 1 are the cosine and sine of one pair of uniforms, 2 the
+// cosine of another. Every kernel takes its normals from here, whether a thread
+// draws one component or three, so that all draw the same bits.
+__device__ __forceinline__ float normal_f32(const philox_out &o, int c) {
   const float k = 1.0f / 16777216.0f;
-  float u1 = ((float)(o.v[0] >> 8) + 0.5f) * k, u2 = ((float)(o.v[1] >> 8) + 0.5f) * k;
-  float u3 = ((float)(o.v[2] >> 8) + 0.5f) * k, u4 = ((float)(o.v[3] >> 8) + 0.5f) * k;
-  float rad = sqrtf(-2.0f * logf(u1)), sn, cs;
-  sincospif(2.0f * u2, &sn, &cs);
-  n[0] = rad * cs;
-  n[1] = rad * sn;
-  n[2] = sqrtf(-2.0f * logf(u3)) * cospif(2.0f * u4);
+  const float ua = ((float)((c == 2 ? o.v[2] : o.v[0]) >> 8) + 0.5f) * k;
+  const float ub = ((float)((c == 2 ? o.v[3] : o.v[1]) >> 8) + 0.5f) * k;
+  const float rad = sqrtf(-2.0f * logf(ua));
+  float sn, cs;
+  sincospif(2.0f * ub, &sn, &cs);
+  return rad * (c == 1 ? sn : cs);
 }
-__device__ __forceinline__ void normals3_f32(uint64_t seed, uint32_t stream, uint64_t step, int v, double n[3]) {
-  float f[3];
-  normals3_f32(seed, stream, step, v, f);
-  n[0] = f[0];
-  n[1] = f[1];
-  n[2] = f[2];
-}
-
-__device__ __forceinline__ void normals3(uint64_t seed, uint32_t stream, uint64_t step, int v, double n[3]) {
-  philox_out o = philox4x32_10((uint32_t)v, (uint32_t)step, (uint32_t)(step >> 32), stream, (uint32_t)seed,
-                               (uint32_t)(seed >> 32));
-  double u1 = philox_u53(o.v[0], o.v[1]), u2 = philox_u53(o.v[2], o.v[3]);
-  double rad = sqrt(-2.0 * log(u1)), sn, cs;
+__device__ __forceinline__ double normal_f64(const philox_out &o, int c) {
+  const double u1 = philox_u53(o.v[0], o.v[1]), u2 = philox_u53(o.v[2], o.v[3]);
+  const double rad = sqrt(-2.0 * log(u1));
+  double sn, cs;
   sincospi(2.0 * u2, &sn, &cs);
-  n[0] = rad * cs;
-  n[1] = rad * sn;
-  o = philox4x32_10((uint32_t)v, (uint32_t)step, (uint32_t)(step >> 32), stream | 0x80000000u, (uint32_t)seed,
-                    (uint32_t)(seed >> 32));
-  u1 = philox_u53(o.v[0], o.v[1]);
-  u2 = philox_u53(o.v[2], o.v[3]);
-  rad = sqrt(-2.0 * log(u1));
-  n[2] = rad * cospi(2.0 * u2);
+  return rad * (c == 1 ? sn : cs);
+}
+// The Philox draw that component c's normal comes from.
+template <typename T>
+__device__ __forceinline__ philox_out normal_draw(uint64_t seed, uint32_t stream, uint64_t step, int v, int c) {
+  if (sizeof(T) == 8 && c == 2) stream |= 0x80000000u;
+  return philox4x32_10((uint32_t)v, (uint32_t)step, (uint32_t)(step >> 32), stream, (uint32_t)seed,
+                       (uint32_t)(seed >> 32));
+}
+__device__ __forceinline__ void normals3_f32(uint64_t seed, uint32_t stream, uint64_t step, int v, float n[3]) {
+  const philox_out o = normal_draw<float>(seed, stream, step, v, 0);
+#pragma unroll
+  for (int c = 0; c < 3; ++c) n[c] = normal_f32(o, c);
+}
+__device__ __forceinline__ void normals3(uint64_t seed, uint32_t stream, uint64_t step, int v, double n[3]) {
+  const philox_out o = normal_draw<double>(seed, stream, step, v, 0);
+  n[0] = normal_f64(o, 0);
+  n[1] = normal_f64(o, 1);
+  n[2] = normal_f64(normal_draw<double>(seed, stream, step, v, 2), 2);
 }
 
-// Momentum update of the reference leapfrog (src/hd.C:1546-1693), one vertex.
+// Momentum update of the reference leapfrog (src/hd.C:1546-1693), one coordinate.
 // Every product and sum is rounded on its own (no fused multiply-add), in the
 // reference's order of operations, so each kernel that uses it rounds alike.
-__device__ __forceinline__ void kick(const StepArgs &a, const double n[3], double pp[3], const double gg[3]) {
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    double q = pp[c];
-    if (a.kind == 2) q = __dsub_rn(q, __dmul_rn(__dmul_rn(a.gamma, a.AK), q));  // friction
-    const double half = __dmul_rn(__dmul_rn(-gg[c], a.AK), 0.5);                 // half kick
-    q = __dadd_rn(q, half);
-    if (a.kind == 1)
-      q = __dadd_rn(q, __ddiv_rn(__dmul_rn(__dmul_rn(__ddiv_rn(1.0, a.gamma), a.sigma), n[c]), a.AK));
-    else
-      q = __dadd_rn(q, __dmul_rn(a.sigma, n[c]));
-    q = __dadd_rn(q, half);
-    pp[c] = q;
-  }
+__device__ __forceinline__ double kick(const StepArgs &a, double n, double p, double g) {
+  double q = p;
+  if (a.kind == 2) q = __dsub_rn(q, __dmul_rn(__dmul_rn(a.gamma, a.AK), q));  // friction
+  const double half = __dmul_rn(__dmul_rn(-g, a.AK), 0.5);                     // half kick
+  q = __dadd_rn(q, half);
+  if (a.kind == 1)
+    q = __dadd_rn(q, __ddiv_rn(__dmul_rn(__dmul_rn(__ddiv_rn(1.0, a.gamma), a.sigma), n), a.AK));
+  else
+    q = __dadd_rn(q, __dmul_rn(a.sigma, n));
+  return __dadd_rn(q, half);
 }
 
-// The vertex-local update of one step with identity mass: overdamped BD
+// The update of one coordinate of one step with identity mass: overdamped BD
 // (r += -(D dt/kT) g + sqrt(2 D dt) xi), or the leapfrog kick followed by
 // r += p AK (p reset for BD). Rounded as kick() is.
-__device__ __forceinline__ void vertex_update(const StepArgs &a, const double gg[3], const double n[3], double rn[3],
-                                              double pp[3]) {
-  if (a.kind == 0) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c)
-      rn[c] = __dadd_rn(rn[c], __dadd_rn(__dmul_rn(-a.mob_dt, gg[c]), __dmul_rn(a.sigma, n[c])));
-    return;
-  }
-  kick(a, n, pp, gg);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) rn[c] = __dadd_rn(rn[c], __dmul_rn(pp[c], a.AK));
+__device__ __forceinline__ double coordinate_update(const StepArgs &a, double g, double n, double r, double *p) {
+  if (a.kind == 0) return __dadd_rn(r, __dadd_rn(__dmul_rn(-a.mob_dt, g), __dmul_rn(a.sigma, n)));
+  const double q = kick(a, n, *p, g);
+  *p = a.kind == 1 ? 0.0 : q;
+  return __dadd_rn(r, __dmul_rn(q, a.AK));
 }
 
 // Step index of the current step: the run's first step plus the run index,
@@ -1223,6 +1230,9 @@ __device__ __forceinline__ uint64_t current_step(const uint64_t *cnt) { return c
 // then taken. The FP64 work is the position and its copies only: 8 operations
 // per coordinate instead of 14 on GB300's narrow FP64 pipe. Explicitly
 // rounded, so every kernel that inlines it rounds alike.
+__device__ __forceinline__ double bd_coordinate_f32(const StepArgs &a, float g, float n, double r) {
+  return __dadd_rn(r, (double)__fmaf_rn(-a.mob_dt_f, g, __fmul_rn(a.sigma_f, n)));
+}
 __device__ __forceinline__ void bd_vertex_f32(const float *__restrict__ partial, const int *__restrict__ off, int v,
                                               const StepArgs &a, uint64_t st, double *__restrict__ r,
                                               float *__restrict__ rhi, float *__restrict__ rlo,
@@ -1233,15 +1243,18 @@ __device__ __forceinline__ void bd_vertex_f32(const float *__restrict__ partial,
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const size_t i = 3 * (size_t)v + c;
-    const float d = __fmaf_rn(-a.mob_dt_f, g[c], __fmul_rn(a.sigma_f, n[c]));
-    const double x = __dadd_rn(r[i], (double)d);
+    const double x = bd_coordinate_f32(a, g[c], n[c], r[i]);
     r[i] = x;
     if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
   }
 }
 
-// Gather fused with the vertex-local update (overdamped BD, or the leapfrog
-// kinds with identity mass).
+// Gather fused with the update of the coordinate (overdamped BD, or the
+// leapfrog kinds with identity mass), one thread per coordinate: the chain of a
+// coordinate (24 adds, a Box-Muller normal, the update) is a third of a
+// vertex's, and a 642-vertex mesh spreads over 31 blocks instead of three. The
+// redundant Philox rounds are integer work beside it. 642-vertex FP64 BD step:
+// 45.6 -> 32.5 us; 128 x 128 membrane, FP32: 39.6 -> 35.6 us.
 template <typename T>
 __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off, StepArgs a,
                                    const uint64_t *__restrict__ cnt, double *__restrict__ r, double *__restrict__ p,
@@ -1250,31 +1263,28 @@ __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const 
   grid_dependency_wait();  // the partials and the status come from the face launches
   if (*status) return;
   const uint64_t st = current_step(cnt);
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
+    const int v = i / 3, c = i - 3 * v;
+    const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
+    const philox_out o = normal_draw<T>(a.seed, a.stream, st, v, c);
+    double x;
     if constexpr (sizeof(T) == 4) {
       if (a.kind == 0) {
-        bd_vertex_f32((const float *)partial, off, v, a, st, r, rhi, rlo, r0, dsp);
+        const GradSum s = coordinate_sum(partial, at.x, at.y, c);
+        x = bd_coordinate_f32(a, s.hi - s.lo, normal_f32(o, c), r[i]);
+        r[i] = x;
+        if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
         continue;
       }
     }
-    double gg[3], n[3];
-    vertex_gradient(partial, off, v, gg);
-    if constexpr (sizeof(T) == 8) normals3(a.seed, a.stream, st, v, n);
-    else normals3_f32(a.seed, a.stream, st, v, n);
-    double rn[3] = {r[3 * (size_t)v], r[3 * (size_t)v + 1], r[3 * (size_t)v + 2]};
-    double pp[3] = {0, 0, 0};
-    if (a.kind != 0)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) pp[c] = p[3 * (size_t)v + c];
-    vertex_update(a, gg, n, rn, pp);
-    if (a.kind != 0)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) p[3 * (size_t)v + c] = (a.kind == 1) ? 0.0 : pp[c];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      r[3 * (size_t)v + c] = rn[c];
-      if (rhi) store_f32_position(3 * (size_t)v + c, rn[c], rhi, rlo, r0, dsp);
-    }
+    const double g = coordinate_gradient(partial, at.x, at.y, c);
+    double n, q = a.kind != 0 ? p[i] : 0.0;
+    if constexpr (sizeof(T) == 8) n = normal_f64(o, c);
+    else n = (double)normal_f32(o, c);
+    x = coordinate_update(a, g, n, r[i], &q);
+    if (a.kind != 0) p[i] = q;
+    r[i] = x;
+    if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
   }
 }
 
@@ -1283,13 +1293,9 @@ __global__ void kick_kernel(int nv, StepArgs a, const uint64_t *__restrict__ cnt
   grid_dependency_wait();
   if (*status) return;
   const uint64_t st = current_step(cnt);
-  for (int v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    double n[3], gg[3] = {g[3 * (size_t)v], g[3 * (size_t)v + 1], g[3 * (size_t)v + 2]};
-    normals3(a.seed, a.stream, st, v, n);
-    double pp[3] = {p[3 * (size_t)v], p[3 * (size_t)v + 1], p[3 * (size_t)v + 2]};
-    kick(a, n, pp, gg);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) p[3 * (size_t)v + c] = pp[c];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
+    const int v = i / 3, c = i - 3 * v;
+    p[i] = kick(a, normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c), p[i], g[i]);
   }
 }
 
@@ -1889,22 +1895,21 @@ __global__ void batch_gather_step_kernel(const BatchJob *__restrict__ jobs, cons
     }
     double gg[3], n[3];
     vertex_gradient((const T *)J.f.partial, J.off, v, gg);
-    if constexpr (sizeof(T) == 8) normals3(a.seed, a.stream, st, v, n);
-    else normals3_f32(a.seed, a.stream, st, v, n);
-    double *r = J.r, *p = J.p;
-    double rn[3] = {r[3 * (size_t)v], r[3 * (size_t)v + 1], r[3 * (size_t)v + 2]};
-    double pp[3] = {0, 0, 0};
-    if (a.kind != 0)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) pp[c] = p[3 * (size_t)v + c];
-    vertex_update(a, gg, n, rn, pp);
-    if (a.kind != 0)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) p[3 * (size_t)v + c] = (a.kind == 1) ? 0.0 : pp[c];
+    if constexpr (sizeof(T) == 8) {
+      normals3(a.seed, a.stream, st, v, n);
+    } else {
+      float nf[3];
+      normals3_f32(a.seed, a.stream, st, v, nf);
+      for (int c = 0; c < 3; ++c) n[c] = nf[c];
+    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
-      r[3 * (size_t)v + c] = rn[c];
-      if (J.rhi) store_f32_position(3 * (size_t)v + c, rn[c], J.rhi, J.rlo, J.r0, J.dsp);
+      const size_t i = 3 * (size_t)v + c;
+      double q = a.kind != 0 ? J.p[i] : 0.0;
+      const double x = coordinate_update(a, gg[c], n[c], J.r[i], &q);
+      if (a.kind != 0) J.p[i] = q;
+      J.r[i] = x;
+      if (J.rhi) store_f32_position(i, x, J.rhi, J.rlo, J.r0, J.dsp);
     }
   }
 }
@@ -2751,11 +2756,13 @@ cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s) {
   return cudaGetLastError();
 }
 
+// Small blocks, so that a small mesh's gather spreads over the SMs.
+constexpr int kGatherThreads = 64;
 template <typename T>
 cudaError_t launch_gather(int nv, const T *partial, const int *off, double *g, cudaStream_t s) {
   if (nv <= 0) return cudaSuccess;
-  dev::gather_kernel<T><<<grid_for(nv, 256), 256, 0, s>>>(nv, partial, off, g);
-  return cudaGetLastError();
+  return launch_after(dev::gather_kernel<T>, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, partial, off,
+                      g);
 }
 template cudaError_t launch_gather<double>(int, const double *, const int *, double *, cudaStream_t);
 template cudaError_t launch_gather<float>(int, const float *, const int *, double *, cudaStream_t);
@@ -2763,8 +2770,8 @@ template cudaError_t launch_gather<float>(int, const float *, const int *, doubl
 template <typename T>
 cudaError_t launch_gather_step(int nv, const T *partial, const int *off, const StepArgs &a, const uint64_t *cnt,
                                double *r, double *p, const F32Pos &f, const int *status, cudaStream_t s) {
-  return launch_after(dev::gather_step_kernel<T>, grid_for(nv, 256), 256, 0, s, nv, partial, off, a, cnt, r, p, f.hi,
-                      f.lo, f.r0, f.dsp, status);
+  return launch_after(dev::gather_step_kernel<T>, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, partial,
+                      off, a, cnt, r, p, f.hi, f.lo, f.r0, f.dsp, status);
 }
 template cudaError_t launch_gather_step<double>(int, const double *, const int *, const StepArgs &, const uint64_t *,
                                                 double *, double *, const F32Pos &, const int *, cudaStream_t);
@@ -2773,7 +2780,8 @@ template cudaError_t launch_gather_step<float>(int, const float *, const int *, 
 
 cudaError_t launch_kick(int nv, const StepArgs &a, const uint64_t *cnt, double *p, const double *g, const int *status,
                         cudaStream_t s) {
-  return launch_after(dev::kick_kernel, grid_for(nv, 256), 256, 0, s, nv, a, cnt, p, g, status);
+  return launch_after(dev::kick_kernel, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, a, cnt, p, g,
+                      status);
 }
 cudaError_t launch_drift(int nv, const StepArgs &a, double *r, double *p, const double *qdot, const F32Pos &f,
                          const int *status, cudaStream_t s) {
