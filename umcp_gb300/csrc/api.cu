@@ -395,6 +395,10 @@ class MeshArena {
 };
 }  // namespace
 
+// Whether a regular group of the precision form takes the thread-per-face
+// kernel instead of the half-warp one.
+static bool use_tpf(int ncp, int nfaces) { return ncp == 12 && nfaces >= kTpfFaces; }
+
 extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, const umcp_params *prm, umcp_mesh **out) {
   if (!ctx || !plan || !out) return fail(UMCP_ERR_INVALID, "null argument");
   umcp_params defaults;
@@ -474,13 +478,15 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
       for (int k = 0; k < 5; ++k)
         for (int x = 0; x < G->ncp; ++x) basis[((size_t)p * 5 + k) * ncpp + x] = B.at(k + 1, p, x);
     G->tc = prm->precision == UMCP_FP32_CENTRED && prm->face_kernel == 1 && G->ncp == 12 && G->npt == 15;
-    G->nblocks = group_blocks(prm->precision, G->tc, G->ncp, G->npt, G->nfaces);
+    G->tpf = prm->precision == UMCP_FP32_CENTRED && !G->tc && use_tpf(G->ncp, G->nfaces);
+    G->nblocks = group_blocks(prm->precision, G->tc, G->ncp, G->nfaces);
     G->block_base = block_base;
     block_base += G->nblocks;
-    block_rows += group_block_rows(prm->precision, G->ncp, G->npt, G->nfaces);
+    block_rows += group_block_rows(prm->precision, G->ncp, G->nfaces);
     arena.stage(G->cp, cp);
     arena.stage(G->basis, basis);
     if (prm->precision == UMCP_FP64) arena.stage(G->table, fixed::basis_table(basis, G->ncp, G->npt, ncpp));
+    else arena.stage(G->table, f32_table(basis, B.weight, G->ncp));
     if (prm->precision == UMCP_FP32_CENTRED) {  // the precision form's kernels read only the FP32 copies
       arena.stage(G->g0f, std::vector<float>(g0.begin(), g0.end()));
       arena.stage(G->rr0f, std::vector<float>(rr0.begin(), rr0.end()));
@@ -597,14 +603,15 @@ size_t umcp::interleave_slots(const std::vector<int> &counts, std::vector<int> *
   return base;
 }
 
-int umcp::group_blocks(int precision, bool tc, int ncp, int npt, int nfaces) {
+int umcp::group_blocks(int precision, bool tc, int ncp, int nfaces) {
   if (tc) return face_blocks_tc(nfaces);
-  return precision == UMCP_FP64 ? face_blocks64(nfaces) : face_blocks(nfaces, ncp, npt);
+  if (precision == UMCP_FP64) return face_blocks64(nfaces);
+  return use_tpf(ncp, nfaces) ? face_blocks_tpf(nfaces) : face_blocks32(nfaces);
 }
 
-int umcp::group_block_rows(int precision, int ncp, int npt, int nfaces) {
-  int b = group_blocks(precision, false, ncp, npt, nfaces);
-  if (precision == UMCP_FP32_CENTRED && ncp == 12 && npt == 15) b = std::max(b, face_blocks_tc(nfaces));
+int umcp::group_block_rows(int precision, int ncp, int nfaces) {
+  int b = group_blocks(precision, false, ncp, nfaces);
+  if (precision == UMCP_FP32_CENTRED && ncp == 12) b = std::max(b, face_blocks_tc(nfaces));
   return b;
 }
 
@@ -659,11 +666,11 @@ struct FaceBuffers {
   int *status;
 };
 
-// The face launches of every group. Plain path: one launch. Precision form:
-// one per group, the irregular ones on the ctx's side stream beside the regular
-// one when fork is set. Every block counts toward the finish
-// (FinishArgs::nblk), so whichever block is the last of all sums the block
-// partials.
+// The face launches of every group: one launch where all of them take a
+// half-warp kernel; else the regular group's own kernel on the ctx's stream, with
+// the irregular groups' launch on its side stream beside it when fork is set.
+// Every block counts toward the finish (FinishArgs::nblk), so whichever block is
+// the last of all sums the block partials.
 static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const FinishArgs &fin, bool fork) {
   cudaStream_t s = m->ctx->stream;
   if (m->precision == UMCP_FP64) {
@@ -674,39 +681,44 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
                                      G->ncp, G->nblocks, G->block_base};
     return launch_faces64(F, m->P, B.r, (double *)B.partial, B.blockpart, fin, s);
   }
-  fork = fork && m->groups.size() > 1;
+  FaceSet32 F{};
+  const Group *own = nullptr;
+  for (auto &G : m->groups) {
+    if (G->tc || G->tpf) own = G.get();
+    else
+      F.g[F.ngroups++] = FaceGroup32{G->cp.as<uint32_t>(), G->g0f.as<float>(), G->rr0f.as<float>(),
+                                     G->compf.as<float>(), G->table.as<float>(), G->dest.as<int>(), G->dudv, G->nfaces,
+                                     G->ncp, G->nblocks, G->block_base};
+  }
+  float *partial = (float *)B.partial;
+  if (!own) return launch_faces32(F, m->P, B.r, B.f32, partial, B.blockpart, fin, s, true);
+  fork = fork && F.ngroups > 0;
+  cudaError_t e = cudaSuccess;
   if (fork) {
-    cudaError_t e = cudaEventRecord(m->ctx->fork, s);
+    e = cudaEventRecord(m->ctx->fork, s);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(m->ctx->side, m->ctx->fork, 0);
     if (e != cudaSuccess) return e;
   }
-  for (size_t gi = 0; gi < m->groups.size(); ++gi) {
-    auto &G = m->groups[gi];
-    const cudaStream_t on = (fork && gi > 0) ? m->ctx->side : s;
-    dev::FaceLaunch L;
-    L.nfaces = G->nfaces;
-    L.block_base = G->block_base;
-    L.cp = G->cp.as<uint32_t>();
-    L.g0f = G->g0f.as<float>();
-    L.rr0f = G->rr0f.as<float>();
-    L.compf = G->compf.as<float>();
-    L.basis = G->basis.as<double>();
-    L.weight = G->weight.as<double>();
-    L.dudv = G->dudv;
-    L.irregular = G->irregular;
-    const cudaError_t e =
-        G->tc ? launch_faces_tc(L, G->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, (float *)B.partial,
-                                B.blockpart, B.status, G->nblocks, fin, on)
-              : launch_faces(L, G->dest.as<int>(), G->ncp, G->npt, m->P, B.r, B.f32, (float *)B.partial, B.blockpart,
-                             B.status, G->nblocks, fin, on);
-    if (e != cudaSuccess) return e;
-  }
-  if (fork) {
-    cudaError_t e = cudaEventRecord(m->ctx->join, m->ctx->side);
-    if (e == cudaSuccess) e = cudaStreamWaitEvent(s, m->ctx->join, 0);
-    if (e != cudaSuccess) return e;
-  }
-  return cudaSuccess;
+  dev::FaceLaunch L;
+  L.nfaces = own->nfaces;
+  L.block_base = own->block_base;
+  L.cp = own->cp.as<uint32_t>();
+  L.g0f = own->g0f.as<float>();
+  L.rr0f = own->rr0f.as<float>();
+  L.compf = own->compf.as<float>();
+  L.table = own->table.as<float>();
+  L.basis = own->basis.as<double>();
+  L.weight = own->weight.as<double>();
+  L.dudv = own->dudv;
+  e = own->tc ? launch_faces_tc(L, own->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, partial, B.blockpart,
+                                B.status, own->nblocks, fin, s)
+              : launch_faces_tpf(L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
+                                 fin, s);
+  if (e == cudaSuccess)
+    e = launch_faces32(F, m->P, B.r, B.f32, partial, B.blockpart, fin, fork ? m->ctx->side : s, !fork);
+  if (e == cudaSuccess && fork) e = cudaEventRecord(m->ctx->join, m->ctx->side);
+  if (e == cudaSuccess && fork) e = cudaStreamWaitEvent(s, m->ctx->join, 0);
+  return e;
 }
 
 // Face launches of an evaluation at d_r. With restraints on, the area and
@@ -863,10 +875,10 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
     const size_t ncpp = (size_t)(B.ncp + 3) / 4 * 4;
     b += nf * B.ncp * 4 + (size_t)B.npt * 5 * ncpp * 8 + B.weight.size() * 8 + nf * B.ncp * 4 +
          (size_t)B.npt * B.ncp * 8;
-    if (!f32) b += (size_t)fixed::table_ints(B.ncp, B.npt) * 4;
+    b += 4 * (size_t)(f32 ? f32_table_floats(B.ncp) : fixed::table_ints(B.ncp, B.npt));
     const size_t es = f32 ? 4 : 8;  // g0, reference angles and composition in the form's own type
     b += 2 * nf * B.npt * es + nf * 3 * es;
-    nblocks += group_block_rows(precision, B.ncp, B.npt, (int)nf);
+    nblocks += group_block_rows(precision, B.ncp, (int)nf);
   };
   group(PL.regular, PL.reg_faces.size());
   for (int val : {5, 7}) {

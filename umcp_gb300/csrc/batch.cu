@@ -54,13 +54,11 @@ struct umcp_batch {
   long long tuned_faces = 0;  // faces in the batch when the tile size was last timed
   std::vector<Job> jobs;
   bool dirty = true;
-  // Each patch type's basis (the same for every mesh: it depends on the
-  // valence only), copied from the first job that has the type.
+  // Each patch type's staged table (the same for every mesh of the precision:
+  // it depends on the valence only), copied from the first job that has the type.
   bool have_type[kTypes] = {false, false, false};
-  int npt[kTypes] = {0, 0, 0};
   double dudv[kTypes] = {0, 0, 0};
-  DevBuf basis[kTypes], weight[kTypes];
-  DevBuf table[kTypes];  // FP64: the fixed-point rows instead of basis (fixed64.h)
+  DevBuf table[kTypes], weight[kTypes];
   int face_grid[kTypes] = {0, 0, 0};
   int vgrid = 0;
   // device tables
@@ -181,7 +179,7 @@ static umcp_status rebuild(umcp_batch *b) {
   // Irregular faces (a few dozen per closed vesicle) go in tiles of at most
   // four faces per half-warp of their kernel, so that they spread over the
   // grid instead of queueing on one block per job.
-  const int hw = b->precision == UMCP_FP64 ? kHalfWarps64 : kHalfWarps32;
+  const int hw = kHalfWarps;
   for (int t = 0; t < kTypes; ++t) {
     b->counts[kCountTileBase + t] = (int)tiles.size();
     const int tft = t == 0 ? tf : (b->irr_tile > 0 ? b->irr_tile : std::min(tf, 4 * hw));
@@ -308,10 +306,13 @@ static cudaError_t queue_faces(umcp_batch *b) {
       return launch_batch_faces64(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
                                   b->table[t].as<int>(), b->weight[t].as<double>(), kTypeNcp[t], b->dudv[t],
                                   b->d_tile_sums.as<double>(), b->face_grid[t], on);
-    return launch_batch_faces(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
-                                 b->basis[t].as<double>(), b->weight[t].as<double>(), kTypeNcp[t], b->npt[t],
-                                 b->dudv[t], t > 0, b->d_tile_sums.as<double>(), b->face_grid[t],
-                                 b->d_next_tile.as<int>(), on);
+    if (t > 0)
+      return launch_batch_faces32(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
+                                  b->table[t].as<float>(), kTypeNcp[t], b->dudv[t], b->d_tile_sums.as<double>(),
+                                  b->face_grid[t], on);
+    return launch_batch_faces_tpf(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
+                                  b->table[t].as<float>(), b->dudv[t], b->d_tile_sums.as<double>(), b->face_grid[t],
+                                  b->d_next_tile.as<int>(), on);
   };
   cudaError_t e = cudaSuccess;
   const bool irregular = b->have_type[1] || b->have_type[2];
@@ -478,7 +479,7 @@ static umcp_status autotune(umcp_batch *b, long long faces) {
     }
   }
   const bool f64 = b->precision == UMCP_FP64;
-  const int hw = f64 ? kHalfWarps64 : kHalfWarps32;
+  const int hw = kHalfWarps;
   int sms = 0;
   UMCP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->ctx->device));
   const int max_bps = std::max(1, b->max_grid[0] / std::max(sms, 1));
@@ -493,7 +494,7 @@ static umcp_status autotune(umcp_batch *b, long long faces) {
     L.face_ms = time_face_launches(b, e0, e1, &st);
     if (st == UMCP_OK && (best.tile_faces == 0 || L.face_ms < best.face_ms)) best = L;
   };
-  const int unit = f64 ? kHalfWarps64 : 32;
+  const int unit = f64 ? kHalfWarps : 32;
   for (int mult : {1, 2, 4, 8, 16, 32, 64}) {
     if ((f64 && mult > 32) || (!f64 && mult < 4)) continue;
     trial(Layout{unit * mult, 4 * hw, max_bps, 0});
@@ -541,8 +542,9 @@ extern "C" umcp_status umcp_batch_create(umcp_ctx *ctx, int precision, const umc
   int sms = 0;
   UMCP_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device));
   for (int t = 0; t < kTypes; ++t) {
-    const int npt = t == 0 ? 15 : 16;
-    int g = precision == UMCP_FP64 ? batch_face_blocks64(kTypeNcp[t]) : batch_face_blocks(kTypeNcp[t], npt);
+    int g = precision == UMCP_FP64 ? batch_face_blocks64(kTypeNcp[t])
+            : t > 0                ? batch_face_blocks32(kTypeNcp[t])
+                                   : batch_face_blocks_tpf();
     b->max_grid[t] = std::max(g, 1);
     if (b->opt_blocks_per_sm > 0) g = std::min(g, b->opt_blocks_per_sm * sms);
     b->face_grid[t] = std::max(g, 1);
@@ -593,13 +595,10 @@ extern "C" umcp_status umcp_batch_add(umcp_batch *b, umcp_mesh *m, const umcp_in
     const Group &G = *Gp;
     const int t = type_of(G);
     if (b->have_type[t]) continue;
-    DevBuf &rows = b->precision == UMCP_FP64 ? b->table[t] : b->basis[t];
-    const DevBuf &from = b->precision == UMCP_FP64 ? G.table : G.basis;
-    UMCP_CUDA(rows.alloc(from.bytes));
+    UMCP_CUDA(b->table[t].alloc(G.table.bytes));
     UMCP_CUDA(b->weight[t].alloc(G.weight.bytes));
-    UMCP_CUDA(cudaMemcpyAsync(rows.p, from.p, from.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
+    UMCP_CUDA(cudaMemcpyAsync(b->table[t].p, G.table.p, G.table.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
     UMCP_CUDA(cudaMemcpyAsync(b->weight[t].p, G.weight.p, G.weight.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
-    b->npt[t] = G.npt;
     b->dudv[t] = G.dudv;
     b->have_type[t] = true;
     b->drop_graphs();  // the captured steps do not launch this type yet

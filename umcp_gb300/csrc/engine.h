@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/umcp_gpu.h"
+#include "face32_table.h"
 #include "fixed64.h"
 #include "launch.h"
 
@@ -49,11 +50,12 @@ struct Group {
   int valence = 6;                  // of the patch type's lowest corner
   std::vector<int> face_index;      // each face's index in the plan (regular faces, then irregular)
   bool tc = false;                  // regular faces of the precision form on the tensor cores
+  bool tpf = false;                 // ... or one per thread (large meshes); else half-warps
   int nblocks = 0, block_base = 0;  // persistent face-pass grid and its block-partial rows
   double dudv = 0.5;
   DevBuf cp, g0, rr0, comp, basis, weight, dest;
   DevBuf basis_w;           // value rows [npt][ncp] (area and volume terms)
-  DevBuf table;             // plain path: the basis rows in fixed point (fixed64.h)
+  DevBuf table;             // staged rows: fixed point in the plain path (fixed64.h), else FP32 (face32_table.h)
   DevBuf g0f, rr0f, compf;  // FP32 copies for the precision form
   DevBuf geo_tab;           // FP32 restraint tables (GeoGroup::tab), built when restraints are first set
 };
@@ -194,9 +196,9 @@ void batch_mesh_changed(umcp_batch *b);
 // Block-partial rows of a group's face launch, and the rows its footprint
 // reserves (the larger of the two kernels' grids, so the footprint does not
 // depend on the kernel choice).
-int group_blocks(int precision, bool tc, int ncp, int npt, int nfaces);
+int group_blocks(int precision, bool tc, int ncp, int nfaces);
 size_t interleave_slots(const std::vector<int> &counts, std::vector<int> *loc);
-int group_block_rows(int precision, int ncp, int npt, int nfaces);
+int group_block_rows(int precision, int ncp, int nfaces);
 
 inline uint32_t pack_cp(int v, const int8_t img[3]) {
   int code = (img[0] + 1) + 3 * (img[1] + 1) + 9 * (img[2] + 1);

@@ -1,0 +1,53 @@
+// The precision form's staged table of a patch type: the image of the leading
+// part of the half-warp face kernel's shared memory (face32.cuh), then the
+// quadrature weights. Formed once per mesh on the host, so that no block
+// converts rows from FP64.
+#pragma once
+#include <string.h>
+
+#include <vector>
+
+namespace umcp {
+
+template <int NCP, int NPT>
+struct F32Table {
+  static constexpr int NC4 = (NCP + 3) / 4;       // control points in fours
+  static constexpr int ROW4 = (5 * NC4) | 1;      // float4 stride of a point's rows: odd, free of bank conflicts
+  static constexpr int kRows = 0;                 // [NPT][ROW4][4]: rows u, v, uu, uv, vv
+  static constexpr int kPoint4 = NPT * ROW4 * 4;  // [NPT][NCP][4]: u, v, uu, uv of each control point
+  static constexpr int kPoint1 = kPoint4 + NPT * NCP * 4;  // [NPT][16]: vv
+  static constexpr int kWeights = kPoint1 + NPT * 16;      // [16] doubles
+  static constexpr int kFloats = kWeights + 32;
+};
+
+// Floats of a patch type's table.
+inline int f32_table_floats(int ncp) {
+  return ncp == 12 ? F32Table<12, 15>::kFloats : ncp == 11 ? F32Table<11, 16>::kFloats : F32Table<13, 16>::kFloats;
+}
+
+template <int NCP, int NPT>
+void fill_f32_table(const std::vector<double> &basis, const std::vector<double> &weight, std::vector<float> *t) {
+  using L = F32Table<NCP, NPT>;
+  t->assign(L::kFloats, 0.f);
+  for (int p = 0; p < NPT; ++p) {
+    for (int k = 0; k < 5; ++k)
+      for (int x = 0; x < NCP; ++x) {
+        const float b = (float)basis[((size_t)p * 5 + k) * (4 * L::NC4) + x];
+        (*t)[(size_t)(p * L::ROW4 + k * L::NC4) * 4 + x] = b;
+        if (k < 4) (*t)[L::kPoint4 + (p * NCP + x) * 4 + k] = b;
+        else (*t)[L::kPoint1 + p * 16 + x] = b;
+      }
+  }
+  memcpy(t->data() + L::kWeights, weight.data(), NPT * sizeof(double));
+}
+
+// The table from rows basis[npt][5][ncp rounded up to 4] and the weights.
+inline std::vector<float> f32_table(const std::vector<double> &basis, const std::vector<double> &weight, int ncp) {
+  std::vector<float> t;
+  if (ncp == 12) fill_f32_table<12, 15>(basis, weight, &t);
+  else if (ncp == 11) fill_f32_table<11, 16>(basis, weight, &t);
+  else if (ncp == 13) fill_f32_table<13, 16>(basis, weight, &t);
+  return t;
+}
+
+}  // namespace umcp

@@ -15,9 +15,10 @@ namespace f64 {
 // Bytes of the largest patch type's shared memory.
 constexpr size_t kSmemBytes = sizeof(Smem<13, 16>);
 static_assert(kSmemBytes >= sizeof(Smem<12, 15>) && kSmemBytes >= sizeof(Smem<11, 16>), "largest patch type");
-// Blocks per SM the registers are capped for (128 a thread): four warps a
+// Blocks per SM the registers are capped for (168 a thread): three warps a
 // scheduler, so that one warp's integer contractions run beside another's FP64.
-constexpr int kMinBlocks = 6;
+// (Four spill.)
+constexpr int kMinBlocks = 3;
 
 // Sum of q over each warp's lanes into red[warp][i], then over the block into out.
 __device__ __forceinline__ void block_row(double (*red)[6], const double *v, int n, double *out) {

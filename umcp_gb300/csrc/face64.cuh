@@ -26,7 +26,7 @@ namespace umcp {
 namespace dev {
 namespace f64 {
 
-constexpr int kThreads = 64, kHW = kThreads / 16, kWarps = kThreads / 32;
+constexpr int kThreads = 128, kHW = kThreads / 16, kWarps = kThreads / 32;
 
 template <int NCP, int NPT>
 struct Smem {

@@ -82,10 +82,6 @@ struct F32Pos {
   float *dsp = nullptr;
 };
 
-// Persistent grid of the face pass for one patch type (fixed per device and
-// face count, so the order of every sum is fixed).
-int face_blocks(int nfaces, int ncp, int npt);
-
 // The FP64 face pass (face64.cu): every patch type of a mesh in one launch. A
 // group's blocks write the block-partial rows [block_base, block_base + nblocks),
 // the groups' rows following one another from 0.
@@ -104,18 +100,47 @@ int face_blocks64(int nfaces);
 cudaError_t launch_faces64(const FaceSet64 &F, const dev::SurfaceParams &P, const double *r, double *partial,
                            double *blockpart, const FinishArgs &fin, cudaStream_t s);
 
-// Face pass of the precision form for one patch type (ncp 12/npt 15 regular;
-// ncp 11 or 13, npt 16 irregular). partial[dest[f*ncp+x]] receives the
-// alpha-scaled gradient of control point x of face f; blockpart[L.block_base
-// + b] receives block b's sums {E_area, E_curvature, E_angle, dE/dalpha_xyz}.
-// f: the FP32 positions and displacements.
-cudaError_t launch_faces(const dev::FaceLaunch &L, const int *dest, int ncp, int npt, const dev::SurfaceParams &P,
-                         const double *r, const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                         const FinishArgs &fin, cudaStream_t s);
+// The precision form's half-warp face pass (face32.cu): any of a mesh's patch
+// types in one launch. partial[dest[f*ncp+x]] receives the alpha-scaled gradient
+// of control point x of face f; blockpart[block_base + b] the sums of block b of
+// the group, {E_area, E_curvature, E_angle, dE/dalpha_xyz}.
+struct FaceGroup32 {
+  const uint32_t *cp;
+  const float *g0, *rr0, *comp, *table;  // table: face32_table.h
+  const int *dest;
+  double dudv;
+  int nfaces, ncp, nblocks, block_base;
+};
+struct FaceSet32 {
+  FaceGroup32 g[3];
+  int ngroups;
+};
+struct F32View {
+  const float *hi, *lo, *dsp;
+};
+int face_blocks32(int nfaces);
+// chained: s's previous kernel is the one whose results it reads (the launch may
+// then start while that one drains).
+cudaError_t launch_faces32(const FaceSet32 &F, const dev::SurfaceParams &P, const double *r, const F32Pos &f,
+                           float *partial, double *blockpart, const FinishArgs &fin, cudaStream_t s, bool chained);
+
+// Regular faces (ncp 12, npt 15) of the precision form, one per thread
+// (face_tpf_kernel): the same outputs; the same gradient bits.
+// From kTpfFaces faces on. With fewer, a thread per face leaves the schedulers
+// one warp each or none, and a face's serial chain (about 14 us) is the pass; a
+// half-warp per face shortens it to about 3 us but issues 1.6 times the
+// instructions per face. BD step, half-warps against a thread per face: 320
+// faces 11.0 / 25.7 us, 8,192 18.7 / 23.7, 20,400 25.9 / 29.8, 32,768 34.6 /
+// 29.8, 131,072 103 / 68.
+constexpr int kTpfFaces = 24000;
+int face_blocks_tpf(int nfaces);
+cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
+                             const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
+                             const FinishArgs &fin, cudaStream_t s);
 
 // The regular faces of the precision form on the tensor cores (face_tc_kernel):
-// the same outputs as launch_faces<float> for ncp 12 / npt 15, in 128-face
-// tiles; grid from face_blocks_tc.
+// the same outputs as launch_faces_tpf, in 128-face tiles; grid from
+// face_blocks_tc.
 int face_blocks_tc(int nfaces);
 cudaError_t launch_faces_tc(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
                             const float *rhi, const float *rlo, const float *dsp, float *partial, double *blockpart,
@@ -189,16 +214,17 @@ struct BatchTile {
 enum : int { kCountTiles = 0, kCountTileBase = 3, kCountJobs = 6, kCountVertexTiles = 7, kCountWords = 8 };
 constexpr int kVertexTile = 256;  // vertices per vertex tile (one thread each)
 
-// Face launch of patch type `group` over its tiles (counts[group] of them,
+// Face launches of patch type `group` over its tiles (counts[group] of them,
 // from counts[3 + group] in tiles); tile_sums[3 * global tile] receives each
-// tile's energy terms. Persistent grid; tiles of stopped or finished jobs are
-// skipped.
-// next_tile: {tiles handed out, blocks done} of the regular launch, which leaves
-// both zero.
-cudaError_t launch_batch_faces(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
-                               const double *basis, const double *weight, int ncp, int npt, double dudv,
-                               int irregular, double *tile_sums, int grid, int *next_tile, cudaStream_t s);
-// The same in FP64 (table: the patch type's fixed-point rows, fixed64.h).
+// tile's energy terms. Persistent grids; tiles of stopped or finished jobs are
+// skipped. Regular faces of the precision form (tpf; next_tile: {tiles handed
+// out, blocks done}, which the launch leaves zero), its irregular ones (32), and
+// FP64 (64); table: the patch type's (face32_table.h, fixed64.h).
+cudaError_t launch_batch_faces_tpf(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
+                                   const float *table, double dudv, double *tile_sums, int grid, int *next_tile,
+                                   cudaStream_t s);
+cudaError_t launch_batch_faces32(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
+                                 const float *table, int ncp, double dudv, double *tile_sums, int grid, cudaStream_t s);
 cudaError_t launch_batch_faces64(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
                                  const int *table, const double *weight, int ncp, double dudv, double *tile_sums,
                                  int grid, cudaStream_t s);
@@ -221,12 +247,12 @@ cudaError_t launch_batch_unpack(const BatchJob *jobs, const BatchTile *vtiles, c
                                 const long long *off, const double *pack, int grid, cudaStream_t s);
 cudaError_t launch_batch_pack(const BatchJob *jobs, const BatchTile *vtiles, const int *counts, const long long *off,
                               double *pack, double *E, int grid, cudaStream_t s);
-// Device-filling grid of a batch face launch for a patch type.
-int batch_face_blocks(int ncp, int npt);
+// Device-filling grids of the batch face launches.
+int batch_face_blocks_tpf();
+int batch_face_blocks32(int ncp);
 int batch_face_blocks64(int ncp);
-// Faces in flight per block of the half-warp kernels, FP64 and FP32: the units
-// of a batch's tile sizes.
-constexpr int kHalfWarps64 = 4, kHalfWarps32 = 8;
+// Faces in flight per block of the half-warp kernels: the unit of a batch's tile sizes.
+constexpr int kHalfWarps = 8;
 
 // out[3i+c] (+)= scale/alpha_c^2 * (scalev ? scalev[c*nrow+i] : 1) * sum_k val[k] in[3 col[k]+c].
 // accumulate=0 overwrites out. alphas: device pointer to 3 doubles (or NULL = 1).

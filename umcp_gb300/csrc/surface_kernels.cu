@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include "device_common.cuh"
+#include "face32.cuh"
 #include "kernels.cuh"
 #include "launch.h"
 #include "launch_host.h"
@@ -18,466 +19,6 @@ template <typename T>
 struct alignas(4 * sizeof(T)) Q4 {
   T x, y, z, w;
 };
-
-template <typename T, int NCP, int NPT>
-struct FaceSmem {
-  static constexpr int NC4 = (NCP + 3) / 4;  // control points in chunks of four
-  static constexpr int NCPP = NC4 * 4;
-  static constexpr int HW = FaceCfg<T>::half_warps;
-  Q4<T> B[NPT][5][NC4];           // basis rows u,v,uu,uv,vv of point p
-  Q4<T> X[HW][NCPP];              // centred, alpha-scaled control points
-  Q4<T> Tc[HW][NPT][NCPP + 1];    // point p's contribution to each control point (+1 row pad: no bank conflicts)
-  T W[NPT];
-  double red[HW][6];
-  __device__ __forceinline__ void *scratch() { return &Tc[0][0][0]; }
-};
-
-// Precision form (the half-warp kernel runs the irregular faces there; the
-// regular ones take face_tpf_kernel): control points and per-point contributions are stored
-// coordinate-major, so four control points of one coordinate are one float4
-// and both contractions run as paired FP32 multiply-adds (two control points
-// per instruction).
-//  Xt[hw][c][cp]                 coordinate c of the centred control points
-//  Tc[hw][(c * NPT + p) * TROW + cp]  point p's contribution to control point cp
-// TROW makes the 16-byte row stride odd (conflict-free float4 stores by the
-// point lanes); THW puts the two half-warps of a warp 16 banks apart, so the
-// control-point lanes' scalar reads do not conflict either.
-template <int NCP, int NPT>
-struct FaceSmem<float, NCP, NPT> {
-  static constexpr int NC4 = (NCP + 3) / 4;
-  static constexpr int NCPP = NC4 * 4;
-  static constexpr int HW = FaceCfg<float>::half_warps;
-  static constexpr int TROW = NCPP + ((NC4 % 2 == 0) ? 4 : 0);
-  static constexpr int TSZ = 3 * NPT * TROW;
-  static constexpr int THW = TSZ + (48 - TSZ % 32) % 32;
-  static_assert(THW % 32 == 16 && THW % 4 == 0, "half-warp stride");
-  Q4<float> B[NPT][5][NC4];
-  alignas(16) float Xt[HW][3][NCPP];
-  alignas(16) float Dt[HW][3][NCPP];  // the same control points' change from the reference state
-  alignas(16) float Tc[HW][THW];
-  float W[NPT];
-  double red[HW][6];
-  __device__ __forceinline__ void *scratch() { return &Tc[0][0]; }
-};
-
-// Error-free sum: s + e == a + b exactly (Knuth's two-sum).
-__device__ __forceinline__ void two_sum(float a, float b, float &s, float &e) {
-  s = a + b;
-  float bb = s - a;
-  e = (a - (s - bb)) + (b - bb);
-}
-
-// Per-half-warp sums of a face's energy terms and dE/dalpha: FP64 in the
-// plain path; FP32 with Kahan compensation in the precision form, which keeps
-// the FP64 pipe out of the face loop.
-template <typename T>
-struct HalfWarpSums;
-template <>
-struct HalfWarpSums<double> {
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  __device__ __forceinline__ void add(int q, double v) { s[q] += v; }
-  __device__ __forceinline__ double get(int q) const { return s[q]; }
-};
-template <>
-struct HalfWarpSums<float> {
-  float s[6] = {0, 0, 0, 0, 0, 0}, c[6] = {0, 0, 0, 0, 0, 0};
-  __device__ __forceinline__ void add(int q, float v) {
-    float y = v - c[q], t = s[q] + y;
-    c[q] = (t - s[q]) - y;
-    s[q] = t;
-  }
-  __device__ __forceinline__ double get(int q) const { return (double)s[q] - (double)c[q]; }
-};
-
-template <typename T>
-__device__ __forceinline__ T point_data(const double *d64, const float *d32, size_t i) {
-  if constexpr (sizeof(T) == 8) return d64[i];
-  else return d32[i];
-}
-
-// The moduli in the arithmetic type, converted once per launch (or per
-// tile) rather than per face: conversions from FP64 run on the narrow FP64 pipe.
-template <typename T>
-struct Moduli {
-  T kc, KA, kg, k_reg;
-  __device__ __forceinline__ explicit Moduli(const SurfaceParams &P)
-      : kc((T)P.kc), KA((T)P.KA), kg((T)P.kg), k_reg((T)P.k_reg) {}
-};
-
-// Global data of one face, loaded one face ahead (control-point indices two
-// ahead) so the loads are in flight while the previous face computes.
-template <typename T>
-struct FaceAhead {
-  int img[3] = {0, 0, 0};
-  float hi[3] = {0, 0, 0}, lo[3] = {0, 0, 0};  // precision form
-  float dsp[3] = {0, 0, 0};                    // precision form: r - r0
-  double X[3] = {0, 0, 0};                     // plain path (image position)
-  T g0 = 1, rr0 = 0, P2 = 0, Hbar = 0, Pres = 0;
-  int dest = 0;
-};
-
-// Faces at or past end are not loaded.
-template <int NCP>
-__device__ __forceinline__ uint32_t load_cp(const FaceSrc &S, int f, int end, int lane) {
-  return (f >= 0 && f < end && lane < NCP) ? __ldg(&S.cp[(size_t)f * NCP + lane]) : 0u;
-}
-
-template <typename T, int NCP, int NPT>
-__device__ __forceinline__ void load_ahead(const FaceSrc &S, const SurfaceParams &P, int f, int end, uint32_t packed,
-                                           int lane, FaceAhead<T> &a) {
-  if (f < 0 || f >= end) return;
-  if (lane < NCP) {
-    const int v = (int)(packed & kVertexMask), code = (int)(packed >> kVertexBits);
-    a.img[0] = code % 3 - 1; a.img[1] = (code / 3) % 3 - 1; a.img[2] = code / 9 - 1;
-    if constexpr (sizeof(T) == 8) {
-#pragma unroll
-      for (int c = 0; c < 3; ++c)
-        a.X[c] = S.r[3 * (size_t)v + c] + a.img[0] * P.box[0][c] + a.img[1] * P.box[1][c] + a.img[2] * P.box[2][c];
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        a.hi[c] = S.rhi[3 * (size_t)v + c];
-        a.lo[c] = S.rlo[3 * (size_t)v + c];
-        a.dsp[c] = S.dsp[3 * (size_t)v + c];
-      }
-    }
-    a.dest = __ldg(&S.dest[(size_t)f * NCP + lane]);
-  }
-  if (lane < NPT) {
-    const size_t pi = (size_t)f * NPT + lane;
-    a.g0 = point_data<T>(S.g0, S.g0f, pi);
-    a.rr0 = point_data<T>(S.rr0, S.rr0f, pi);
-  }
-  a.P2 = point_data<T>(S.comp, S.compf, 3 * (size_t)f);
-  a.Hbar = point_data<T>(S.comp, S.compf, 3 * (size_t)f + 1);
-  a.Pres = point_data<T>(S.comp, S.compf, 3 * (size_t)f + 2);
-}
-
-// Stage the block's copy of the patch type's basis rows and weights.
-template <typename T, int NCP, int NPT, int NT>
-__device__ __forceinline__ void stage_basis(FaceSmem<T, NCP, NPT> &sm, const double *basis, const double *weight) {
-  constexpr int NCPP = FaceSmem<T, NCP, NPT>::NCPP, HW = FaceSmem<T, NCP, NPT>::HW;
-  T *b = &sm.B[0][0][0].x;
-  for (int i = threadIdx.x; i < NPT * 5 * NCPP; i += NT) b[i] = (T)basis[i];
-  for (int i = threadIdx.x; i < NPT; i += NT) sm.W[i] = (T)weight[i];
-  // padding control points stay zero
-  if constexpr (sizeof(T) == 4)
-    for (int i = threadIdx.x; i < HW * 3 * NCPP; i += NT) (&sm.Xt[0][0][0])[i] = (&sm.Dt[0][0][0])[i] = 0.f;
-  else
-    for (int i = threadIdx.x; i < HW * NCPP; i += NT) sm.X[i / NCPP][i % NCPP] = Q4<T>{0, 0, 0, 0};
-}
-
-// Precision form, lane = quadrature point p: the five contractions, the
-// pointwise energy and adjoint, and p's contribution to every control point.
-// Both contractions use paired FP32 multiply-adds over two control points at
-// once (__ffma2_rn), which halves their instruction count:
-//   K[k]_c = sum_j B[p][k][j] X_c[j]    even j in the pair's first half, odd j
-//                                       in its second; the halves added last
-//   T_c[j] = sum_k B[p][k][j] Kb[k]_c   j, j+1 in one pair, Kb duplicated
-template <int NCP, int NPT>
-__device__ __forceinline__ void point_pass_f32(FaceSmem<float, NCP, NPT> &sm, int hw, int lane,
-                                               const FaceAhead<float> &cur, float dudv, const Moduli<float> &mod,
-                                               bool reg_alpha, float *ea, float *ec, float *er, float dreg[3]) {
-  using S = FaceSmem<float, NCP, NPT>;
-  constexpr int NC4 = S::NC4, TROW = S::TROW;
-  float2 A[5][3], Ad[2][3];  // Ad: the u and v rows contracted with the displacements (Dt)
-#pragma unroll
-  for (int k = 0; k < 5; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) A[k][c] = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 2; ++k)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) Ad[k][c] = make_float2(0.f, 0.f);
-#pragma unroll 1
-  for (int c4 = 0; c4 < NC4; ++c4) {
-    float4 x[3], d[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      x[c] = *reinterpret_cast<const float4 *>(&sm.Xt[hw][c][4 * c4]);
-      d[c] = *reinterpret_cast<const float4 *>(&sm.Dt[hw][c][4 * c4]);
-    }
-#pragma unroll
-    for (int k = 0; k < 5; ++k) {
-      const Q4<float> b = sm.B[lane][k][c4];
-      const float2 b01 = make_float2(b.x, b.y), b23 = make_float2(b.z, b.w);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        A[k][c] = __ffma2_rn(b01, make_float2(x[c].x, x[c].y), A[k][c]);
-        A[k][c] = __ffma2_rn(b23, make_float2(x[c].z, x[c].w), A[k][c]);
-        if (k < 2) {
-          Ad[k][c] = __ffma2_rn(b01, make_float2(d[c].x, d[c].y), Ad[k][c]);
-          Ad[k][c] = __ffma2_rn(b23, make_float2(d[c].z, d[c].w), Ad[k][c]);
-        }
-      }
-    }
-  }
-  Vec3<float> K[5], dR[2];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) K[k] = {A[k][0].x + A[k][0].y, A[k][1].x + A[k][1].y, A[k][2].x + A[k][2].y};
-#pragma unroll
-  for (int k = 0; k < 2; ++k) dR[k] = {Ad[k][0].x + Ad[k][0].y, Ad[k][1].x + Ad[k][1].y, Ad[k][2].x + Ad[k][2].y};
-  Vec3<float> Kb[5], Kreg[2];
-  point_adjoint<float>(K, sm.W[lane], cur.g0, cur.rr0, dudv, cur.P2, cur.Hbar, cur.Pres, mod.kc, mod.KA, mod.kg,
-                       mod.k_reg, ea, ec, er, Kb, Kreg, dR);
-  float2 Kd[5][3];
-#pragma unroll
-  for (int k = 0; k < 5; ++k) {
-    Kd[k][0] = make_float2(Kb[k].x, Kb[k].x);
-    Kd[k][1] = make_float2(Kb[k].y, Kb[k].y);
-    Kd[k][2] = make_float2(Kb[k].z, Kb[k].z);
-  }
-  float *tc = &sm.Tc[hw][lane * TROW];
-#pragma unroll 1
-  for (int c4 = 0; c4 < NC4; ++c4) {
-    Q4<float> b[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) b[k] = sm.B[lane][k][c4];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      float2 t01 = __fmul2_rn(make_float2(b[0].x, b[0].y), Kd[0][c]);
-      float2 t23 = __fmul2_rn(make_float2(b[0].z, b[0].w), Kd[0][c]);
-#pragma unroll
-      for (int k = 1; k < 5; ++k) {
-        t01 = __ffma2_rn(make_float2(b[k].x, b[k].y), Kd[k][c], t01);
-        t23 = __ffma2_rn(make_float2(b[k].z, b[k].w), Kd[k][c], t23);
-      }
-      *reinterpret_cast<float4 *>(&tc[c * NPT * TROW + 4 * c4]) = make_float4(t01.x, t01.y, t23.x, t23.y);
-    }
-    if (reg_alpha) {
-      // igrad's box-scale derivative takes the angle-term adjoint with one
-      // more alpha factor (src/grad.C:7414-7421).
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float bk0 = (&b[0].x)[j], bk1 = (&b[1].x)[j];
-        dreg[0] += (bk0 * Kreg[0].x + bk1 * Kreg[1].x) * sm.Xt[hw][0][4 * c4 + j];
-        dreg[1] += (bk0 * Kreg[0].y + bk1 * Kreg[1].y) * sm.Xt[hw][1][4 * c4 + j];
-        dreg[2] += (bk0 * Kreg[0].z + bk1 * Kreg[1].z) * sm.Xt[hw][2][4 * c4 + j];
-      }
-    }
-  }
-}
-
-// Energy, adjoint and gradient partials of one face by one half-warp:
-//  1. lanes = control points: the control point's position relative to the
-//     patch corner (control point 0) in its lattice image, times alpha. The
-//     plain path forms it in FP64; the precision form from FP32 hi/lo pairs
-//     with error-free sums, so the local coordinates carry full FP32
-//     precision even across periodic images.
-//  2. lanes = quadrature points: the five contractions (basis rows held per
-//     point, control points broadcast), pointwise energy and adjoint, and the
-//     adjoint's contribution to every control point (written transposed).
-//  3. lanes = control points: sum the contributions over the points; write the
-//     alpha-scaled gradient partial to its slot.
-// Returns the face's energy terms and dE/dalpha summed over the half-warp.
-template <typename T, int NCP, int NPT>
-__device__ __forceinline__ void face_compute(FaceSmem<T, NCP, NPT> &sm, int hw, int lane, unsigned hmask,
-                                             const FaceAhead<T> &cur, const SurfaceParams &P, const T alpha[3],
-                                             const T ialpha[3], const T am1[3], const Moduli<T> &mod, T dudv,
-                                             bool reg_alpha, T *__restrict__ partial, T e3[3], T da[3]) {
-  constexpr int NC4 = FaceSmem<T, NCP, NPT>::NC4;
-  const T kc = mod.kc, KA = mod.KA, kg = mod.kg, k_reg = mod.k_reg;
-  // ---- 1. control points, relative to the patch corner
-  T xl[3] = {0, 0, 0}, dx[3] = {0, 0, 0};
-  if constexpr (sizeof(T) == 8) {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const double a = __shfl_sync(hmask, cur.X[c], 0, 16);
-      xl[c] = alpha[c] * (cur.X[c] - a);
-    }
-  } else {
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const float ahi = __shfl_sync(hmask, cur.hi[c], 0, 16), alo = __shfl_sync(hmask, cur.lo[c], 0, 16);
-      // lattice shift hi + lo (each term exact: images are -1, 0 or +1)
-      float sh = 0.f, she = 0.f, shl = 0.f;
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        float t, e;
-        two_sum(sh, (float)cur.img[d] * P.box_hi[d][c], t, e);
-        sh = t;
-        she += e;
-        shl += (float)cur.img[d] * P.box_lo[d][c];
-      }
-      float s1, e1, s2, e2;
-      two_sum(cur.hi[c], sh, s1, e1);
-      two_sum(s1, -ahi, s2, e2);
-      const float lc = s2 + ((e1 + e2) + ((cur.lo[c] - alo) + (she + shl)));
-      xl[c] = alpha[c] * lc;
-      // change from the reference state (box scales 1 there): alpha L - L0 = (alpha - 1) L + (L - L0),
-      // L - L0 = dsp - dsp of the corner (the lattice shifts cancel)
-      const float d0 = __shfl_sync(hmask, cur.dsp[c], 0, 16);
-      dx[c] = fmaf(am1[c], lc, cur.dsp[c] - d0);
-    }
-  }
-  if constexpr (sizeof(T) == 4) {
-    if (lane < NCP) {
-      sm.Xt[hw][0][lane] = xl[0];
-      sm.Xt[hw][1][lane] = xl[1];
-      sm.Xt[hw][2][lane] = xl[2];
-      sm.Dt[hw][0][lane] = dx[0];
-      sm.Dt[hw][1][lane] = dx[1];
-      sm.Dt[hw][2][lane] = dx[2];
-    }
-  } else {
-    if (lane < NCP) sm.X[hw][lane] = Q4<T>{xl[0], xl[1], xl[2], T(0)};
-  }
-  __syncwarp(hmask);
-
-  // ---- 2. lanes as quadrature points
-  T ea = 0, ec = 0, er = 0;
-  T dreg[3] = {0, 0, 0};
-  if constexpr (sizeof(T) == 4) {
-    if (lane < NPT) point_pass_f32<NCP, NPT>(sm, hw, lane, cur, dudv, mod, reg_alpha, &ea, &ec, &er, dreg);
-  } else if (lane < NPT) {
-    Vec3<T> K[5];
-#pragma unroll
-    for (int k = 0; k < 5; ++k) K[k] = {0, 0, 0};
-#pragma unroll 1
-    for (int c4 = 0; c4 < NC4; ++c4) {
-      const Q4<T> x0 = sm.X[hw][4 * c4], x1 = sm.X[hw][4 * c4 + 1], x2 = sm.X[hw][4 * c4 + 2],
-                  x3 = sm.X[hw][4 * c4 + 3];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) {
-        const Q4<T> b = sm.B[lane][k][c4];
-        K[k].x += b.x * x0.x + b.y * x1.x + b.z * x2.x + b.w * x3.x;
-        K[k].y += b.x * x0.y + b.y * x1.y + b.z * x2.y + b.w * x3.y;
-        K[k].z += b.x * x0.z + b.y * x1.z + b.z * x2.z + b.w * x3.z;
-      }
-    }
-    Vec3<T> Kb[5], Kreg[2];
-    point_adjoint<T>(K, sm.W[lane], cur.g0, cur.rr0, dudv, cur.P2, cur.Hbar, cur.Pres, kc, KA, kg, k_reg, &ea, &ec,
-                     &er, Kb, Kreg);
-#pragma unroll 1
-    for (int c4 = 0; c4 < NC4; ++c4) {
-      Q4<T> b[5];
-#pragma unroll
-      for (int k = 0; k < 5; ++k) b[k] = sm.B[lane][k][c4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const T bk0 = (&b[0].x)[j], bk1 = (&b[1].x)[j], bk2 = (&b[2].x)[j], bk3 = (&b[3].x)[j],
-                bk4 = (&b[4].x)[j];
-        Q4<T> t;
-        t.x = bk0 * Kb[0].x + bk1 * Kb[1].x + bk2 * Kb[2].x + bk3 * Kb[3].x + bk4 * Kb[4].x;
-        t.y = bk0 * Kb[0].y + bk1 * Kb[1].y + bk2 * Kb[2].y + bk3 * Kb[3].y + bk4 * Kb[4].y;
-        t.z = bk0 * Kb[0].z + bk1 * Kb[1].z + bk2 * Kb[2].z + bk3 * Kb[3].z + bk4 * Kb[4].z;
-        t.w = T(0);
-        sm.Tc[hw][lane][4 * c4 + j] = t;
-        if (reg_alpha) {
-          // igrad's box-scale derivative takes the angle-term adjoint with
-          // one more alpha factor (src/grad.C:7414-7421).
-          const Q4<T> xx = sm.X[hw][4 * c4 + j];
-          dreg[0] += (bk0 * Kreg[0].x + bk1 * Kreg[1].x) * xx.x;
-          dreg[1] += (bk0 * Kreg[0].y + bk1 * Kreg[1].y) * xx.y;
-          dreg[2] += (bk0 * Kreg[0].z + bk1 * Kreg[1].z) * xx.z;
-        }
-      }
-    }
-  }
-  __syncwarp(hmask);
-
-  // ---- 3. lanes as control points
-  da[0] = da[1] = da[2] = 0;
-  if (lane < NCP) {
-    T G0 = 0, G1 = 0, G2 = 0;
-    if constexpr (sizeof(T) == 4) {
-      constexpr int TROW = FaceSmem<T, NCP, NPT>::TROW;
-      const float *tc = &sm.Tc[hw][lane];
-#pragma unroll
-      for (int p = 0; p < NPT; ++p) {
-        G0 += tc[p * TROW];
-        G1 += tc[(NPT + p) * TROW];
-        G2 += tc[(2 * NPT + p) * TROW];
-      }
-    } else {
-#pragma unroll
-      for (int p = 0; p < NPT; ++p) {
-        const Q4<T> t = sm.Tc[hw][p][lane];
-        G0 += t.x;
-        G1 += t.y;
-        G2 += t.z;
-      }
-    }
-    const int d = cur.dest;
-    partial[3 * (size_t)d] = alpha[0] * G0;
-    partial[3 * (size_t)d + 1] = alpha[1] * G1;
-    partial[3 * (size_t)d + 2] = alpha[2] * G2;
-    // dE/dalpha_c = sum_x G_xc (X - X_0)_xc: the patch gradient sums to
-    // zero, so coordinates relative to the corner give the same sum.
-    da[0] = G0 * xl[0] * ialpha[0];
-    da[1] = G1 * xl[1] * ialpha[1];
-    da[2] = G2 * xl[2] * ialpha[2];
-  }
-  if (reg_alpha)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) da[c] += (alpha[c] - T(1)) * ialpha[c] * dreg[c];
-  e3[0] = ea; e3[1] = ec; e3[2] = er;
-#pragma unroll
-  for (int off = 8; off >= 1; off >>= 1)
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      e3[c] += __shfl_xor_sync(hmask, e3[c], off, 16);
-      da[c] += __shfl_xor_sync(hmask, da[c], off, 16);
-    }
-}
-
-// Single mesh: one half-warp per face, persistent over the mesh's faces.
-// Energy terms and dE/dalpha are summed per half-warp, then per block in a
-// fixed order, and written as one block partial (no atomics on floats).
-template <typename T, int NCP, int NPT>
-__global__ void __launch_bounds__(FaceCfg<T>::threads, FaceCfg<T>::min_blocks)
-    face_kernel(FaceLaunch L, const int *__restrict__ dest, SurfaceParams P, const double *__restrict__ r,
-                const float *__restrict__ rhi, const float *__restrict__ rlo, const float *__restrict__ dsp,
-                T *__restrict__ partial, double *__restrict__ blockpart, int *__restrict__ status, FinishArgs fin) {
-  using S = FaceSmem<T, NCP, NPT>;
-  constexpr int HW = S::HW, NT = FaceCfg<T>::threads;
-  __shared__ S sm;
-  stage_basis<T, NCP, NPT, NT>(sm, L.basis, L.weight);
-  __syncthreads();
-  grid_dependency_wait();  // the state comes from the kernels before
-
-  const int hw = threadIdx.x >> 4, lane = threadIdx.x & 15;
-  const unsigned hmask = (threadIdx.x & 16) ? 0xFFFF0000u : 0x0000FFFFu;
-  const T alpha[3] = {(T)r[3 * P.nv], (T)r[3 * P.nv + 1], (T)r[3 * P.nv + 2]};
-  const T ialpha[3] = {T(1) / alpha[0], T(1) / alpha[1], T(1) / alpha[2]};
-  const T am1[3] = {(T)(r[3 * P.nv] - 1.0), (T)(r[3 * P.nv + 1] - 1.0), (T)(r[3 * P.nv + 2] - 1.0)};
-  const T dudv = (T)L.dudv;
-  const bool reg_alpha = L.irregular && P.k_reg != 0.0;
-  const Moduli<T> mod(P);
-  const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
-  HalfWarpSums<T> acc;
-
-  const int stride = gridDim.x * HW;
-  int f = blockIdx.x * HW + hw;
-  FaceAhead<T> cur, nxt;
-  const int end = L.nfaces;
-  uint32_t cp_next = load_cp<NCP>(src, f + stride, end, lane);
-  load_ahead<T, NCP, NPT>(src, P, f, end, load_cp<NCP>(src, f, end, lane), lane, cur);
-
-  for (; f < end; f += stride) {
-    const uint32_t cp_after = load_cp<NCP>(src, f + 2 * stride, end, lane);
-    load_ahead<T, NCP, NPT>(src, P, f + stride, end, cp_next, lane, nxt);
-    cp_next = cp_after;
-    T e3[3], da[3];
-    face_compute<T, NCP, NPT>(sm, hw, lane, hmask, cur, P, alpha, ialpha, am1, mod, dudv, reg_alpha, partial, e3, da);
-    acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
-    acc.add(3, da[0]); acc.add(4, da[1]); acc.add(5, da[2]);
-    if (lane == 0 && !isfinite(e3[0] + e3[1] + e3[2])) atomicOr(status, kStatusNonFinite);
-    cur = nxt;
-    __syncwarp(hmask);
-  }
-  if (lane == 0)
-#pragma unroll
-    for (int q = 0; q < 6; ++q) sm.red[hw][q] = acc.get(q);
-  __syncthreads();
-  if (threadIdx.x < 6) {
-    double s = 0;
-#pragma unroll
-    for (int h = 0; h < HW; ++h) s += sm.red[h][threadIdx.x];
-    blockpart[6 * (size_t)(L.block_base + blockIdx.x) + threadIdx.x] = s;
-  }
-  count_and_finish<NT>(fin, blockpart);
-}
 
 // ---------------------------------------------------------------- tensor-core face pass
 //
@@ -539,7 +80,7 @@ struct Smem {
   float xmax[2][3][kFaces];       // per-row maxima exchanged between the two thread halves
   float Dd[3][kNcp][kFaces];      // control points' change from the reference state (FP32, per face)
   float Buv[kNpt][2][kNcp];       // basis rows u, v in FP32, for the area strain's tangent changes
-  float W[16];
+  f32::Coef C[16];                // each point's coefficients
   uint64_t mbar;
   uint32_t tmem;
   int abort;
@@ -640,8 +181,9 @@ __device__ __forceinline__ void split_pair(float x0, float x1, uint32_t &hi, uin
   lo = cvt2(__fsub_rn(x0, h0), __fsub_rn(x1, h1));
 }
 
-// CTA set-up: mbarrier, TMEM, the basis operands of every chunk, the weights.
-__device__ void setup(Smem &sm, const double *__restrict__ basis, const double *__restrict__ weight) {
+// CTA set-up: mbarrier, TMEM, the basis operands of every chunk, the points' coefficients.
+__device__ void setup(Smem &sm, const double *__restrict__ basis, const double *__restrict__ weight,
+                      const SurfaceParams &P, double dudv) {
   const int tid = threadIdx.x;
   // fp16 hi or lo part of the scaled basis value of point p, derivative d, control point x
   auto bval = [&](int p, int d, int x, bool lo) -> __half {
@@ -678,7 +220,7 @@ __device__ void setup(Smem &sm, const double *__restrict__ basis, const double *
     }
     b2[(size_t)j * kN2 * kK2 + core_off(n, k, kSbo2) / 2] = v;
   }
-  if (tid < 16) sm.W[tid] = tid < kNpt ? (float)weight[tid] : 0.f;
+  if (tid < kNpt) sm.C[tid] = f32::point_coef(P, weight[tid], dudv);
   for (int e = tid; e < kNpt * 2 * kNcp; e += kThreads) {
     const int p = e / (2 * kNcp), k = (e / kNcp) % 2, x = e % kNcp;
     sm.Buv[p][k][x] = (float)basis[((size_t)p * 5 + k) * kNcp + x];
@@ -741,9 +283,9 @@ __device__ __forceinline__ void gather_d2(uint32_t tmem, uint32_t lane_base, int
 // One tile of up to 128 faces [first, first + count) of source S. Returns
 // false if a wait gave up (the CTA then stops).
 __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const float alpha[3], const float ialpha[3],
-                     const float am1[3], const Moduli<float> &mod, float dudv, int first, int count,
+                     const float am1[3], float k_reg, int first, int count,
                      float *__restrict__ partial,
-                     HalfWarpSums<float> &acc, uint32_t &phase) {
+                     KahanSums<6> &acc, uint32_t &phase) {
   const int tid = threadIdx.x, fs = tid & (kFaces - 1), h = tid >> 7;
   const uint32_t tmem = sm.tmem, lane_base = (uint32_t)(32 * ((tid >> 5) & 3)) << 16;
   const bool active = fs < count;
@@ -887,7 +429,7 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
       const int p = 4 * j + 2 * h + q;
       K[q][0].x += Eu[0]; K[q][0].y += Eu[1]; K[q][0].z += Eu[2];
       K[q][1].x += Ev[0]; K[q][1].y += Ev[1]; K[q][1].z += Ev[2];
-      Vec3<float> Kb[5], Kreg[2];
+      Vec3<float> Kb[5];
       if (active && p < kNpt) {
         // the tangents' change from the reference state, for the area strain
         Vec3<float> dR[2] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
@@ -898,10 +440,13 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
           dR[0].x = fmaf(bu, d0, dR[0].x); dR[0].y = fmaf(bu, d1, dR[0].y); dR[0].z = fmaf(bu, d2, dR[0].z);
           dR[1].x = fmaf(bv, d0, dR[1].x); dR[1].y = fmaf(bv, d1, dR[1].y); dR[1].z = fmaf(bv, d2, dR[1].z);
         }
-        float ea = 0, ec = 0, er = 0;
-        point_adjoint<float>(K[q], sm.W[p], g0[q], rr0[q], dudv, P2, Hbar, Pres, mod.kc, mod.KA, mod.kg, mod.k_reg,
-                             &ea, &ec, &er, Kb, Kreg, dR);
-        e3[0] += ea; e3[1] += ec; e3[2] += er;
+        const f32::Point o = f32::point<true>(K[q], dR, sm.C[p], k_reg, g0[q], rr0[q], P2, Hbar, Pres);
+        e3[0] += o.ea; e3[1] += o.ec; e3[2] += o.er;
+        Kb[0] = o.Ku;
+        Kb[1] = o.Kv;
+        Kb[2] = {o.lb * o.m.x, o.lb * o.m.y, o.lb * o.m.z};
+        Kb[3] = {o.kb * o.m.x, o.kb * o.m.y, o.kb * o.m.z};
+        Kb[4] = {o.nb * o.m.x, o.nb * o.m.y, o.nb * o.m.z};
       } else {
 #pragma unroll
         for (int d = 0; d < 5; ++d) Kb[d] = {0.f, 0.f, 0.f};
@@ -988,7 +533,7 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
 
 // Fixed-order block sum of the six per-thread sums into out[6] (global). The
 // reduction buffer lies over the Kb operand, which no MMA reads any more.
-__device__ void block_sums(Smem &sm, const HalfWarpSums<float> &acc, double *out) {
+__device__ void block_sums(Smem &sm, const KahanSums<6> &acc, double *out) {
   double(*red)[6] = reinterpret_cast<double(*)[6]>(&sm.A2[0][0]);
   for (int q = 0; q < 6; ++q) red[threadIdx.x][q] = acc.get(q);
   __syncthreads();
@@ -1010,19 +555,18 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
                    FinishArgs fin) {
   extern __shared__ uint8_t tc_smem_raw[];
   tc::Smem &sm = *reinterpret_cast<tc::Smem *>((reinterpret_cast<uintptr_t>(tc_smem_raw) + 1023) & ~(uintptr_t)1023);
-  tc::setup(sm, L.basis, L.weight);
+  tc::setup(sm, L.basis, L.weight, P, L.dudv);
   const float alpha[3] = {(float)r[3 * P.nv], (float)r[3 * P.nv + 1], (float)r[3 * P.nv + 2]};
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
   const float am1[3] = {(float)(r[3 * P.nv] - 1.0), (float)(r[3 * P.nv + 1] - 1.0), (float)(r[3 * P.nv + 2] - 1.0)};
-  const Moduli<float> mod(P);
   const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
-  HalfWarpSums<float> acc;
+  KahanSums<6> acc;
   uint32_t phase = 0;
   bool ok = true;
   const int ntiles = (L.nfaces + tc::kFaces - 1) / tc::kFaces;
   for (int t = blockIdx.x; t < ntiles && ok; t += gridDim.x) {
     const int first = t * tc::kFaces;
-    ok = tc::tile(sm, src, P, alpha, ialpha, am1, mod, (float)L.dudv, first, min(tc::kFaces, L.nfaces - first), partial,
+    ok = tc::tile(sm, src, P, alpha, ialpha, am1, (float)P.k_reg, first, min(tc::kFaces, L.nfaces - first), partial,
                   acc, phase);
   }
   if (!ok && threadIdx.x == 0) atomicOr(status, kStatusTimeout);
@@ -1059,8 +603,7 @@ __global__ void status_merge_kernel(const int *__restrict__ src, int *__restrict
 // Sum of coordinate c of vertex v's gradient partials: its slots are
 // loc[2 v] + 32 k for k < loc[2 v + 1] (32 vertices interleaved, so the lanes of
 // a warp read consecutive slots), summed in k order (FP64, or FP32 with Kahan
-// compensation: hi - lo). Eight slots' loads are issued before they are added;
-// every partial is read once (evict-first).
+// compensation: hi - lo). Eight slots' loads are issued before they are added.
 template <typename T, class F>
 __device__ __forceinline__ void each_partial(const T *__restrict__ partial, int base, int n, int c, F add) {
   const T *q = partial + 3 * (size_t)base + c;
@@ -1068,11 +611,11 @@ __device__ __forceinline__ void each_partial(const T *__restrict__ partial, int 
   for (; k + 8 <= n; k += 8) {
     T x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = __ldcs(q + 96 * (size_t)(k + i));
+    for (int i = 0; i < 8; ++i) x[i] = q[96 * (size_t)(k + i)];
 #pragma unroll
     for (int i = 0; i < 8; ++i) add(x[i]);
   }
-  for (; k < n; ++k) add(__ldcs(q + 96 * (size_t)k));
+  for (; k < n; ++k) add(q[96 * (size_t)k]);
 }
 struct GradSum {
   float hi, lo;
@@ -1322,74 +865,6 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
 // depend on what else is in the batch. Tile and job counts are read from
 // device memory, so a captured step stays valid when the membership changes.
 
-template <typename T, int NCP, int NPT>
-__global__ void __launch_bounds__(FaceCfg<T>::threads, FaceCfg<T>::min_blocks)
-    batch_face_kernel(const BatchJob *__restrict__ jobs, int group, const BatchTile *__restrict__ tiles,
-                      const int *__restrict__ counts, const double *__restrict__ basis,
-                      const double *__restrict__ weight, double dudv_d, int irregular,
-                      double *__restrict__ tile_sums) {
-  using S = FaceSmem<T, NCP, NPT>;
-  constexpr int HW = S::HW, NT = FaceCfg<T>::threads;
-  __shared__ S sm;
-  __shared__ BatchFaceJob sj;
-  __shared__ int s_active;
-  const int ntiles = counts[group], tile_base = counts[3 + group];
-  if ((int)blockIdx.x >= ntiles) return;
-  stage_basis<T, NCP, NPT, NT>(sm, basis, weight);
-  const int hw = threadIdx.x >> 4, lane = threadIdx.x & 15;
-  const unsigned hmask = (threadIdx.x & 16) ? 0xFFFF0000u : 0x0000FFFFu;
-  const T dudv = (T)dudv_d;
-  for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
-    const BatchTile tile = tiles[tile_base + t];
-    __syncthreads();  // the previous tile's readers of sj and sm.red are done
-    {
-      const int *src = reinterpret_cast<const int *>(&jobs[tile.job].f);
-      int *dst = reinterpret_cast<int *>(&sj);
-      for (int i = threadIdx.x; i < (int)(sizeof(BatchFaceJob) / sizeof(int)); i += NT) dst[i] = src[i];
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) s_active = job_active(sj);  // one read for the whole block
-    __syncthreads();
-    HalfWarpSums<T> acc;
-    if (s_active) {
-      const FaceSrc &src = sj.src[group];
-      const SurfaceParams &P = sj.P;
-      const double *r = src.r;
-      const T alpha[3] = {(T)r[3 * P.nv], (T)r[3 * P.nv + 1], (T)r[3 * P.nv + 2]};
-      const T ialpha[3] = {T(1) / alpha[0], T(1) / alpha[1], T(1) / alpha[2]};
-      const T am1[3] = {(T)(r[3 * P.nv] - 1.0), (T)(r[3 * P.nv + 1] - 1.0), (T)(r[3 * P.nv + 2] - 1.0)};
-      const bool reg_alpha = irregular && P.k_reg != 0.0;
-      const Moduli<T> mod(P);
-      const int end = tile.first + tile.count;
-      int f = tile.first + hw;
-      FaceAhead<T> cur, nxt;
-      uint32_t cp_next = load_cp<NCP>(src, f + HW, end, lane);
-      load_ahead<T, NCP, NPT>(src, P, f, end, load_cp<NCP>(src, f, end, lane), lane, cur);
-      for (; f < end; f += HW) {
-        const uint32_t cp_after = load_cp<NCP>(src, f + 2 * HW, end, lane);
-        load_ahead<T, NCP, NPT>(src, P, f + HW, end, cp_next, lane, nxt);
-        cp_next = cp_after;
-        T e3[3], da[3];
-        face_compute<T, NCP, NPT>(sm, hw, lane, hmask, cur, P, alpha, ialpha, am1, mod, dudv, reg_alpha,
-                                  (T *)sj.partial, e3, da);
-        acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
-        cur = nxt;
-        __syncwarp(hmask);
-      }
-    }
-    if (lane == 0)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) sm.red[hw][q] = acc.get(q);
-    __syncthreads();
-    if (threadIdx.x < 3) {
-      double s = 0;
-#pragma unroll
-      for (int h = 0; h < HW; ++h) s += sm.red[h][threadIdx.x];
-      tile_sums[3 * (size_t)(tile_base + t) + threadIdx.x] = s;
-    }
-  }
-}
-
 // ---------------------------------------------------------------- thread-per-face pass
 //
 // Regular faces of the precision form (12 control points, 15 quadrature
@@ -1417,7 +892,8 @@ struct Smem {
   // conflict
   float4 X[kThreads][9];
   float4 D[kThreads][9];  // the same control points' change from the reference state, same layout
-  float W[kNpt];
+  float2 C[kNpt];  // each point's coefficients curv, area (f32::Coef)
+  float Cg[kNpt];  // and gauss
   double red[kWarps][6];
 };
 constexpr size_t kSumBytes = sizeof(float) * 12 * kThreads;  // per-thread Kahan totals (dynamic shared memory)
@@ -1444,10 +920,25 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 constexpr int kPrefetchPoint = 10;
 }  // namespace tpf
 
-__device__ __forceinline__ void tpf_stage(tpf::Smem &sm, const double *basis, const double *weight) {
-  float *b = &sm.B[0][0][0].x;
-  for (int i = threadIdx.x; i < tpf::kNpt * 5 * tpf::kNc4 * 4; i += blockDim.x) b[i] = (float)basis[i];
-  for (int i = threadIdx.x; i < tpf::kNpt; i += blockDim.x) sm.W[i] = (float)weight[i];
+// table: the patch type's staged table, whose leading rows are B's image.
+__device__ __forceinline__ void tpf_stage(tpf::Smem &sm, const float *__restrict__ table) {
+  using L = F32Table<tpf::kNcp, tpf::kNpt>;
+  static_assert(L::ROW4 == 5 * tpf::kNc4, "the table's rows are B's image");
+  const float4 *t = reinterpret_cast<const float4 *>(table);
+  Q4<float> *b = &sm.B[0][0][0];
+  for (int i = threadIdx.x; i < tpf::kNpt * L::ROW4; i += blockDim.x) {
+    const float4 v = __ldg(t + i);
+    b[i] = Q4<float>{v.x, v.y, v.z, v.w};
+  }
+}
+// The points' coefficients for a mesh's moduli, by the block's first threads.
+__device__ __forceinline__ void tpf_coefs(tpf::Smem &sm, const float *__restrict__ table, const SurfaceParams &P,
+                                          double dudv) {
+  if ((int)threadIdx.x >= tpf::kNpt) return;
+  const double w = __ldg(reinterpret_cast<const double *>(table + F32Table<tpf::kNcp, tpf::kNpt>::kWeights) + threadIdx.x);
+  const f32::Coef c = f32::point_coef(P, w, dudv);
+  sm.C[threadIdx.x] = make_float2(c.curv, c.area);
+  sm.Cg[threadIdx.x] = c.gauss;
 }
 
 // Face f's energy terms and dE/dalpha; writes its alpha-scaled gradient
@@ -1458,7 +949,7 @@ __device__ __forceinline__ void tpf_stage(tpf::Smem &sm, const double *basis, co
 template <bool KG_REG>
 __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const SurfaceParams &P, int f,
                                          const float alpha[3], const float ialpha[3], const float am1[3],
-                                         const Moduli<float> &mod, float dudv, bool vec, float *__restrict__ partial,
+                                         float k_reg, bool vec, float *__restrict__ partial,
                                          float e3[3], float da[3], int fn) {
   using namespace tpf;
   uint32_t cp[kNcp];
@@ -1505,38 +996,11 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
         lo[c] = __ldg(&S.rlo[3 * (size_t)v + c]);
         dv[c] = __ldg(&S.dsp[3 * (size_t)v + c]);
       }
-      if (code == 13) {  // the home image (every control point of a closed vesicle)
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          float s2, e2;
-          two_sum(hi[c], -ahi[c], s2, e2);
-          l[c] = s2 + (e2 + (lo[c] - alo[c]));
-        }
-      } else {  // a periodic image: the lattice shift as hi + lo (each term exact)
-        const int img[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
-        float sh[3] = {0.f, 0.f, 0.f}, she[3] = {0.f, 0.f, 0.f}, shl[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-        for (int c = 0; c < 3; ++c)
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            float t, e;
-            two_sum(sh[c], (float)img[d] * P.box_hi[d][c], t, e);
-            sh[c] = t;
-            she[c] += e;
-            shl[c] += (float)img[d] * P.box_lo[d][c];
-          }
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          float s1, e1, s2, e2;
-          two_sum(hi[c], sh[c], s1, e1);
-          two_sum(s1, -ahi[c], s2, e2);
-          l[c] = s2 + ((e1 + e2) + ((lo[c] - alo[c]) + (she[c] + shl[c])));
-        }
-      }
+      f32::local_position(hi, lo, code, ahi, alo, P, l);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        X[jj][c] = alpha[c] * l[c];
-        Dx[jj][c] = fmaf(am1[c], l[c], dv[c] - ad[c]);
+        X[jj][c] = f32::mul(alpha[c], l[c]);
+        Dx[jj][c] = fmaf(am1[c], l[c], f32::sub(dv[c], ad[c]));
       }
     }
 #pragma unroll
@@ -1549,7 +1013,8 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
   float G[kNcp][3];  // gradient sums
 #pragma unroll
   for (int j = 0; j < kNcp; ++j) G[j][0] = G[j][1] = G[j][2] = 0.f;
-  float ea = 0.f, ec = 0.f, er = 0.f, dax = 0.f, day = 0.f, daz = 0.f;
+  float ea = 0.f, ec = 0.f, er = 0.f;
+  Vec3<float> da3 = {0.f, 0.f, 0.f};
 #pragma unroll 1
   for (int p = 0; p < kNpt; ++p) {
     if (p == kPrefetchPoint && fn >= 0) {
@@ -1597,30 +1062,23 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
     }
     Vec3<float> K[5], dR[2];
 #pragma unroll
-    for (int k = 0; k < 5; ++k) K[k] = {A[k][0].x + A[k][0].y, A[k][1].x + A[k][1].y, A[k][2].x + A[k][2].y};
+    for (int k = 0; k < 5; ++k)
+      K[k] = {f32::add(A[k][0].x, A[k][0].y), f32::add(A[k][1].x, A[k][1].y), f32::add(A[k][2].x, A[k][2].y)};
 #pragma unroll
-    for (int k = 0; k < 2; ++k) dR[k] = {Ad[k][0].x + Ad[k][0].y, Ad[k][1].x + Ad[k][1].y, Ad[k][2].x + Ad[k][2].y};
-    Vec3<float> Kb[5], Kreg[2], m;
-    float a, c, r, lkn[3];
-    point_adjoint<float, KG_REG>(K, sm.W[p], g0, rr0, dudv, P2, Hbar, Pres, mod.kc, mod.KA, mod.kg, mod.k_reg, &a,
-                                 &c, &r, Kb, Kreg, dR, lkn, &m);
-    ea += a;
-    ec += c;
-    er += r;
-    // alpha_c dE/dalpha_c over this point: sum_k Kb[k]_c K[k]_c, with Kb[2..4] = (lb, kb, nb) m
-    {
-      const float t[3] = {lkn[0] * K[2].x + lkn[1] * K[3].x + lkn[2] * K[4].x,
-                          lkn[0] * K[2].y + lkn[1] * K[3].y + lkn[2] * K[4].y,
-                          lkn[0] * K[2].z + lkn[1] * K[3].z + lkn[2] * K[4].z};
-      dax = fmaf(Kb[0].x, K[0].x, fmaf(Kb[1].x, K[1].x, fmaf(m.x, t[0], dax)));
-      day = fmaf(Kb[0].y, K[0].y, fmaf(Kb[1].y, K[1].y, fmaf(m.y, t[1], day)));
-      daz = fmaf(Kb[0].z, K[0].z, fmaf(Kb[1].z, K[1].z, fmaf(m.z, t[2], daz)));
-    }
+    for (int k = 0; k < 2; ++k)
+      dR[k] = {f32::add(Ad[k][0].x, Ad[k][0].y), f32::add(Ad[k][1].x, Ad[k][1].y), f32::add(Ad[k][2].x, Ad[k][2].y)};
+    const float2 cf = sm.C[p];
+    const f32::Coef M{cf.x, cf.y, KG_REG ? sm.Cg[p] : 0.f};
+    const f32::Point o = f32::point<KG_REG>(K, dR, M, k_reg, g0, rr0, P2, Hbar, Pres);
+    ea += o.ea;
+    ec += o.ec;
+    er += o.er;
+    da3 = f32::scale_derivative(o, K, da3);
     // G[j]_c += B[u][j] Kb[u]_c + B[v][j] Kb[v]_c + s[j] m_c in scalar multiply-adds: with the
     // forward contraction in paired ones, the mix keeps both FP32 multiply-add pipes busy
     // (all paired: 763 us, this mix: 747 us, all scalar: 776 us on the 256-vesicle pass)
     {
-      const float ku[3] = {Kb[0].x, Kb[0].y, Kb[0].z}, kv[3] = {Kb[1].x, Kb[1].y, Kb[1].z}, md[3] = {m.x, m.y, m.z};
+      const float ku[3] = {o.Ku.x, o.Ku.y, o.Ku.z}, kv[3] = {o.Kv.x, o.Kv.y, o.Kv.z}, md[3] = {o.m.x, o.m.y, o.m.z};
 #pragma unroll
       for (int c4 = 0; c4 < kNc4; ++c4) {
         const Q4<float> bu = sm.B[p][0][c4], bv = sm.B[p][1][c4], buu = sm.B[p][2][c4], buv = sm.B[p][3][c4],
@@ -1630,7 +1088,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
                     vv[4] = {bvv.x, bvv.y, bvv.z, bvv.w};
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-          const float sj = fmaf(vv[jj], lkn[2], fmaf(uv[jj], lkn[1], uu[jj] * lkn[0]));
+          const float sj = fmaf(vv[jj], o.nb, fmaf(uv[jj], o.kb, __fmul_rn(uu[jj], o.lb)));
           float *g = G[4 * c4 + jj];
 #pragma unroll
           for (int cc = 0; cc < 3; ++cc) g[cc] = fmaf(sj, md[cc], fmaf(v[jj], kv[cc], fmaf(u[jj], ku[cc], g[cc])));
@@ -1640,7 +1098,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
   }
   // ---- dE/dalpha_c: K is linear in the alpha-scaled coordinates, so
   // alpha_c dE/dalpha_c = sum over points and k of Kb[k]_c K[k]_c
-  da[0] = dax * ialpha[0]; da[1] = day * ialpha[1]; da[2] = daz * ialpha[2];
+  da[0] = da3.x * ialpha[0]; da[1] = da3.y * ialpha[1]; da[2] = da3.z * ialpha[2];
   int d[kNcp];
   if (vec) {
     const int4 *q = reinterpret_cast<const int4 *>(S.dest + (size_t)f * kNcp);
@@ -1657,7 +1115,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
   for (int j = 0; j < kNcp; ++j) {
     float *o = partial + 3 * (size_t)d[j];
 #pragma unroll
-    for (int c = 0; c < 3; ++c) o[c] = alpha[c] * G[j][c];
+    for (int c = 0; c < 3; ++c) o[c] = f32::mul(alpha[c], G[j][c]);
   }
   e3[0] = ea; e3[1] = ec; e3[2] = er;
 }
@@ -1681,8 +1139,8 @@ struct SharedSums {
     s[(2 * q + 1) * tpf::kThreads] = (t - sum) - y;
     s[2 * q * tpf::kThreads] = t;
   }
-  __device__ __forceinline__ double get(int q) const {
-    return (double)s[2 * q * tpf::kThreads] - (double)s[(2 * q + 1) * tpf::kThreads];
+  __device__ __forceinline__ double total(int q) const {  // over the warp
+    return warp_sum(s[2 * q * tpf::kThreads], s[(2 * q + 1) * tpf::kThreads]);
   }
 };
 
@@ -1698,18 +1156,18 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   using namespace tpf;
   __shared__ Smem sm;
   extern __shared__ __align__(16) unsigned char tpf_dyn[];
-  tpf_stage(sm, L.basis, L.weight);
+  tpf_stage(sm, L.table);
+  tpf_coefs(sm, L.table, P, L.dudv);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float alpha[3] = {(float)r[3 * P.nv], (float)r[3 * P.nv + 1], (float)r[3 * P.nv + 2]};
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
   const float am1[3] = {(float)(r[3 * P.nv] - 1.0), (float)(r[3 * P.nv + 1] - 1.0), (float)(r[3 * P.nv + 2] - 1.0)};
-  const Moduli<float> mod(P);
   const FaceSrc src{L.cp, nullptr, nullptr, nullptr, L.g0f, L.rr0f, L.compf, dest, r, rhi, rlo, dsp, L.nfaces};
   const bool vec = tpf_vec(src);
-  const float dudv = (float)L.dudv;
   const bool kg_reg = P.kg != 0.0 || P.k_reg != 0.0;  // else the pointwise step leaves those terms out
+  const float k_reg = (float)P.k_reg;
   const int n = L.nfaces, stride = gridDim.x * kThreads;
   SharedSums acc{reinterpret_cast<float *>(tpf_dyn) + threadIdx.x};
   acc.zero();
@@ -1719,8 +1177,8 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
       float e3[3], da[3];
       // no prefetch: a thread's next face is a grid stride away, and on the
       // 512 x 512 planar pass the prefetch cost 1% instead of gaining
-      if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, mod, dudv, vec, partial, e3, da, -1);
-      else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, mod, dudv, vec, partial, e3, da, -1);
+      if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, -1);
+      else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, -1);
       acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
       acc.add(3, da[0]); acc.add(4, da[1]); acc.add(5, da[2]);
       if (!isfinite(e3[0] + e3[1] + e3[2])) atomicOr(status, kStatusNonFinite);
@@ -1728,7 +1186,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   }
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
-    const double s = warp_sum(acc.get(q));
+    const double s = acc.total(q);
     if (lane == 0) sm.red[warp][q] = s;
   }
   __syncthreads();  // every thread has read its sums: the finish may reuse their space
@@ -1749,18 +1207,16 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
 // the faces), and copies a job's header only when the tile's job changes.
 __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
     batch_face_tpf_kernel(const BatchJob *__restrict__ jobs, int group, const BatchTile *__restrict__ tiles,
-                          const int *__restrict__ counts, const double *__restrict__ basis,
-                          const double *__restrict__ weight, double dudv_d, double *__restrict__ tile_sums,
-                          int *__restrict__ counter) {
+                          const int *__restrict__ counts, const float *__restrict__ table, double dudv,
+                          double *__restrict__ tile_sums, int *__restrict__ counter) {
   using namespace tpf;
   __shared__ Smem sm;
   __shared__ BatchFaceJob sj;
   __shared__ int s_active, s_tile[2];
-  tpf_stage(sm, basis, weight);  // constant tables: before the wait
+  tpf_stage(sm, table);     // constant table: before the wait
   grid_dependency_wait();        // positions, job states and the counter come from the kernels before
   const int ntiles = counts[group], tile_base = counts[3 + group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const float dudv = (float)dudv_d;
   // Tiles are handed out by a counter (zeroed before the launch), so blocks
   // that draw cheap tiles take more; each tile's sums go to its own row, so
   // the results do not depend on which block took which tile. Draw k is read
@@ -1779,11 +1235,12 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
       int *dst = reinterpret_cast<int *>(&sj);
       for (int i = threadIdx.x; i < (int)(sizeof(BatchFaceJob) / sizeof(int)); i += kThreads) dst[i] = src[i];
       if (threadIdx.x == 0) s_active = job_active(jobs[tile.job].f);
+      tpf_coefs(sm, table, jobs[tile.job].f.P, dudv);
       job = tile.job;
       __syncthreads();
     }
     if (threadIdx.x == 0) s_tile[(k + 1) & 1] = atomicAdd(&counter[0], 1);
-    HalfWarpSums<float> acc;
+    KahanSums<3> acc;
     if (s_active) {
       const FaceSrc &src = sj.src[group];
       const SurfaceParams &P = sj.P;
@@ -1792,25 +1249,25 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
       const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
       const float am1[3] = {(float)(r[3 * P.nv] - 1.0), (float)(r[3 * P.nv + 1] - 1.0),
                             (float)(r[3 * P.nv + 2] - 1.0)};
-      const Moduli<float> mod(P);
       const int end = tile.first + tile.count;
       float *partial = (float *)sj.partial;
       const bool kg_reg = P.kg != 0.0 || P.k_reg != 0.0;  // else the pointwise step leaves those terms out
+      const float k_reg = (float)P.k_reg;
       const bool vec = tpf_vec(src);
       for (int fb = tile.first + warp * 32; fb < end; fb += kThreads) {
         const int f = fb + lane;
         if (f < end) {
           float e3[3], da[3];
           const int fn = f + kThreads < end ? f + kThreads : -1;
-          if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, mod, dudv, vec, partial, e3, da, fn);
-          else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, mod, dudv, vec, partial, e3, da, fn);
+          if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, fn);
+          else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, fn);
           acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
         }
       }
     }
 #pragma unroll
     for (int q = 0; q < 3; ++q) {
-      const double s = warp_sum(acc.get(q));
+      const double s = warp_sum(acc.s[q], acc.c[q]);
       if (lane == 0) sm.red[warp][q] = s;
     }
     __syncthreads();
@@ -2613,7 +2070,7 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
     f[c] = scale / (a * a);
   }
   for (int i = warp; i < nrow; i += nwarps) {
-    HalfWarpSums<float> acc;
+    KahanSums<3> acc;
     const int beg = row_ptr[i], end = row_ptr[i + 1];
     for (int w = 32 * lane; w < 32 * kSpmvAhead; w += 32 * 32) {  // the row's first windows
       if (w < end - beg) {
@@ -2689,23 +2146,8 @@ static cudaError_t tc_opt_in() {
                                      (int)dev::tc::kSmemBytes);
   });
 }
-template <typename T, int NCP, int NPT>
-static int face_grid_size(int nfaces) {
-  // Persistent grid: as many blocks as fit on the device at once (a fixed
-  // number per device, so the face-to-block assignment and the sums' order are fixed).
-  static PerDevice pd;
-  const int cached = per_device(pd, [] {
-    int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::face_kernel<T, NCP, NPT>,
-                                                  dev::FaceCfg<T>::threads, 0);
-    return sm_count() * (per_sm > 0 ? per_sm : 1);
-  });
-  int need = grid_for(nfaces, dev::FaceCfg<T>::half_warps);
-  return need < cached ? need : cached;
-}
-
 // The thread-per-face kernel's persistent grid (precision form, regular faces).
-static int face_grid_size_tpf(int nfaces) {
+int face_blocks_tpf(int nfaces) {
   static PerDevice pd;
   const int cached = per_device(pd, [] {
     int per_sm = 0;
@@ -2717,31 +2159,13 @@ static int face_grid_size_tpf(int nfaces) {
   return need < cached ? need : cached;
 }
 
-int face_blocks(int nfaces, int ncp, int npt) {
-  if (nfaces <= 0) return 0;
-  if (ncp == 12 && npt == 15) return face_grid_size_tpf(nfaces);
-  if (ncp == 11 && npt == 16) return face_grid_size<float, 11, 16>(nfaces);
-  if (ncp == 13 && npt == 16) return face_grid_size<float, 13, 16>(nfaces);
-  return 0;
-}
-
-cudaError_t launch_faces(const dev::FaceLaunch &L, const int *dest, int ncp, int npt, const dev::SurfaceParams &P,
-                         const double *r, const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                         const FinishArgs &fin, cudaStream_t s) {
+cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
+                             const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
+                             const FinishArgs &fin, cudaStream_t s) {
   if (L.nfaces <= 0) return cudaSuccess;
-  constexpr int NT = dev::FaceCfg<float>::threads;
-  const float *rhi = f.hi, *rlo = f.lo, *dsp = f.dsp;
-  if (!rhi || !rlo || !dsp) return cudaErrorInvalidValue;
-  if (ncp == 12 && npt == 15)
-    return launch_after(dev::face_tpf_kernel, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, rhi,
-                        rlo, dsp, partial, blockpart, status, fin);
-  if (ncp == 11 && npt == 16)
-    dev::face_kernel<float, 11, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status, fin);
-  else if (ncp == 13 && npt == 16)
-    dev::face_kernel<float, 13, 16><<<grid, NT, 0, s>>>(L, dest, P, r, rhi, rlo, dsp, partial, blockpart, status, fin);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
+  if (!f.hi || !f.lo || !f.dsp) return cudaErrorInvalidValue;
+  return launch_after(dev::face_tpf_kernel, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, f.hi, f.lo,
+                      f.dsp, partial, blockpart, status, fin);
 }
 
 cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cudaStream_t s) {
@@ -2826,36 +2250,21 @@ cudaError_t launch_spmv(int nrow, const int *row_ptr, const int *col, const doub
 
 namespace umcp {
 
-int batch_face_blocks(int ncp, int npt) {
-  if (ncp == 12 && npt == 15) {  // the batched thread-per-face kernel's own occupancy
-    static PerDevice pd;
-    return per_device(pd, [] {
-      int per_sm = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::batch_face_tpf_kernel, dev::tpf::kThreads, 0);
-      return sm_count() * (per_sm > 0 ? per_sm : 1);
-    });
-  }
-  return face_blocks(1 << 30, ncp, npt);  // device-filling persistent grid
+int batch_face_blocks_tpf() {
+  static PerDevice pd;
+  return per_device(pd, [] {
+    int per_sm = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::batch_face_tpf_kernel, dev::tpf::kThreads, 0);
+    return sm_count() * (per_sm > 0 ? per_sm : 1);
+  });
 }
 
-cudaError_t launch_batch_faces(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
-                               const double *basis, const double *weight, int ncp, int npt, double dudv,
-                               int irregular, double *tile_sums, int grid, int *next_tile, cudaStream_t s) {
-  constexpr int NT = dev::FaceCfg<float>::threads;
-  if (ncp == 12 && npt == 15) {
-    if (!next_tile) return cudaErrorInvalidValue;
-    return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, jobs, group, tiles, counts, basis,
-                        weight, dudv, tile_sums, next_tile);
-  }
-  if (ncp == 11 && npt == 16)
-    dev::batch_face_kernel<float, 11, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv,
-                                                              irregular, tile_sums);
-  else if (ncp == 13 && npt == 16)
-    dev::batch_face_kernel<float, 13, 16><<<grid, NT, 0, s>>>(jobs, group, tiles, counts, basis, weight, dudv,
-                                                              irregular, tile_sums);
-  else
-    return cudaErrorInvalidValue;
-  return cudaGetLastError();
+cudaError_t launch_batch_faces_tpf(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
+                                   const float *table, double dudv, double *tile_sums, int grid, int *next_tile,
+                                   cudaStream_t s) {
+  if (!next_tile) return cudaErrorInvalidValue;
+  return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, jobs, group, tiles, counts, table,
+                      dudv, tile_sums, next_tile);
 }
 
 cudaError_t launch_batch_reduce(const BatchJob *jobs, const int *counts, int max_jobs, const int *tile_off,
