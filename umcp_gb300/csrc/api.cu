@@ -542,7 +542,6 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
   arena.uninit(m->cnt, 2 * sizeof(uint64_t));
   arena.uninit(m->r_eval, nst * sizeof(double));
   arena.zeroed(m->done, sizeof(unsigned));
-  arena.uninit(m->alphas, 3 * sizeof(double));
   if (m->precision == UMCP_FP32_CENTRED) {
     arena.uninit(m->rhi, 3 * (size_t)ME.nv * sizeof(float));
     arena.uninit(m->rlo, 3 * (size_t)ME.nv * sizeof(float));
@@ -890,7 +889,7 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
   b += (size_t)std::max(nblocks, 1) * 6 * 8;          // blockpart
   b += slots * 3 * (f32 ? 4 : 8);                     // partial
   b += 3 * nst * 8 + 2 * 3 * nv * 8;                  // r, g, r_eval; p, qdot
-  b += 8 + 3 * 8 + 4 + 2 * 8 + 4 + 3 * 8;             // E, parts, status, cnt, done, alphas
+  b += 8 + 3 * 8 + 4 + 2 * 8 + 4;                     // E, parts, status, cnt, done
   if (f32) b += 3 * 3 * nv * 4 + 3 * nv * 8;          // rhi, rlo, dsp; r0
   b += (size_t)n_energies * 8;                        // energy record
   *bytes = b;
@@ -921,12 +920,22 @@ extern "C" umcp_status umcp_mass_set(umcp_mesh *m, int nrow, const int *row_ptr,
   else UMCP_CUDA(upload(m->mcol, std::vector<int>(col, col + nnz)));
   if (m->mass_f32) UMCP_CUDA(upload(m->mval, std::vector<float>(val, val + nnz)));
   else UMCP_CUDA(upload(m->mval, std::vector<double>(val, val + nnz)));
-  UMCP_CUDA(m->min32.alloc(m->mass_f32 ? (size_t)nrow * sizeof(float4) : 0));
   UMCP_CUDA(m->mdense.alloc(0));
   m->mass_dense = false;
+  UMCP_CUDA(alloc_mass_input(m, nrow));
   m->mrows = nrow;
   m->drop_graphs();
   return UMCP_OK;
+}
+
+// The apply's factors for host box scales (NULL: 1), as the device formed them.
+static MassScale mass_scale(double scale, const double *alphas) {
+  MassScale f;
+  for (int c = 0; c < 3; ++c) {
+    const double a = alphas ? alphas[c] : 1.0;
+    f.f[c] = scale / (a * a);
+  }
+  return f;
 }
 
 extern "C" umcp_status umcp_mass_apply_device(umcp_mesh *m, const double *d_in, double *d_out, const double *d_scalev,
@@ -934,37 +943,33 @@ extern "C" umcp_status umcp_mass_apply_device(umcp_mesh *m, const double *d_in, 
   if (!m || !d_in || !d_out) return fail(UMCP_ERR_INVALID, "null argument");
   if (!m->mrows) return fail(UMCP_ERR_INVALID, "no mass matrix installed");
   UMCP_CUDA(cudaSetDevice(m->ctx->device));
-  double a[3] = {1, 1, 1};
-  if (alphas) { a[0] = alphas[0]; a[1] = alphas[1]; a[2] = alphas[2]; }
-  UMCP_CUDA(cudaMemcpyAsync(m->alphas.p, a, sizeof a, cudaMemcpyHostToDevice, m->ctx->stream));
-  UMCP_CUDA(queue_mass_apply(m, d_scalev, scale, m->alphas.as<double>(), d_in, d_out, 1, m->ctx->stream));
+  UMCP_CUDA(queue_mass_apply(m, d_scalev, mass_scale(scale, alphas), d_in, d_out, 1, m->ctx->stream));
   UMCP_CUDA(cudaStreamSynchronize(m->ctx->stream));
   return UMCP_OK;
 }
 
+// Host pointers: the input through the mesh's pinned staging and its scratch
+// vectors (r_eval, qdot, g hold nothing between calls); the product is added to
+// out here, as the device would.
 extern "C" umcp_status umcp_mass_apply(umcp_mesh *m, const double *in, double *out, const double *scalev, double scale,
                                        const double *alphas) {
   if (!m || !in || !out) return fail(UMCP_ERR_INVALID, "null argument");
   if (!m->mrows) return fail(UMCP_ERR_INVALID, "no mass matrix installed");
   UMCP_CUDA(cudaSetDevice(m->ctx->device));
+  UMCP_CUDA(ensure_pinned(m));
   cudaStream_t s = m->ctx->stream;
-  const size_t n3 = 3 * (size_t)m->nv;
-  DevBuf din, dout, dsc;
-  UMCP_CUDA(din.alloc(n3 * sizeof(double)));
-  UMCP_CUDA(dout.alloc(n3 * sizeof(double)));
-  UMCP_CUDA(cudaMemcpyAsync(din.p, in, n3 * sizeof(double), cudaMemcpyHostToDevice, s));
-  UMCP_CUDA(cudaMemcpyAsync(dout.p, out, n3 * sizeof(double), cudaMemcpyHostToDevice, s));
+  const size_t n3 = 3 * (size_t)m->nv, bytes = n3 * sizeof(double);
+  memcpy(m->h_stage, in, bytes);
+  UMCP_CUDA(cudaMemcpyAsync(m->r_eval.p, m->h_stage, bytes, cudaMemcpyHostToDevice, s));
   if (scalev) {
-    UMCP_CUDA(dsc.alloc(n3 * sizeof(double)));
-    UMCP_CUDA(cudaMemcpyAsync(dsc.p, scalev, n3 * sizeof(double), cudaMemcpyHostToDevice, s));
+    memcpy(m->h_stage2, scalev, bytes);
+    UMCP_CUDA(cudaMemcpyAsync(m->qdot.p, m->h_stage2, bytes, cudaMemcpyHostToDevice, s));
   }
-  double a[3] = {1, 1, 1};
-  if (alphas) { a[0] = alphas[0]; a[1] = alphas[1]; a[2] = alphas[2]; }
-  UMCP_CUDA(cudaMemcpyAsync(m->alphas.p, a, sizeof a, cudaMemcpyHostToDevice, s));
-  UMCP_CUDA(queue_mass_apply(m, scalev ? dsc.as<double>() : nullptr, scale, m->alphas.as<double>(),
-                             din.as<double>(), dout.as<double>(), 1, s));
-  UMCP_CUDA(cudaMemcpyAsync(out, dout.p, n3 * sizeof(double), cudaMemcpyDeviceToHost, s));
+  UMCP_CUDA(queue_mass_apply(m, scalev ? m->qdot.as<double>() : nullptr, mass_scale(scale, alphas),
+                             m->r_eval.as<double>(), m->g.as<double>(), 0, s));
+  UMCP_CUDA(cudaMemcpyAsync(m->h_stage, m->g.p, bytes, cudaMemcpyDeviceToHost, s));
   UMCP_CUDA(cudaStreamSynchronize(s));
+  for (size_t i = 0; i < n3; ++i) out[i] += m->h_stage[i];
   return UMCP_OK;
 }
 
@@ -1141,7 +1146,7 @@ static cudaError_t queue_step_t(umcp_mesh *m, const StepArgs &a, int use_mass, d
   if (e == cudaSuccess)
     e = launch_kick(m->nv, a, m->cnt.as<uint64_t>(), m->p.as<double>(), m->g.as<double>(), m->status.as<int>(), s);
   if (e == cudaSuccess)
-    e = queue_mass_apply(m, nullptr, 1.0, nullptr, m->p.as<double>(), m->qdot.as<double>(), 0, s);
+    e = queue_mass_apply(m, nullptr, MassScale{{1.0, 1.0, 1.0}}, m->p.as<double>(), m->qdot.as<double>(), 0, s);
   if (e == cudaSuccess)
     e = launch_drift(m->nv, a, m->r.as<double>(), m->p.as<double>(), m->qdot.as<double>(), m->f32pos(),
                      m->status.as<int>(), s);

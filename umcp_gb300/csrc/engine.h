@@ -124,9 +124,11 @@ struct umcp_mesh {
   uint64_t *h_cnt = nullptr;  // pinned, 2 counters
   // effective inverse mass: CSR (mrow, mcol, mval) or dense row-major (mdense);
   // FP64 values, or FP32 ones for meshes of the precision form (mass_f32),
-  // whose apply reads an FP32 copy of its input (min32, nv float4 {x, y, z, 0})
+  // whose apply reads an FP32 copy of its input (min32: CSR nv float4 {x, y, z,
+  // 0}, dense three vectors) and pads the dense rows (dense32_ld)
   int mrows = 0;
-  umcp::DevBuf mrow, mcol, mval, alphas, mdense, min32;
+  umcp::DevBuf mrow, mcol, mval, mdense, min32;
+  umcp::DevBuf mpart;  // slots of the dense FP32 apply's partial sums
   bool mass_dense = false, mass_f32 = false;
   // the FP32 CSR's column indices as uint16 (meshes of at most 65,536 vertices:
   // 6 bytes per nonzero instead of 8 for an apply that HBM bounds)
@@ -154,7 +156,7 @@ struct umcp_mesh {
                                     &G->rr0f, &G->compf, &G->basis_w, &G->table, &G->geo_tab})
         b += x->bytes;
     for (const umcp::DevBuf *x : {&partial, &off, &blockpart, &r, &g, &p, &qdot, &E, &parts, &status, &cnt, &rhi,
-                                  &rlo, &r0, &dsp, &r_eval, &done, &energies, &mrow, &mcol, &mval, &alphas, &mdense, &min32, &geo_block, &gterm,
+                                  &rlo, &r0, &dsp, &r_eval, &done, &energies, &mrow, &mcol, &mval, &mdense, &min32, &mpart, &geo_block, &gterm,
                                   &geo_done})
       b += x->bytes;
     return b;
@@ -183,8 +185,10 @@ const Plan &plan_of(const umcp_plan *p);
 
 // out (+)= M^-1 in with the installed inverse mass, dense or CSR (see launch_spmv
 // for the scaling arguments).
-cudaError_t queue_mass_apply(umcp_mesh *m, const double *scalev, double scale, const double *alphas,
-                             const double *in, double *out, int accumulate, cudaStream_t s);
+cudaError_t queue_mass_apply(umcp_mesh *m, const double *scalev, const MassScale &f, const double *in, double *out,
+                             int accumulate, cudaStream_t s);
+// The apply's input copy and scratch for the form just installed (n rows).
+cudaError_t alloc_mass_input(umcp_mesh *m, int n);
 
 // Integrator settings of a run on mesh m (validates it).
 umcp_status make_step_args(const umcp_mesh *m, const umcp_integrator *it, StepArgs *a);

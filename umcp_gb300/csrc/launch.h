@@ -254,17 +254,27 @@ int batch_face_blocks64(int ncp);
 // Faces in flight per block of the half-warp kernels: the unit of a batch's tile sizes.
 constexpr int kHalfWarps = 8;
 
-// out[3i+c] (+)= scale/alpha_c^2 * (scalev ? scalev[c*nrow+i] : 1) * sum_k val[k] in[3 col[k]+c].
-// accumulate=0 overwrites out. alphas: device pointer to 3 doubles (or NULL = 1).
-// launch_spmv on FP32 values and an FP32 input packed as float4 {x, y, z, 0}
-// per row (spmv32_kernel).
-cudaError_t launch_spmv32(int nrow, const int *row_ptr, const void *col, bool col16, const float *val, const double *scalev,
-                          double scale, const double *alphas, const float4 *in, double *out, int accumulate,
-                          cudaStream_t s);
-// out[i] = {(float)in[3i], (float)in[3i+1], (float)in[3i+2], 0}, i < n.
-cudaError_t launch_to_f32x4(int n, const double *in, float4 *out, cudaStream_t s);
+// Factors of an M^-1 apply per component, scale / alpha_c^2.
+struct MassScale {
+  double f[3];
+};
+// out[3i+c] (+)= f_c (scalev ? scalev[c*nrow+i] : 1) * sum_k val[k] in[3 col[k]+c].
+// accumulate=0 overwrites out.
 cudaError_t launch_spmv(int nrow, const int *row_ptr, const int *col, const double *val, const double *scalev,
-                        double scale, const double *alphas, const double *in, double *out, int accumulate,
-                        cudaStream_t s);
+                        const MassScale &f, const double *in, double *out, int accumulate, cudaStream_t s);
+// The same on FP32 values and an FP32 input packed as float4 {x, y, z, 0} per
+// row (spmv32_kernel).
+cudaError_t launch_spmv32(int nrow, const int *row_ptr, const void *col, bool col16, const float *val,
+                          const double *scalev, const MassScale &f, const float4 *in, double *out, int accumulate,
+                          cudaStream_t s);
+// The same on a dense FP32 matrix, rows padded with zeros to dense32_ld(n)
+// floats, and the input as three vectors x[c][dense32_ld(n)], padded with zeros.
+inline int dense32_ld(int n) { return (n + 31) / 32 * 32; }
+size_t dense32_scratch_doubles(int n);
+cudaError_t launch_dense_apply32(int n, const float *A, const float *x, double *scratch, const MassScale &f,
+                                 const double *scalev, double *out, int accumulate, cudaStream_t s);
+// The FP32 input of those: out4[i] = {in[3i], in[3i+1], in[3i+2], 0}, or (ld > 0)
+// out[c ld + i] = in[3i+c].
+cudaError_t launch_mass_input32(int n, const double *in, float *out, int ld, cudaStream_t s);
 
 }  // namespace umcp

@@ -146,117 +146,54 @@ __global__ void truncate_kernel(int n, double rel_tol, double *__restrict__ A, u
   if ((threadIdx.x & 31) == 0) atomicAdd(kept, k);
 }
 
-// out[3i+c] (+)= scale/alpha_c^2 * (scalev ? scalev[c*n+i] : 1) * sum_j A[i][j] in[3j+c].
-// One block per row (grid-stride), fixed-order block reduction.
-__global__ void dense_apply_kernel(int n, const double *__restrict__ A, const double *__restrict__ scalev, double scale,
-                                   const double *__restrict__ alphas, const double *__restrict__ in,
-                                   double *__restrict__ out, int accumulate) {
-  __shared__ double red[3][8];
-  for (int i = blockIdx.x; i < n; i += gridDim.x) {
+// out[3i+c] (+)= f_c (scalev ? scalev[c*n+i] : 1) * sum_j A[i][j] in[3j+c] in
+// FP64, one warp per row. It is bound by the FP64 pipe (64 cycles per warp
+// instruction and scheduler): three multiply-adds per 32 elements, and the sums
+// over the lanes, which exchange halves of the three components (6 adds a row
+// instead of 15). A block of eight warps per row spent most of a 642-column row
+// on its sums.
+constexpr int kDense64Threads = 128;
+__global__ void __launch_bounds__(kDense64Threads)
+    dense_apply_kernel(int n, const double *__restrict__ A, const double *__restrict__ scalev, MassScale F,
+                       const double *__restrict__ in, double *__restrict__ out, int accumulate) {
+  const int lane = threadIdx.x & 31, warps = gridDim.x * (kDense64Threads / 32);
+  for (int i = blockIdx.x * (kDense64Threads / 32) + (threadIdx.x >> 5); i < n; i += warps) {
     const double *row = A + (size_t)i * n;
-    double a0 = 0, a1 = 0, a2 = 0;
-    for (int j = threadIdx.x; j < n; j += blockDim.x) {
+    double a[4] = {0, 0, 0, 0};
+    int j = lane;
+    for (; j + 96 < n; j += 128) {  // four columns' loads in flight
+      double m[4], x[4][3];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        m[u] = row[j + 32 * u];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) x[u][c] = in[3 * (size_t)(j + 32 * u) + c];
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) a[c] = fma(m[u], x[u][c], a[c]);
+    }
+    for (; j < n; j += 32) {
       const double m = row[j];
-      a0 += m * in[3 * (size_t)j];
-      a1 += m * in[3 * (size_t)j + 1];
-      a2 += m * in[3 * (size_t)j + 2];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) a[c] = fma(m, in[3 * (size_t)j + c], a[c]);
     }
-    for (int off = 16; off >= 1; off >>= 1) {
-      a0 += __shfl_xor_sync(0xffffffffu, a0, off);
-      a1 += __shfl_xor_sync(0xffffffffu, a1, off);
-      a2 += __shfl_xor_sync(0xffffffffu, a2, off);
-    }
-    const int w = threadIdx.x >> 5;
-    if ((threadIdx.x & 31) == 0) { red[0][w] = a0; red[1][w] = a1; red[2][w] = a2; }
-    __syncthreads();
-    if (threadIdx.x < 3) {
-      const int c = threadIdx.x;
-      double s = 0;
-      for (int k = 0; k < (int)(blockDim.x >> 5); ++k) s += red[c][k];
-      const double al = alphas ? alphas[c] : 1.0;
-      double f = scale / (al * al);
+    // lanes with bit 4 keep component 2 (and the zero), the others 0 and 1; bit 3 picks one of the two
+    const bool b4 = lane & 16, b3 = lane & 8;
+    const double s0 = __shfl_xor_sync(0xffffffffu, b4 ? a[0] : a[2], 16);
+    const double s1 = __shfl_xor_sync(0xffffffffu, b4 ? a[1] : a[3], 16);
+    const double k0 = (b4 ? a[2] : a[0]) + s0, k1 = (b4 ? a[3] : a[1]) + s1;
+    double v = (b3 ? k1 : k0) + __shfl_xor_sync(0xffffffffu, b3 ? k0 : k1, 8);
+#pragma unroll
+    for (int off = 4; off >= 1; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    const int c = 2 * b4 + b3;
+    if ((lane & 7) == 0 && c < 3) {
+      double f = F.f[c];
       if (scalev) f *= scalev[(size_t)c * n + i];
-      const double v = f * s;
-      out[3 * (size_t)i + c] = accumulate ? out[3 * (size_t)i + c] + v : v;
+      const size_t o = 3 * (size_t)i + c;
+      out[o] = accumulate ? out[o] + f * v : f * v;
     }
-    __syncthreads();
-  }
-}
-
-// dense_apply_kernel on FP32 values and an FP32 input packed as one float4
-// per row. One warp takes kDenseRows rows at once, so each coalesced load of
-// the input serves all of them; every lane keeps kDenseAhead columns' loads of
-// each row in flight (the matrix streams from HBM once, with an evict-first
-// hint, while the input stays cached). Kahan-compensated FP32 sums per lane
-// and row, then the lanes' sums in FP64 in a fixed butterfly order, and the
-// scaling in FP64. (L2 prefetches 8 iterations ahead of each row's loads, as
-// the CSR apply makes, took 10,242 rows from 153.5 to 163.9 us; two warps per
-// nine rows, one per half of the columns, with twice the loads in flight per
-// SM, took 164-166 us.)
-constexpr int kDenseRows = 4;
-constexpr int kDenseAhead = 4;
-constexpr int kDenseThreads = 256;
-__global__ void __launch_bounds__(kDenseThreads, 3) dense_apply32_kernel(int n, const float *__restrict__ A,
-                                                                      const double *__restrict__ scalev, double scale,
-                                                                      const double *__restrict__ alphas,
-                                                                      const float4 *__restrict__ in4,
-                                                                      double *__restrict__ out, int accumulate) {
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (kDenseThreads / 32);
-  for (int i0 = (blockIdx.x * (kDenseThreads / 32) + (threadIdx.x >> 5)) * kDenseRows; i0 < n;
-       i0 += warps * kDenseRows) {
-    const int nr = n - i0 < kDenseRows ? n - i0 : kDenseRows;
-    float s[kDenseRows][3], c[kDenseRows][3];
-#pragma unroll
-    for (int r = 0; r < kDenseRows; ++r)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) s[r][q] = c[r][q] = 0.f;
-    for (int j0 = lane; j0 < n; j0 += 32 * kDenseAhead) {
-      float4 x[kDenseAhead];
-      float m[kDenseRows][kDenseAhead];
-#pragma unroll
-      for (int u = 0; u < kDenseAhead; ++u) {
-        const int j = j0 + 32 * u;
-        x[u] = j < n ? __ldg(&in4[j]) : make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-        for (int r = 0; r < kDenseRows; ++r)
-          m[r][u] = (j < n && r < nr) ? __ldcs(&A[(size_t)(i0 + r) * n + j]) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < kDenseAhead; ++u) {
-        if (j0 + 32 * u >= n) break;
-        const float xv[3] = {x[u].x, x[u].y, x[u].z};
-#pragma unroll
-        for (int r = 0; r < kDenseRows; ++r)
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            const float y = fmaf(m[r][u], xv[q], -c[r][q]), t = s[r][q] + y;
-            c[r][q] = (t - s[r][q]) - y;
-            s[r][q] = t;
-          }
-      }
-    }
-    double a[kDenseRows][3];
-#pragma unroll
-    for (int r = 0; r < kDenseRows; ++r)
-#pragma unroll
-      for (int q = 0; q < 3; ++q) {
-        a[r][q] = (double)s[r][q] - (double)c[r][q];
-        for (int off = 16; off >= 1; off >>= 1) a[r][q] += __shfl_xor_sync(0xffffffffu, a[r][q], off);
-      }
-    // lane 3 r + q writes component q of row i0 + r
-#pragma unroll
-    for (int r = 0; r < kDenseRows; ++r)
-#pragma unroll
-      for (int q = 0; q < 3; ++q)
-        if (lane == 3 * r + q && r < nr) {
-          const int i = i0 + r;
-          const double al = alphas ? alphas[q] : 1.0;
-          double f = scale / (al * al);
-          if (scalev) f *= scalev[(size_t)q * n + i];
-          const double v = f * a[r][q];
-          out[3 * (size_t)i + q] = accumulate ? out[3 * (size_t)i + q] + v : v;
-        }
   }
 }
 
@@ -296,38 +233,45 @@ __global__ void row_fill_kernel(int n, const double *__restrict__ A, const int *
   }
 }
 
-__global__ void dense_to_f32_kernel(size_t total, const double *__restrict__ A, float *__restrict__ B) {
-  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x)
-    B[e] = (float)A[e];
+// A rounded to FP32, rows padded with zeros to ld columns.
+__global__ void dense_to_f32_kernel(int n, int ld, const double *__restrict__ A, float *__restrict__ B) {
+  const size_t total = (size_t)n * ld;
+  for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < total; e += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = e / ld, j = e % ld;
+    B[e] = j < (size_t)n ? (float)A[i * n + j] : 0.f;
+  }
 }
 
 }  // namespace
 
-cudaError_t umcp::queue_mass_apply(umcp_mesh *m, const double *scalev, double scale, const double *alphas,
-                                   const double *in, double *out, int accumulate, cudaStream_t s) {
+cudaError_t umcp::queue_mass_apply(umcp_mesh *m, const double *scalev, const MassScale &f, const double *in,
+                                   double *out, int accumulate, cudaStream_t s) {
+  const int n = m->mrows;
   if (m->mass_f32) {
-    cudaError_t e = launch_to_f32x4(m->mrows, in, m->min32.as<float4>(), s);
+    const cudaError_t e = launch_mass_input32(n, in, m->min32.as<float>(), m->mass_dense ? dense32_ld(n) : 0, s);
     if (e != cudaSuccess) return e;
-    if (!m->mass_dense)
-      return launch_spmv32(m->mrows, m->mrow.as<int>(), m->mcol.p, m->mcol16, m->mval.as<float>(), scalev, scale, alphas,
-                           m->min32.as<float4>(), out, accumulate, s);
+    if (m->mass_dense)
+      return launch_dense_apply32(n, m->mdense.as<float>(), m->min32.as<float>(), m->mpart.as<double>(), f, scalev, out,
+                                  accumulate, s);
+    return launch_spmv32(n, m->mrow.as<int>(), m->mcol.p, m->mcol16, m->mval.as<float>(), scalev, f,
+                         m->min32.as<float4>(), out, accumulate, s);
   }
   if (m->mass_dense) {
-    int sms = 152;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->ctx->device);
-    const int grid = m->mrows < sms * 8 ? m->mrows : sms * 8;
-    if (m->mass_f32) {
-      const int groups = (m->mrows + kDenseRows - 1) / kDenseRows, per_block = kDenseThreads / 32;
-      const int blocks = (groups + per_block - 1) / per_block;
-      dense_apply32_kernel<<<blocks < sms * 8 ? blocks : sms * 8, kDenseThreads, 0, s>>>(
-          m->mrows, m->mdense.as<float>(), scalev, scale, alphas, m->min32.as<float4>(), out, accumulate);
-    } else
-      dense_apply_kernel<<<grid, 256, 0, s>>>(m->mrows, m->mdense.as<double>(), scalev, scale, alphas, in, out,
-                                              accumulate);
+    const int per_block = kDense64Threads / 32, blocks = (n + per_block - 1) / per_block;
+    dense_apply_kernel<<<blocks, kDense64Threads, 0, s>>>(n, m->mdense.as<double>(), scalev, f, in, out, accumulate);
     return cudaGetLastError();
   }
-  return launch_spmv(m->mrows, m->mrow.as<int>(), m->mcol.as<int>(), m->mval.as<double>(), scalev, scale, alphas, in,
-                     out, accumulate, s);
+  return launch_spmv(n, m->mrow.as<int>(), m->mcol.as<int>(), m->mval.as<double>(), scalev, f, in, out, accumulate, s);
+}
+
+cudaError_t umcp::alloc_mass_input(umcp_mesh *m, int n) {
+  // float4 per row (CSR), or three padded vectors (dense); the padding stays zero
+  const size_t bytes = !m->mass_f32 ? 0 : m->mass_dense ? 3 * (size_t)dense32_ld(n) * sizeof(float) : n * sizeof(float4);
+  cudaError_t e = m->min32.alloc(bytes);
+  if (e == cudaSuccess && bytes) e = cudaMemset(m->min32.p, 0, bytes);
+  if (e == cudaSuccess)
+    e = m->mpart.alloc(m->mass_f32 && m->mass_dense ? dense32_scratch_doubles(n) * sizeof(double) : 0);
+  return e;
 }
 
 static umcp_status fail(umcp_status s, const std::string &msg) { return umcp::set_error(s, msg); }
@@ -423,8 +367,8 @@ extern "C" umcp_status umcp_mass_build(umcp_mesh *m, const umcp_plan *plan, cons
   const bool f32 = m->precision == UMCP_FP32_CENTRED;
   if (fill >= 0.3) {
     if (f32) {
-      UMCP_CUDA(m->mdense.alloc((size_t)n * n * sizeof(float)));
-      dense_to_f32_kernel<<<sms * 8, 256, 0, s>>>((size_t)n * n, A.as<double>(), m->mdense.as<float>());
+      UMCP_CUDA(m->mdense.alloc((size_t)n * dense32_ld(n) * sizeof(float)));
+      dense_to_f32_kernel<<<sms * 8, 256, 0, s>>>(n, dense32_ld(n), A.as<double>(), m->mdense.as<float>());
       UMCP_CUDA(cudaGetLastError());
       UMCP_CUDA(cudaStreamSynchronize(s));
     } else {
@@ -468,7 +412,7 @@ extern "C" umcp_status umcp_mass_build(umcp_mesh *m, const umcp_plan *plan, cons
     m->mass_dense = false;
   }
   m->mass_f32 = f32;
-  UMCP_CUDA(m->min32.alloc(f32 ? (size_t)n * sizeof(float4) : 0));
+  UMCP_CUDA(alloc_mass_input(m, n));
   m->mrows = n;
   if (info) {
     const auto t_end = std::chrono::steady_clock::now();
@@ -499,7 +443,8 @@ extern "C" umcp_status umcp_mass_get(umcp_mesh *m, double *dense) {
   if (m->mass_dense) {
     if (m->mass_f32) {
       std::vector<float> a((size_t)n * n);
-      UMCP_CUDA(cudaMemcpy(a.data(), m->mdense.p, a.size() * sizeof(float), cudaMemcpyDeviceToHost));
+      UMCP_CUDA(cudaMemcpy2D(a.data(), n * sizeof(float), m->mdense.p, dense32_ld(n) * sizeof(float), n * sizeof(float), n,
+                             cudaMemcpyDeviceToHost));
       for (size_t e = 0; e < a.size(); ++e) dense[e] = a[e];
     } else {
       UMCP_CUDA(cudaMemcpy(dense, m->mdense.p, (size_t)n * n * sizeof(double), cudaMemcpyDeviceToHost));

@@ -1999,19 +1999,13 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
 // One warp per row; lanes stride the row's nonzeros (coalesced reads of the
 // value/column streams), warp-shuffle sum in fixed order.
 __global__ void spmv_kernel(int nrow, const int *__restrict__ row_ptr, const int *__restrict__ col,
-                            const double *__restrict__ val, const double *__restrict__ scalev, double scale,
-                            const double *__restrict__ alphas, const double *__restrict__ in, double *__restrict__ out,
-                            int accumulate) {
+                            const double *__restrict__ val, const double *__restrict__ scalev, MassScale F,
+                            const double *__restrict__ in, double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  double f[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    double a = alphas ? alphas[c] : 1.0;
-    f[c] = scale / (a * a);
-  }
+  const double f[3] = {F.f[0], F.f[1], F.f[2]};
   for (int i = warp; i < nrow; i += nwarps) {
     double s0 = 0, s1 = 0, s2 = 0;
     for (int k = row_ptr[i] + lane; k < row_ptr[i + 1]; k += 32) {
@@ -2056,19 +2050,14 @@ constexpr int kSpmvAhead = 32;
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 template <typename C>  // column index type: int, or uint16_t for up to 65,536 columns
 __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C *__restrict__ col,
-                              const float *__restrict__ val, const double *__restrict__ scalev, double scale,
-                              const double *__restrict__ alphas, const float4 *__restrict__ in4,
+                              const float *__restrict__ val, const double *__restrict__ scalev, MassScale F,
+                              const float4 *__restrict__ in4,
                               double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
-  double f[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    double a = alphas ? alphas[c] : 1.0;
-    f[c] = scale / (a * a);
-  }
+  const double f[3] = {F.f[0], F.f[1], F.f[2]};
   for (int i = warp; i < nrow; i += nwarps) {
     KahanSums<3> acc;
     const int beg = row_ptr[i], end = row_ptr[i + 1];
@@ -2128,11 +2117,13 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
   }
 }
 
-// Rows of three doubles to float4 {x, y, z, 0}.
-__global__ void to_f32x4_kernel(int n, const double *__restrict__ in, float4 *__restrict__ out) {
+// Rows of three doubles to float4 {x, y, z, 0}, or (ld > 0) to three vectors.
+__global__ void mass_input32_kernel(int n, const double *__restrict__ in, float *__restrict__ out, int ld) {
   grid_dependency_wait();
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-    out[i] = make_float4((float)in[3 * (size_t)i], (float)in[3 * (size_t)i + 1], (float)in[3 * (size_t)i + 2], 0.f);
+  for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * n; t += gridDim.x * blockDim.x) {
+    const int i = t / 3, c = t - 3 * i;
+    out[ld > 0 ? (size_t)c * ld + i : 4 * (size_t)i + c] = (float)in[t];
+  }
 }
 
 }  // namespace dev
@@ -2213,8 +2204,8 @@ cudaError_t launch_drift(int nv, const StepArgs &a, double *r, double *p, const 
                       status);
 }
 cudaError_t launch_spmv32(int nrow, const int *row_ptr, const void *col, bool col16, const float *val,
-                          const double *scalev, double scale, const double *alphas, const float4 *in, double *out,
-                          int accumulate, cudaStream_t s) {
+                          const double *scalev, const MassScale &f, const float4 *in, double *out, int accumulate,
+                          cudaStream_t s) {
   if (nrow <= 0) return cudaSuccess;
   int warps_per_block = 8;
   int grid = grid_for(nrow, warps_per_block);
@@ -2224,26 +2215,24 @@ cudaError_t launch_spmv32(int nrow, const int *row_ptr, const void *col, bool co
   // 16-byte value loads, was slower: 0.80 against 0.55 ms at 40,962 rows)
   if (col16)
     return launch_after(dev::spmv32_kernel<uint16_t>, grid, 32 * warps_per_block, 0, s, nrow, row_ptr,
-                        static_cast<const uint16_t *>(col), val, scalev, scale, alphas, in, out, accumulate);
+                        static_cast<const uint16_t *>(col), val, scalev, f, in, out, accumulate);
   return launch_after(dev::spmv32_kernel<int>, grid, 32 * warps_per_block, 0, s, nrow, row_ptr,
-                      static_cast<const int *>(col), val, scalev, scale, alphas, in, out, accumulate);
+                      static_cast<const int *>(col), val, scalev, f, in, out, accumulate);
 }
 
-cudaError_t launch_to_f32x4(int n, const double *in, float4 *out, cudaStream_t s) {
+cudaError_t launch_mass_input32(int n, const double *in, float *out, int ld, cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const int g = grid_for(n, 256);
-  return launch_after(dev::to_f32x4_kernel, g < 152 * 8 ? g : 152 * 8, 256, 0, s, n, in, out);
+  return launch_after(dev::mass_input32_kernel, grid_for(3 * n, 256), 256, 0, s, n, in, out, ld);
 }
 
 cudaError_t launch_spmv(int nrow, const int *row_ptr, const int *col, const double *val, const double *scalev,
-                        double scale, const double *alphas, const double *in, double *out, int accumulate,
-                        cudaStream_t s) {
+                        const MassScale &f, const double *in, double *out, int accumulate, cudaStream_t s) {
   if (nrow <= 0) return cudaSuccess;
   int warps_per_block = 8;
   int grid = grid_for(nrow, warps_per_block);
   if (grid > 152 * 16) grid = 152 * 16;
-  return launch_after(dev::spmv_kernel, grid, 32 * warps_per_block, 0, s, nrow, row_ptr, col, val, scalev, scale,
-                      alphas, in, out, accumulate);
+  return launch_after(dev::spmv_kernel, grid, 32 * warps_per_block, 0, s, nrow, row_ptr, col, val, scalev, f, in, out,
+                      accumulate);
 }
 
 }  // namespace umcp
