@@ -342,12 +342,13 @@ cudaError_t ensure_pinned(umcp_mesh *m) {
   if (m->h_pinned) return cudaSuccess;
   const size_t nst = 3 * (size_t)m->nv + 3;
   const size_t a = (nst * sizeof(double) + 63) & ~(size_t)63, b = (3 * (size_t)m->nv * sizeof(double) + 63) & ~(size_t)63;
-  cudaError_t e = cudaMallocHost(&m->h_pinned, a + b + 2 * sizeof(uint64_t));
+  cudaError_t e = cudaMallocHost(&m->h_pinned, a + b + 2 * sizeof(uint64_t) + (nst + 5) * sizeof(double));
   if (e != cudaSuccess) return e;
   unsigned char *h = (unsigned char *)m->h_pinned;
   m->h_stage = (double *)h;
   m->h_stage2 = (double *)(h + a);
   m->h_cnt = (uint64_t *)(h + a + b);
+  m->h_eval = (double *)(m->h_cnt + 2);
   return cudaSuccess;
 }
 
@@ -743,10 +744,12 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
 }
 
 // Energy and gradient of state d_r: E -> d_E (parts -> d_parts), gradient
-// ADDED into d_g (3*nv+3) when d_g is given.
+// ADDED into d_g (3*nv+3) when d_g is given. host_status: the call of a host
+// pointer, whose state is staged (and split) already; the outputs lie in
+// page-locked host memory and are overwritten, the status word goes along.
 template <typename T>
 static cudaError_t queue_energy_grad(umcp_mesh *m, const double *d_r, double *d_E, double *d_parts, double *d_g,
-                                     bool faces_only) {
+                                     bool faces_only, int *host_status) {
   cudaStream_t s = m->ctx->stream;
   cudaError_t e = cudaSuccess;
   if (faces_only) {
@@ -755,35 +758,44 @@ static cudaError_t queue_energy_grad(umcp_mesh *m, const double *d_r, double *d_
     m->split_valid = true;
     return e == cudaSuccess ? queue_faces<T>(m, m->r.as<double>(), nullptr) : e;
   }
-  if (sizeof(T) == 4) {
+  if (sizeof(T) == 4 && !host_status) {
     e = launch_split_positions(3 * m->nv, d_r, m->f32pos(), s);
     m->split_valid = (d_r == m->r.as<double>());
   }
   if (e != cudaSuccess) return e;
+  const int store = host_status != nullptr;
   FinishArgs fin{m->nblocks, d_E, d_parts, d_g ? d_g + 3 * m->nv : nullptr, nullptr, nullptr, 0.0,
-                 m->status.as<int>(), m->done.as<unsigned>()};
+                 m->status.as<int>(), m->done.as<unsigned>(), nullptr, host_status, store};
   e = queue_faces<T>(m, d_r, &fin);
   if (e != cudaSuccess) return e;
-  if (d_g) e = launch_gather<T>(m->nv, m->partial.as<T>(), m->off.as<int>(), d_g, s);
+  if (d_g) e = launch_gather<T>(m->nv, m->partial.as<T>(), m->off.as<int>(), d_g, store, s);
   return e;
 }
 
 static cudaError_t queue_eg(umcp_mesh *m, const double *d_r, double *d_E, double *d_parts, double *d_g,
-                            bool faces_only = false) {
-  return (m->precision == UMCP_FP64) ? queue_energy_grad<double>(m, d_r, d_E, d_parts, d_g, faces_only)
-                                     : queue_energy_grad<float>(m, d_r, d_E, d_parts, d_g, faces_only);
+                            bool faces_only = false, int *host_status = nullptr) {
+  return (m->precision == UMCP_FP64) ? queue_energy_grad<double>(m, d_r, d_E, d_parts, d_g, faces_only, host_status)
+                                     : queue_energy_grad<float>(m, d_r, d_E, d_parts, d_g, faces_only, host_status);
 }
 
-static umcp_status check_status(umcp_mesh *m) {
-  int st = 0;
-  UMCP_CUDA(cudaMemcpyAsync(&st, m->status.p, sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
-  UMCP_CUDA(cudaStreamSynchronize(m->ctx->stream));
+static umcp_status status_result(int st) {
   if (st & kStatusNonFinite) return fail(UMCP_ERR_NONFINITE, "non-finite energy (the reference stops with \"nan en.\")");
   if (st & kStatusDiverged) return fail(UMCP_ERR_DIVERGED, "energy rose above the divergence threshold");
   if (st & kStatusTimeout) return fail(UMCP_ERR_TIMEOUT, "a tensor-core wait in the face pass gave up");
   return UMCP_OK;
 }
 
+static umcp_status check_status(umcp_mesh *m) {
+  int st = 0;
+  UMCP_CUDA(cudaMemcpyAsync(&st, m->status.p, sizeof(int), cudaMemcpyDeviceToHost, m->ctx->stream));
+  UMCP_CUDA(cudaStreamSynchronize(m->ctx->stream));
+  return status_result(st);
+}
+
+// Host pointers. The kernels read the state from the mesh's page-locked staging
+// and write their results there, so a call is three launches and a wait: with
+// copy commands and memsets in between (nine calls) a 162-vertex vesicle took
+// 60 us, of which its kernels were 12.
 static umcp_status host_energy_grad(umcp_mesh *m, const double *r, double *E, double *terms, double *g) {
   if (!m || !r) return fail(UMCP_ERR_INVALID, "null argument");
   UMCP_CUDA(cudaSetDevice(m->ctx->device));
@@ -791,21 +803,17 @@ static umcp_status host_energy_grad(umcp_mesh *m, const double *r, double *E, do
   cudaStream_t s = m->ctx->stream;
   const size_t nst = 3 * (size_t)m->nv + 3;
   memcpy(m->h_stage, r, nst * sizeof(double));
-  UMCP_CUDA(cudaMemcpyAsync(m->r_eval.p, m->h_stage, nst * sizeof(double), cudaMemcpyHostToDevice, s));
-  UMCP_CUDA(cudaMemsetAsync(m->status.p, 0, sizeof(int), s));
-  if (g) UMCP_CUDA(cudaMemsetAsync(m->g.p, 0, nst * sizeof(double), s));
-  UMCP_CUDA(queue_eg(m, m->r_eval.as<double>(), m->E.as<double>(), m->parts.as<double>(),
-                     g ? m->g.as<double>() : nullptr));
-  double e_parts[4];
-  UMCP_CUDA(cudaMemcpyAsync(&e_parts[0], m->E.p, sizeof(double), cudaMemcpyDeviceToHost, s));
-  UMCP_CUDA(cudaMemcpyAsync(&e_parts[1], m->parts.p, 3 * sizeof(double), cudaMemcpyDeviceToHost, s));
-  if (g) UMCP_CUDA(cudaMemcpyAsync(m->h_stage, m->g.p, nst * sizeof(double), cudaMemcpyDeviceToHost, s));
-  umcp_status st = check_status(m);  // synchronizes
-  if (E) *E = e_parts[0];
-  if (terms) { terms[0] = e_parts[1]; terms[1] = e_parts[2]; terms[2] = e_parts[3]; }
+  double *out_g = m->h_eval, *out_E = m->h_eval + nst;  // E, then its three parts
+  int *out_status = (int *)(out_E + 4);
+  UMCP_CUDA(launch_stage_in((int)nst, m->h_stage, m->r_eval.as<double>(), m->f32pos(), m->status.as<int>(), s));
+  m->split_valid = false;  // the FP32 positions are this state's
+  UMCP_CUDA(queue_eg(m, m->r_eval.as<double>(), out_E, out_E + 1, g ? out_g : nullptr, false, out_status));
+  UMCP_CUDA(cudaStreamSynchronize(s));
+  if (E) *E = out_E[0];
+  if (terms) { terms[0] = out_E[1]; terms[1] = out_E[2]; terms[2] = out_E[3]; }
   if (g)
-    for (size_t i = 0; i < nst; ++i) g[i] += m->h_stage[i];
-  return st;
+    for (size_t i = 0; i < nst; ++i) g[i] += out_g[i];
+  return status_result(*out_status);
 }
 
 extern "C" umcp_status umcp_energy(umcp_mesh *mesh, const double *r, double *E, double *terms) {
@@ -835,10 +843,14 @@ extern "C" umcp_status umcp_mesh_info_get(const umcp_mesh *m, umcp_mesh_info *in
   info->n_points = npts;
   info->n_slots = m->nslots;
   const int groups = (int)m->groups.size();
-  // face kernels (the last one also sums the energy) + fused gather/update;
-  // the mass path replaces the fused kernel with memset + gather + kick + spmv + drift.
-  info->kernels_per_step = groups + 1;
-  info->kernels_per_step_mass = groups + 5;
+  // face launches (the last one also sums the energy): one, or the regular
+  // group's own kernel and the irregular groups' one; then the fused
+  // gather/update, or gather and kick, the M^-1 apply and the drift (the dense
+  // FP32 apply's drift is its second kernel)
+  int faces = 1;
+  for (auto &G : m->groups) faces += (G->tc || G->tpf) && groups > 1;
+  info->kernels_per_step = faces + 1;
+  info->kernels_per_step_mass = faces + 3;
   info->precision = m->precision;
   info->device_bytes = (long long)m->device_bytes();
   // bytes umcp_mesh_create copied in: face tables, bases, slot offsets, positions
@@ -948,9 +960,9 @@ extern "C" umcp_status umcp_mass_apply_device(umcp_mesh *m, const double *d_in, 
   return UMCP_OK;
 }
 
-// Host pointers: the input through the mesh's pinned staging and its scratch
-// vectors (r_eval, qdot, g hold nothing between calls); the product is added to
-// out here, as the device would.
+// Host pointers: the kernels read the input from the mesh's page-locked staging
+// (r_eval and qdot are scratch) and write the product there; it is added to out
+// here, as the device would.
 extern "C" umcp_status umcp_mass_apply(umcp_mesh *m, const double *in, double *out, const double *scalev, double scale,
                                        const double *alphas) {
   if (!m || !in || !out) return fail(UMCP_ERR_INVALID, "null argument");
@@ -959,17 +971,21 @@ extern "C" umcp_status umcp_mass_apply(umcp_mesh *m, const double *in, double *o
   UMCP_CUDA(ensure_pinned(m));
   cudaStream_t s = m->ctx->stream;
   const size_t n3 = 3 * (size_t)m->nv, bytes = n3 * sizeof(double);
+  const MassScale f = mass_scale(scale, alphas);
   memcpy(m->h_stage, in, bytes);
-  UMCP_CUDA(cudaMemcpyAsync(m->r_eval.p, m->h_stage, bytes, cudaMemcpyHostToDevice, s));
   if (scalev) {
     memcpy(m->h_stage2, scalev, bytes);
     UMCP_CUDA(cudaMemcpyAsync(m->qdot.p, m->h_stage2, bytes, cudaMemcpyHostToDevice, s));
   }
-  UMCP_CUDA(queue_mass_apply(m, scalev ? m->qdot.as<double>() : nullptr, mass_scale(scale, alphas),
-                             m->r_eval.as<double>(), m->g.as<double>(), 0, s));
-  UMCP_CUDA(cudaMemcpyAsync(m->h_stage, m->g.p, bytes, cudaMemcpyDeviceToHost, s));
+  const double *d_sv = scalev ? m->qdot.as<double>() : nullptr;
+  if (m->mass_f32) {  // the FP32 copy of the input is made from the staging
+    UMCP_CUDA(queue_mass_apply(m, d_sv, f, m->h_stage, m->h_eval, 0, s));
+  } else {
+    UMCP_CUDA(launch_stage_in((int)n3, m->h_stage, m->r_eval.as<double>(), F32Pos{}, nullptr, s));
+    UMCP_CUDA(queue_mass_product(m, d_sv, f, m->r_eval.as<double>(), m->h_eval, 0, s));
+  }
   UMCP_CUDA(cudaStreamSynchronize(s));
-  for (size_t i = 0; i < n3; ++i) out[i] += m->h_stage[i];
+  for (size_t i = 0; i < n3; ++i) out[i] += m->h_eval[i];
   return UMCP_OK;
 }
 
@@ -1141,12 +1157,15 @@ static cudaError_t queue_step_t(umcp_mesh *m, const StepArgs &a, int use_mass, d
   if (a.kind == 0 || !use_mass)
     return launch_gather_step<T>(m->nv, m->partial.as<T>(), m->off.as<int>(), a, m->cnt.as<uint64_t>(),
                                  m->r.as<double>(), m->p.as<double>(), m->f32pos(), m->status.as<int>(), s);
-  e = cudaMemsetAsync(m->g.p, 0, 3 * (size_t)m->nv * sizeof(double), s);
-  if (e == cudaSuccess) e = launch_gather<T>(m->nv, m->partial.as<T>(), m->off.as<int>(), m->g.as<double>(), s);
+  const int n = m->mrows, ld = m->mass_dense ? dense32_ld(n) : 0;
+  float *x32 = m->mass_f32 ? m->min32.as<float>() : nullptr;
+  e = launch_gather_kick<T>(m->nv, m->partial.as<T>(), m->off.as<int>(), a, m->cnt.as<uint64_t>(), m->p.as<double>(), x32,
+                            ld, m->status.as<int>(), s);
+  if (e == cudaSuccess && x32 && m->mass_dense)
+    return launch_dense_drift32(n, m->mdense.as<float>(), x32, m->mpart.as<double>(), a, m->r.as<double>(),
+                                m->p.as<double>(), m->f32pos(), m->status.as<int>(), s);
   if (e == cudaSuccess)
-    e = launch_kick(m->nv, a, m->cnt.as<uint64_t>(), m->p.as<double>(), m->g.as<double>(), m->status.as<int>(), s);
-  if (e == cudaSuccess)
-    e = queue_mass_apply(m, nullptr, MassScale{{1.0, 1.0, 1.0}}, m->p.as<double>(), m->qdot.as<double>(), 0, s);
+    e = queue_mass_product(m, nullptr, MassScale{{1.0, 1.0, 1.0}}, m->p.as<double>(), m->qdot.as<double>(), 0, s);
   if (e == cudaSuccess)
     e = launch_drift(m->nv, a, m->r.as<double>(), m->p.as<double>(), m->qdot.as<double>(), m->f32pos(),
                      m->status.as<int>(), s);
@@ -1333,8 +1352,8 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
   cudaError_t e = queue_groups(m, B, fin, false);
   if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("face pass: ") + cudaGetErrorString(e));
   if (d_g) {
-    e = fp32 ? launch_gather<float>(m->nv, (float *)(base + off_partial), m->off.as<int>(), d_g, s)
-                         : launch_gather<double>(m->nv, (double *)(base + off_partial), m->off.as<int>(), d_g, s);
+    e = fp32 ? launch_gather<float>(m->nv, (float *)(base + off_partial), m->off.as<int>(), d_g, 0, s)
+                         : launch_gather<double>(m->nv, (double *)(base + off_partial), m->off.as<int>(), d_g, 0, s);
     if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("gather: ") + cudaGetErrorString(e));
   }
   // The next call clears the array's status word: hand its bits (non-finite

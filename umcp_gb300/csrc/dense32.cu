@@ -110,6 +110,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   float4 m[kRows], nx[kRows];
   load(g, c, m);
   grid_dependency_wait();  // the vectors come from the kernel before; the matrix does not
+  grid_dependents();
   for (long long u = u0; u < u1; ++u) {
     int gn = g, cn = c + 1;
     if (cn == chunks) { cn = 0; ++gn; }
@@ -160,21 +161,40 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 }
 
-// out (+)= f_c (scalev ? scalev[c n + i] : 1) (sum of row i's slots), one thread per coordinate.
-__global__ void dense_finish32_kernel(int n, int chunks, long long units, long long W, const double *__restrict__ part,
-                                      int slots, MassScale f, const double *__restrict__ scalev,
-                                      double *__restrict__ out, int accumulate) {
-  grid_dependency_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * n) return;
+// Sum of the slots of coordinate t = 3 i + k of the product.
+__device__ __forceinline__ double slot_sum(int t, int chunks, long long units, long long W,
+                                           const double *__restrict__ part, int slots) {
   const int i = t / 3, k = t - 3 * i, g = i / kRows, q = 3 * (i - g * kRows) + k;
   const int ns = (int)(warp_of((long long)(g + 1) * chunks - 1, units, W) - warp_of((long long)g * chunks, units, W)) + 1;
   double s = 0;
   for (int a = 0; a < ns; ++a) s += part[((size_t)g * slots + a) * kSums + q];
+  return s;
+}
+
+// out (+)= f_c (scalev ? scalev[c n + i] : 1) (A x), one thread per coordinate.
+__global__ void dense_finish32_kernel(int n, int chunks, long long units, long long W, const double *__restrict__ part,
+                                      int slots, MassScale f, const double *__restrict__ scalev,
+                                      double *__restrict__ out, int accumulate) {
+  grid_dependency_wait();
+  grid_dependents();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * n) return;
+  const int i = t / 3, k = t - 3 * i;
   double v = f.f[k];
   if (scalev) v *= scalev[(size_t)k * n + i];
-  v *= s;
+  v *= slot_sum(t, chunks, units, W, part, slots);
   out[t] = accumulate ? out[t] + v : v;
+}
+
+__global__ void dense_drift32_kernel(int n, int chunks, long long units, long long W, const double *__restrict__ part,
+                                     int slots, StepArgs a, double *__restrict__ r, double *__restrict__ p,
+                                     float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
+                                     float *__restrict__ dsp, const int *__restrict__ status) {
+  grid_dependency_wait();
+  grid_dependents();
+  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= 3 * n || *status) return;
+  drift(a, t, slot_sum(t, chunks, units, W, part, slots), r, p, rhi, rlo, r0, dsp);
 }
 
 }  // namespace dense32
@@ -205,17 +225,32 @@ size_t dense32_scratch_doubles(int n) {
   return (size_t)p.groups * p.slots * dev::dense32::kSums;
 }
 
+static cudaError_t launch_units(int n, const float *A, const float *x, double *scratch, const Plan32 &p,
+                                cudaStream_t s) {
+  using namespace dev::dense32;
+  return launch_after(dense_apply32_kernel, p.grid, kThreads, 0, s, n, dense32_ld(n), p.chunks, p.units, A, x, scratch,
+                      p.slots);
+}
+
 cudaError_t launch_dense_apply32(int n, const float *A, const float *x, double *scratch, const MassScale &f,
                                  const double *scalev, double *out, int accumulate, cudaStream_t s) {
-  using namespace dev::dense32;
   if (n <= 0) return cudaSuccess;
-  const int ld = dense32_ld(n);
-  const Plan32 p = plan32(n, ld);
-  const cudaError_t e = launch_after(dense_apply32_kernel, p.grid, kThreads, 0, s, n, ld, p.chunks, p.units, A, x,
-                                     scratch, p.slots);
+  const Plan32 p = plan32(n, dense32_ld(n));
+  const cudaError_t e = launch_units(n, A, x, scratch, p, s);
   if (e != cudaSuccess) return e;
-  return launch_after(dense_finish32_kernel, grid_for(3 * n, 128), 128, 0, s, n, p.chunks, p.units,
-                      (long long)p.grid * kWarps, scratch, p.slots, f, scalev, out, accumulate);
+  return launch_after(dev::dense32::dense_finish32_kernel, grid_for(3 * n, 128), 128, 0, s, n, p.chunks, p.units,
+                      (long long)p.grid * dev::dense32::kWarps, scratch, p.slots, f, scalev, out, accumulate);
+}
+
+cudaError_t launch_dense_drift32(int n, const float *A, const float *x, double *scratch, const StepArgs &a, double *r,
+                                 double *p, const F32Pos &f, const int *status, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const Plan32 q = plan32(n, dense32_ld(n));
+  const cudaError_t e = launch_units(n, A, x, scratch, q, s);
+  if (e != cudaSuccess) return e;
+  return launch_after(dev::dense32::dense_drift32_kernel, grid_for(3 * n, 128), 128, 0, s, n, q.chunks, q.units,
+                      (long long)q.grid * dev::dense32::kWarps, scratch, q.slots, a, r, p, f.hi, f.lo, f.r0, f.dsp,
+                      status);
 }
 
 }  // namespace umcp

@@ -9,13 +9,43 @@ namespace umcp {
 namespace dev {
 
 // Programmatic dependent launch: a kernel launched with programmatic stream
-// serialization may start while the kernel before it on the stream finishes;
-// it waits here, before its first read of that kernel's results (a no-op
-// when it was launched without the attribute).
+// serialization may start while the kernel before it on the stream runs; it
+// waits here, before its first read of that kernel's results (a no-op when it
+// was launched without the attribute).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the kernel after this one be scheduled once every block has come this
+// far; it then waits for this kernel's end in grid_dependency_wait. The kernels
+// of a step call it right after their own wait: the next one's blocks are up
+// when this one drains. The long restraint kernels do not: the next kernel's
+// blocks, waiting on the SMs for all of their time, cost other streams' kernels
+// their place (three restrained evaluations in flight: 179 -> 217 us each).
+__device__ __forceinline__ void grid_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // A job takes the step when it has neither stopped nor reached its limit.
 __device__ __forceinline__ bool job_active(const BatchFaceJob &J) { return !*J.status && J.cnt[1] < J.limit; }
+
+// The precision form's FP32 copies of one position coordinate x = r[i]:
+// x = hi + lo to about 2^-48 relative, and dsp = x - r0[i] (the displacement
+// from the reference state, rounded once from FP64).
+__device__ __forceinline__ void store_f32_position(size_t i, double x, float *__restrict__ hi,
+                                                   float *__restrict__ lo, const double *__restrict__ r0,
+                                                   float *__restrict__ dsp) {
+  const float h = (float)x;
+  hi[i] = h;
+  lo[i] = (float)(x - (double)h);
+  dsp[i] = (float)(x - r0[i]);
+}
+
+// Second half of a leapfrog step with M^-1 for coordinate i: r += qdot AK (and
+// p reset for BD), and the precision form's FP32 copies (rhi NULL: none).
+__device__ __forceinline__ void drift(const StepArgs &a, size_t i, double qdot, double *__restrict__ r,
+                                      double *__restrict__ p, float *__restrict__ rhi, float *__restrict__ rlo,
+                                      const double *__restrict__ r0, float *__restrict__ dsp) {
+  const double x = __dadd_rn(r[i], __dmul_rn(qdot, a.AK));
+  r[i] = x;
+  if (a.kind == 1) p[i] = 0.0;
+  if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
+}
 
 // Sum of q over the warp in a fixed (xor-tree) order.
 __device__ __forceinline__ double warp_sum(double q) {
@@ -48,8 +78,12 @@ __device__ void finish_sums(const FinishArgs &F, const double *__restrict__ bloc
     if (F.E) F.E[0] = e;
     if (F.parts) { F.parts[0] = tot[0]; F.parts[1] = tot[1]; F.parts[2] = tot[2]; }
     if (F.galpha)
-      for (int c = 0; c < 3; ++c) F.galpha[c] += tot[3 + c] + (F.gterm ? F.gterm[kGeoDAlpha + c] : 0.0);
+      for (int c = 0; c < 3; ++c) {
+        const double d = tot[3 + c] + (F.gterm ? F.gterm[kGeoDAlpha + c] : 0.0);
+        F.galpha[c] = F.store_galpha ? d : F.galpha[c] + d;
+      }
     if (!isfinite(e)) atomicOr(F.status, kStatusNonFinite);
+    if (F.host_status) *F.host_status = atomicOr(F.status, 0);
     if (F.energies) {
       const uint64_t idx = F.cnt[1];
       F.energies[idx] = e;

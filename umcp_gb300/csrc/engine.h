@@ -122,6 +122,8 @@ struct umcp_mesh {
   double *h_stage = nullptr;  // pinned, 3*nv+3 doubles
   double *h_stage2 = nullptr; // pinned, 3*nv doubles
   uint64_t *h_cnt = nullptr;  // pinned, 2 counters
+  // pinned, written by the kernels of a host call: gradient (3*nv+3 doubles), energy, its three parts, the status word
+  double *h_eval = nullptr;
   // effective inverse mass: CSR (mrow, mcol, mval) or dense row-major (mdense);
   // FP64 values, or FP32 ones for meshes of the precision form (mass_f32),
   // whose apply reads an FP32 copy of its input (min32: CSR nv float4 {x, y, z,
@@ -187,6 +189,10 @@ const Plan &plan_of(const umcp_plan *p);
 // for the scaling arguments).
 cudaError_t queue_mass_apply(umcp_mesh *m, const double *scalev, const MassScale &f, const double *in, double *out,
                              int accumulate, cudaStream_t s);
+// The same once the precision form's FP32 copy of the input is in place (in is
+// read by the plain path only).
+cudaError_t queue_mass_product(umcp_mesh *m, const double *scalev, const MassScale &f, const double *in, double *out,
+                               int accumulate, cudaStream_t s);
 // The apply's input copy and scratch for the form just installed (n rows).
 cudaError_t alloc_mass_input(umcp_mesh *m, int n);
 

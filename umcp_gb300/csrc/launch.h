@@ -24,6 +24,8 @@ struct FinishArgs {
   int *status;
   unsigned *done;
   const double *gterm; // global restraint terms to add (NULL: none), see GeoArgs
+  int *host_status;    // page-locked host word that receives the status (NULL: none)
+  int store_galpha;    // galpha is overwritten instead of added to
 };
 
 // Global area and volume of the limit surface and their restraint (one
@@ -153,10 +155,15 @@ cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cuda
 // *dst |= *src on the device (one thread).
 cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s);
 
-// Per vertex: g[3v+c] += sum of its partial slots off[2v] + 32 k, k < off[2v+1]
-// (32 vertices interleaved per group, see interleave_slots).
+// Per vertex: g[3v+c] += (store: =) sum of its partial slots off[2v] + 32 k, k <
+// off[2v+1] (32 vertices interleaved per group, see interleave_slots).
 template <typename T>
-cudaError_t launch_gather(int nv, const T *partial, const int *off, double *g, cudaStream_t s);
+cudaError_t launch_gather(int nv, const T *partial, const int *off, double *g, int store, cudaStream_t s);
+
+// A host call's state from page-locked host memory (n doubles) into r, without
+// a copy command; the status word cleared (status may be NULL); f.hi given: the
+// FP32 positions of the first n - 3, as launch_split_positions.
+cudaError_t launch_stage_in(int n, const double *host_r, double *r, const F32Pos &f, int *status, cudaStream_t s);
 
 // Integrator kernels. r, p: 3*nv doubles. Noise from Philox4x32-10 keyed by
 // seed, counter (vertex, step, stream) with step = cnt[0] + cnt[1] - 1.
@@ -175,10 +182,12 @@ struct StepArgs {
 template <typename T>
 cudaError_t launch_gather_step(int nv, const T *partial, const int *off, const StepArgs &a, const uint64_t *cnt,
                                double *r, double *p, const F32Pos &f, const int *status, cudaStream_t s);
-// Kinds 1/2 with a mass matrix: kick p (friction, kicks, noise); then
-// qdot = M^-1 p by launch_spmv; then r += qdot AK (and p reset for BD).
-cudaError_t launch_kick(int nv, const StepArgs &a, const uint64_t *cnt, double *p, const double *g, const int *status,
-                        cudaStream_t s);
+// Kinds 1/2 with a mass matrix: gather the gradient and kick p (friction, kicks,
+// noise), with p's FP32 copy for the apply (see launch_mass_input32; NULL in the
+// plain path); then qdot = M^-1 p; then r += qdot AK (and p reset for BD).
+template <typename T>
+cudaError_t launch_gather_kick(int nv, const T *partial, const int *off, const StepArgs &a, const uint64_t *cnt,
+                               double *p, float *x32, int ld, const int *status, cudaStream_t s);
 cudaError_t launch_drift(int nv, const StepArgs &a, double *r, double *p, const double *qdot, const F32Pos &f,
                          const int *status, cudaStream_t s);
 
@@ -273,6 +282,10 @@ inline int dense32_ld(int n) { return (n + 31) / 32 * 32; }
 size_t dense32_scratch_doubles(int n);
 cudaError_t launch_dense_apply32(int n, const float *A, const float *x, double *scratch, const MassScale &f,
                                  const double *scalev, double *out, int accumulate, cudaStream_t s);
+// A leapfrog step's apply and drift: as launch_dense_apply32 into qdot, then
+// launch_drift, with the drift done where the product is formed.
+cudaError_t launch_dense_drift32(int n, const float *A, const float *x, double *scratch, const StepArgs &a, double *r,
+                                 double *p, const F32Pos &f, const int *status, cudaStream_t s);
 // The FP32 input of those: out4[i] = {in[3i], in[3i+1], in[3i+2], 0}, or (ld > 0)
 // out[c ld + i] = in[3i+c].
 cudaError_t launch_mass_input32(int n, const double *in, float *out, int ld, cudaStream_t s);

@@ -28,7 +28,9 @@
 #include <cmath>
 #include <vector>
 
+#include "device_common.cuh"
 #include "engine.h"
+#include "launch_host.h"
 #include "plan.h"
 
 using namespace umcp;
@@ -157,6 +159,8 @@ __global__ void __launch_bounds__(kDense64Threads)
     dense_apply_kernel(int n, const double *__restrict__ A, const double *__restrict__ scalev, MassScale F,
                        const double *__restrict__ in, double *__restrict__ out, int accumulate) {
   const int lane = threadIdx.x & 31, warps = gridDim.x * (kDense64Threads / 32);
+  dev::grid_dependency_wait();
+  dev::grid_dependents();
   for (int i = blockIdx.x * (kDense64Threads / 32) + (threadIdx.x >> 5); i < n; i += warps) {
     const double *row = A + (size_t)i * n;
     double a[4] = {0, 0, 0, 0};
@@ -250,16 +254,23 @@ cudaError_t umcp::queue_mass_apply(umcp_mesh *m, const double *scalev, const Mas
   if (m->mass_f32) {
     const cudaError_t e = launch_mass_input32(n, in, m->min32.as<float>(), m->mass_dense ? dense32_ld(n) : 0, s);
     if (e != cudaSuccess) return e;
-    if (m->mass_dense)
-      return launch_dense_apply32(n, m->mdense.as<float>(), m->min32.as<float>(), m->mpart.as<double>(), f, scalev, out,
-                                  accumulate, s);
+  }
+  return queue_mass_product(m, scalev, f, in, out, accumulate, s);
+}
+
+cudaError_t umcp::queue_mass_product(umcp_mesh *m, const double *scalev, const MassScale &f, const double *in,
+                                     double *out, int accumulate, cudaStream_t s) {
+  const int n = m->mrows;
+  if (m->mass_f32 && m->mass_dense)
+    return launch_dense_apply32(n, m->mdense.as<float>(), m->min32.as<float>(), m->mpart.as<double>(), f, scalev, out,
+                                accumulate, s);
+  if (m->mass_f32)
     return launch_spmv32(n, m->mrow.as<int>(), m->mcol.p, m->mcol16, m->mval.as<float>(), scalev, f,
                          m->min32.as<float4>(), out, accumulate, s);
-  }
   if (m->mass_dense) {
     const int per_block = kDense64Threads / 32, blocks = (n + per_block - 1) / per_block;
-    dense_apply_kernel<<<blocks, kDense64Threads, 0, s>>>(n, m->mdense.as<double>(), scalev, f, in, out, accumulate);
-    return cudaGetLastError();
+    return launch_after(dense_apply_kernel, blocks, kDense64Threads, 0, s, n, m->mdense.as<double>(), scalev, f, in, out,
+                        accumulate);
   }
   return launch_spmv(n, m->mrow.as<int>(), m->mcol.as<int>(), m->mval.as<double>(), scalev, f, in, out, accumulate, s);
 }

@@ -575,23 +575,27 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
   count_and_finish<tc::kThreads>(fin, blockpart);
 }
 
-// The precision form's FP32 copies of one position coordinate x = r[i]:
-// x = hi + lo to about 2^-48 relative, and dsp = x - r0[i] (the displacement
-// from the reference state, rounded once from FP64).
-__device__ __forceinline__ void store_f32_position(size_t i, double x, float *__restrict__ hi,
-                                                   float *__restrict__ lo, const double *__restrict__ r0,
-                                                   float *__restrict__ dsp) {
-  const float h = (float)x;
-  hi[i] = h;
-  lo[i] = (float)(x - (double)h);
-  dsp[i] = (float)(x - r0[i]);
-}
-
 __global__ void split_positions_kernel(int n, const double *__restrict__ r, float *__restrict__ hi,
                                        float *__restrict__ lo, const double *__restrict__ r0,
                                        float *__restrict__ dsp) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
     store_f32_position(i, r[i], hi, lo, r0, dsp);
+}
+
+// A host call's state, read from page-locked host memory where it lies: one
+// kernel in place of a copy, a memset and (precision form) the split, and the
+// kernel after it follows without a copy engine in between.
+__global__ void stage_in_kernel(int n, const double *__restrict__ host_r, double *__restrict__ r,
+                                float *__restrict__ hi, float *__restrict__ lo, const double *__restrict__ r0,
+                                float *__restrict__ dsp, int *__restrict__ status) {
+  grid_dependency_wait();
+  grid_dependents();
+  if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const double x = host_r[i];
+    r[i] = x;
+    if (hi && i < n - 3) store_f32_position(i, x, hi, lo, r0, dsp);
+  }
 }
 
 // dst |= *src (one thread): a status word handed on to another.
@@ -687,12 +691,14 @@ __device__ __forceinline__ void vertex_gradient_f32(const float *__restrict__ pa
 // adds (64 cycles each in FP64) ran one after another.
 template <typename T>
 __global__ void gather_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off,
-                              double *__restrict__ g) {
+                              double *__restrict__ g, int store) {
   grid_dependency_wait();  // the partials come from the face launches
+  grid_dependents();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
     const int v = i / 3, c = i - 3 * v;
     const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
-    g[i] += coordinate_gradient(partial, at.x, at.y, c);
+    const double a = coordinate_gradient(partial, at.x, at.y, c);
+    g[i] = store ? a : g[i] + a;
   }
 }
 
@@ -804,6 +810,7 @@ __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const 
                                    float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
                                    float *__restrict__ dsp, const int *__restrict__ status) {
   grid_dependency_wait();  // the partials and the status come from the face launches
+  grid_dependents();
   if (*status) return;
   const uint64_t st = current_step(cnt);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
@@ -831,14 +838,24 @@ __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const 
   }
 }
 
-__global__ void kick_kernel(int nv, StepArgs a, const uint64_t *__restrict__ cnt, double *__restrict__ p,
-                            const double *__restrict__ g, const int *__restrict__ status) {
+// The mass path's first half, one thread per coordinate: gather the gradient,
+// kick the momentum, and leave its FP32 copy where the precision form's M^-1
+// apply reads it (x32: see launch_mass_input32; NULL in the plain path).
+template <typename T>
+__global__ void gather_kick_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off, StepArgs a,
+                                   const uint64_t *__restrict__ cnt, double *__restrict__ p, float *__restrict__ x32,
+                                   int ld, const int *__restrict__ status) {
   grid_dependency_wait();
+  grid_dependents();
   if (*status) return;
   const uint64_t st = current_step(cnt);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
     const int v = i / 3, c = i - 3 * v;
-    p[i] = kick(a, normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c), p[i], g[i]);
+    const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
+    const double n = normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c);
+    const double q = kick(a, n, p[i], coordinate_gradient(partial, at.x, at.y, c));
+    p[i] = q;
+    if (x32) x32[ld > 0 ? (size_t)c * ld + v : 4 * (size_t)v + c] = (float)q;
   }
 }
 
@@ -846,13 +863,10 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
                              const double *__restrict__ qdot, float *__restrict__ rhi, float *__restrict__ rlo,
                              const double *__restrict__ r0, float *__restrict__ dsp, const int *__restrict__ status) {
   grid_dependency_wait();
+  grid_dependents();
   if (*status) return;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
-    const double x = __dadd_rn(r[i], __dmul_rn(qdot[i], a.AK));
-    r[i] = x;
-    if (a.kind == 1) p[i] = 0.0;
-    if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
-  }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x)
+    drift(a, i, qdot[i], r, p, rhi, rlo, r0, dsp);
 }
 
 // ---------------------------------------------------------------- batches
@@ -1160,6 +1174,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   tpf_coefs(sm, L.table, P, L.dudv);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
+  grid_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float alpha[3] = {(float)r[3 * P.nv], (float)r[3 * P.nv + 1], (float)r[3 * P.nv + 2]};
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
@@ -1215,6 +1230,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   __shared__ int s_active, s_tile[2];
   tpf_stage(sm, table);     // constant table: before the wait
   grid_dependency_wait();        // positions, job states and the counter come from the kernels before
+  grid_dependents();
   const int ntiles = counts[group], tile_base = counts[3 + group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Tiles are handed out by a counter (zeroed before the launch), so blocks
@@ -1294,6 +1310,7 @@ __global__ void batch_reduce_kernel(const BatchJob *__restrict__ jobs, const int
                                     const double *__restrict__ tile_sums, int *__restrict__ live,
                                     unsigned long long *__restrict__ prog) {
   grid_dependency_wait();
+  grid_dependents();
   const int lane = threadIdx.x & 31;
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (j >= counts[6]) return;
@@ -1336,6 +1353,7 @@ template <typename T>
 __global__ void batch_gather_step_kernel(const BatchJob *__restrict__ jobs, const BatchTile *__restrict__ vtiles,
                                          const int *__restrict__ counts, const int *__restrict__ live) {
   grid_dependency_wait();
+  grid_dependents();
   const int nvtiles = counts[7];
   for (int t = blockIdx.x; t < nvtiles; t += gridDim.x) {
     const BatchTile tile = vtiles[t];
@@ -2002,6 +2020,7 @@ __global__ void spmv_kernel(int nrow, const int *__restrict__ row_ptr, const int
                             const double *__restrict__ val, const double *__restrict__ scalev, MassScale F,
                             const double *__restrict__ in, double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
+  grid_dependents();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2054,6 +2073,7 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
                               const float4 *__restrict__ in4,
                               double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
+  grid_dependents();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2120,6 +2140,7 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
 // Rows of three doubles to float4 {x, y, z, 0}, or (ld > 0) to three vectors.
 __global__ void mass_input32_kernel(int n, const double *__restrict__ in, float *__restrict__ out, int ld) {
   grid_dependency_wait();
+  grid_dependents();
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * n; t += gridDim.x * blockDim.x) {
     const int i = t / 3, c = t - 3 * i;
     out[ld > 0 ? (size_t)c * ld + i : 4 * (size_t)i + c] = (float)in[t];
@@ -2166,6 +2187,10 @@ cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cuda
   return cudaGetLastError();
 }
 
+cudaError_t launch_stage_in(int n, const double *host_r, double *r, const F32Pos &f, int *status, cudaStream_t s) {
+  return launch_after(dev::stage_in_kernel, grid_for(n, 128), 128, 0, s, n, host_r, r, f.hi, f.lo, f.r0, f.dsp, status);
+}
+
 cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s) {
   dev::status_merge_kernel<<<1, 1, 0, s>>>(src, dst);
   return cudaGetLastError();
@@ -2174,13 +2199,13 @@ cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s) {
 // Small blocks, so that a small mesh's gather spreads over the SMs.
 constexpr int kGatherThreads = 64;
 template <typename T>
-cudaError_t launch_gather(int nv, const T *partial, const int *off, double *g, cudaStream_t s) {
+cudaError_t launch_gather(int nv, const T *partial, const int *off, double *g, int store, cudaStream_t s) {
   if (nv <= 0) return cudaSuccess;
   return launch_after(dev::gather_kernel<T>, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, partial, off,
-                      g);
+                      g, store);
 }
-template cudaError_t launch_gather<double>(int, const double *, const int *, double *, cudaStream_t);
-template cudaError_t launch_gather<float>(int, const float *, const int *, double *, cudaStream_t);
+template cudaError_t launch_gather<double>(int, const double *, const int *, double *, int, cudaStream_t);
+template cudaError_t launch_gather<float>(int, const float *, const int *, double *, int, cudaStream_t);
 
 template <typename T>
 cudaError_t launch_gather_step(int nv, const T *partial, const int *off, const StepArgs &a, const uint64_t *cnt,
@@ -2193,11 +2218,16 @@ template cudaError_t launch_gather_step<double>(int, const double *, const int *
 template cudaError_t launch_gather_step<float>(int, const float *, const int *, const StepArgs &, const uint64_t *,
                                                double *, double *, const F32Pos &, const int *, cudaStream_t);
 
-cudaError_t launch_kick(int nv, const StepArgs &a, const uint64_t *cnt, double *p, const double *g, const int *status,
-                        cudaStream_t s) {
-  return launch_after(dev::kick_kernel, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, a, cnt, p, g,
-                      status);
+template <typename T>
+cudaError_t launch_gather_kick(int nv, const T *partial, const int *off, const StepArgs &a, const uint64_t *cnt,
+                               double *p, float *x32, int ld, const int *status, cudaStream_t s) {
+  return launch_after(dev::gather_kick_kernel<T>, grid_for(3 * nv, kGatherThreads), kGatherThreads, 0, s, nv, partial,
+                      off, a, cnt, p, x32, ld, status);
 }
+template cudaError_t launch_gather_kick<double>(int, const double *, const int *, const StepArgs &, const uint64_t *,
+                                                double *, float *, int, const int *, cudaStream_t);
+template cudaError_t launch_gather_kick<float>(int, const float *, const int *, const StepArgs &, const uint64_t *,
+                                               double *, float *, int, const int *, cudaStream_t);
 cudaError_t launch_drift(int nv, const StepArgs &a, double *r, double *p, const double *qdot, const F32Pos &f,
                          const int *status, cudaStream_t s) {
   return launch_after(dev::drift_kernel, grid_for(3 * nv, 256), 256, 0, s, nv, a, r, p, qdot, f.hi, f.lo, f.r0, f.dsp,
