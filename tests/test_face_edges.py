@@ -132,3 +132,24 @@ def test_non_finite_coordinates_are_reported(tmp_path, value, precision):
     with pytest.raises(U.UmcpError, match="non-finite"):
         mesh.energy_grad(r)
     mesh.energy_grad(plan.positions())  # and the mesh is usable after it
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("level", [5, 6])
+def test_restrained_gradient_of_large_meshes(tmp_path, level):
+    """Below and above the size where a thread per face takes over: the FP32
+    form's restrained energy and gradient against the FP64 path's."""
+    path = tmp_path / "m.mesh"
+    U.generate_icosphere(path, level, 160.0 * 2 ** (level - 4), 1.0, 11)
+    ctx, got = U.Context(0), {}
+    for precision in (U.FP64, U.FP32_CENTRED):
+        prm = U.params(kc=U.kc_from_kT(20.0), precision=precision)
+        plan = U.Plan(path, prm)
+        mesh = U.Mesh(ctx, plan, prm)
+        mesh.restraints_set(K_area=0.2, K_volume=1e-4)
+        r = plan.positions()
+        r[:-3] += np.random.default_rng(5).normal(0.0, 0.05, r.size - 3)
+        got[precision] = mesh.energy_grad(r)
+    (E64, g64), (E32, g32) = got[U.FP64], got[U.FP32_CENTRED]
+    assert abs(E32 - E64) <= TOL[U.FP32_CENTRED] * abs(E64)
+    assert rel_inf(g32, g64) <= TOL[U.FP32_CENTRED]

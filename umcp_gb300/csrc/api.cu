@@ -487,7 +487,6 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
     arena.stage(G->cp, cp);
     arena.stage(G->basis, basis);
     if (prm->precision == UMCP_FP64) arena.stage(G->table, fixed::basis_table(basis, G->ncp, G->npt, ncpp));
-    else arena.stage(G->table, f32_table(basis, B.weight, G->ncp));
     if (prm->precision == UMCP_FP32_CENTRED) {  // the precision form's kernels read only the FP32 copies
       arena.stage(G->g0f, std::vector<float>(g0.begin(), g0.end()));
       arena.stage(G->rr0f, std::vector<float>(rr0.begin(), rr0.end()));
@@ -503,6 +502,7 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
       for (int p = 0; p < G->npt; ++p)
         for (int x = 0; x < G->ncp; ++x) bw[(size_t)p * G->ncp + x] = B.at(0, p, x);
       arena.stage(G->basis_w, bw);
+      if (prm->precision == UMCP_FP32_CENTRED) arena.stage(G->table, f32_table(basis, bw, B.weight, G->ncp));
     }
     face_base += G->nfaces;
     slot_base += G->nfaces * G->ncp;
@@ -671,7 +671,7 @@ struct FaceBuffers {
 // the irregular groups' launch on its side stream beside it when fork is set.
 // Every block counts toward the finish (FinishArgs::nblk), so whichever block is
 // the last of all sums the block partials.
-static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const FinishArgs &fin, bool fork) {
+static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const FinishArgs &fin, bool fork, bool geo) {
   cudaStream_t s = m->ctx->stream;
   if (m->precision == UMCP_FP64) {
     FaceSet64 F{};
@@ -682,6 +682,7 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
     return launch_faces64(F, m->P, B.r, (double *)B.partial, B.blockpart, fin, s);
   }
   FaceSet32 F{};
+  F.geo = geo;
   const Group *own = nullptr;
   for (auto &G : m->groups) {
     if (G->tc || G->tpf) own = G.get();
@@ -713,7 +714,7 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
   e = own->tc ? launch_faces_tc(L, own->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, partial, B.blockpart,
                                 B.status, own->nblocks, fin, s)
               : launch_faces_tpf(L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
-                                 fin, s);
+                                 fin, geo, s);
   if (e == cudaSuccess)
     e = launch_faces32(F, m->P, B.r, B.f32, partial, B.blockpart, fin, fork ? m->ctx->side : s, !fork);
   if (e == cudaSuccess && fork) e = cudaEventRecord(m->ctx->join, m->ctx->side);
@@ -722,24 +723,28 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
 }
 
 // Face launches of an evaluation at d_r. With restraints on, the area and
-// volume sums run first (the face pass's finish adds their energy) and their
-// gradient is added into the partial slots after it.
+// volume sums run first (the face pass's finish adds their energy); their
+// gradient goes along in the precision form's face kernels, or is added into the
+// partial slots after them (plain path, tensor-core kernel).
 template <typename T>
 static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs *fin_in) {
   cudaStream_t s = m->ctx->stream;
   FinishArgs fin = fin_in ? *fin_in : FinishArgs{};
   const bool geo = m->rs.on && fin_in;
+  // the precision form's SIMT face kernels add the restraints' gradient themselves
+  bool fused = geo && sizeof(T) == 4;
+  for (auto &G : m->groups) fused = fused && !G->tc;
   GeoArgs GA{};
   if (geo) {
     GA = geo_args(m, d_r);
-    cudaError_t e = launch_geo_sums(GA, m->precision == UMCP_FP64, s);
+    cudaError_t e = launch_geo_sums(GA, m->precision == UMCP_FP64, fused, s);
     if (e != cudaSuccess) return e;
     fin.gterm = m->gterm.as<double>();
   }
   const FaceBuffers B{d_r, m->f32pos(), m->partial.p, m->blockpart.as<double>(), m->status.as<int>()};
-  const cudaError_t e = queue_groups(m, B, fin, true);
+  const cudaError_t e = queue_groups(m, B, fin, true, fused);
   if (e != cudaSuccess) return e;
-  if (geo) return launch_geo_grad<T>(GA, m->partial.as<T>(), s);
+  if (geo && !fused) return launch_geo_grad<T>(GA, m->partial.as<T>(), s);
   return cudaSuccess;
 }
 
@@ -1087,7 +1092,7 @@ extern "C" umcp_status umcp_restraints_set(umcp_mesh *m, const umcp_restraints *
     if (m->precision == UMCP_FP32_CENTRED && !m->split_valid)
       UMCP_CUDA(launch_split_positions(3 * m->nv, m->r.as<double>(), m->f32pos(), s));
     m->split_valid = true;
-    UMCP_CUDA(launch_geo_sums(geo_args(m, m->r.as<double>()), m->precision == UMCP_FP64, s));
+    UMCP_CUDA(launch_geo_sums(geo_args(m, m->r.as<double>()), m->precision == UMCP_FP64, true, s));
     double gt[kGeoWords];
     UMCP_CUDA(cudaMemcpyAsync(gt, m->gterm.p, sizeof gt, cudaMemcpyDeviceToHost, s));
     UMCP_CUDA(cudaStreamSynchronize(s));
@@ -1349,7 +1354,7 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
   if (fp32) UMCP_CUDA(launch_split_positions(3 * m->nv, d_r, f32, s));
   FinishArgs fin{m->nblocks, d_E, nullptr, d_g ? d_g + 3 * m->nv : nullptr, nullptr, nullptr, 0.0, status, done};
   const FaceBuffers B{d_r, f32, base + off_partial, blockpart, status};
-  cudaError_t e = queue_groups(m, B, fin, false);
+  cudaError_t e = queue_groups(m, B, fin, false, false);
   if (e != cudaSuccess) return fail(UMCP_ERR_CUDA, std::string("face pass: ") + cudaGetErrorString(e));
   if (d_g) {
     e = fp32 ? launch_gather<float>(m->nv, (float *)(base + off_partial), m->off.as<int>(), d_g, 0, s)

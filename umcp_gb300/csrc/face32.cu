@@ -19,7 +19,7 @@ constexpr int kMinBlocks = 4;
 
 // Faces [first, end) by this block's warps, two at a time, from pair `pair` in
 // strides of `stride` pairs.
-template <int NCP, int NPT, bool KG_REG>
+template <int NCP, int NPT, bool KG_REG, bool GEO>
 __device__ __forceinline__ void faces(Smem<NCP, NPT> &sm, const FaceSrc &S, const SurfaceParams &P, int first, int end,
                                       int pair, int stride, double w, double dudv, bool want_da,
                                       float *__restrict__ partial, KahanSums<6> &sums) {
@@ -36,7 +36,7 @@ __device__ __forceinline__ void faces(Smem<NCP, NPT> &sm, const FaceSrc &S, cons
   for (; f < end; f += 2 * stride) {
     const int fn = f + 2 * stride;
     if (fn < end) load<NCP, NPT, KG_REG>(S, fn + half, end, lane, nxt);
-    face<NCP, NPT, KG_REG>(sm, hw, lane, cur, P, alpha, am1, M, k_reg, reg_alpha, want_da, partial, sums);
+    face<NCP, NPT, KG_REG, GEO>(sm, hw, lane, cur, P, alpha, am1, M, k_reg, reg_alpha, want_da, partial, sums);
     cur = nxt;
   }
 }
@@ -63,7 +63,7 @@ __device__ __forceinline__ void block_row(double (*red)[6], const KahanSums<6> &
 template <int NCP, int NPT>
 __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block, const SurfaceParams &P,
                                       const double *__restrict__ r, const F32View &f, float *__restrict__ partial,
-                                      double *__restrict__ row, bool want_da) {
+                                      double *__restrict__ row, bool want_da, const double *__restrict__ gterm) {
   Smem<NCP, NPT> &sm = *reinterpret_cast<Smem<NCP, NPT> *>(raw);
   const double w = stage(sm, G.table);
   __syncthreads();
@@ -74,10 +74,16 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block
   S.r = r; S.rhi = f.hi; S.rlo = f.lo; S.dsp = f.dsp;
   KahanSums<6> sums;
   const int pair = block * kWarps + (threadIdx.x >> 5), stride = G.nblocks * kWarps;
-  if (P.kg != 0.0 || P.k_reg != 0.0)
-    faces<NCP, NPT, true>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
-  else
-    faces<NCP, NPT, false>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
+  const bool kg_reg = P.kg != 0.0 || P.k_reg != 0.0;
+  if (gterm) {  // restraints: their coefficients come from the sums kernel
+    if (threadIdx.x < NPT) sm.geo[threadIdx.x] = geo_coef(gterm, w, G.dudv);
+    __syncthreads();
+    if (kg_reg) faces<NCP, NPT, true, true>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
+    else faces<NCP, NPT, false, true>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
+  } else {
+    if (kg_reg) faces<NCP, NPT, true, false>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
+    else faces<NCP, NPT, false, false>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
+  }
   block_row(sm.red, sums, r + 3 * (size_t)P.nv, want_da ? 6 : 3, row);
 }
 
@@ -96,9 +102,10 @@ __global__ void __launch_bounds__(f32::kThreads, f32::kMinBlocks)
   const FaceGroup32 &G = F.g[k];
   double *row = blockpart + 6 * (size_t)(G.block_base + b);
   const bool want_da = fin.galpha != nullptr;  // a run's steps leave the box scales alone
-  if (G.ncp == 12) f32::group<12, 15>(raw, G, b, P, r, f, partial, row, want_da);
-  else if (G.ncp == 11) f32::group<11, 16>(raw, G, b, P, r, f, partial, row, want_da);
-  else f32::group<13, 16>(raw, G, b, P, r, f, partial, row, want_da);
+  const double *gterm = F.geo ? fin.gterm : nullptr;
+  if (G.ncp == 12) f32::group<12, 15>(raw, G, b, P, r, f, partial, row, want_da, gterm);
+  else if (G.ncp == 11) f32::group<11, 16>(raw, G, b, P, r, f, partial, row, want_da, gterm);
+  else f32::group<13, 16>(raw, G, b, P, r, f, partial, row, want_da, gterm);
   count_and_finish<f32::kThreads>(fin, blockpart);
 }
 
@@ -133,9 +140,9 @@ __global__ void __launch_bounds__(f32::kThreads, f32::kMinBlocks)
       const FaceSrc &src = sj.src[group];
       const int pair = threadIdx.x >> 5, end = tile.first + tile.count;
       if (sj.P.kg != 0.0 || sj.P.k_reg != 0.0)
-        faces<NCP, NPT, true>(sm, src, sj.P, tile.first, end, pair, kWarps, w, dudv, false, (float *)sj.partial, sums);
+        faces<NCP, NPT, true, false>(sm, src, sj.P, tile.first, end, pair, kWarps, w, dudv, false, (float *)sj.partial, sums);
       else
-        faces<NCP, NPT, false>(sm, src, sj.P, tile.first, end, pair, kWarps, w, dudv, false, (float *)sj.partial, sums);
+        faces<NCP, NPT, false, false>(sm, src, sj.P, tile.first, end, pair, kWarps, w, dudv, false, (float *)sj.partial, sums);
     }
     block_row(sm.red, sums, nullptr, 3, tile_sums + 3 * (size_t)(tile_base + t));
   }

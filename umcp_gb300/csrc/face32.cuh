@@ -5,6 +5,7 @@
 
 #include "face32_table.h"
 #include "kernels.cuh"
+#include "launch.h"
 
 namespace umcp {
 namespace dev {
@@ -112,6 +113,16 @@ __device__ __forceinline__ Coef point_coef(const SurfaceParams &P, double w, dou
   return {(float)(0.25 * P.kc * w), (float)(dudv * w * P.KA), (float)(dudv * w * P.kg)};
 }
 
+// The global restraints at a point: dE_r/dA and dE_r/dV times the point's area
+// and volume weights (cA cw, cV cw / 3), and the limit point (GEO).
+struct GeoPoint {
+  float kA, kV;
+  Vec3<float> R;
+};
+__device__ __forceinline__ float2 geo_coef(const double *gterm, double w, double dudv) {
+  return make_float2((float)(gterm[kGeoCA] * (dudv * w)), (float)(gterm[kGeoCV] * (dudv * w) / 3.0));
+}
+
 // One quadrature point's energy terms and adjoints.
 struct Point {
   float ea, ec, er;       // area, curvature, angle
@@ -132,12 +143,16 @@ struct Point {
 // state that rounding is the whole area force, on coarse patches up to 1e-5
 // of the gradient.
 // KG_REG = false: kg and k_reg are zero and their terms are left out.
+// GEO: the restraints' gradient goes along, dE_r/dg = kA (g = |m|), dE_r/dm =
+// kV R and dE_r/dR = kV m (the last for the caller: one more coefficient of m
+// beside lb, kb, nb, on the value row).
 // Products and sums are rounded as written (no contraction is left to the
 // compiler), so every kernel that inlines this rounds alike: a batch's job
 // follows its single-mesh trajectory bit for bit whichever kernels run it.
-template <bool KG_REG>
+template <bool KG_REG, bool GEO = false>
 __device__ __forceinline__ Point point(const Vec3<float> K[5], const Vec3<float> dR[2], const Coef &M, float k_reg,
-                                       float g0, float rr0, float P2, float Hbar, float Pres) {
+                                       float g0, float rr0, float P2, float Hbar, float Pres,
+                                       const GeoPoint &geo = GeoPoint{}) {
   const Vec3<float> &Ru = K[0], &Rv = K[1], &Suu = K[2], &Suv = K[3], &Svv = K[4], &a = dR[0], &b = dR[1];
   Point o;
   const Vec3<float> m = cross(Ru, Rv);
@@ -181,10 +196,12 @@ __device__ __forceinline__ Point point(const Vec3<float> K[5], const Vec3<float>
     F12 = add(F12, o.r12);
     F22 = add(F22, o.r22);
   }
+  if constexpr (GEO) W2 = fma(geo.kA, ig, W2);
   const float lb = o.lb, kb = o.kb, nb = o.nb;
-  const Vec3<float> mb = {fma(lb, Suu.x, fma(kb, Suv.x, fma(nb, Svv.x, mul(W2, m.x)))),
-                          fma(lb, Suu.y, fma(kb, Suv.y, fma(nb, Svv.y, mul(W2, m.y)))),
-                          fma(lb, Suu.z, fma(kb, Suv.z, fma(nb, Svv.z, mul(W2, m.z))))};
+  Vec3<float> mb = {fma(lb, Suu.x, fma(kb, Suv.x, fma(nb, Svv.x, mul(W2, m.x)))),
+                    fma(lb, Suu.y, fma(kb, Suv.y, fma(nb, Svv.y, mul(W2, m.y)))),
+                    fma(lb, Suu.z, fma(kb, Suv.z, fma(nb, Svv.z, mul(W2, m.z))))};
+  if constexpr (GEO) mb = {fma(geo.kV, geo.R.x, mb.x), fma(geo.kV, geo.R.y, mb.y), fma(geo.kV, geo.R.z, mb.z)};
   // F11 Ru + F12 Rv + Rv x mb and F22 Rv + F12 Ru + mb x Ru
   o.Ku = {fma(Rv.y, mb.z, fma(-Rv.z, mb.y, fma(F11, Ru.x, mul(F12, Rv.x)))),
           fma(Rv.z, mb.x, fma(-Rv.x, mb.z, fma(F11, Ru.y, mul(F12, Rv.y)))),
@@ -205,6 +222,10 @@ __device__ __forceinline__ Vec3<float> scale_derivative(const Point &o, const Ve
   return {one(o.Ku.x, K[0].x, o.Kv.x, K[1].x, o.m.x, K[2].x, K[3].x, K[4].x, s.x),
           one(o.Ku.y, K[0].y, o.Kv.y, K[1].y, o.m.y, K[2].y, K[3].y, K[4].y, s.y),
           one(o.Ku.z, K[0].z, o.Kv.z, K[1].z, o.m.z, K[2].z, K[3].z, K[4].z, s.z)};
+}
+// The restraints' value-row part of it, kV m . R.
+__device__ __forceinline__ Vec3<float> geo_scale_derivative(const Point &o, const GeoPoint &geo, const Vec3<float> &s) {
+  return {fma(mul(geo.kV, o.m.x), geo.R.x, s.x), fma(mul(geo.kV, o.m.y), geo.R.y, s.y), fma(mul(geo.kV, o.m.z), geo.R.z, s.z)};
 }
 
 }  // namespace f32
@@ -238,9 +259,11 @@ struct Smem {
   float4 B[NPT][L::ROW4];           // rows u, v, uu, uv, vv of point p, control points in fours (forward)
   float4 G4[NPT][NCP];              // u, v, uu, uv of control point j (gradient)
   float G1[NPT][16];                // vv of control point j
+  float4 V[NPT][L::NC4];            // value rows
   float4 X[kHW][3][L::NC4];         // coordinate c of the local control points
   float4 D[kHW][3][L::NC4];         // the same points' change from the reference state
   float4 A[kHW][NPT][3];            // {Ku, lb}, {Kv, kb}, {m, nb} of each point
+  float2 geo[16];                   // restraints: each point's kA, kV
   double red[kWarps][6];
 };
 
@@ -298,7 +321,7 @@ __device__ __forceinline__ double stage(Smem<NCP, NPT> &sm, const float *__restr
   return lane < NPT ? __ldg(reinterpret_cast<const double *>(table + L::kWeights) + lane) : 0.0;
 }
 
-template <int NCP, int NPT, bool KG_REG>
+template <int NCP, int NPT, bool KG_REG, bool GEO>
 __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const Ahead &cur, const SurfaceParams &P,
                                      const float alpha[3], const float am1[3], const Coef &M, float k_reg, bool reg_alpha, bool want_da, float *__restrict__ partial, KahanSums<6> &sums) {
   constexpr int NC4 = F32Table<NCP, NPT>::NC4;
@@ -306,6 +329,7 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
   // in their lattice images, times alpha, with error-free sums on the hi/lo
   // pairs; and their change from the reference state, alpha L - L0 =
   // (alpha - 1) L + (dsp - dsp of the corner)
+  GeoPoint geo{0.f, 0.f, {0.f, 0.f, 0.f}};
   {
     float ahi[3], alo[3], ad[3], l[3];
 #pragma unroll
@@ -322,16 +346,19 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
         reinterpret_cast<float *>(sm.D[hw][c])[lane] = fma(am1[c], l[c], sub(cur.dsp[c], ad[c]));
       }
     }
+    if constexpr (GEO)  // the corner, absolute (it carries no image)
+      geo.R = {mul(alpha[0], add(ahi[0], alo[0])), mul(alpha[1], add(ahi[1], alo[1])), mul(alpha[2], add(ahi[2], alo[2]))};
   }
   __syncwarp();
   // ---- lanes as quadrature points; K[k]_c as two partial sums (even and odd
   // control points) in one paired multiply-add
   if (lane < NPT) {
-    float2 A[5][3], Ad[2][3];
+    float2 A[5][3], Ad[2][3], Av[3];
 #pragma unroll
     for (int k = 0; k < 5; ++k) A[k][0] = A[k][1] = A[k][2] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 2; ++k) Ad[k][0] = Ad[k][1] = Ad[k][2] = make_float2(0.f, 0.f);
+    Av[0] = Av[1] = Av[2] = make_float2(0.f, 0.f);
 #pragma unroll 1
     for (int c4 = 0; c4 < NC4; ++c4) {
       float4 x[3], d[3];
@@ -354,6 +381,14 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
           }
         }
       }
+      if constexpr (GEO) {
+        const float4 b = sm.V[lane][c4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          Av[c] = __ffma2_rn(make_float2(b.x, b.y), make_float2(x[c].x, x[c].y), Av[c]);
+          Av[c] = __ffma2_rn(make_float2(b.z, b.w), make_float2(x[c].z, x[c].w), Av[c]);
+        }
+      }
     }
     Vec3<float> K[5], dR[2];
 #pragma unroll
@@ -361,7 +396,12 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
 #pragma unroll
     for (int k = 0; k < 2; ++k)
       dR[k] = {add(Ad[k][0].x, Ad[k][0].y), add(Ad[k][1].x, Ad[k][1].y), add(Ad[k][2].x, Ad[k][2].y)};
-    const Point o = point<KG_REG>(K, dR, M, k_reg, cur.g0, cur.rr0, cur.P2, cur.Hbar, cur.Pres);
+    if constexpr (GEO) {
+      geo.R = {add(geo.R.x, add(Av[0].x, Av[0].y)), add(geo.R.y, add(Av[1].x, Av[1].y)), add(geo.R.z, add(Av[2].x, Av[2].y))};
+      geo.kA = sm.geo[lane].x;
+      geo.kV = sm.geo[lane].y;
+    }
+    const Point o = point<KG_REG, GEO>(K, dR, M, k_reg, cur.g0, cur.rr0, cur.P2, cur.Hbar, cur.Pres, geo);
     sm.A[hw][lane][0] = make_float4(o.Ku.x, o.Ku.y, o.Ku.z, o.lb);
     sm.A[hw][lane][1] = make_float4(o.Kv.x, o.Kv.y, o.Kv.z, o.kb);
     sm.A[hw][lane][2] = make_float4(o.m.x, o.m.y, o.m.z, o.nb);
@@ -371,6 +411,7 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
       if constexpr (KG_REG) sums.add(2, o.er);
       if (want_da) {
         Vec3<float> d = scale_derivative(o, K, {0.f, 0.f, 0.f});
+        if constexpr (GEO) d = geo_scale_derivative(o, geo, d);
         if (KG_REG && reg_alpha) {
           // the angle term's extra box-scale part (src/grad.C:7414-7421):
           // sum_x (b_u Kreg_u + b_v Kreg_v) X = Kreg_u Ru + Kreg_v Rv, times alpha - 1
@@ -392,7 +433,8 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
 #pragma unroll 3
     for (int p = 0; p < NPT; ++p) {
       const float4 u = sm.A[hw][p][0], v = sm.A[hw][p][1], m = sm.A[hw][p][2], b = sm.G4[p][lane];
-      const float s = fma(sm.G1[p][lane], m.w, fma(b.w, v.w, mul(b.z, u.w)));
+      float s = fma(sm.G1[p][lane], m.w, fma(b.w, v.w, mul(b.z, u.w)));
+      if constexpr (GEO) s = fma(reinterpret_cast<const float *>(sm.V[p])[lane], sm.geo[p].y, s);
       g[0] = fma(s, m.x, fma(b.y, v.x, fma(b.x, u.x, g[0])));
       g[1] = fma(s, m.y, fma(b.y, v.y, fma(b.x, u.y, g[1])));
       g[2] = fma(s, m.z, fma(b.y, v.z, fma(b.x, u.z, g[2])));

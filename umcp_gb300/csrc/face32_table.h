@@ -16,7 +16,8 @@ struct F32Table {
   static constexpr int kRows = 0;                 // [NPT][ROW4][4]: rows u, v, uu, uv, vv
   static constexpr int kPoint4 = NPT * ROW4 * 4;  // [NPT][NCP][4]: u, v, uu, uv of each control point
   static constexpr int kPoint1 = kPoint4 + NPT * NCP * 4;  // [NPT][16]: vv
-  static constexpr int kWeights = kPoint1 + NPT * 16;      // [16] doubles
+  static constexpr int kValue = kPoint1 + NPT * 16;        // [NPT][4 NC4]: the value row (restraints)
+  static constexpr int kWeights = kValue + NPT * 4 * NC4;  // [16] doubles
   static constexpr int kFloats = kWeights + 32;
 };
 
@@ -26,7 +27,8 @@ inline int f32_table_floats(int ncp) {
 }
 
 template <int NCP, int NPT>
-void fill_f32_table(const std::vector<double> &basis, const std::vector<double> &weight, std::vector<float> *t) {
+void fill_f32_table(const std::vector<double> &basis, const std::vector<double> &value,
+                    const std::vector<double> &weight, std::vector<float> *t) {
   using L = F32Table<NCP, NPT>;
   t->assign(L::kFloats, 0.f);
   for (int p = 0; p < NPT; ++p) {
@@ -37,16 +39,18 @@ void fill_f32_table(const std::vector<double> &basis, const std::vector<double> 
         if (k < 4) (*t)[L::kPoint4 + (p * NCP + x) * 4 + k] = b;
         else (*t)[L::kPoint1 + p * 16 + x] = b;
       }
+    for (int x = 0; x < NCP; ++x) (*t)[L::kValue + p * 4 * L::NC4 + x] = (float)value[(size_t)p * NCP + x];
   }
   memcpy(t->data() + L::kWeights, weight.data(), NPT * sizeof(double));
 }
 
-// The table from rows basis[npt][5][ncp rounded up to 4] and the weights.
-inline std::vector<float> f32_table(const std::vector<double> &basis, const std::vector<double> &weight, int ncp) {
+// The table from rows basis[npt][5][ncp rounded up to 4], value rows [npt][ncp] and the weights.
+inline std::vector<float> f32_table(const std::vector<double> &basis, const std::vector<double> &value,
+                                    const std::vector<double> &weight, int ncp) {
   std::vector<float> t;
-  if (ncp == 12) fill_f32_table<12, 15>(basis, weight, &t);
-  else if (ncp == 11) fill_f32_table<11, 16>(basis, weight, &t);
-  else if (ncp == 13) fill_f32_table<13, 16>(basis, weight, &t);
+  if (ncp == 12) fill_f32_table<12, 15>(basis, value, weight, &t);
+  else if (ncp == 11) fill_f32_table<11, 16>(basis, value, weight, &t);
+  else if (ncp == 13) fill_f32_table<13, 16>(basis, value, weight, &t);
   return t;
 }
 

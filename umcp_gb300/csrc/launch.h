@@ -69,7 +69,9 @@ inline int geo_blocks(int nfaces) {
 }
 // Sums A, V and their alpha derivatives; the last block writes gterm.
 // alpha64: the area and the box-scale derivatives in FP64 as well (plain path).
-cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, cudaStream_t s);
+// fused: the face launches form the restraints' gradient (and with it dE_r/dalpha,
+// which gterm then has as zero): the precision form's SIMT kernels.
+cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, bool fused, cudaStream_t s);
 // partial[slot] += alpha * (dE_r/dA dA/dX + dE_r/dV dV/dX) for every (face, control point).
 template <typename T>
 cudaError_t launch_geo_grad(const GeoArgs &G, T *partial, cudaStream_t s);
@@ -116,6 +118,7 @@ struct FaceGroup32 {
 struct FaceSet32 {
   FaceGroup32 g[3];
   int ngroups;
+  int geo;  // the restraints' gradient goes along (coefficients at FinishArgs::gterm)
 };
 struct F32View {
   const float *hi, *lo, *dsp;
@@ -138,7 +141,7 @@ constexpr int kTpfFaces = 24000;
 int face_blocks_tpf(int nfaces);
 cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
                              const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                             const FinishArgs &fin, cudaStream_t s);
+                             const FinishArgs &fin, int geo, cudaStream_t s);
 
 // The regular faces of the precision form on the tensor cores (face_tc_kernel):
 // the same outputs as launch_faces_tpf, in 128-face tiles; grid from

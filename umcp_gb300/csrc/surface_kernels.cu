@@ -908,6 +908,8 @@ struct Smem {
   float4 D[kThreads][9];  // the same control points' change from the reference state, same layout
   float2 C[kNpt];  // each point's coefficients curv, area (f32::Coef)
   float Cg[kNpt];  // and gauss
+  Q4<float> V[kNpt][kNc4];  // value rows and each point's kA, kV (restraints)
+  float2 geo[kNpt];
   double red[kWarps][6];
 };
 constexpr size_t kSumBytes = sizeof(float) * 12 * kThreads;  // per-thread Kahan totals (dynamic shared memory)
@@ -945,6 +947,19 @@ __device__ __forceinline__ void tpf_stage(tpf::Smem &sm, const float *__restrict
     b[i] = Q4<float>{v.x, v.y, v.z, v.w};
   }
 }
+// The restraints' tables: value rows, and the points' coefficients (which come from the sums kernel).
+__device__ __forceinline__ void tpf_stage_geo(tpf::Smem &sm, const float *__restrict__ table,
+                                              const double *__restrict__ gterm, double dudv) {
+  using L = F32Table<tpf::kNcp, tpf::kNpt>;
+  const float4 *t = reinterpret_cast<const float4 *>(table + L::kValue);
+  Q4<float> *v = &sm.V[0][0];
+  for (int i = threadIdx.x; i < tpf::kNpt * tpf::kNc4; i += blockDim.x) {
+    const float4 x = __ldg(t + i);
+    v[i] = Q4<float>{x.x, x.y, x.z, x.w};
+  }
+  if ((int)threadIdx.x < tpf::kNpt)
+    sm.geo[threadIdx.x] = f32::geo_coef(gterm, __ldg(reinterpret_cast<const double *>(table + L::kWeights) + threadIdx.x), dudv);
+}
 // The points' coefficients for a mesh's moduli, by the block's first threads.
 __device__ __forceinline__ void tpf_coefs(tpf::Smem &sm, const float *__restrict__ table, const SurfaceParams &P,
                                           double dudv) {
@@ -960,10 +975,10 @@ __device__ __forceinline__ void tpf_coefs(tpf::Smem &sm, const float *__restrict
 // am1 = alpha - 1 (formed in FP64): the box scales' part of the change from
 // the reference state. fn: the face this thread takes next (its rows are
 // prefetched), or -1.
-template <bool KG_REG>
+template <bool KG_REG, bool GEO>
 __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const SurfaceParams &P, int f,
                                          const float alpha[3], const float ialpha[3], const float am1[3],
-                                         float k_reg, bool vec, float *__restrict__ partial,
+                                         float k_reg, bool vec, bool want_da, float *__restrict__ partial,
                                          float e3[3], float da[3], int fn) {
   using namespace tpf;
   uint32_t cp[kNcp];
@@ -1046,11 +1061,12 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
     // K[k]_c as two partial sums (even, odd control points) in one pair; the
     // u and v rows also over the displacements (dR, the tangents' change
     // from the reference state)
-    float2 A[5][3], Ad[2][3];
+    float2 A[5][3], Ad[2][3], Av[3];
 #pragma unroll
     for (int k = 0; k < 5; ++k) A[k][0] = A[k][1] = A[k][2] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int k = 0; k < 2; ++k) Ad[k][0] = Ad[k][1] = Ad[k][2] = make_float2(0.f, 0.f);
+    Av[0] = Av[1] = Av[2] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int c4 = 0; c4 < kNc4; ++c4) {
       float4 x[3], d[3];  // coordinate c of control points 4 c4 .. 4 c4 + 3
@@ -1073,6 +1089,14 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
           }
         }
       }
+      if constexpr (GEO) {
+        const Q4<float> b = sm.V[p][c4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          Av[c] = __ffma2_rn(make_float2(b.x, b.y), make_float2(x[c].x, x[c].y), Av[c]);
+          Av[c] = __ffma2_rn(make_float2(b.z, b.w), make_float2(x[c].z, x[c].w), Av[c]);
+        }
+      }
     }
     Vec3<float> K[5], dR[2];
 #pragma unroll
@@ -1083,11 +1107,23 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
       dR[k] = {f32::add(Ad[k][0].x, Ad[k][0].y), f32::add(Ad[k][1].x, Ad[k][1].y), f32::add(Ad[k][2].x, Ad[k][2].y)};
     const float2 cf = sm.C[p];
     const f32::Coef M{cf.x, cf.y, KG_REG ? sm.Cg[p] : 0.f};
-    const f32::Point o = f32::point<KG_REG>(K, dR, M, k_reg, g0, rr0, P2, Hbar, Pres);
+    f32::GeoPoint geo{0.f, 0.f, {0.f, 0.f, 0.f}};
+    if constexpr (GEO) {
+      geo.kA = sm.geo[p].x;
+      geo.kV = sm.geo[p].y;
+      // the corner's absolute position (it carries no image) plus the local limit point
+      geo.R = {f32::add(f32::mul(alpha[0], f32::add(ahi[0], alo[0])), f32::add(Av[0].x, Av[0].y)),
+               f32::add(f32::mul(alpha[1], f32::add(ahi[1], alo[1])), f32::add(Av[1].x, Av[1].y)),
+               f32::add(f32::mul(alpha[2], f32::add(ahi[2], alo[2])), f32::add(Av[2].x, Av[2].y))};
+    }
+    const f32::Point o = f32::point<KG_REG, GEO>(K, dR, M, k_reg, g0, rr0, P2, Hbar, Pres, geo);
     ea += o.ea;
     ec += o.ec;
     er += o.er;
-    da3 = f32::scale_derivative(o, K, da3);
+    if (want_da) {
+      da3 = f32::scale_derivative(o, K, da3);
+      if constexpr (GEO) da3 = f32::geo_scale_derivative(o, geo, da3);
+    }
     // G[j]_c += B[u][j] Kb[u]_c + B[v][j] Kb[v]_c + s[j] m_c in scalar multiply-adds: with the
     // forward contraction in paired ones, the mix keeps both FP32 multiply-add pipes busy
     // (all paired: 763 us, this mix: 747 us, all scalar: 776 us on the 256-vesicle pass)
@@ -1102,7 +1138,8 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
                     vv[4] = {bvv.x, bvv.y, bvv.z, bvv.w};
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-          const float sj = fmaf(vv[jj], o.nb, fmaf(uv[jj], o.kb, __fmul_rn(uu[jj], o.lb)));
+          float sj = fmaf(vv[jj], o.nb, fmaf(uv[jj], o.kb, __fmul_rn(uu[jj], o.lb)));
+          if constexpr (GEO) sj = fmaf((&sm.V[p][c4].x)[jj], geo.kV, sj);
           float *g = G[4 * c4 + jj];
 #pragma unroll
           for (int cc = 0; cc < 3; ++cc) g[cc] = fmaf(sj, md[cc], fmaf(v[jj], kv[cc], fmaf(u[jj], ku[cc], g[cc])));
@@ -1162,6 +1199,7 @@ struct SharedSums {
 // grid takes faces 32 w .. 32 w + 31, then 32 (w + warps in the grid) ...
 // Writes one block partial of the energy terms and dE/dalpha; the last block
 // to finish sums them (as face_kernel does).
+template <bool GEO>  // the restraints' gradient goes along
 __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
     face_tpf_kernel(FaceLaunch L, const int *__restrict__ dest, SurfaceParams P, const double *__restrict__ r,
                     const float *__restrict__ rhi, const float *__restrict__ rlo, const float *__restrict__ dsp,
@@ -1175,6 +1213,11 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
   grid_dependents();
+  if constexpr (GEO) {
+    tpf_stage_geo(sm, L.table, fin.gterm, L.dudv);
+    __syncthreads();
+  }
+  const bool want_da = fin.galpha != nullptr;  // a run's steps leave the box scales alone
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float alpha[3] = {(float)r[3 * P.nv], (float)r[3 * P.nv + 1], (float)r[3 * P.nv + 2]};
   const float ialpha[3] = {1.f / alpha[0], 1.f / alpha[1], 1.f / alpha[2]};
@@ -1192,8 +1235,8 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
       float e3[3], da[3];
       // no prefetch: a thread's next face is a grid stride away, and on the
       // 512 x 512 planar pass the prefetch cost 1% instead of gaining
-      if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, -1);
-      else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, -1);
+      if (kg_reg) tpf_face<true, GEO>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
+      else tpf_face<false, GEO>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
       acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
       acc.add(3, da[0]); acc.add(4, da[1]); acc.add(5, da[2]);
       if (!isfinite(e3[0] + e3[1] + e3[2])) atomicOr(status, kStatusNonFinite);
@@ -1275,8 +1318,8 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
         if (f < end) {
           float e3[3], da[3];
           const int fn = f + kThreads < end ? f + kThreads : -1;
-          if (kg_reg) tpf_face<true>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, fn);
-          else tpf_face<false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, partial, e3, da, fn);
+          if (kg_reg) tpf_face<true, false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
+          else tpf_face<false, false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
           acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
         }
       }
@@ -1681,6 +1724,13 @@ __device__ __forceinline__ FF ff_of(double x) {
   return {h, (float)(x - (double)h)};
 }
 
+// (The gradient goes along in the face kernels, which have the tangents and the
+// normal at hand: 10% more of their work instead of a pass of its own over every
+// face, 40 to 50 us at 81,920 faces, with a read and write of every partial.
+// Three restrained evaluations of a 40,962-vertex vesicle in flight: 179 -> 135
+// us each. The pass below remains for the plain path and for meshes whose
+// regular faces run on the tensor cores.)
+//
 // The precision form's sums: V from float-float contractions of float-float
 // local coordinates (formed from the FP32 hi/lo position pairs with error-free
 // sums) and summed in float-float per thread; the area and the box-scale
@@ -1709,7 +1759,7 @@ struct Rows {
 constexpr size_t kDynBytes = sizeof(float) * kCol * kThreads;
 }  // namespace geo_tpf
 
-template <int NCP, int NPT>
+template <int NCP, int NPT, bool DA>
 __device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g, const geo_tpf::Rows &rows, int gi,
                                             int lf, const FF alpha[3], const float ialpha[3], float *col, FF &accV,
                                             float ks[kGeoWords], float kc[kGeoWords]) {
@@ -1811,6 +1861,7 @@ __device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g,
     const float ig = rsqrtf(gg2), gg = gg2 * ig;
     const float cwf = rows.cw[gi][p], c3f = rows.c3[gi][p].hi;
     kahan(0, cwf * gg);
+    if constexpr (!DA) continue;
     float n[3] = {mf[0] * ig, mf[1] * ig, mf[2] * ig}, a1[3], a2[3], v1[3], v2[3];
     cross3(Vf, n, a1);
     cross3(n, Uf, a2);
@@ -1824,6 +1875,8 @@ __device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g,
   }
 }
 
+// DA: the box-scale derivatives too (else the face launches form them).
+template <bool DA>
 __global__ void __launch_bounds__(geo_tpf::kThreads, 3) geo_sums_ff_tpf_kernel(GeoArgs G) {
   using namespace geo_tpf;
   __shared__ Rows rows;
@@ -1860,9 +1913,9 @@ __global__ void __launch_bounds__(geo_tpf::kThreads, 3) geo_sums_ff_tpf_kernel(G
     int lf;
     const int gi = geo_group(G, f, &lf);
     const GeoGroup &g = G.g[gi];
-    if (g.ncp == 12) geo_face_ff<12, 15>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
-    else if (g.ncp == 11) geo_face_ff<11, 16>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
-    else geo_face_ff<13, 16>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
+    if (g.ncp == 12) geo_face_ff<12, 15, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
+    else if (g.ncp == 11) geo_face_ff<11, 16, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
+    else geo_face_ff<13, 16, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
   }
   double acc[kGeoWords];
 #pragma unroll
@@ -2163,7 +2216,7 @@ int face_blocks_tpf(int nfaces) {
   static PerDevice pd;
   const int cached = per_device(pd, [] {
     int per_sm = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::face_tpf_kernel, dev::tpf::kThreads,
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, dev::face_tpf_kernel<false>, dev::tpf::kThreads,
                                                   dev::tpf::kSumBytes);
     return sm_count() * (per_sm > 0 ? per_sm : 1);
   });
@@ -2173,10 +2226,10 @@ int face_blocks_tpf(int nfaces) {
 
 cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
                              const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                             const FinishArgs &fin, cudaStream_t s) {
+                             const FinishArgs &fin, int geo, cudaStream_t s) {
   if (L.nfaces <= 0) return cudaSuccess;
   if (!f.hi || !f.lo || !f.dsp) return cudaErrorInvalidValue;
-  return launch_after(dev::face_tpf_kernel, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, f.hi, f.lo,
+  return launch_after(geo ? dev::face_tpf_kernel<true> : dev::face_tpf_kernel<false>, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, f.hi, f.lo,
                       f.dsp, partial, blockpart, status, fin);
 }
 
@@ -2325,16 +2378,16 @@ cudaError_t launch_batch_pack(const BatchJob *jobs, const BatchTile *vtiles, con
 
 namespace umcp {
 
-cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, cudaStream_t s) {
+cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, bool fused, cudaStream_t s) {
   if (alpha64) return launch_after(dev::geo_sums_kernel, geo_blocks(G.nfaces), kGeoThreads, 0, s, G);
   // the thread-per-face form: a grid that depends on the face count only (the sums' order is fixed)
-  const cudaError_t e = cudaFuncSetAttribute(dev::geo_sums_ff_tpf_kernel,
-                                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)dev::geo_tpf::kDynBytes);
+  auto kernel = fused ? dev::geo_sums_ff_tpf_kernel<false> : dev::geo_sums_ff_tpf_kernel<true>;
+  const cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dev::geo_tpf::kDynBytes);
   if (e != cudaSuccess) return e;
   const int per_block = dev::geo_tpf::kThreads, want = (G.nfaces + per_block - 1) / per_block;
   const int grid = want < 1 ? 1 : (want < geo_blocks(G.nfaces) ? want : geo_blocks(G.nfaces));
-  return launch_after(dev::geo_sums_ff_tpf_kernel, grid, dev::geo_tpf::kThreads, dev::geo_tpf::kDynBytes, s, G);
+  return launch_after(kernel, grid, dev::geo_tpf::kThreads, dev::geo_tpf::kDynBytes, s, G);
 }
 
 template <typename T>
