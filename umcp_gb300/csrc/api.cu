@@ -544,10 +544,8 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
   arena.uninit(m->r_eval, nst * sizeof(double));
   arena.zeroed(m->done, sizeof(unsigned));
   if (m->precision == UMCP_FP32_CENTRED) {
-    arena.uninit(m->rhi, 3 * (size_t)ME.nv * sizeof(float));
-    arena.uninit(m->rlo, 3 * (size_t)ME.nv * sizeof(float));
+    arena.uninit(m->pos32, dev::kPosStride * (size_t)ME.nv * sizeof(float));
     arena.stage(m->r0, PL.ref_r);  // the state the reference metric g0 was taken at
-    arena.uninit(m->dsp, 3 * (size_t)ME.nv * sizeof(float));
   }
   UMCP_CUDA(arena.commit(m->arena));
   if (m->precision == UMCP_FP32_CENTRED) {
@@ -638,8 +636,8 @@ static GeoArgs geo_args(umcp_mesh *m, const double *d_r) {
   G.nfaces = base;
   G.nv = m->nv;
   G.r = d_r;
-  G.rhi = m->rhi.as<float>();
-  G.rlo = m->rlo.as<float>();
+  G.rhi = m->f32pos().hi;
+  G.rlo = m->f32pos().lo;
   for (int d = 0; d < 3; ++d)
     for (int c = 0; c < 3; ++c) {
       G.box[d][c] = m->P.box[d][c];
@@ -907,7 +905,7 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
   b += slots * 3 * (f32 ? 4 : 8);                     // partial
   b += 3 * nst * 8 + 2 * 3 * nv * 8;                  // r, g, r_eval; p, qdot
   b += 8 + 3 * 8 + 4 + 2 * 8 + 4;                     // E, parts, status, cnt, done
-  if (f32) b += 3 * 3 * nv * 4 + 3 * nv * 8;          // rhi, rlo, dsp; r0
+  if (f32) b += dev::kPosStride * nv * 4 + 3 * nv * 8;  // hi, lo, dsp; r0
   b += (size_t)n_energies * 8;                        // energy record
   *bytes = b;
   return UMCP_OK;
@@ -1302,8 +1300,9 @@ extern "C" umcp_status umcp_step_host(umcp_mesh *m, const umcp_integrator *it, u
 // word and the FP32 position pairs) lives in this file-scope array, which
 // every GPU that loads the library holds until the process exits.
 
-static constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // 32 MiB per device
-static __device__ __align__(256) unsigned char g_static_scratch[kStaticScratchBytes];
+static constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // per device, of the layout that meshes are admitted by
+static constexpr size_t kStaticArrayBytes = (size_t)34 << 20;    // the array: the positions take a third more since
+static __device__ __align__(256) unsigned char g_static_scratch[kStaticArrayBytes];
 static void *g_static_scratch_addr[128];  // device address of the array, per device (host-side)
 
 static size_t align256(size_t x) { return (x + 255) / 256 * 256; }
@@ -1330,10 +1329,10 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
   // layout: [status, done] | block partials | gradient partials | FP32 position pairs and displacements
   const size_t off_flags = 0, off_block = 256;
   const size_t off_partial = off_block + align256((size_t)m->nblocks * 6 * sizeof(double));
-  const size_t f32_bytes = fp32 ? align256((size_t)3 * m->nv * sizeof(float)) : 0;
   const size_t off_hi = off_partial + align256((size_t)m->nslot_cap * 3 * esize);
-  const size_t off_lo = off_hi + f32_bytes, off_dsp = off_lo + f32_bytes;
-  const size_t need = off_dsp + f32_bytes;
+  // a mesh is admitted by three packed arrays of positions (9 floats a vertex); they lie 12 apart
+  const size_t need = off_hi + (fp32 ? 3 * align256((size_t)3 * m->nv * sizeof(float)) : 0);
+  static_assert(kStaticArrayBytes >= kStaticScratchBytes + kStaticScratchBytes / 3 / 9, "12 floats a vertex for 9");
   if (need > kStaticScratchBytes)
     return fail(UMCP_ERR_NOMEM, "mesh needs " + std::to_string(need) + " bytes of scratch; the static area holds " +
                                     std::to_string(kStaticScratchBytes) + " bytes");
@@ -1343,9 +1342,9 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
   F32Pos f32;
   if (fp32) {
     f32.hi = (float *)(base + off_hi);
-    f32.lo = (float *)(base + off_lo);
+    f32.lo = f32.hi + 3;
     f32.r0 = m->r0.as<double>();
-    f32.dsp = (float *)(base + off_dsp);
+    f32.dsp = f32.hi + 6;
   }
   cudaStream_t s = m->ctx->stream;
   // The array keeps the previous call's contents: the status word and the

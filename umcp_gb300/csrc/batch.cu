@@ -144,7 +144,8 @@ static BatchJob job_entry(const Job &J) {
     s.g0f = G.g0f.as<float>(); s.rr0f = G.rr0f.as<float>(); s.compf = G.compf.as<float>();
     s.dest = G.dest.as<int>();
     s.r = m->r.as<double>();
-    s.rhi = m->rhi.as<float>(); s.rlo = m->rlo.as<float>(); s.dsp = m->dsp.as<float>();
+    const F32Pos f = m->f32pos();
+    s.rhi = f.hi; s.rlo = f.lo; s.dsp = f.dsp;
     s.nfaces = G.nfaces;
   }
   e.f.P = m->P;
@@ -155,11 +156,11 @@ static BatchJob job_entry(const Job &J) {
   e.off = m->off.as<int>();
   e.r = m->r.as<double>();
   e.p = m->p.as<double>();
-  const bool f32 = m->precision == UMCP_FP32_CENTRED;
-  e.rhi = f32 ? m->rhi.as<float>() : nullptr;
-  e.rlo = f32 ? m->rlo.as<float>() : nullptr;
-  e.r0 = f32 ? m->r0.as<double>() : nullptr;
-  e.dsp = f32 ? m->dsp.as<float>() : nullptr;
+  const F32Pos f = m->f32pos();
+  e.rhi = f.hi;
+  e.rlo = f.lo;
+  e.r0 = f.r0;
+  e.dsp = f.dsp;
   e.E = m->E.as<double>();
   e.parts = m->parts.as<double>();
   e.energies = m->energies.as<double>();

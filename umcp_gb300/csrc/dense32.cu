@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   float4 m[kRows], nx[kRows];
   load(g, c, m);
   grid_dependency_wait();  // the vectors come from the kernel before; the matrix does not
-  grid_dependents();
+  grid_dependents(gridDim.x);  // the finish is short and its blocks few
   for (long long u = u0; u < u1; ++u) {
     int gn = g, cn = c + 1;
     if (cn == chunks) { cn = 0; ++gn; }
@@ -176,7 +176,6 @@ __global__ void dense_finish32_kernel(int n, int chunks, long long units, long l
                                       int slots, MassScale f, const double *__restrict__ scalev,
                                       double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
-  grid_dependents();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3 * n) return;
   const int i = t / 3, k = t - 3 * i;
@@ -191,7 +190,6 @@ __global__ void dense_drift32_kernel(int n, int chunks, long long units, long lo
                                      float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
                                      float *__restrict__ dsp, const int *__restrict__ status) {
   grid_dependency_wait();
-  grid_dependents();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= 3 * n || *status) return;
   drift(a, t, slot_sum(t, chunks, units, W, part, slots), r, p, rhi, rlo, r0, dsp);

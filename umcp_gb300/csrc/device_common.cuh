@@ -14,12 +14,17 @@ namespace dev {
 // was launched without the attribute).
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Lets the kernel after this one be scheduled once every block has come this
-// far; it then waits for this kernel's end in grid_dependency_wait. The kernels
-// of a step call it right after their own wait: the next one's blocks are up
-// when this one drains. The long restraint kernels do not: the next kernel's
-// blocks, waiting on the SMs for all of their time, cost other streams' kernels
-// their place (three restrained evaluations in flight: 179 -> 217 us each).
-__device__ __forceinline__ void grid_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// far; it then waits for this kernel's end in grid_dependency_wait. A kernel
+// calls it right after its own wait, so that the next one's blocks are up when it
+// drains, but only where its grid is small (few_blocks: the most it may have).
+// With a large one the next kernel's blocks go wherever this one's leave room
+// first: its own blocks end up uneven over the SMs, and other streams' kernels
+// lose their place. BD step with / without: 1,280 faces 11.3 / 12.5 us, 16,000
+// faces 24.8 / 23.4, 131,072 faces 81 / 64.
+constexpr unsigned kFewFaceBlocks = 320, kFewGatherBlocks = 96;
+__device__ __forceinline__ void grid_dependents(unsigned few_blocks) {
+  if (gridDim.x <= few_blocks) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 
 // A job takes the step when it has neither stopped nor reached its limit.
 __device__ __forceinline__ bool job_active(const BatchFaceJob &J) { return !*J.status && J.cnt[1] < J.limit; }
@@ -31,9 +36,27 @@ __device__ __forceinline__ void store_f32_position(size_t i, double x, float *__
                                                    float *__restrict__ lo, const double *__restrict__ r0,
                                                    float *__restrict__ dsp) {
   const float h = (float)x;
-  hi[i] = h;
-  lo[i] = (float)(x - (double)h);
-  dsp[i] = (float)(x - r0[i]);
+  const size_t at = pos_at(i);
+  hi[at] = h;
+  lo[at] = (float)(x - (double)h);
+  dsp[at] = (float)(x - r0[i]);
+}
+
+// The same for a vertex whose three coordinates one thread has, in the two
+// 16-byte stores and the 4-byte one that load_vertex reads (hi: F32Pos::hi).
+__device__ __forceinline__ void store_f32_vertex(int v, const double x[3], float *__restrict__ hi,
+                                                 const double *__restrict__ r0) {
+  float h[3], l[3], d[3];
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    h[c] = (float)x[c];
+    l[c] = (float)(x[c] - (double)h[c]);
+    d[c] = (float)(x[c] - r0[3 * (size_t)v + c]);
+  }
+  float *q = hi + kPosStride * (size_t)v;
+  reinterpret_cast<float4 *>(q)[0] = make_float4(h[0], h[1], h[2], l[0]);
+  reinterpret_cast<float4 *>(q)[1] = make_float4(l[1], l[2], d[0], d[1]);
+  q[8] = d[2];
 }
 
 // Second half of a leapfrog step with M^-1 for coordinate i: r += qdot AK (and

@@ -102,8 +102,8 @@ struct umcp_mesh {
   umcp::DevBuf partial, off, blockpart;
   int nblocks = 0;
   umcp::DevBuf r, g, p, qdot, E, parts, status, cnt;  // cnt: {first step of the run, run index}
-  umcp::DevBuf rhi, rlo;  // FP32 hi/lo pairs of r (precision form)
-  umcp::DevBuf r0, dsp;   // precision form: reference state (FP64) and r - r0 (FP32)
+  umcp::DevBuf pos32;     // precision form: FP32 positions hi, lo (r = hi + lo) and r - r0 (dev::kPosStride floats a vertex)
+  umcp::DevBuf r0;        // precision form: reference state (FP64)
   umcp::DevBuf r_eval;    // staging for host-pointer energy/gradient calls (keeps the resident state)
   umcp::DevBuf done;      // finished-block counter of the face pass
   bool split_valid = false;  // rhi/rlo hold the resident state r
@@ -157,8 +157,8 @@ struct umcp_mesh {
       for (const umcp::DevBuf *x : {&G->cp, &G->g0, &G->rr0, &G->comp, &G->basis, &G->weight, &G->dest, &G->g0f,
                                     &G->rr0f, &G->compf, &G->basis_w, &G->table, &G->geo_tab})
         b += x->bytes;
-    for (const umcp::DevBuf *x : {&partial, &off, &blockpart, &r, &g, &p, &qdot, &E, &parts, &status, &cnt, &rhi,
-                                  &rlo, &r0, &dsp, &r_eval, &done, &energies, &mrow, &mcol, &mval, &mdense, &min32, &mpart, &geo_block, &gterm,
+    for (const umcp::DevBuf *x : {&partial, &off, &blockpart, &r, &g, &p, &qdot, &E, &parts, &status, &cnt, &pos32,
+                                  &r0, &r_eval, &done, &energies, &mrow, &mcol, &mval, &mdense, &min32, &mpart, &geo_block, &gterm,
                                   &geo_done})
       b += x->bytes;
     return b;
@@ -168,7 +168,7 @@ struct umcp_mesh {
   umcp::F32Pos f32pos() const {
     umcp::F32Pos f;
     if (precision == UMCP_FP32_CENTRED) {
-      f.hi = rhi.as<float>(); f.lo = rlo.as<float>(); f.r0 = r0.as<double>(); f.dsp = dsp.as<float>();
+      f.hi = pos32.as<float>(); f.lo = f.hi + 3; f.dsp = f.hi + 6; f.r0 = r0.as<double>();
     }
     return f;
   }

@@ -68,7 +68,7 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block
   const double w = stage(sm, G.table);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
-  grid_dependents();
+  grid_dependents(kFewFaceBlocks);
   FaceSrc S{};
   S.cp = G.cp; S.g0f = G.g0; S.rr0f = G.rr0; S.compf = G.comp; S.dest = G.dest;
   S.r = r; S.rhi = f.hi; S.rlo = f.lo; S.dsp = f.dsp;

@@ -70,6 +70,15 @@ __device__ __forceinline__ float rcp(float x) {
   return fma(y, fma(-x, y, 1.f), y);
 }
 
+// A vertex's FP32 positions (hi: F32Pos::hi).
+__device__ __forceinline__ void load_vertex(const float *__restrict__ hi, int v, float h[3], float l[3], float d[3]) {
+  const float *q = hi + kPosStride * (size_t)v;
+  const float4 a = __ldg(reinterpret_cast<const float4 *>(q)), b = __ldg(reinterpret_cast<const float4 *>(q) + 1);
+  h[0] = a.x; h[1] = a.y; h[2] = a.z;
+  l[0] = a.w; l[1] = b.x; l[2] = b.y;
+  d[0] = b.z; d[1] = b.w; d[2] = __ldg(q + 8);
+}
+
 // Control point (hi + lo) in lattice image `code`, relative to the patch corner
 // (ahi + alo, home image): error-free sums, so the local coordinates carry full
 // FP32 precision even across periodic images.
@@ -284,14 +293,8 @@ __device__ __forceinline__ void load(const FaceSrc &S, int f, int end, int lane,
   f = min(f, end - 1);
   if (lane < NCP) {
     const uint32_t packed = __ldg(&S.cp[(size_t)f * NCP + lane]);
-    const size_t v = 3 * (size_t)(packed & kVertexMask);
     a.code = (int)(packed >> kVertexBits);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      a.hi[c] = S.rhi[v + c];
-      a.lo[c] = S.rlo[v + c];
-      a.dsp[c] = S.dsp[v + c];
-    }
+    load_vertex(S.rhi, (int)(packed & kVertexMask), a.hi, a.lo, a.dsp);
     a.dest = a.on ? __ldg(&S.dest[(size_t)f * NCP + lane]) : -1;
   }
   if (lane < NPT) {

@@ -74,7 +74,7 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup64 &G, int block
   const double w = lane < NPT ? __ldg(G.weight + lane) : 0.0;
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
-  grid_dependents();
+  grid_dependents(kFewFaceBlocks);
   FaceSrc S{};
   S.cp = G.cp; S.g0 = G.g0; S.rr0 = G.rr0; S.comp = G.comp; S.dest = G.dest; S.r = r;
   Sums sums;

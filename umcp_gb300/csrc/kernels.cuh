@@ -34,6 +34,15 @@ constexpr int kVertexBits = 27;  // packed control point: vertex | image_code <<
 constexpr uint32_t kVertexMask = (1u << kVertexBits) - 1u;
 constexpr double kSafety = 1e-12;  // SAFETY, src/interp.h:14
 
+// The precision form's FP32 positions of a vertex lie together, 12 floats on a
+// 16-byte boundary: hi.xyz, lo.xyz, dsp.xyz and three of padding, so a face
+// kernel fetches a control point with two 16-byte loads and a 4-byte one instead
+// of nine 4-byte ones from three arrays. F32Pos::hi, lo and dsp point at the first
+// vertex's hi, lo and dsp.
+constexpr int kPosStride = 12;
+// Offset of coordinate i = 3 v + c from those pointers.
+__host__ __device__ constexpr size_t pos_at(size_t i) { return kPosStride * (i / 3) + i % 3; }
+
 struct SurfaceParams {
   double kc, KA, kg, k_reg;
   double box[3][3];
@@ -61,7 +70,7 @@ struct FaceSrc {
   const int *dest;
   const double *r;
   const float *rhi, *rlo;
-  const float *dsp;  // precision form: r - r0 per coordinate (displacement from the reference state)
+  const float *dsp;  // precision form: r - r0 per coordinate (displacement from the reference state); see kPosStride
   int nfaces;
 };
 

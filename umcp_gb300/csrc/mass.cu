@@ -160,7 +160,6 @@ __global__ void __launch_bounds__(kDense64Threads)
                        const double *__restrict__ in, double *__restrict__ out, int accumulate) {
   const int lane = threadIdx.x & 31, warps = gridDim.x * (kDense64Threads / 32);
   dev::grid_dependency_wait();
-  dev::grid_dependents();
   for (int i = blockIdx.x * (kDense64Threads / 32) + (threadIdx.x >> 5); i < n; i += warps) {
     const double *row = A + (size_t)i * n;
     double a[4] = {0, 0, 0, 0};

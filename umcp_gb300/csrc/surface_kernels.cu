@@ -304,9 +304,10 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
       float chi[3], clo[3], cd[3];
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        chi[c] = S.rhi[3 * (size_t)v0 + c];
-        clo[c] = S.rlo[3 * (size_t)v0 + c];
-        cd[c] = S.dsp[3 * (size_t)v0 + c];
+        const size_t at = kPosStride * (size_t)v0 + c;
+        chi[c] = S.rhi[at];
+        clo[c] = S.rlo[at];
+        cd[c] = S.dsp[at];
       }
       // out = alpha L; with d given, d = (alpha - 1) L + (dsp - dsp of the corner), the change from
       // the reference state (as in the thread-per-face kernel)
@@ -325,12 +326,13 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
             shl += (float)im[d] * P.box_lo[d][c];
           }
           float s1, e1, s2, e2;
-          const float hi = S.rhi[3 * (size_t)v + c], lo = S.rlo[3 * (size_t)v + c];
+          const size_t at = kPosStride * (size_t)v + c;
+          const float hi = S.rhi[at], lo = S.rlo[at];
           two_sum(hi, sh, s1, e1);
           two_sum(s1, -chi[c], s2, e2);
           const float l = s2 + ((e1 + e2) + ((lo - clo[c]) + (she + shl)));
           out[c] = alpha[c] * l;
-          if (d) d[c] = fmaf(am1[c], l, S.dsp[3 * (size_t)v + c] - cd[c]);
+          if (d) d[c] = fmaf(am1[c], l, S.dsp[at] - cd[c]);
         }
       };
       local(__ldg(&cp[1]), Ev);  // lattice (0,1)
@@ -589,7 +591,7 @@ __global__ void stage_in_kernel(int n, const double *__restrict__ host_r, double
                                 float *__restrict__ hi, float *__restrict__ lo, const double *__restrict__ r0,
                                 float *__restrict__ dsp, int *__restrict__ status) {
   grid_dependency_wait();
-  grid_dependents();
+  grid_dependents(kFewGatherBlocks);
   if (status && blockIdx.x == 0 && threadIdx.x == 0) *status = 0;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double x = host_r[i];
@@ -693,7 +695,7 @@ template <typename T>
 __global__ void gather_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off,
                               double *__restrict__ g, int store) {
   grid_dependency_wait();  // the partials come from the face launches
-  grid_dependents();
+  grid_dependents(kFewGatherBlocks);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
     const int v = i / 3, c = i - 3 * v;
     const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
@@ -784,18 +786,18 @@ __device__ __forceinline__ double bd_coordinate_f32(const StepArgs &a, float g, 
 }
 __device__ __forceinline__ void bd_vertex_f32(const float *__restrict__ partial, const int *__restrict__ off, int v,
                                               const StepArgs &a, uint64_t st, double *__restrict__ r,
-                                              float *__restrict__ rhi, float *__restrict__ rlo,
-                                              const double *__restrict__ r0, float *__restrict__ dsp) {
+                                              float *__restrict__ rhi, const double *__restrict__ r0) {
   float g[3], n[3];
   vertex_gradient_f32(partial, off, v, g);
   normals3_f32(a.seed, a.stream, st, v, n);
+  double x[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const size_t i = 3 * (size_t)v + c;
-    const double x = bd_coordinate_f32(a, g[c], n[c], r[i]);
-    r[i] = x;
-    if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
+    x[c] = bd_coordinate_f32(a, g[c], n[c], r[i]);
+    r[i] = x[c];
   }
+  store_f32_vertex(v, x, rhi, r0);
 }
 
 // Gather fused with the update of the coordinate (overdamped BD, or the
@@ -810,7 +812,7 @@ __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const 
                                    float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
                                    float *__restrict__ dsp, const int *__restrict__ status) {
   grid_dependency_wait();  // the partials and the status come from the face launches
-  grid_dependents();
+  grid_dependents(kFewGatherBlocks);
   if (*status) return;
   const uint64_t st = current_step(cnt);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
@@ -846,7 +848,7 @@ __global__ void gather_kick_kernel(int nv, const T *__restrict__ partial, const 
                                    const uint64_t *__restrict__ cnt, double *__restrict__ p, float *__restrict__ x32,
                                    int ld, const int *__restrict__ status) {
   grid_dependency_wait();
-  grid_dependents();
+  grid_dependents(gridDim.x);  // the apply's first loads do not depend on this
   if (*status) return;
   const uint64_t st = current_step(cnt);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
@@ -863,7 +865,6 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
                              const double *__restrict__ qdot, float *__restrict__ rhi, float *__restrict__ rlo,
                              const double *__restrict__ r0, float *__restrict__ dsp, const int *__restrict__ status) {
   grid_dependency_wait();
-  grid_dependents();
   if (*status) return;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x)
     drift(a, i, qdot[i], r, p, rhi, rlo, r0, dsp);
@@ -1002,15 +1003,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
   // dsp of the corner). Formed and stored four control points at a time.
   float4 *xs = sm.X[threadIdx.x], *ds = sm.D[threadIdx.x];
   float ahi[3], alo[3], ad[3];
-  {
-    const int v0 = (int)(cp[0] & kVertexMask);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      ahi[c] = __ldg(&S.rhi[3 * (size_t)v0 + c]);
-      alo[c] = __ldg(&S.rlo[3 * (size_t)v0 + c]);
-      ad[c] = __ldg(&S.dsp[3 * (size_t)v0 + c]);
-    }
-  }
+  f32::load_vertex(S.rhi, (int)(cp[0] & kVertexMask), ahi, alo, ad);
 #pragma unroll
   for (int c4 = 0; c4 < kNc4; ++c4) {
     float X[4][3], Dx[4][3];
@@ -1019,12 +1012,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
       const int j = 4 * c4 + jj;
       const int v = (int)(cp[j] & kVertexMask), code = (int)(cp[j] >> kVertexBits);
       float hi[3], lo[3], dv[3], l[3];
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        hi[c] = __ldg(&S.rhi[3 * (size_t)v + c]);
-        lo[c] = __ldg(&S.rlo[3 * (size_t)v + c]);
-        dv[c] = __ldg(&S.dsp[3 * (size_t)v + c]);
-      }
+      f32::load_vertex(S.rhi, v, hi, lo, dv);
       f32::local_position(hi, lo, code, ahi, alo, P, l);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
@@ -1212,7 +1200,6 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   tpf_coefs(sm, L.table, P, L.dudv);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
-  grid_dependents();
   if constexpr (GEO) {
     tpf_stage_geo(sm, L.table, fin.gterm, L.dudv);
     __syncthreads();
@@ -1273,7 +1260,6 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
   __shared__ int s_active, s_tile[2];
   tpf_stage(sm, table);     // constant table: before the wait
   grid_dependency_wait();        // positions, job states and the counter come from the kernels before
-  grid_dependents();
   const int ntiles = counts[group], tile_base = counts[3 + group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // Tiles are handed out by a counter (zeroed before the launch), so blocks
@@ -1353,7 +1339,7 @@ __global__ void batch_reduce_kernel(const BatchJob *__restrict__ jobs, const int
                                     const double *__restrict__ tile_sums, int *__restrict__ live,
                                     unsigned long long *__restrict__ prog) {
   grid_dependency_wait();
-  grid_dependents();
+  grid_dependents(kFewGatherBlocks);
   const int lane = threadIdx.x & 31;
   const int j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (j >= counts[6]) return;
@@ -1396,7 +1382,6 @@ template <typename T>
 __global__ void batch_gather_step_kernel(const BatchJob *__restrict__ jobs, const BatchTile *__restrict__ vtiles,
                                          const int *__restrict__ counts, const int *__restrict__ live) {
   grid_dependency_wait();
-  grid_dependents();
   const int nvtiles = counts[7];
   for (int t = blockIdx.x; t < nvtiles; t += gridDim.x) {
     const BatchTile tile = vtiles[t];
@@ -1407,7 +1392,7 @@ __global__ void batch_gather_step_kernel(const BatchJob *__restrict__ jobs, cons
     const uint64_t st = J.f.cnt[0] + J.f.cnt[1] - 1;
     if constexpr (sizeof(T) == 4) {
       if (a.kind == 0) {
-        bd_vertex_f32((const float *)J.f.partial, J.off, v, a, st, J.r, J.rhi, J.rlo, J.r0, J.dsp);
+        bd_vertex_f32((const float *)J.f.partial, J.off, v, a, st, J.r, J.rhi, J.r0);
         continue;
       }
     }
@@ -1449,8 +1434,7 @@ __global__ void batch_start_kernel(const BatchJob *__restrict__ jobs, const Batc
     }
     if (J.rhi && (int)threadIdx.x < tile.count) {
       const int v = tile.first + threadIdx.x;
-      for (int c = 0; c < 3; ++c)
-        store_f32_position(3 * (size_t)v + c, J.r[3 * (size_t)v + c], J.rhi, J.rlo, J.r0, J.dsp);
+      store_f32_vertex(v, J.r + 3 * (size_t)v, J.rhi, J.r0);
     }
   }
 }
@@ -1469,13 +1453,17 @@ __global__ void batch_unpack_kernel(const BatchJob *__restrict__ jobs, const Bat
     const double *src = pack + off[tile.job];
     if ((int)threadIdx.x < tile.count) {
       const size_t v = (size_t)(tile.first + threadIdx.x);
+      double x[3];
+      bool changed = false;
       for (int c = 0; c < 3; ++c) {
-        const double x = src[3 * v + c];
-        // a coordinate the caller left as it was keeps its FP32 copies (compared
-        // bit for bit, on the integer pipe): most of the unpacking's FP64 work
-        if (__double_as_longlong(x) == __double_as_longlong(J.r[3 * v + c])) continue;
-        J.r[3 * v + c] = x;
-        if (J.rhi) store_f32_position(3 * v + c, x, J.rhi, J.rlo, J.r0, J.dsp);
+        x[c] = src[3 * v + c];
+        changed = changed || __double_as_longlong(x[c]) != __double_as_longlong(J.r[3 * v + c]);
+      }
+      // a vertex the caller left as it was keeps its FP32 copies (compared bit
+      // for bit, on the integer pipe): most of the unpacking's FP64 work
+      if (changed) {
+        for (int c = 0; c < 3; ++c) J.r[3 * v + c] = x[c];
+        if (J.rhi) store_f32_vertex((int)v, x, J.rhi, J.r0);
       }
     }
     if (tile.first == 0 && threadIdx.x < 3) {
@@ -1771,12 +1759,8 @@ __device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g,
   };
   // ---- local coordinates (float-float, relative to the corner, in their images, times alpha)
   const uint32_t *cp = g.cp + (size_t)lf * NCP;
-  float ahi[3], alo[3];
-  {
-    const int v0 = (int)(__ldg(&cp[0]) & kVertexMask);
-#pragma unroll
-    for (int c = 0; c < 3; ++c) { ahi[c] = G.rhi[3 * (size_t)v0 + c]; alo[c] = G.rlo[3 * (size_t)v0 + c]; }
-  }
+  float ahi[3], alo[3], dsp[3];  // dsp: not used here
+  f32::load_vertex(G.rhi, (int)(__ldg(&cp[0]) & kVertexMask), ahi, alo, dsp);
   FF X0[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) X0[c] = ff_mul(alpha[c], FF{ahi[c], alo[c]});  // the corner carries no image
@@ -1787,9 +1771,11 @@ __device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g,
       const uint32_t packed = __ldg(&cp[j]);
       const int v = (int)(packed & kVertexMask), code = (int)(packed >> kVertexBits);
       const int img[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
+      float vh[3], vl[3];
+      f32::load_vertex(G.rhi, v, vh, vl, dsp);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
-        const float hi = G.rhi[3 * (size_t)v + c], lo = G.rlo[3 * (size_t)v + c];
+        const float hi = vh[c], lo = vl[c];
         float sh = 0.f, she = 0.f, shl = 0.f;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -1988,7 +1974,10 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
         const int v = (int)(packed & kVertexMask), code = (int)(packed >> kVertexBits);
         img[0] = code % 3 - 1; img[1] = (code / 3) % 3 - 1; img[2] = code / 9 - 1;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) { hi[c] = G.rhi[3 * (size_t)v + c]; lo[c] = G.rlo[3 * (size_t)v + c]; }
+        for (int c = 0; c < 3; ++c) {
+          hi[c] = G.rhi[kPosStride * (size_t)v + c];
+          lo[c] = G.rlo[kPosStride * (size_t)v + c];
+        }
         dest = __ldg(&g.dest[(size_t)lf * g.ncp + lane]);
       }
 #pragma unroll
@@ -2073,7 +2062,6 @@ __global__ void spmv_kernel(int nrow, const int *__restrict__ row_ptr, const int
                             const double *__restrict__ val, const double *__restrict__ scalev, MassScale F,
                             const double *__restrict__ in, double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
-  grid_dependents();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2126,7 +2114,6 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
                               const float4 *__restrict__ in4,
                               double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
-  grid_dependents();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -2193,7 +2180,7 @@ __global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C
 // Rows of three doubles to float4 {x, y, z, 0}, or (ld > 0) to three vectors.
 __global__ void mass_input32_kernel(int n, const double *__restrict__ in, float *__restrict__ out, int ld) {
   grid_dependency_wait();
-  grid_dependents();
+  grid_dependents(kFewGatherBlocks);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * n; t += gridDim.x * blockDim.x) {
     const int i = t / 3, c = t - 3 * i;
     out[ld > 0 ? (size_t)c * ld + i : 4 * (size_t)i + c] = (float)in[t];
