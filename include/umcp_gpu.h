@@ -164,10 +164,10 @@ umcp_status umcp_energy_grad_device(umcp_mesh *mesh, const double *d_r, double *
  * another runtime). Same inputs and outputs as umcp_energy_grad_device (the
  * mesh's plan tables, made at set-up, plus the caller's d_r, d_E, d_g; g is
  * accumulated; d_E may be NULL, the energy then goes to the mesh's own
- * slot); every scratch buffer lives in one 32 MiB file-scope device array
+ * slot); every scratch buffer lives in one 43 MiB file-scope device array
  * that each GPU loading the library holds until exit. Meshes whose scratch
- * exceeds 32 MiB (about 110,000 faces in FP64, 190,000 in the FP32 form) are
- * rejected with UMCP_ERR_NOMEM. The first call on a device looks up the
+ * (without padding) exceeds 32 MiB (about 110,000 faces in FP64, 190,000 in the
+ * FP32 form) are rejected with UMCP_ERR_NOMEM. The first call on a device looks up the
  * array's device address (cudaGetSymbolAddress), so make that first call
  * before any stream capture. All calls on one device share that device's
  * array and it keeps the last call's contents: calls whose work overlaps on

@@ -396,6 +396,11 @@ class MeshArena {
 };
 }  // namespace
 
+// Bytes of a gradient-partial slot.
+static size_t slot_bytes(int precision) {
+  return precision == UMCP_FP64 ? dev::kSlot<double> * sizeof(double) : dev::kSlot<float> * sizeof(float);
+}
+
 // Whether a regular group of the precision form takes the thread-per-face
 // kernel instead of the half-warp one.
 static bool use_tpf(int ncp, int nfaces) { return ncp == 12 && nfaces >= kTpfFaces; }
@@ -526,8 +531,7 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
   arena.stage(m->off, off);
   m->nblocks = block_base;
   arena.zeroed(m->blockpart, (size_t)(block_rows > 0 ? block_rows : 1) * 6 * sizeof(double));
-  const size_t elem = (m->precision == UMCP_FP64) ? sizeof(double) : sizeof(float);
-  arena.uninit(m->partial, (size_t)m->nslot_cap * 3 * elem);
+  arena.uninit(m->partial, (size_t)m->nslot_cap * slot_bytes(m->precision));
   const size_t nst = 3 * (size_t)ME.nv + 3;
   // Initial state: the plan's positions, alpha = 1.
   std::vector<double> r0(nst);
@@ -902,7 +906,7 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
   }
   b += 2 * nv * 4;                                    // slot locations
   b += (size_t)std::max(nblocks, 1) * 6 * 8;          // blockpart
-  b += slots * 3 * (f32 ? 4 : 8);                     // partial
+  b += slots * slot_bytes(precision);                 // partial
   b += 3 * nst * 8 + 2 * 3 * nv * 8;                  // r, g, r_eval; p, qdot
   b += 8 + 3 * 8 + 4 + 2 * 8 + 4;                     // E, parts, status, cnt, done
   if (f32) b += dev::kPosStride * nv * 4 + 3 * nv * 8;  // hi, lo, dsp; r0
@@ -1300,8 +1304,12 @@ extern "C" umcp_status umcp_step_host(umcp_mesh *m, const umcp_integrator *it, u
 // word and the FP32 position pairs) lives in this file-scope array, which
 // every GPU that loads the library holds until the process exits.
 
-static constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // per device, of the layout that meshes are admitted by
-static constexpr size_t kStaticArrayBytes = (size_t)34 << 20;    // the array: the positions take a third more since
+// Meshes are admitted by the packed layout (12 and 9 floats for a slot's and a
+// vertex's FP32 values), whatever padding they lie with: the array holds any
+// mesh that the limit admits, padded.
+static constexpr size_t kStaticScratchBytes = (size_t)32 << 20;  // the limit, per device
+static constexpr size_t kStaticArrayBytes = (size_t)43 << 20;
+static_assert(3 * kStaticArrayBytes >= 4 * kStaticScratchBytes, "16 bytes a slot for 12, 12 floats a vertex for 9");
 static __device__ __align__(256) unsigned char g_static_scratch[kStaticArrayBytes];
 static void *g_static_scratch_addr[128];  // device address of the array, per device (host-side)
 
@@ -1329,10 +1337,9 @@ extern "C" umcp_status umcp_energy_grad_static(umcp_mesh *m, const double *d_r, 
   // layout: [status, done] | block partials | gradient partials | FP32 position pairs and displacements
   const size_t off_flags = 0, off_block = 256;
   const size_t off_partial = off_block + align256((size_t)m->nblocks * 6 * sizeof(double));
-  const size_t off_hi = off_partial + align256((size_t)m->nslot_cap * 3 * esize);
-  // a mesh is admitted by three packed arrays of positions (9 floats a vertex); they lie 12 apart
-  const size_t need = off_hi + (fp32 ? 3 * align256((size_t)3 * m->nv * sizeof(float)) : 0);
-  static_assert(kStaticArrayBytes >= kStaticScratchBytes + kStaticScratchBytes / 3 / 9, "12 floats a vertex for 9");
+  const size_t need = off_partial + align256((size_t)m->nslot_cap * 3 * esize) +
+                      (fp32 ? 3 * align256((size_t)3 * m->nv * sizeof(float)) : 0);
+  const size_t off_hi = off_partial + align256((size_t)m->nslot_cap * slot_bytes(m->precision));
   if (need > kStaticScratchBytes)
     return fail(UMCP_ERR_NOMEM, "mesh needs " + std::to_string(need) + " bytes of scratch; the static area holds " +
                                     std::to_string(kStaticScratchBytes) + " bytes");

@@ -443,8 +443,8 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
       g[2] = fma(s, m.z, fma(b.y, v.z, fma(b.x, u.z, g[2])));
     }
     if (cur.dest >= 0)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) partial[3 * (size_t)cur.dest + c] = mul(alpha[c], g[c]);
+      reinterpret_cast<float4 *>(partial)[cur.dest] =
+          make_float4(mul(alpha[0], g[0]), mul(alpha[1], g[1]), mul(alpha[2], g[2]), 0.f);
   }
   __syncwarp();  // the next face overwrites X, D and A
 }

@@ -34,6 +34,14 @@ constexpr int kVertexBits = 27;  // packed control point: vertex | image_code <<
 constexpr uint32_t kVertexMask = (1u << kVertexBits) - 1u;
 constexpr double kSafety = 1e-12;  // SAFETY, src/interp.h:14
 
+// Elements of a gradient-partial slot. The precision form pads its slots to 16
+// bytes: a face kernel writes each with one store instead of three 4-byte ones
+// (whose 32 scattered sectors per warp instruction were 16% of the 256-vesicle
+// face pass), and the gather reads them with 16-byte loads. FP64 slots stay at
+// 24 bytes: that pass is bound by the FP64 pipe.
+template <typename T>
+constexpr int kSlot = sizeof(T) == 8 ? 3 : 4;
+
 // The precision form's FP32 positions of a vertex lie together, 12 floats on a
 // 16-byte boundary: hi.xyz, lo.xyz, dsp.xyz and three of padding, so a face
 // kernel fetches a control point with two 16-byte loads and a 4-byte one instead

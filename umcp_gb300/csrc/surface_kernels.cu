@@ -518,7 +518,7 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
           const __half ll = __ushort_as_half((unsigned short)(lw[i / 2] >> (16 * (i & 1))));
           const float xl = (__half2float(hh) + __half2float(ll)) * ia + (float)kLatU[x] * Eu[c] + (float)kLatV[x] * Ev[c];
           const int dst = __ldg(&S.dest[(size_t)f * kNcp + x]);
-          partial[3 * (size_t)dst + c] = alpha[c] * G[c][i];
+          partial[kSlot<float> * (size_t)dst + c] = alpha[c] * G[c][i];
           da[c] += G[c][i] * xl * ialpha[c];
         }
       }
@@ -612,16 +612,17 @@ __global__ void status_merge_kernel(const int *__restrict__ src, int *__restrict
 // compensation: hi - lo). Eight slots' loads are issued before they are added.
 template <typename T, class F>
 __device__ __forceinline__ void each_partial(const T *__restrict__ partial, int base, int n, int c, F add) {
-  const T *q = partial + 3 * (size_t)base + c;
+  constexpr int kStep = 32 * kSlot<T>;
+  const T *q = partial + kSlot<T> * (size_t)base + c;
   int k = 0;
   for (; k + 8 <= n; k += 8) {
     T x[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) x[i] = q[96 * (size_t)(k + i)];
+    for (int i = 0; i < 8; ++i) x[i] = q[kStep * (size_t)(k + i)];
 #pragma unroll
     for (int i = 0; i < 8; ++i) add(x[i]);
   }
-  for (; k < n; ++k) add(q[96 * (size_t)k]);
+  for (; k < n; ++k) add(q[kStep * (size_t)k]);
 }
 struct GradSum {
   float hi, lo;
@@ -654,7 +655,7 @@ __device__ __forceinline__ void vertex_gradient(const T *__restrict__ partial, c
 
 // The same sum in the precision form, its compensated total rounded to FP32.
 // Eight slots' loads are issued before they are summed (in the same order), so
-// each thread keeps 96 bytes in flight; the partials are read once, so the
+// each thread keeps 128 bytes in flight; the partials are read once, so the
 // loads are marked evict-first. 839 -> 827 us per 256-vesicle step.
 __device__ __forceinline__ void vertex_gradient_f32(const float *__restrict__ partial, const int *__restrict__ loc,
                                                     int v, float g[3]) {
@@ -665,25 +666,21 @@ __device__ __forceinline__ void vertex_gradient_f32(const float *__restrict__ pa
     c3[c] = (t - s3[c]) - y;
     s3[c] = t;
   };
+  const float4 *q = reinterpret_cast<const float4 *>(partial) + base;
+  auto add3 = [&](float4 x) {
+    add(0, x.x);
+    add(1, x.y);
+    add(2, x.z);
+  };
   int k = 0;
   for (; k + 8 <= n; k += 8) {
-    float x[8][3];
+    float4 x[8];
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const size_t s = (size_t)base + 32 * (size_t)(k + q);
+    for (int i = 0; i < 8; ++i) x[i] = __ldcs(q + 32 * (size_t)(k + i));
 #pragma unroll
-      for (int c = 0; c < 3; ++c) x[q][c] = __ldcs(&partial[3 * s + c]);
-    }
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-#pragma unroll
-      for (int c = 0; c < 3; ++c) add(c, x[q][c]);
+    for (int i = 0; i < 8; ++i) add3(x[i]);
   }
-  for (; k < n; ++k) {
-    const size_t s = (size_t)base + 32 * (size_t)k;
-#pragma unroll
-    for (int c = 0; c < 3; ++c) add(c, __ldcs(&partial[3 * s + c]));
-  }
+  for (; k < n; ++k) add3(__ldcs(q + 32 * (size_t)k));
 #pragma unroll
   for (int c = 0; c < 3; ++c) g[c] = s3[c] - c3[c];
 }
@@ -1151,11 +1148,9 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
     for (int j = 0; j < kNcp; ++j) d[j] = __ldg(&S.dest[(size_t)f * kNcp + j]);
   }
 #pragma unroll
-  for (int j = 0; j < kNcp; ++j) {
-    float *o = partial + 3 * (size_t)d[j];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) o[c] = f32::mul(alpha[c], G[j][c]);
-  }
+  for (int j = 0; j < kNcp; ++j)
+    reinterpret_cast<float4 *>(partial)[d[j]] =
+        make_float4(f32::mul(alpha[0], G[j][0]), f32::mul(alpha[1], G[j][1]), f32::mul(alpha[2], G[j][2]), 0.f);
   e3[0] = ea; e3[1] = ec; e3[2] = er;
 }
 
@@ -2004,7 +1999,7 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
     T old[3] = {0, 0, 0};
     if (lane < g.ncp)
 #pragma unroll
-      for (int k = 0; k < 3; ++k) old[k] = partial[3 * (size_t)dest + k];
+      for (int k = 0; k < 3; ++k) old[k] = partial[kSlot<T> * (size_t)dest + k];
     __syncwarp(hmask);
     if (lane < g.npt) {
       T R[3] = {0, 0, 0}, Ru[3] = {0, 0, 0}, Rv[3] = {0, 0, 0};
@@ -2050,7 +2045,7 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
         for (int k = 0; k < 3; ++k) Gx[k] += w * Es[hw][p][k] + u * Es[hw][p][3 + k] + v * Es[hw][p][6 + k];
       }
 #pragma unroll
-      for (int k = 0; k < 3; ++k) partial[3 * (size_t)dest + k] = old[k] + alpha[k] * Gx[k];
+      for (int k = 0; k < 3; ++k) partial[kSlot<T> * (size_t)dest + k] = old[k] + alpha[k] * Gx[k];
     }
     __syncwarp(hmask);
   }
