@@ -507,7 +507,11 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
       for (int p = 0; p < G->npt; ++p)
         for (int x = 0; x < G->ncp; ++x) bw[(size_t)p * G->ncp + x] = B.at(0, p, x);
       arena.stage(G->basis_w, bw);
-      if (prm->precision == UMCP_FP32_CENTRED) arena.stage(G->table, f32_table(basis, bw, B.weight, G->ncp));
+      if (prm->precision == UMCP_FP32_CENTRED) {
+        const std::vector<float> table = f32_table(basis, bw, B.weight, G->ncp);
+        if (G->ncp == 12) G->rows = tpf_rows(table);
+        arena.stage(G->table, table);
+      }
     }
     face_base += G->nfaces;
     slot_base += G->nfaces * G->ncp;
@@ -715,7 +719,7 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
   L.dudv = own->dudv;
   e = own->tc ? launch_faces_tc(L, own->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, partial, B.blockpart,
                                 B.status, own->nblocks, fin, s)
-              : launch_faces_tpf(L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
+              : launch_faces_tpf(own->rows, L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
                                  fin, geo, s);
   if (e == cudaSuccess)
     e = launch_faces32(F, m->P, B.r, B.f32, partial, B.blockpart, fin, fork ? m->ctx->side : s, !fork);

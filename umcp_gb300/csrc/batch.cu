@@ -59,6 +59,7 @@ struct umcp_batch {
   bool have_type[kTypes] = {false, false, false};
   double dudv[kTypes] = {0, 0, 0};
   DevBuf table[kTypes], weight[kTypes];
+  TpfRows rows;
   int face_grid[kTypes] = {0, 0, 0};
   int vgrid = 0;
   // device tables
@@ -311,8 +312,8 @@ static cudaError_t queue_faces(umcp_batch *b) {
       return launch_batch_faces32(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
                                   b->table[t].as<float>(), kTypeNcp[t], b->dudv[t], b->d_tile_sums.as<double>(),
                                   b->face_grid[t], on);
-    return launch_batch_faces_tpf(b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(), b->d_counts.as<int>(),
-                                  b->table[t].as<float>(), b->dudv[t], b->d_tile_sums.as<double>(), b->face_grid[t],
+    return launch_batch_faces_tpf(b->rows, b->d_jobs.as<BatchJob>(), t, b->d_tiles.as<BatchTile>(),
+                                  b->d_counts.as<int>(), b->table[t].as<float>(), b->dudv[t], b->d_tile_sums.as<double>(), b->face_grid[t],
                                   b->d_next_tile.as<int>(), on);
   };
   cudaError_t e = cudaSuccess;
@@ -600,6 +601,7 @@ extern "C" umcp_status umcp_batch_add(umcp_batch *b, umcp_mesh *m, const umcp_in
     UMCP_CUDA(b->weight[t].alloc(G.weight.bytes));
     UMCP_CUDA(cudaMemcpyAsync(b->table[t].p, G.table.p, G.table.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
     UMCP_CUDA(cudaMemcpyAsync(b->weight[t].p, G.weight.p, G.weight.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
+    if (t == 0) b->rows = G.rows;
     b->dudv[t] = G.dudv;
     b->have_type[t] = true;
     b->drop_graphs();  // the captured steps do not launch this type yet

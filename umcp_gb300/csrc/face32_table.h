@@ -21,6 +21,14 @@ struct F32Table {
   static constexpr int kFloats = kWeights + 32;
 };
 
+// The regular patch's rows for the thread-per-face kernel, which takes them as a
+// launch parameter: all threads of a warp are at the same quadrature point, so its
+// multiply-adds read them through the constant cache.
+struct TpfRows {
+  float B[15][5][12];  // rows u, v, uu, uv, vv of each point
+  float V[15][12];     // value rows (restraints)
+};
+
 // Floats of a patch type's table.
 inline int f32_table_floats(int ncp) {
   return ncp == 12 ? F32Table<12, 15>::kFloats : ncp == 11 ? F32Table<11, 16>::kFloats : F32Table<13, 16>::kFloats;
@@ -52,6 +60,17 @@ inline std::vector<float> f32_table(const std::vector<double> &basis, const std:
   else if (ncp == 11) fill_f32_table<11, 16>(basis, value, weight, &t);
   else if (ncp == 13) fill_f32_table<13, 16>(basis, value, weight, &t);
   return t;
+}
+
+// The thread-per-face kernel's rows: the same values as the table's (12 control points).
+inline TpfRows tpf_rows(const std::vector<float> &table) {
+  using L = F32Table<12, 15>;
+  TpfRows r;
+  for (int p = 0; p < 15; ++p) {
+    memcpy(r.B[p], &table[(size_t)p * L::ROW4 * 4], sizeof r.B[p]);
+    memcpy(r.V[p], &table[L::kValue + (size_t)p * 12], sizeof r.V[p]);
+  }
+  return r;
 }
 
 }  // namespace umcp

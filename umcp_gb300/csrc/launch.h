@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "face32_table.h"
 #include "kernels.cuh"
 
 namespace umcp {
@@ -135,13 +136,15 @@ cudaError_t launch_faces32(const FaceSet32 &F, const dev::SurfaceParams &P, cons
 // one warp each or none, and a face's serial chain (about 14 us) is the pass; a
 // half-warp per face shortens it to about 3 us but issues 1.6 times the
 // instructions per face. BD step, half-warps against a thread per face: 320
-// faces 11.0 / 25.7 us, 8,192 18.7 / 23.7, 20,400 25.9 / 29.8, 32,768 34.6 /
-// 29.8, 131,072 103 / 68.
+// faces 10.0 / 25 us, 8,192 18.4 / 22.1, 16,000 23.5 / 22.5, 20,400 26.7 / 25.6,
+// 32,768 34 / 26.3, 131,072 103 / 65. In between the line lies on the half-warps'
+// side of the crossing: with irregular patches beside and three evaluations in
+// flight on separate streams, 20,480 faces take 43 against 49 us.
 constexpr int kTpfFaces = 24000;
 int face_blocks_tpf(int nfaces);
-cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
-                             const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                             const FinishArgs &fin, int geo, cudaStream_t s);
+cudaError_t launch_faces_tpf(const TpfRows &rows, const dev::FaceLaunch &L, const int *dest,
+                             const dev::SurfaceParams &P, const double *r, const F32Pos &f, float *partial,
+                             double *blockpart, int *status, int grid, const FinishArgs &fin, int geo, cudaStream_t s);
 
 // The regular faces of the precision form on the tensor cores (face_tc_kernel):
 // the same outputs as launch_faces_tpf, in 128-face tiles; grid from
@@ -232,9 +235,9 @@ constexpr int kVertexTile = 256;  // vertices per vertex tile (one thread each)
 // skipped. Regular faces of the precision form (tpf; next_tile: {tiles handed
 // out, blocks done}, which the launch leaves zero), its irregular ones (32), and
 // FP64 (64); table: the patch type's (face32_table.h, fixed64.h).
-cudaError_t launch_batch_faces_tpf(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
-                                   const float *table, double dudv, double *tile_sums, int grid, int *next_tile,
-                                   cudaStream_t s);
+cudaError_t launch_batch_faces_tpf(const TpfRows &rows, const BatchJob *jobs, int group, const BatchTile *tiles,
+                                   const int *counts, const float *table, double dudv, double *tile_sums, int grid,
+                                   int *next_tile, cudaStream_t s);
 cudaError_t launch_batch_faces32(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
                                  const float *table, int ncp, double dudv, double *tile_sums, int grid, cudaStream_t s);
 cudaError_t launch_batch_faces64(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,

@@ -15,10 +15,6 @@
 namespace umcp {
 namespace dev {
 
-template <typename T>
-struct alignas(4 * sizeof(T)) Q4 {
-  T x, y, z, w;
-};
 
 // ---------------------------------------------------------------- tensor-core face pass
 //
@@ -884,8 +880,8 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
 // points X[12][3] (and their displacements from the reference state) in its
 // own columns of shared memory, its gradient sums G[12][3] in registers, and
 // walks the 15 points; every thread of a warp reads the same basis row at the
-// same time, so the basis comes out of shared memory as broadcasts (one
-// wavefront per float4) and both contractions are plain multiply-adds:
+// same time, so the rows come as a launch parameter through the constant cache
+// and both contractions are plain multiply-adds:
 //   K[k]_c = sum_j B[p][k][j] X[j]_c          (Ru, Rv, Suu, Suv, Svv)
 //   G[j]_c += B[p][u][j] Kb[u]_c + B[p][v][j] Kb[v]_c + s[j] m_c,
 //   s[j] = B[p][uu][j] lb + B[p][uv][j] kb + B[p][vv][j] nb
@@ -893,11 +889,18 @@ __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double 
 // point times the normal instead of three vector rows). Nothing is shuffled
 // or transposed per face. Energy terms and dE/dalpha are Kahan-summed per
 // thread over its faces and reduced once at the end, in a fixed order.
+//
+// Bound by issue and the FP32 pipe (64% busy, 0.6 instructions a cycle and
+// scheduler). With the rows in shared memory their broadcasts took the 27 reads a
+// point of a data path that X and D also need, and registers to hold them: 256
+// vesicles of 5,120 faces 657 us, 320,000 planar faces 122 us; as a parameter 550
+// and 111 us. Blocks: the batch kernel gains from a fourth a SM (579 us with
+// three); the single-mesh kernel's code for three is the faster one (111 against
+// 113 us; both reach four).
 namespace tpf {
 constexpr int kNcp = 12, kNpt = 15, kNc4 = 3;
-constexpr int kThreads = 128, kWarps = kThreads / 32, kMinBlocks = 3;
+constexpr int kThreads = 128, kWarps = kThreads / 32, kMinBlocks = 3, kBatchMinBlocks = 4;
 struct Smem {
-  Q4<float> B[kNpt][5][kNc4];  // basis rows u, v, uu, uv, vv of point p, control points in fours
   // each thread's centred control points, coordinate-major: float4 3 c + q
   // holds coordinate c of control points 4 q .. 4 q + 3; the 144-byte stride
   // is an odd number of 16-byte chunks, so the float4 reads of a warp do not
@@ -906,8 +909,7 @@ struct Smem {
   float4 D[kThreads][9];  // the same control points' change from the reference state, same layout
   float2 C[kNpt];  // each point's coefficients curv, area (f32::Coef)
   float Cg[kNpt];  // and gauss
-  Q4<float> V[kNpt][kNc4];  // value rows and each point's kA, kV (restraints)
-  float2 geo[kNpt];
+  float2 geo[kNpt];  // and kA, kV (restraints)
   double red[kWarps][6];
 };
 constexpr size_t kSumBytes = sizeof(float) * 12 * kThreads;  // per-thread Kahan totals (dynamic shared memory)
@@ -934,27 +936,10 @@ __device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefe
 constexpr int kPrefetchPoint = 10;
 }  // namespace tpf
 
-// table: the patch type's staged table, whose leading rows are B's image.
-__device__ __forceinline__ void tpf_stage(tpf::Smem &sm, const float *__restrict__ table) {
-  using L = F32Table<tpf::kNcp, tpf::kNpt>;
-  static_assert(L::ROW4 == 5 * tpf::kNc4, "the table's rows are B's image");
-  const float4 *t = reinterpret_cast<const float4 *>(table);
-  Q4<float> *b = &sm.B[0][0][0];
-  for (int i = threadIdx.x; i < tpf::kNpt * L::ROW4; i += blockDim.x) {
-    const float4 v = __ldg(t + i);
-    b[i] = Q4<float>{v.x, v.y, v.z, v.w};
-  }
-}
-// The restraints' tables: value rows, and the points' coefficients (which come from the sums kernel).
+// The restraints' coefficients of the points (which come from the sums kernel).
 __device__ __forceinline__ void tpf_stage_geo(tpf::Smem &sm, const float *__restrict__ table,
                                               const double *__restrict__ gterm, double dudv) {
   using L = F32Table<tpf::kNcp, tpf::kNpt>;
-  const float4 *t = reinterpret_cast<const float4 *>(table + L::kValue);
-  Q4<float> *v = &sm.V[0][0];
-  for (int i = threadIdx.x; i < tpf::kNpt * tpf::kNc4; i += blockDim.x) {
-    const float4 x = __ldg(t + i);
-    v[i] = Q4<float>{x.x, x.y, x.z, x.w};
-  }
   if ((int)threadIdx.x < tpf::kNpt)
     sm.geo[threadIdx.x] = f32::geo_coef(gterm, __ldg(reinterpret_cast<const double *>(table + L::kWeights) + threadIdx.x), dudv);
 }
@@ -974,7 +959,7 @@ __device__ __forceinline__ void tpf_coefs(tpf::Smem &sm, const float *__restrict
 // the reference state. fn: the face this thread takes next (its rows are
 // prefetched), or -1.
 template <bool KG_REG, bool GEO>
-__device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const SurfaceParams &P, int f,
+__device__ __forceinline__ void tpf_face(tpf::Smem &sm, const TpfRows &rows, const FaceSrc &S, const SurfaceParams &P, int f,
                                          const float alpha[3], const float ialpha[3], const float am1[3],
                                          float k_reg, bool vec, bool want_da, float *__restrict__ partial,
                                          float e3[3], float da[3], int fn) {
@@ -1062,8 +1047,8 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
       }
 #pragma unroll
       for (int k = 0; k < 5; ++k) {
-        const Q4<float> b = sm.B[p][k][c4];
-        const float2 b01 = make_float2(b.x, b.y), b23 = make_float2(b.z, b.w);
+        const float *b = &rows.B[p][k][4 * c4];
+        const float2 b01 = make_float2(b[0], b[1]), b23 = make_float2(b[2], b[3]);
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
           A[k][c] = __ffma2_rn(b01, make_float2(x[c].x, x[c].y), A[k][c]);
@@ -1075,11 +1060,11 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
         }
       }
       if constexpr (GEO) {
-        const Q4<float> b = sm.V[p][c4];
+        const float *b = &rows.V[p][4 * c4];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          Av[c] = __ffma2_rn(make_float2(b.x, b.y), make_float2(x[c].x, x[c].y), Av[c]);
-          Av[c] = __ffma2_rn(make_float2(b.z, b.w), make_float2(x[c].z, x[c].w), Av[c]);
+          Av[c] = __ffma2_rn(make_float2(b[0], b[1]), make_float2(x[c].x, x[c].y), Av[c]);
+          Av[c] = __ffma2_rn(make_float2(b[2], b[3]), make_float2(x[c].z, x[c].w), Av[c]);
         }
       }
     }
@@ -1111,20 +1096,17 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const FaceSrc &S, const 
     }
     // G[j]_c += B[u][j] Kb[u]_c + B[v][j] Kb[v]_c + s[j] m_c in scalar multiply-adds: with the
     // forward contraction in paired ones, the mix keeps both FP32 multiply-add pipes busy
-    // (all paired: 763 us, this mix: 747 us, all scalar: 776 us on the 256-vesicle pass)
+    // (256-vesicle pass: this mix 550 us, all scalar 591, all paired 727 with spills)
     {
       const float ku[3] = {o.Ku.x, o.Ku.y, o.Ku.z}, kv[3] = {o.Kv.x, o.Kv.y, o.Kv.z}, md[3] = {o.m.x, o.m.y, o.m.z};
 #pragma unroll
       for (int c4 = 0; c4 < kNc4; ++c4) {
-        const Q4<float> bu = sm.B[p][0][c4], bv = sm.B[p][1][c4], buu = sm.B[p][2][c4], buv = sm.B[p][3][c4],
-                        bvv = sm.B[p][4][c4];
-        const float u[4] = {bu.x, bu.y, bu.z, bu.w}, v[4] = {bv.x, bv.y, bv.z, bv.w};
-        const float uu[4] = {buu.x, buu.y, buu.z, buu.w}, uv[4] = {buv.x, buv.y, buv.z, buv.w},
-                    vv[4] = {bvv.x, bvv.y, bvv.z, bvv.w};
+        const float *u = &rows.B[p][0][4 * c4], *v = &rows.B[p][1][4 * c4], *uu = &rows.B[p][2][4 * c4],
+                    *uv = &rows.B[p][3][4 * c4], *vv = &rows.B[p][4][4 * c4];
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
           float sj = fmaf(vv[jj], o.nb, fmaf(uv[jj], o.kb, __fmul_rn(uu[jj], o.lb)));
-          if constexpr (GEO) sj = fmaf((&sm.V[p][c4].x)[jj], geo.kV, sj);
+          if constexpr (GEO) sj = fmaf(rows.V[p][4 * c4 + jj], geo.kV, sj);
           float *g = G[4 * c4 + jj];
 #pragma unroll
           for (int cc = 0; cc < 3; ++cc) g[cc] = fmaf(sj, md[cc], fmaf(v[jj], kv[cc], fmaf(u[jj], ku[cc], g[cc])));
@@ -1184,14 +1166,13 @@ struct SharedSums {
 // to finish sums them (as face_kernel does).
 template <bool GEO>  // the restraints' gradient goes along
 __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
-    face_tpf_kernel(FaceLaunch L, const int *__restrict__ dest, SurfaceParams P, const double *__restrict__ r,
+    face_tpf_kernel(const __grid_constant__ TpfRows rows, FaceLaunch L, const int *__restrict__ dest, SurfaceParams P, const double *__restrict__ r,
                     const float *__restrict__ rhi, const float *__restrict__ rlo, const float *__restrict__ dsp,
                     float *__restrict__ partial, double *__restrict__ blockpart, int *__restrict__ status,
                     FinishArgs fin) {
   using namespace tpf;
   __shared__ Smem sm;
   extern __shared__ __align__(16) unsigned char tpf_dyn[];
-  tpf_stage(sm, L.table);
   tpf_coefs(sm, L.table, P, L.dudv);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
@@ -1217,8 +1198,8 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
       float e3[3], da[3];
       // no prefetch: a thread's next face is a grid stride away, and on the
       // 512 x 512 planar pass the prefetch cost 1% instead of gaining
-      if (kg_reg) tpf_face<true, GEO>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
-      else tpf_face<false, GEO>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
+      if (kg_reg) tpf_face<true, GEO>(sm, rows, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
+      else tpf_face<false, GEO>(sm, rows, src, P, f, alpha, ialpha, am1, k_reg, vec, want_da, partial, e3, da, -1);
       acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
       acc.add(3, da[0]); acc.add(4, da[1]); acc.add(5, da[2]);
       if (!isfinite(e3[0] + e3[1] + e3[2])) atomicOr(status, kStatusNonFinite);
@@ -1245,15 +1226,14 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
 // and the last of them zeroes both for the next launch. A block draws its next
 // tile while it works on the current one (the draw's round trip hides behind
 // the faces), and copies a job's header only when the tile's job changes.
-__global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
-    batch_face_tpf_kernel(const BatchJob *__restrict__ jobs, int group, const BatchTile *__restrict__ tiles,
+__global__ void __launch_bounds__(tpf::kThreads, tpf::kBatchMinBlocks)
+    batch_face_tpf_kernel(const __grid_constant__ TpfRows rows, const BatchJob *__restrict__ jobs, int group, const BatchTile *__restrict__ tiles,
                           const int *__restrict__ counts, const float *__restrict__ table, double dudv,
                           double *__restrict__ tile_sums, int *__restrict__ counter) {
   using namespace tpf;
   __shared__ Smem sm;
   __shared__ BatchFaceJob sj;
   __shared__ int s_active, s_tile[2];
-  tpf_stage(sm, table);     // constant table: before the wait
   grid_dependency_wait();        // positions, job states and the counter come from the kernels before
   const int ntiles = counts[group], tile_base = counts[3 + group];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1299,8 +1279,8 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
         if (f < end) {
           float e3[3], da[3];
           const int fn = f + kThreads < end ? f + kThreads : -1;
-          if (kg_reg) tpf_face<true, false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
-          else tpf_face<false, false>(sm, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
+          if (kg_reg) tpf_face<true, false>(sm, rows, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
+          else tpf_face<false, false>(sm, rows, src, P, f, alpha, ialpha, am1, k_reg, vec, false, partial, e3, da, fn);
           acc.add(0, e3[0]); acc.add(1, e3[1]); acc.add(2, e3[2]);
         }
       }
@@ -2206,13 +2186,14 @@ int face_blocks_tpf(int nfaces) {
   return need < cached ? need : cached;
 }
 
-cudaError_t launch_faces_tpf(const dev::FaceLaunch &L, const int *dest, const dev::SurfaceParams &P, const double *r,
-                             const F32Pos &f, float *partial, double *blockpart, int *status, int grid,
-                             const FinishArgs &fin, int geo, cudaStream_t s) {
+cudaError_t launch_faces_tpf(const TpfRows &rows, const dev::FaceLaunch &L, const int *dest,
+                             const dev::SurfaceParams &P, const double *r, const F32Pos &f, float *partial,
+                             double *blockpart, int *status, int grid, const FinishArgs &fin, int geo,
+                             cudaStream_t s) {
   if (L.nfaces <= 0) return cudaSuccess;
   if (!f.hi || !f.lo || !f.dsp) return cudaErrorInvalidValue;
-  return launch_after(geo ? dev::face_tpf_kernel<true> : dev::face_tpf_kernel<false>, grid, dev::tpf::kThreads, dev::tpf::kSumBytes, s, L, dest, P, r, f.hi, f.lo,
-                      f.dsp, partial, blockpart, status, fin);
+  return launch_after(geo ? dev::face_tpf_kernel<true> : dev::face_tpf_kernel<false>, grid, dev::tpf::kThreads,
+                      dev::tpf::kSumBytes, s, rows, L, dest, P, r, f.hi, f.lo, f.dsp, partial, blockpart, status, fin);
 }
 
 cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cudaStream_t s) {
@@ -2313,12 +2294,12 @@ int batch_face_blocks_tpf() {
   });
 }
 
-cudaError_t launch_batch_faces_tpf(const BatchJob *jobs, int group, const BatchTile *tiles, const int *counts,
-                                   const float *table, double dudv, double *tile_sums, int grid, int *next_tile,
-                                   cudaStream_t s) {
+cudaError_t launch_batch_faces_tpf(const TpfRows &rows, const BatchJob *jobs, int group, const BatchTile *tiles,
+                                   const int *counts, const float *table, double dudv, double *tile_sums, int grid,
+                                   int *next_tile, cudaStream_t s) {
   if (!next_tile) return cudaErrorInvalidValue;
-  return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, jobs, group, tiles, counts, table,
-                      dudv, tile_sums, next_tile);
+  return launch_after(dev::batch_face_tpf_kernel, grid, dev::tpf::kThreads, 0, s, rows, jobs, group, tiles, counts,
+                      table, dudv, tile_sums, next_tile);
 }
 
 cudaError_t launch_batch_reduce(const BatchJob *jobs, const int *counts, int max_jobs, const int *tile_off,
