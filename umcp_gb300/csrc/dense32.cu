@@ -12,9 +12,11 @@
 // own slot and the finish adds a row's slots in order. Results depend on the
 // device's SM count only.
 // Measured (one call on device arrays, about 19 us of it launch and wait):
-// 10,242 rows 152 -> 103 us, 2,562 rows 46 -> 25 us, against four whole rows per
-// warp with 4-byte loads. (The loads ahead through a shared-memory ring of two or
-// three units: 99.5 us, not kept.)
+// 10,242 rows 152 -> 98 us, 2,562 rows 46 -> 25 us, against four whole rows per
+// warp with 4-byte loads. (Two units of loads ahead in registers instead of one:
+// no gain at 10,242 rows, a Langevin step of 2,562 vertices 9% slower; through a
+// shared-memory ring of two or three units: 3% faster than in registers before the
+// vectors kept their L1 lines, not kept.)
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -56,6 +58,14 @@ __device__ __forceinline__ f2 sub2(f2 a, f2 b) {
   return r;
 }
 
+// A load of the matrix, which is read once: it leaves the L1 cache to the vectors
+// (a warp reads their next chunk only when it sums it, so a miss is a stall: 10,242
+// rows 106 us a call with evict-first loads, 98 with these).
+__device__ __forceinline__ float4 load_once(const float *p) {
+  float4 v;
+  asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
+}
 // Units of warp w of W: [w U / W, (w + 1) U / W); the warp of unit u.
 __host__ __device__ __forceinline__ long long first_unit(long long w, long long U, long long W) { return w * U / W; }
 __host__ __device__ __forceinline__ long long warp_of(long long u, long long U, long long W) {
@@ -101,7 +111,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
 #pragma unroll
     for (int r = 0; r < kRows; ++r) {
       const int i = gg * kRows + r;
-      m[r] = (i < n && j < ld) ? __ldcs(reinterpret_cast<const float4 *>(A + (size_t)i * ld + j)) : zero4;
+      m[r] = (i < n && j < ld) ? load_once(A + (size_t)i * ld + j) : zero4;
     }
   };
   f2 s[kSums], nc[kSums];  // Kahan sums of even and odd columns, and minus their compensations
