@@ -632,7 +632,7 @@ static GeoArgs geo_args(umcp_mesh *m, const double *d_r) {
     g.basis = Gp->basis.as<double>();
     g.basis_w = Gp->basis_w.as<double>();
     g.weight = Gp->weight.as<double>();
-    g.tab = Gp->geo_tab.as<float>();
+    g.tab = Gp->geo_tab.p;
     g.ncp = Gp->ncp;
     g.npt = Gp->npt;
     g.ncpp = (Gp->ncp + 3) / 4 * 4;
@@ -743,7 +743,7 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
   GeoArgs GA{};
   if (geo) {
     GA = geo_args(m, d_r);
-    cudaError_t e = launch_geo_sums(GA, m->precision == UMCP_FP64, fused, s);
+    cudaError_t e = sizeof(T) == 8 ? launch_geo_sums(GA, s) : launch_geo_sums32(GA, fused, s);
     if (e != cudaSuccess) return e;
     fin.gterm = m->gterm.as<double>();
   }
@@ -1053,30 +1053,21 @@ extern "C" umcp_status umcp_restraints_set(umcp_mesh *m, const umcp_restraints *
   if (m->precision == UMCP_FP32_CENTRED)
     for (auto &G : m->groups) {
       if (G->geo_tab.p || G->nfaces == 0) continue;
-      // FP32 tables of the restraint kernels: the value and first-derivative
-      // rows split as hi + lo, and the point weights
+      // tables of the restraint kernels
       const int ncp = G->ncp, npt = G->npt, ncpp = (ncp + 3) / 4 * 4;
       std::vector<double> basis((size_t)npt * 5 * ncpp), bw((size_t)npt * ncp), w(npt);
       UMCP_CUDA(cudaMemcpy(basis.data(), G->basis.p, basis.size() * sizeof(double), cudaMemcpyDeviceToHost));
       UMCP_CUDA(cudaMemcpy(bw.data(), G->basis_w.p, bw.size() * sizeof(double), cudaMemcpyDeviceToHost));
       UMCP_CUDA(cudaMemcpy(w.data(), G->weight.p, w.size() * sizeof(double), cudaMemcpyDeviceToHost));
-      std::vector<float> tab(geo_tab_floats(ncp, npt));
-      const size_t nrow = (size_t)npt * 3 * ncp;
-      for (int p = 0; p < npt; ++p)
-        for (int k = 0; k < 3; ++k)
-          for (int x = 0; x < ncp; ++x) {
-            const double b = k == 0 ? bw[(size_t)p * ncp + x] : basis[((size_t)p * 5 + (k - 1)) * ncpp + x];
-            const size_t i = ((size_t)p * 3 + k) * ncp + x;
-            tab[i] = (float)b;
-            tab[nrow + i] = (float)(b - (double)tab[i]);
-          }
-      for (int p = 0; p < npt; ++p) {
-        const double cw = G->dudv * w[p], c3 = cw / 3.0;
-        tab[2 * nrow + p] = (float)cw;
-        tab[2 * nrow + npt + p] = (float)c3;
-        tab[2 * nrow + 2 * npt + p] = (float)(c3 - (double)(float)c3);
+      if (geo_padded(ncp) == 12) {
+        std::vector<GeoRows<12>> tab(1);
+        fill_geo_rows(basis, bw, w, G->dudv, ncp, npt, ncpp, &tab[0]);
+        UMCP_CUDA(upload(G->geo_tab, tab));
+      } else {
+        std::vector<GeoRows<16>> tab(1);
+        fill_geo_rows(basis, bw, w, G->dudv, ncp, npt, ncpp, &tab[0]);
+        UMCP_CUDA(upload(G->geo_tab, tab));
       }
-      UMCP_CUDA(upload(G->geo_tab, tab));
     }
   if (!m->gterm.p) {
     int nblk = geo_blocks(m->nfaces);
@@ -1098,7 +1089,8 @@ extern "C" umcp_status umcp_restraints_set(umcp_mesh *m, const umcp_restraints *
     if (m->precision == UMCP_FP32_CENTRED && !m->split_valid)
       UMCP_CUDA(launch_split_positions(3 * m->nv, m->r.as<double>(), m->f32pos(), s));
     m->split_valid = true;
-    UMCP_CUDA(launch_geo_sums(geo_args(m, m->r.as<double>()), m->precision == UMCP_FP64, true, s));
+    const GeoArgs GA = geo_args(m, m->r.as<double>());
+    UMCP_CUDA(m->precision == UMCP_FP64 ? launch_geo_sums(GA, s) : launch_geo_sums32(GA, true, s));
     double gt[kGeoWords];
     UMCP_CUDA(cudaMemcpyAsync(gt, m->gterm.p, sizeof gt, cudaMemcpyDeviceToHost, s));
     UMCP_CUDA(cudaStreamSynchronize(s));

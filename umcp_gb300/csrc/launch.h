@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "face32_table.h"
+#include "geo32_table.h"
 #include "kernels.cuh"
 
 namespace umcp {
@@ -40,15 +41,10 @@ struct GeoGroup {
   const double *basis;     // [npt][5][ncpp] rows u,v,uu,uv,vv
   const double *basis_w;   // [npt][ncp] value rows
   const double *weight;    // [npt]
-  // FP32 tables of the precision form: rows w,u,v as hi [npt][3][ncp] then
-  // lo [npt][3][ncp] (row = hi + lo), then cw = dudv w [npt], then
-  // c3 = dudv w / 3 as hi [npt] and lo [npt]
-  const float *tab;
+  const void *tab;         // the precision form's rows: GeoRows<geo_padded(ncp)> (geo32_table.h)
   int ncp, npt, ncpp, nfaces, face_base;
   double dudv;
 };
-// Floats of GeoGroup::tab for a patch type.
-inline size_t geo_tab_floats(int ncp, int npt) { return (size_t)6 * npt * ncp + 3 * (size_t)npt; }
 enum : int { kGeoA = 0, kGeoV, kGeoE, kGeoCA, kGeoCV, kGeoDAlpha, kGeoWords = 8 };
 struct GeoArgs {
   GeoGroup g[3];
@@ -68,11 +64,12 @@ inline int geo_blocks(int nfaces) {
   const int b = nfaces > 0 ? (nfaces + 4 * (kGeoThreads / 16) - 1) / (4 * (kGeoThreads / 16)) : 1;  // >= 4 faces per half-warp
   return b < 152 * 8 ? b : 152 * 8;
 }
-// Sums A, V and their alpha derivatives; the last block writes gterm.
-// alpha64: the area and the box-scale derivatives in FP64 as well (plain path).
-// fused: the face launches form the restraints' gradient (and with it dE_r/dalpha,
-// which gterm then has as zero): the precision form's SIMT kernels.
-cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, bool fused, cudaStream_t s);
+// Sums A, V and their alpha derivatives; the last block writes gterm. The plain
+// path, in FP64 throughout.
+cudaError_t launch_geo_sums(const GeoArgs &G, cudaStream_t s);
+// The precision form (geo32.cu). fused: the face launches form the restraints' gradient (and with it dE_r/dalpha, which gterm then
+// has as zero): its SIMT kernels.
+cudaError_t launch_geo_sums32(const GeoArgs &G, bool fused, cudaStream_t s);
 // partial[slot] += alpha * (dE_r/dA dA/dX + dE_r/dV dV/dX) for every (face, control point).
 template <typename T>
 cudaError_t launch_geo_grad(const GeoArgs &G, T *partial, cudaStream_t s);

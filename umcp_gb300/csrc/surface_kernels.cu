@@ -7,6 +7,8 @@
 
 #include "device_common.cuh"
 #include "face32.cuh"
+#include "geo.cuh"
+#include "geo32_table.h"
 #include "kernels.cuh"
 #include "launch.h"
 #include "launch_host.h"
@@ -1486,7 +1488,6 @@ __global__ void batch_pack_kernel(const BatchJob *__restrict__ jobs, const Batch
 // pairs, as the face pass forms them).
 
 constexpr int kGeoHW = kGeoThreads / 16;  // faces in flight per block
-constexpr int kGeoPt = 16;                // quadrature points of the largest rule
 
 template <typename T>
 struct GeoBasis {
@@ -1529,64 +1530,6 @@ __device__ __forceinline__ void geo_abs64(const GeoArgs &G, const GeoGroup &g, i
 }
 
 __device__ __forceinline__ double shfl_d(unsigned mask, double v, int src) { return __shfl_sync(mask, v, src, 16); }
-
-template <typename T>
-__device__ __forceinline__ void cross3(const T a[3], const T b[3], T o[3]) {
-  o[0] = a[1] * b[2] - a[2] * b[1];
-  o[1] = a[2] * b[0] - a[0] * b[2];
-  o[2] = a[0] * b[1] - a[1] * b[0];
-}
-
-// Block sums of the per-thread accumulators in a fixed order; the last block
-// to finish sums the block rows (in block order) and forms E_r, dE_r/dA,
-// dE_r/dV and dE_r/dalpha.
-__device__ void geo_finish(const GeoArgs &G, const double acc[kGeoWords], double (*red)[kGeoThreads]) {
-  __shared__ bool last;
-#pragma unroll
-  for (int q = 0; q < kGeoWords; ++q) red[q][threadIdx.x] = acc[q];
-  __syncthreads();
-  for (int w = kGeoThreads / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-#pragma unroll
-      for (int q = 0; q < kGeoWords; ++q) red[q][threadIdx.x] += red[q][threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x < kGeoWords) G.block[(size_t)blockIdx.x * kGeoWords + threadIdx.x] = red[threadIdx.x][0];
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) last = (atomicAdd(G.done, 1u) == gridDim.x - 1);
-  __syncthreads();
-  if (!last) return;
-  __threadfence();
-  // Fixed-order sum of the block rows by the whole block: thread (i, q) sums word q
-  // of rows i, i + 16, ..., and the 16 sums of a word are added in order. (One
-  // thread a word is a chain of loads from L2: 27 us for 640 rows, a restrained evaluation
-  // of a 40,962-vertex vesicle alone 206 -> 179 us.)
-  static_assert(kGeoThreads % kGeoWords == 0, "a thread per word and row class");
-  constexpr int kClasses = kGeoThreads / kGeoWords;
-  const int q = threadIdx.x % kGeoWords, i = threadIdx.x / kGeoWords;
-  double t = 0;
-#pragma unroll 8
-  for (unsigned b = i; b < gridDim.x; b += kClasses) t += __ldcg(&G.block[(size_t)b * kGeoWords + q]);
-  red[q][i] = t;
-  __syncthreads();
-  if (i == 0) {
-    for (int k = 1; k < kClasses; ++k) t += red[q][k];
-    red[q][0] = t;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double A = red[0][0], V = red[1][0];
-    const double cA = G.A0 > 0 ? G.KA * (A - G.A0) / G.A0 : 0.0, cV = G.KV * (V - G.V0);
-    G.gterm[kGeoA] = A;
-    G.gterm[kGeoV] = V;
-    G.gterm[kGeoE] = (G.A0 > 0 ? 0.5 * G.KA * (A - G.A0) * (A - G.A0) / G.A0 : 0.0) + 0.5 * G.KV * (V - G.V0) * (V - G.V0);
-    G.gterm[kGeoCA] = cA;
-    G.gterm[kGeoCV] = cV;
-    for (int k = 0; k < 3; ++k) G.gterm[kGeoDAlpha + k] = cA * red[2 + k][0] + cV * red[5 + k][0];
-    *G.done = 0u;
-  }
-}
 
 // Sums A, V and their alpha derivatives in FP64 (the plain path).
 __global__ void __launch_bounds__(kGeoThreads) geo_sums_kernel(GeoArgs G) {
@@ -1654,248 +1597,12 @@ __global__ void __launch_bounds__(kGeoThreads) geo_sums_kernel(GeoArgs G) {
   geo_finish(G, acc, red);
 }
 
-// ---- float-float (double-FP32) arithmetic for the precision form's volume.
-// A value is hi + lo with |lo| <= ulp(hi)/2; the error-free transformations
-// are Knuth's two-sum and the FMA two-product (Dekker's product with a fused
-// multiply-add), so the arithmetic stays on the FP32 pipes and carries about
-// 44 bits. Every product and sum inside them is rounded on its own (no
-// contraction into an FMA), as the transformations require.
-struct FF {
-  float hi, lo;
-};
-__device__ __forceinline__ FF ff_fast_two_sum(float a, float b) {  // |a| >= |b| or a == 0
-  const float s = __fadd_rn(a, b);
-  return {s, __fsub_rn(b, __fsub_rn(s, a))};
-}
-__device__ __forceinline__ FF ff_add(FF x, FF y) {
-  float s, e;
-  two_sum(x.hi, y.hi, s, e);
-  e = __fadd_rn(e, __fadd_rn(x.lo, y.lo));
-  return ff_fast_two_sum(s, e);
-}
-__device__ __forceinline__ FF ff_mul(FF x, FF y) {
-  const float p = __fmul_rn(x.hi, y.hi);
-  float e = __fmaf_rn(x.hi, y.hi, -p);
-  e = __fmaf_rn(x.hi, y.lo, e);
-  e = __fmaf_rn(x.lo, y.hi, e);
-  return ff_fast_two_sum(p, e);
-}
-// acc += b x, without renormalising acc (call ff_norm once at the end).
-__device__ __forceinline__ void ff_acc(FF &acc, float bh, float bl, float xh, float xl) {
-  const float p = __fmul_rn(bh, xh);
-  float e = __fmaf_rn(bh, xh, -p);
-  e = __fmaf_rn(bh, xl, e);
-  e = __fmaf_rn(bl, xh, e);
-  float s, t;
-  two_sum(acc.hi, p, s, t);
-  acc.hi = s;
-  acc.lo = __fadd_rn(acc.lo, __fadd_rn(t, e));
-}
-__device__ __forceinline__ FF ff_norm(FF x) { return ff_fast_two_sum(x.hi, x.lo); }
-__device__ __forceinline__ FF ff_of(double x) {
-  const float h = (float)x;
-  return {h, (float)(x - (double)h)};
-}
-
 // (The gradient goes along in the face kernels, which have the tangents and the
 // normal at hand: 10% more of their work instead of a pass of its own over every
 // face, 40 to 50 us at 81,920 faces, with a read and write of every partial.
 // Three restrained evaluations of a 40,962-vertex vesicle in flight: 179 -> 135
 // us each. The pass below remains for the plain path and for meshes whose
 // regular faces run on the tensor cores.)
-//
-// The precision form's sums: V from float-float contractions of float-float
-// local coordinates (formed from the FP32 hi/lo position pairs with error-free
-// sums) and summed in float-float per thread; the area and the box-scale
-// derivatives from the FP32 leading parts with Kahan sums. FP64 enters only in
-// the per-block and final sums.
-//
-// One face per thread. Each thread keeps its face's
-// float-float local coordinates in its own columns of shared memory
-// (coordinate-major, control points padded to 16, the column 400 bytes, an
-// odd number of 16-byte chunks, so a warp's 16-byte reads do not conflict),
-// and walks the face's points; the value and derivative rows of the point
-// (hi and lo) are the same for every thread of a warp that is on the same
-// patch type, so they come out of shared memory as broadcasts. (A half-warp
-// form, lanes = points with per-lane row reads, took 177.6 us on a 40,962-vertex
-// vesicle against 154.5 us for this one, both issue-bound on the float-float
-// arithmetic.)
-namespace geo_tpf {
-constexpr int kThreads = 128;
-constexpr int kCp = 16;                  // control points, padded
-constexpr int kCol = 3 * kCp * 2 + 4;    // floats of a thread's column: hi [3][16], lo [3][16], pad
-struct Rows {
-  float4 r[3][kGeoPt][6][kCp / 4];       // [group][point][w hi, w lo, u hi, u lo, v hi, v lo][control points in fours]
-  float cw[3][kGeoPt];
-  FF c3[3][kGeoPt];
-};
-constexpr size_t kDynBytes = sizeof(float) * kCol * kThreads;
-}  // namespace geo_tpf
-
-template <int NCP, int NPT, bool DA>
-__device__ __forceinline__ void geo_face_ff(const GeoArgs &G, const GeoGroup &g, const geo_tpf::Rows &rows, int gi,
-                                            int lf, const FF alpha[3], const float ialpha[3], float *col, FF &accV,
-                                            float ks[kGeoWords], float kc[kGeoWords]) {
-  using namespace geo_tpf;
-  auto kahan = [&](int q, float v) {
-    const float y = v - kc[q], t = ks[q] + y;
-    kc[q] = (t - ks[q]) - y;
-    ks[q] = t;
-  };
-  // ---- local coordinates (float-float, relative to the corner, in their images, times alpha)
-  const uint32_t *cp = g.cp + (size_t)lf * NCP;
-  float ahi[3], alo[3], dsp[3];  // dsp: not used here
-  f32::load_vertex(G.rhi, (int)(__ldg(&cp[0]) & kVertexMask), ahi, alo, dsp);
-  FF X0[3];
-#pragma unroll
-  for (int c = 0; c < 3; ++c) X0[c] = ff_mul(alpha[c], FF{ahi[c], alo[c]});  // the corner carries no image
-#pragma unroll
-  for (int j = 0; j < kCp; ++j) {
-    float xh[3] = {0.f, 0.f, 0.f}, xl[3] = {0.f, 0.f, 0.f};
-    if (j < NCP) {
-      const uint32_t packed = __ldg(&cp[j]);
-      const int v = (int)(packed & kVertexMask), code = (int)(packed >> kVertexBits);
-      const int img[3] = {code % 3 - 1, (code / 3) % 3 - 1, code / 9 - 1};
-      float vh[3], vl[3];
-      f32::load_vertex(G.rhi, v, vh, vl, dsp);
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float hi = vh[c], lo = vl[c];
-        float sh = 0.f, she = 0.f, shl = 0.f;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          float t, e;
-          two_sum(sh, __fmul_rn((float)img[d], G.box_hi[d][c]), t, e);
-          sh = t;
-          she = __fadd_rn(she, e);
-          shl = __fadd_rn(shl, __fmul_rn((float)img[d], G.box_lo[d][c]));
-        }
-        float s1, e1, s2, e2;
-        two_sum(hi, sh, s1, e1);
-        two_sum(s1, -ahi[c], s2, e2);
-        const float res = __fadd_rn(__fadd_rn(e1, e2), __fadd_rn(__fsub_rn(lo, alo[c]), __fadd_rn(she, shl)));
-        const FF x = ff_mul(alpha[c], ff_fast_two_sum(s2, res));
-        xh[c] = x.hi;
-        xl[c] = x.lo;
-      }
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      col[c * kCp + j] = xh[c];
-      col[3 * kCp + c * kCp + j] = xl[c];
-    }
-  }
-  // ---- the points
-#pragma unroll 1
-  for (int p = 0; p < NPT; ++p) {
-    FF R[3] = {{0, 0}, {0, 0}, {0, 0}}, Ru[3] = {{0, 0}, {0, 0}, {0, 0}}, Rv[3] = {{0, 0}, {0, 0}, {0, 0}};
-#pragma unroll 1  // rolled: the unrolled body (about 1,900 instructions) missed in the instruction cache
-    for (int q = 0; q < (NCP + 3) / 4; ++q) {
-      const float4 w4h = rows.r[gi][p][0][q], w4l = rows.r[gi][p][1][q], u4h = rows.r[gi][p][2][q],
-                   u4l = rows.r[gi][p][3][q], v4h = rows.r[gi][p][4][q], v4l = rows.r[gi][p][5][q];
-      const float wh[4] = {w4h.x, w4h.y, w4h.z, w4h.w}, wl[4] = {w4l.x, w4l.y, w4l.z, w4l.w};
-      const float uh[4] = {u4h.x, u4h.y, u4h.z, u4h.w}, ul[4] = {u4l.x, u4l.y, u4l.z, u4l.w};
-      const float vh[4] = {v4h.x, v4h.y, v4h.z, v4h.w}, vl[4] = {v4l.x, v4l.y, v4l.z, v4l.w};
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const float4 x4h = *reinterpret_cast<const float4 *>(&col[c * kCp + 4 * q]);
-        const float4 x4l = *reinterpret_cast<const float4 *>(&col[3 * kCp + c * kCp + 4 * q]);
-        const float xh[4] = {x4h.x, x4h.y, x4h.z, x4h.w}, xl[4] = {x4l.x, x4l.y, x4l.z, x4l.w};
-#pragma unroll
-        for (int jj = 0; jj < 4; ++jj) {
-          if (4 * q + jj >= NCP) break;
-          ff_acc(R[c], wh[jj], wl[jj], xh[jj], xl[jj]);
-          ff_acc(Ru[c], uh[jj], ul[jj], xh[jj], xl[jj]);
-          ff_acc(Rv[c], vh[jj], vl[jj], xh[jj], xl[jj]);
-        }
-      }
-    }
-    FF Ra[3], m[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      Ru[c] = ff_norm(Ru[c]);
-      Rv[c] = ff_norm(Rv[c]);
-      Ra[c] = ff_add(X0[c], ff_norm(R[c]));
-    }
-#pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      const int a = (c + 1) % 3, b = (c + 2) % 3;
-      const FF t = ff_mul(Ru[b], Rv[a]);
-      m[c] = ff_add(ff_mul(Ru[a], Rv[b]), FF{-t.hi, -t.lo});
-    }
-    const FF dot = ff_add(ff_add(ff_mul(Ra[0], m[0]), ff_mul(Ra[1], m[1])), ff_mul(Ra[2], m[2]));
-    accV = ff_add(accV, ff_mul(rows.c3[gi][p], dot));
-    // area and box-scale derivatives from the leading parts
-    const float Rf[3] = {Ra[0].hi, Ra[1].hi, Ra[2].hi}, Uf[3] = {Ru[0].hi, Ru[1].hi, Ru[2].hi},
-                Vf[3] = {Rv[0].hi, Rv[1].hi, Rv[2].hi}, mf[3] = {m[0].hi, m[1].hi, m[2].hi};
-    const float gg2 = mf[0] * mf[0] + mf[1] * mf[1] + mf[2] * mf[2];
-    const float ig = rsqrtf(gg2), gg = gg2 * ig;
-    const float cwf = rows.cw[gi][p], c3f = rows.c3[gi][p].hi;
-    kahan(0, cwf * gg);
-    if constexpr (!DA) continue;
-    float n[3] = {mf[0] * ig, mf[1] * ig, mf[2] * ig}, a1[3], a2[3], v1[3], v2[3];
-    cross3(Vf, n, a1);
-    cross3(n, Uf, a2);
-    cross3(Vf, Rf, v1);
-    cross3(Rf, Uf, v2);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      kahan(2 + k, cwf * (a1[k] * Uf[k] + a2[k] * Vf[k]) * ialpha[k]);
-      kahan(5 + k, c3f * (mf[k] * Rf[k] + v1[k] * Uf[k] + v2[k] * Vf[k]) * ialpha[k]);
-    }
-  }
-}
-
-// DA: the box-scale derivatives too (else the face launches form them).
-template <bool DA>
-__global__ void __launch_bounds__(geo_tpf::kThreads, 3) geo_sums_ff_tpf_kernel(GeoArgs G) {
-  using namespace geo_tpf;
-  __shared__ Rows rows;
-  __shared__ FF alpha_s[3];
-  __shared__ float ialpha_s[3];
-  extern __shared__ __align__(16) float geo_cols[];
-  for (int gi = 0; gi < G.ngroups; ++gi) {  // rows hi/lo, control points padded with zeros
-    const GeoGroup &g = G.g[gi];
-    const int nrow = g.npt * 3 * g.ncp;
-    float *r = &rows.r[gi][0][0][0].x;
-    for (int i = threadIdx.x; i < g.npt * 6 * kCp; i += blockDim.x) {
-      const int p = i / (6 * kCp), k = (i / kCp) % 6, x = i % kCp;  // k: row (w, u, v) * 2 + lo
-      const int e = p * 3 * g.ncp + (k / 2) * g.ncp + x;
-      r[((size_t)p * 6 + k) * kCp + x] = x < g.ncp ? g.tab[(k & 1) * nrow + e] : 0.f;
-    }
-    for (int p = threadIdx.x; p < g.npt; p += blockDim.x) {
-      rows.cw[gi][p] = g.tab[2 * nrow + p];
-      rows.c3[gi][p] = FF{g.tab[2 * nrow + g.npt + p], g.tab[2 * nrow + 2 * g.npt + p]};
-    }
-  }
-  grid_dependency_wait();  // the state comes from the kernels before
-  if (threadIdx.x < 3) {
-    const double a = G.r[3 * (size_t)G.nv + threadIdx.x];
-    alpha_s[threadIdx.x] = ff_of(a);
-    ialpha_s[threadIdx.x] = 1.f / (float)a;
-  }
-  __syncthreads();
-  const FF alpha[3] = {alpha_s[0], alpha_s[1], alpha_s[2]};
-  const float ialpha[3] = {ialpha_s[0], ialpha_s[1], ialpha_s[2]};
-  float *col = geo_cols + (size_t)kCol * threadIdx.x;
-  FF accV = {0, 0};
-  float ks[kGeoWords] = {0, 0, 0, 0, 0, 0, 0, 0}, kc[kGeoWords] = {0, 0, 0, 0, 0, 0, 0, 0};
-  for (int f = blockIdx.x * kThreads + threadIdx.x; f < G.nfaces; f += gridDim.x * kThreads) {
-    int lf;
-    const int gi = geo_group(G, f, &lf);
-    const GeoGroup &g = G.g[gi];
-    if (g.ncp == 12) geo_face_ff<12, 15, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
-    else if (g.ncp == 11) geo_face_ff<11, 16, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
-    else geo_face_ff<13, 16, DA>(G, g, rows, gi, lf, alpha, ialpha, col, accV, ks, kc);
-  }
-  double acc[kGeoWords];
-#pragma unroll
-  for (int q = 0; q < kGeoWords; ++q) acc[q] = (double)ks[q] - (double)kc[q];
-  acc[1] = (double)accV.hi + (double)accV.lo;
-  __syncthreads();  // every column is done with: the block sums reuse their space
-  static_assert(kDynBytes >= sizeof(double) * kGeoWords * kThreads, "block sums must fit in the columns");
-  geo_finish(G, acc, reinterpret_cast<double(*)[kThreads]>(geo_cols));
-}
 
 // partial[slot] += alpha * dE_r/dX for every (face, control point):
 //   dE_r/dR  = c_V c/3 m,   dE_r/dRu = c_A c (Rv x n) + c_V c/3 (Rv x R),
@@ -1912,9 +1619,15 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
   if constexpr (sizeof(T) == 4) {
     for (int gi = 0; gi < G.ngroups; ++gi) {
       const GeoGroup &g = G.g[gi];
-      const int nrow = g.npt * 3 * g.ncp;
-      for (int i = threadIdx.x; i < nrow; i += blockDim.x) sb.B[gi][i / (3 * g.ncp)][(i / g.ncp) % 3][i % g.ncp] = g.tab[i];
-      for (int p = threadIdx.x; p < g.npt; p += blockDim.x) sb.cw[gi][p] = g.tab[2 * nrow + p];
+      auto stage = [&](const auto &t) {
+        for (int i = threadIdx.x; i < g.npt * 3 * g.ncp; i += blockDim.x) {
+          const int p = i / (3 * g.ncp), k = (i / g.ncp) % 3, x = i % g.ncp;
+          sb.B[gi][p][k][x] = t.bf[p][k][x];
+        }
+        for (int p = threadIdx.x; p < g.npt; p += blockDim.x) sb.cw[gi][p] = t.cw[p];
+      };
+      if (g.ncp <= 12) stage(*static_cast<const GeoRows<12> *>(g.tab));
+      else stage(*static_cast<const GeoRows<16> *>(g.tab));
     }
   } else {
     stage_geo_basis<T>(G, sb);
@@ -2351,16 +2064,8 @@ cudaError_t launch_batch_pack(const BatchJob *jobs, const BatchTile *vtiles, con
 
 namespace umcp {
 
-cudaError_t launch_geo_sums(const GeoArgs &G, bool alpha64, bool fused, cudaStream_t s) {
-  if (alpha64) return launch_after(dev::geo_sums_kernel, geo_blocks(G.nfaces), kGeoThreads, 0, s, G);
-  // the thread-per-face form: a grid that depends on the face count only (the sums' order is fixed)
-  auto kernel = fused ? dev::geo_sums_ff_tpf_kernel<false> : dev::geo_sums_ff_tpf_kernel<true>;
-  const cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dev::geo_tpf::kDynBytes);
-  if (e != cudaSuccess) return e;
-  const int per_block = dev::geo_tpf::kThreads, want = (G.nfaces + per_block - 1) / per_block;
-  const int grid = want < 1 ? 1 : (want < geo_blocks(G.nfaces) ? want : geo_blocks(G.nfaces));
-  return launch_after(kernel, grid, dev::geo_tpf::kThreads, dev::geo_tpf::kDynBytes, s, G);
+cudaError_t launch_geo_sums(const GeoArgs &G, cudaStream_t s) {
+  return launch_after(dev::geo_sums_kernel, geo_blocks(G.nfaces), kGeoThreads, 0, s, G);
 }
 
 template <typename T>
