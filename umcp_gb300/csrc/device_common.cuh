@@ -3,6 +3,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "convert.h"
 #include "launch.h"
 
 namespace umcp {
@@ -35,11 +36,9 @@ __device__ __forceinline__ bool job_active(const BatchFaceJob &J) { return !*J.s
 __device__ __forceinline__ void store_f32_position(size_t i, double x, float *__restrict__ hi,
                                                    float *__restrict__ lo, const double *__restrict__ r0,
                                                    float *__restrict__ dsp) {
-  const float h = (float)x;
   const size_t at = pos_at(i);
-  hi[at] = h;
-  lo[at] = (float)(x - (double)h);
-  dsp[at] = (float)(x - r0[i]);
+  convert::to_f32_pair(x, hi[at], lo[at]);
+  dsp[at] = convert::to_f32(__dsub_rn(x, r0[i]));
 }
 
 // The same for a vertex whose three coordinates one thread has, in the two
@@ -49,9 +48,8 @@ __device__ __forceinline__ void store_f32_vertex(int v, const double x[3], float
   float h[3], l[3], d[3];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    h[c] = (float)x[c];
-    l[c] = (float)(x[c] - (double)h[c]);
-    d[c] = (float)(x[c] - r0[3 * (size_t)v + c]);
+    convert::to_f32_pair(x[c], h[c], l[c]);
+    d[c] = convert::to_f32(__dsub_rn(x[c], r0[3 * (size_t)v + c]));
   }
   float *q = hi + kPosStride * (size_t)v;
   reinterpret_cast<float4 *>(q)[0] = make_float4(h[0], h[1], h[2], l[0]);

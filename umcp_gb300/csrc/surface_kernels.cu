@@ -636,7 +636,7 @@ __device__ __forceinline__ GradSum coordinate_sum(const float *__restrict__ part
 }
 __device__ __forceinline__ double coordinate_gradient(const float *__restrict__ partial, int base, int n, int c) {
   const GradSum s = coordinate_sum(partial, base, n, c);
-  return (double)s.hi - (double)s.lo;
+  return __dsub_rn(convert::to_f64(s.hi), convert::to_f64(s.lo));
 }
 __device__ __forceinline__ double coordinate_gradient(const double *__restrict__ partial, int base, int n, int c) {
   double a = 0;
@@ -773,11 +773,11 @@ __device__ __forceinline__ uint64_t current_step(const uint64_t *cnt) { return c
 // and the Box-Muller normals stay in FP32, and so does the increment
 // -(D dt / kT) g + sqrt(2 D dt) xi (about 2^-23 relative, 1e-9 A at a 0.02 A
 // step); it is added to the FP64 position, from which the FP32 copies are
-// then taken. The FP64 work is the position and its copies only: 8 operations
-// per coordinate instead of 14 on GB300's narrow FP64 pipe. Explicitly
+// then taken. The FP64 work is two additions a coordinate, the position and its
+// displacement (eight with casts, 14 with the step in FP64; see convert.h). Explicitly
 // rounded, so every kernel that inlines it rounds alike.
 __device__ __forceinline__ double bd_coordinate_f32(const StepArgs &a, float g, float n, double r) {
-  return __dadd_rn(r, (double)__fmaf_rn(-a.mob_dt_f, g, __fmul_rn(a.sigma_f, n)));
+  return __dadd_rn(r, convert::to_f64(__fmaf_rn(-a.mob_dt_f, g, __fmul_rn(a.sigma_f, n))));
 }
 __device__ __forceinline__ void bd_vertex_f32(const float *__restrict__ partial, const int *__restrict__ off, int v,
                                               const StepArgs &a, uint64_t st, double *__restrict__ r,
@@ -827,7 +827,7 @@ __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const 
     const double g = coordinate_gradient(partial, at.x, at.y, c);
     double n, q = a.kind != 0 ? p[i] : 0.0;
     if constexpr (sizeof(T) == 8) n = normal_f64(o, c);
-    else n = (double)normal_f32(o, c);
+    else n = convert::to_f64(normal_f32(o, c));
     x = coordinate_update(a, g, n, r[i], &q);
     if (a.kind != 0) p[i] = q;
     r[i] = x;
@@ -852,7 +852,7 @@ __global__ void gather_kick_kernel(int nv, const T *__restrict__ partial, const 
     const double n = normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c);
     const double q = kick(a, n, p[i], coordinate_gradient(partial, at.x, at.y, c));
     p[i] = q;
-    if (x32) x32[ld > 0 ? (size_t)c * ld + v : 4 * (size_t)v + c] = (float)q;
+    if (x32) x32[ld > 0 ? (size_t)c * ld + v : 4 * (size_t)v + c] = convert::to_f32(q);
   }
 }
 
@@ -1380,7 +1380,7 @@ __global__ void batch_gather_step_kernel(const BatchJob *__restrict__ jobs, cons
     } else {
       float nf[3];
       normals3_f32(a.seed, a.stream, st, v, nf);
-      for (int c = 0; c < 3; ++c) n[c] = nf[c];
+      for (int c = 0; c < 3; ++c) n[c] = convert::to_f64(nf[c]);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -1881,7 +1881,7 @@ __global__ void mass_input32_kernel(int n, const double *__restrict__ in, float 
   grid_dependents(kFewGatherBlocks);
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < 3 * n; t += gridDim.x * blockDim.x) {
     const int i = t / 3, c = t - 3 * i;
-    out[ld > 0 ? (size_t)c * ld + i : 4 * (size_t)i + c] = (float)in[t];
+    out[ld > 0 ? (size_t)c * ld + i : 4 * (size_t)i + c] = convert::to_f32(in[t]);
   }
 }
 
