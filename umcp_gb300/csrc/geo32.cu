@@ -20,8 +20,8 @@
 // from shared memory, what a face needs there is spread over four threads, and a
 // mesh of 1,280 faces still has 40 blocks.
 //
-// Measured on 81,920 faces: the kernel 150 -> 65 us (123 us of it with the block rows
-// summed in parallel), three restrained evaluations in flight 129 -> 89 us each.
+// Measured on 81,920 faces: a restrained evaluation alone 206 -> 121 us (27 us of it by
+// summing the block rows in parallel), three in flight 129 -> 88 us each.
 // The error of V against extended precision is the smaller one, 0.4e-15 to 1.1e-15
 // relative where it was 0.4e-15 to 1.4e-15 (162 to 40,962 vertices). Rows through
 // the constant cache: 3 us slower in the best form, the rows take registers before
@@ -92,10 +92,17 @@ __device__ __forceinline__ long long mad_wide(int a, int b, long long c) {
 // S 2^(e - 56) + c: the bits from 2^kTop up are the high part, exact in FP32 (|S| < 2^58: a
 // row's entries add up to less than 4 in magnitude).
 __device__ __forceinline__ FF from_sum(long long S, float c, int e) {
-  const long long t = (S + (1ll << (kTop - 1))) >> kTop;
-  const int low = (int)((S - (t << kTop)) >> 2);
-  return ff_fast_two_sum(__fmul_rn((float)(int)t, exp2i(e - 2 * kGeoRowBits + kTop)),
+  const int top = ((int)(S >> (kTop - 1)) + 1) >> 1;  // S / 2^kTop, rounded
+  const int low = (int)(S >> 2);                      // the rest: the kTop bits below, as a signed number
+  static_assert(kTop == 34, "low: bits 2 to 33 are a word");
+  return ff_fast_two_sum(__fmul_rn((float)top, exp2i(e - 2 * kGeoRowBits + kTop)),
                          __fmaf_rn((float)low, exp2i(e - 2 * kGeoRowBits + 2), c));
+}
+
+// x y as hi + lo without normalising lo (terms of a sum that is normalised at its end).
+__device__ __forceinline__ FF product(FF x, FF y) {
+  const float p = __fmul_rn(x.hi, y.hi);
+  return {p, __fmaf_rn(x.lo, y.hi, __fmaf_rn(x.hi, y.lo, __fmaf_rn(x.hi, y.hi, -p)))};
 }
 
 // One thread's running sums.
@@ -239,10 +246,19 @@ __device__ __forceinline__ void faces(const GeoRows<NCPP> &rows, const GeoArgs &
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       const int a = (c + 1) % 3, b = (c + 2) % 3;
-      const FF t = ff_mul(Ru[b], Rv[a]);
-      m[c] = ff_add(ff_mul(Ru[a], Rv[b]), FF{-t.hi, -t.lo});
+      const FF p = product(Ru[a], Rv[b]), q = product(Ru[b], Rv[a]);
+      float s, t;
+      two_sum(p.hi, -q.hi, s, t);
+      m[c] = ff_fast_two_sum(s, __fadd_rn(t, __fsub_rn(p.lo, q.lo)));
     }
-    const FF dot = ff_add(ff_add(ff_mul(Ra[0], m[0]), ff_mul(Ra[1], m[1])), ff_mul(Ra[2], m[2]));
+    FF dot;
+    {
+      const FF x = product(Ra[0], m[0]), y = product(Ra[1], m[1]), z = product(Ra[2], m[2]);
+      float s, t, s2, t2;
+      two_sum(x.hi, y.hi, s, t);
+      two_sum(s, z.hi, s2, t2);
+      dot = ff_fast_two_sum(s2, __fadd_rn(__fadd_rn(t, t2), __fadd_rn(__fadd_rn(x.lo, y.lo), z.lo)));
+    }
     const FF c3 = {rows.c3[0][p], rows.c3[1][p]};
     // area and box-scale derivatives from the leading parts
     const float Rf[3] = {Ra[0].hi, Ra[1].hi, Ra[2].hi}, Uf[3] = {Ru[0].hi, Ru[1].hi, Ru[2].hi},
