@@ -85,11 +85,11 @@ SM_COUNT, FP32_LANES_PER_SM = 152, 128
 E2E_GROUPS = 3
 E2E_REPEATS = 3  # K-step e2e runs; the median is reported
 # DRAM bytes per face of the batched face launches, from the ncu capture of
-# the first 64 vesicles of the workload at 512-face tiles (dram__bytes_read.sum
-# + dram__bytes_write.sum of the regular and valence-5 launches: 86.48 +
-# 26.64 + 2.79 + 0.01 MB over 392,960 faces); the benchmark's pass is scaled
+# the first 64 vesicles of the workload at 256-face tiles (dram__bytes_read.sum
+# + dram__bytes_write.sum of the regular and valence-5 launches: 85.06 +
+# 35.11 + 1.86 + 0.00 MB over 392,960 faces); the benchmark's pass is scaled
 # from it by its face count.
-BATCH_FACE_DRAM_BYTES_PER_FACE = 115.92e6 / 392960
+BATCH_FACE_DRAM_BYTES_PER_FACE = 122.03e6 / 392960
 
 
 def parse_args():
@@ -459,7 +459,7 @@ def config1_variant(ctx, U, W, torch, stream, tmpdir: Path, K: int, peak_gbs: fl
             "states_finite": bool(np.all(np.isfinite(r1))),
             "fp64_tflops": flops * K / sec / 1e12, "fp64_frac_of_nominal": flops * K / sec / 1e12 / FP64_NOMINAL_TFLOPS,
             "face_pass_bytes_per_step": byts, "hbm_gbs": byts * K / sec / 1e9, "hbm_frac": byts * K / sec / 1e9 / peak_gbs,
-            "note": "the whole mesh's data (about 0.6 MB) stays in L2; one step is two face launches and a fused "
+            "note": "the whole mesh's data (about 0.6 MB) stays in L2; one step is a face launch and a fused "
                     "gather-update, captured as CUDA graphs of 32 steps, so the step is launch- and latency-bound "
                     "rather than bound by FP64 issue or HBM",
             "cpu_oracle_1core": {"vertex_steps_per_s": plan.nv / cpu_s, "ms_per_step": cpu_s * 1e3, "cores": 1,
@@ -606,7 +606,7 @@ def engine_arm(args) -> None:
                      "small by design, the face work is ~40 flop per byte", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"],
                      "traffic": (BATCH_FACE_DRAM_BYTES_PER_FACE * nfaces) if BATCH_FACE_DRAM_BYTES_PER_FACE else None,
-                     "kernel": "batch_face_tpf_kernel (regular faces) and batch_face_kernel (valence-5 and "
+                     "kernel": "batch_face_tpf_kernel (regular faces) and batch_face32_kernel (valence-5 and "
                                "valence-7 faces): the face launches of one step",
                      "launch_ms": face_ms, "algorithmic_bytes_per_launch": byts, "peak_source": peaks["source"],
                      "compute": {"fp32_tflops": flops / (face_ms / 1e3) / 1e12, "fp32_simt_peak_tflops": fp32_peak,
@@ -718,8 +718,10 @@ def engine_arm(args) -> None:
                                    "fp64_tflops": fl64 * K64 / s64 / 1e12,
                                    "fp64_frac": fl64 * K64 / s64 / 1e12 / FP64_NOMINAL_TFLOPS,
                                    "fp64_peak_note": "face-pass flops of the whole step over its time, against the "
-                                                     "nominal 1.25 TFLOP/s dense FP64 of a GB300: the plain path is "
-                                                     "bound by the FP64 pipe, not by HBM"}
+                                                     "nominal 1.25 TFLOP/s dense FP64 of a GB300. The basis "
+                                                     "contractions, most of those flops, run in fixed point on the "
+                                                     "integer multiply-adds, so the fraction may exceed 1; the "
+                                                     "pointwise step is bound by the FP64 pipe"}
             del b64
             # FP32 form against FP64 on the same states: every vesicle, at its
             # reference state (where the area forces vanish and only rounding

@@ -107,7 +107,7 @@ struct umcp_mesh {
   umcp::DevBuf r0;        // precision form: reference state (FP64)
   umcp::DevBuf r_eval;    // staging for host-pointer energy/gradient calls (keeps the resident state)
   umcp::DevBuf done;      // finished-block counter of the face pass
-  bool split_valid = false;  // rhi/rlo hold the resident state r
+  bool split_valid = false;  // the FP32 positions hold the resident state r
   double kT = 0.592186663194;  // kcal/mol at the params' temperature (src/hd.C:142-143)
   umcp::DevBuf energies;
   size_t energies_cap = 0;

@@ -88,7 +88,7 @@ struct Sums {
   double ea = 0, ec = 0, er = 0, da[3] = {0, 0, 0};
 };
 
-// point_adjoint in FP64 for K = {Ru, Rv, Suu, Suv, Svv}; adds the point's
+// The pointwise energy and adjoint for K = {Ru, Rv, Suu, Suv, Svv}; adds the point's
 // energy terms if on, overwrites K with the adjoints. reg_alpha: also adds the
 // angle term's extra box-scale part (src/grad.C:7414-7421), times alpha - 1.
 template <bool KG_REG>

@@ -1,19 +1,18 @@
 // Device kernels of the membrane-surface hot path (sm_103a).
 //
-// face_tpf_kernel one thread per regular face (precision form): control
-//                 points in thread-private shared memory, basis rows as
-//                 warp-wide broadcasts, gradient sums in registers.
-// face_kernel     one half-warp per face (FP64, and irregular faces): lanes
-//                 are quadrature points while the five basis contractions,
-//                 the pointwise energy and adjoint, and each point's
-//                 contribution to every control point are formed; then lanes
-//                 are control points while those contributions are summed.
-//                 Both write per-face gradient partials and per-block energy
-//                 sums; no float atomics.
-// gather_kernel   per vertex, sums its face partials in a fixed order
-//                 (slots interleaved by groups of 32 vertices), optionally
-//                 fused with an integrator update.
-// finish_kernel   fixed-order sum of the block partials.
+// The face kernels write per-face gradient partials and per-block energy sums; no
+// float atomics. Which takes a face:
+//   face_tpf_kernel, batch_face_tpf_kernel (surface_kernels.cu)  the precision
+//       form's regular faces of large meshes and of batches, one thread per face;
+//   face32_kernel, batch_face32_kernel (face32.cu, face32.cuh)  its irregular
+//       faces, and the regular ones of smaller meshes, a half-warp per face;
+//   face_tc_kernel (surface_kernels.cu)  its regular faces on the tensor cores
+//       (an option);
+//   face64_kernel, batch_face64_kernel (face64.cu, face64.cuh)  FP64, a
+//       half-warp per face, contractions in fixed point.
+// The gather kernels sum each vertex's partials in a fixed order (slots
+// interleaved by groups of 32 vertices), most of them fused with an integrator
+// update. The last block of a pass sums the block sums (count_and_finish).
 //
 // The energy model is the reference's surface::fenergy/ifenergy with
 // FIXED_A and LOCAL_LIPID_ENERGY (src/interpLib.C:3426-3881); the gradient

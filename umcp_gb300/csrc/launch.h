@@ -77,7 +77,7 @@ cudaError_t launch_geo_grad(const GeoArgs &G, T *partial, cudaStream_t s);
 // The precision form's FP32 copies of the positions (all NULL in the plain
 // path): r = hi + lo to about 2^-48 relative, and dsp = r - r0, the
 // displacement from the reference state r0 (setg0's state), rounded once.
-// The face kernels form the area strain from dsp (see point_adjoint).
+// The face kernels form the area strain from dsp (f32::point).
 struct F32Pos {
   float *hi = nullptr, *lo = nullptr;
   const double *r0 = nullptr;

@@ -766,7 +766,7 @@ __device__ __forceinline__ double coordinate_update(const StepArgs &a, double g,
 }
 
 // Step index of the current step: the run's first step plus the run index,
-// which finish_kernel has already advanced past this step.
+// which the face pass has already advanced past this step.
 __device__ __forceinline__ uint64_t current_step(const uint64_t *cnt) { return cnt[0] + cnt[1] - 1; }
 
 // The precision form's overdamped BD step of one vertex: the gradient total
@@ -982,7 +982,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const TpfRows &rows, con
               Pres = __ldg(&S.compf[3 * (size_t)f + 2]);
   // ---- control points relative to the patch corner (control point 0), in
   // their lattice images, times alpha; error-free sums on the hi/lo pairs as
-  // in face_compute, so the local coordinates carry full FP32 precision. Their
+  // in f32::local_position, so the local coordinates carry full FP32 precision. Their
   // change from the reference state: alpha L - L0 = (alpha - 1) L + (dsp -
   // dsp of the corner). Formed and stored four control points at a time.
   float4 *xs = sm.X[threadIdx.x], *ds = sm.D[threadIdx.x];
@@ -1165,7 +1165,7 @@ struct SharedSums {
 // Single mesh, regular faces, precision form: persistent grid, warp w of the
 // grid takes faces 32 w .. 32 w + 31, then 32 (w + warps in the grid) ...
 // Writes one block partial of the energy terms and dE/dalpha; the last block
-// to finish sums them (as face_kernel does).
+// of the pass to finish sums them.
 template <bool GEO>  // the restraints' gradient goes along
 __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
     face_tpf_kernel(const __grid_constant__ TpfRows rows, FaceLaunch L, const int *__restrict__ dest, SurfaceParams P, const double *__restrict__ r,
