@@ -5,6 +5,8 @@
 #include <math.h>
 #include <stdint.h>
 
+#include <type_traits>
+
 #include "device_common.cuh"
 #include "face32.cuh"
 #include "geo.cuh"
@@ -598,16 +600,17 @@ __global__ void stage_in_kernel(int n, const double *__restrict__ host_r, double
   }
 }
 
+__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
+
 // dst |= *src (one thread): a status word handed on to another.
 __global__ void status_merge_kernel(const int *__restrict__ src, int *__restrict__ dst) {
   const int v = *src;
   if (v) *dst |= v;
 }
 
-// Sum of coordinate c of vertex v's gradient partials: its slots are
-// loc[2 v] + 32 k for k < loc[2 v + 1] (32 vertices interleaved, so the lanes of
-// a warp read consecutive slots), summed in k order (FP64, or FP32 with Kahan
-// compensation: hi - lo). Eight slots' loads are issued before they are added.
+// Coordinate c of a vertex's gradient partials, in order: its slots are
+// base + 32 k for k < n (32 vertices interleaved, so the lanes of a warp read
+// consecutive slots). Eight slots' loads are issued before they are handed on.
 template <typename T, class F>
 __device__ __forceinline__ void each_partial(const T *__restrict__ partial, int base, int n, int c, F add) {
   constexpr int kStep = 32 * kSlot<T>;
@@ -622,33 +625,78 @@ __device__ __forceinline__ void each_partial(const T *__restrict__ partial, int 
   }
   for (; k < n; ++k) add(q[kStep * (size_t)k]);
 }
+// The same for a thread with one coordinate to gather: the 24 slots of a vertex of
+// valence 6 are loaded together, before what else the thread loads and before its
+// normals, and added afterwards (each). In rounds of eight behind the normals and
+// the status a BD step took 1.0 to 1.2 us more at every size (320 faces 10.0 ->
+// 8.9 us, 32,768 26.2 -> 25.0; FP64, 1,280 faces 29.6 -> 28.6). gather_kernel, which
+// has no normals to form meanwhile, gained nothing and lost to its registers.
+template <typename T>
+struct Partials {
+  static constexpr int kAhead = 24, kStep = 32 * kSlot<T>;
+  const T *base;
+  int2 at;
+  int c;
+  T x[kAhead];
+  __device__ __forceinline__ Partials(const T *__restrict__ partial, int2 loc, int coordinate)
+      : base(partial), at(loc), c(coordinate) {
+    if (at.y < kAhead) return;
+    const T *q = partial + kSlot<T> * (size_t)at.x + c;
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) x[i] = q[kStep * (size_t)i];
+  }
+  template <class F>
+  __device__ __forceinline__ void each(F add) const {
+    if (at.y < kAhead) {
+      each_partial(base, at.x, at.y, c, add);
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < kAhead; ++i) add(x[i]);
+    for (int k = kAhead; k < at.y; ++k) add(base[kSlot<T> * ((size_t)at.x + 32 * (size_t)k) + c]);
+  }
+};
 struct GradSum {
   float hi, lo;
 };
-__device__ __forceinline__ GradSum coordinate_sum(const float *__restrict__ partial, int base, int n, int c) {
+// Kahan-compensated total hi - lo of FP32 partials.
+struct KahanPartial {
   GradSum s{0.f, 0.f};
-  each_partial(partial, base, n, c, [&](float x) {
+  __device__ __forceinline__ void operator()(float x) {
     const float y = x - s.lo, t = s.hi + y;
     s.lo = (t - s.hi) - y;
     s.hi = t;
-  });
-  return s;
+  }
+  __device__ __forceinline__ double value() const { return __dsub_rn(convert::to_f64(s.hi), convert::to_f64(s.lo)); }
+};
+struct PlainPartial {
+  double s = 0;
+  __device__ __forceinline__ void operator()(double x) { s += x; }
+  __device__ __forceinline__ double value() const { return s; }
+};
+template <typename T>
+using PartialSum = std::conditional_t<sizeof(T) == 4, KahanPartial, PlainPartial>;
+__device__ __forceinline__ GradSum coordinate_sum(const Partials<float> &partials) {
+  KahanPartial s;
+  partials.each([&](float x) { s(x); });
+  return s.s;
 }
-__device__ __forceinline__ double coordinate_gradient(const float *__restrict__ partial, int base, int n, int c) {
-  const GradSum s = coordinate_sum(partial, base, n, c);
-  return __dsub_rn(convert::to_f64(s.hi), convert::to_f64(s.lo));
-}
-__device__ __forceinline__ double coordinate_gradient(const double *__restrict__ partial, int base, int n, int c) {
-  double a = 0;
-  each_partial(partial, base, n, c, [&](double x) { a += x; });
-  return a;
+template <typename T>
+__device__ __forceinline__ double coordinate_gradient(const Partials<T> &partials) {
+  PartialSum<T> s;
+  partials.each([&](T x) { s(x); });
+  return s.value();
 }
 template <typename T>
 __device__ __forceinline__ void vertex_gradient(const T *__restrict__ partial, const int *__restrict__ loc, int v,
                                                 double gg[3]) {
   const int base = loc[2 * (size_t)v], n = loc[2 * (size_t)v + 1];
 #pragma unroll
-  for (int c = 0; c < 3; ++c) gg[c] = coordinate_gradient(partial, base, n, c);
+  for (int c = 0; c < 3; ++c) {
+    PartialSum<T> s;
+    each_partial(partial, base, n, c, [&](T x) { s(x); });
+    gg[c] = s.value();
+  }
 }
 
 // The same sum in the precision form, its compensated total rounded to FP32.
@@ -694,7 +742,9 @@ __global__ void gather_kernel(int nv, const T *__restrict__ partial, const int *
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
     const int v = i / 3, c = i - 3 * v;
     const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
-    const double a = coordinate_gradient(partial, at.x, at.y, c);
+    PartialSum<T> s;
+    each_partial(partial, at.x, at.y, c, [&](T x) { s(x); });
+    const double a = s.value();
     g[i] = store ? a : g[i] + a;
   }
 }
@@ -800,39 +850,43 @@ __device__ __forceinline__ void bd_vertex_f32(const float *__restrict__ partial,
 // coordinate (24 adds, a Box-Muller normal, the update) is a third of a
 // vertex's, and a 642-vertex mesh spreads over 31 blocks instead of three. The
 // redundant Philox rounds are integer work beside it. 642-vertex FP64 BD step:
-// 45.6 -> 32.5 us; 128 x 128 membrane, FP32: 39.6 -> 35.6 us.
+// 45.6 -> 32.5 us; 128 x 128 membrane, FP32: 39.6 -> 35.6 us (see also Partials).
 template <typename T>
 __global__ void gather_step_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off, StepArgs a,
                                    const uint64_t *__restrict__ cnt, double *__restrict__ r, double *__restrict__ p,
                                    float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
                                    float *__restrict__ dsp, const int *__restrict__ status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, v = i / 3, c = i - 3 * v;
+  const bool on = i < 3 * nv;
+  const int2 at = on ? __ldg(reinterpret_cast<const int2 *>(off) + v) : make_int2(0, 0);  // constant: before the wait
   grid_dependency_wait();  // the partials and the status come from the face launches
   grid_dependents(kFewGatherBlocks);
-  if (*status) return;
+  if (!on) return;
+  // every load of the step at once, then the normals, then the sums
+  const Partials<T> partials(partial, at, c);
+  const int stopped = *status;
   const uint64_t st = current_step(cnt);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
-    const int v = i / 3, c = i - 3 * v;
-    const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
-    const philox_out o = normal_draw<T>(a.seed, a.stream, st, v, c);
-    double x;
-    if constexpr (sizeof(T) == 4) {
-      if (a.kind == 0) {
-        const GradSum s = coordinate_sum(partial, at.x, at.y, c);
-        x = bd_coordinate_f32(a, s.hi - s.lo, normal_f32(o, c), r[i]);
-        r[i] = x;
-        if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
-        continue;
-      }
+  const double r_old = r[i];
+  double q = a.kind != 0 ? p[i] : 0.0;
+  if (rhi) prefetch_l1(r0 + i);
+  if (stopped) return;
+  const philox_out o = normal_draw<T>(a.seed, a.stream, st, v, c);
+  double x;
+  if constexpr (sizeof(T) == 4) {
+    const float n = normal_f32(o, c);
+    if (a.kind == 0) {
+      const GradSum s = coordinate_sum(partials);
+      x = bd_coordinate_f32(a, s.hi - s.lo, n, r_old);
+    } else {
+      x = coordinate_update(a, coordinate_gradient(partials), convert::to_f64(n), r_old, &q);
     }
-    const double g = coordinate_gradient(partial, at.x, at.y, c);
-    double n, q = a.kind != 0 ? p[i] : 0.0;
-    if constexpr (sizeof(T) == 8) n = normal_f64(o, c);
-    else n = convert::to_f64(normal_f32(o, c));
-    x = coordinate_update(a, g, n, r[i], &q);
-    if (a.kind != 0) p[i] = q;
-    r[i] = x;
-    if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
+  } else {
+    const double n = normal_f64(o, c);
+    x = coordinate_update(a, coordinate_gradient(partials), n, r_old, &q);
   }
+  if (a.kind != 0) p[i] = q;
+  r[i] = x;
+  if (rhi) store_f32_position(i, x, rhi, rlo, r0, dsp);
 }
 
 // The mass path's first half, one thread per coordinate: gather the gradient,
@@ -842,18 +896,21 @@ template <typename T>
 __global__ void gather_kick_kernel(int nv, const T *__restrict__ partial, const int *__restrict__ off, StepArgs a,
                                    const uint64_t *__restrict__ cnt, double *__restrict__ p, float *__restrict__ x32,
                                    int ld, const int *__restrict__ status) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, v = i / 3, c = i - 3 * v;
+  const bool on = i < 3 * nv;
+  const int2 at = on ? __ldg(reinterpret_cast<const int2 *>(off) + v) : make_int2(0, 0);  // constant: before the wait
   grid_dependency_wait();
   grid_dependents(gridDim.x);  // the apply's first loads do not depend on this
-  if (*status) return;
+  if (!on) return;
+  const Partials<T> partials(partial, at, c);
+  const int stopped = *status;
   const uint64_t st = current_step(cnt);
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < 3 * nv; i += gridDim.x * blockDim.x) {
-    const int v = i / 3, c = i - 3 * v;
-    const int2 at = __ldg(reinterpret_cast<const int2 *>(off) + v);
-    const double n = normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c);
-    const double q = kick(a, n, p[i], coordinate_gradient(partial, at.x, at.y, c));
-    p[i] = q;
-    if (x32) x32[ld > 0 ? (size_t)c * ld + v : 4 * (size_t)v + c] = convert::to_f32(q);
-  }
+  const double p_old = p[i];
+  if (stopped) return;
+  const double n = normal_f64(normal_draw<double>(a.seed, a.stream, st, v, c), c);
+  const double q = kick(a, n, p_old, coordinate_gradient(partials));
+  p[i] = q;
+  if (x32) x32[ld > 0 ? (size_t)c * ld + v : 4 * (size_t)v + c] = convert::to_f32(q);
 }
 
 __global__ void drift_kernel(int nv, StepArgs a, double *__restrict__ r, double *__restrict__ p,
@@ -930,7 +987,6 @@ __device__ __forceinline__ float4 ld4(const float4 *p) {
                : "r"((uint32_t)__cvta_generic_to_shared(p)));
   return v;
 }
-__device__ __forceinline__ void prefetch_l1(const void *p) { asm volatile("prefetch.global.L1 [%0];" ::"l"(p)); }
 // Point of the face loop at which the thread prefetches its next face's table
 // rows (control points, g0, composition, slot destinations) into L1. Those
 // rows are otherwise first touched when the next face starts (control points,
@@ -1648,8 +1704,8 @@ __global__ void __launch_bounds__(kGeoThreads) geo_grad_kernel(GeoArgs G, T *__r
         int lfn;
         const GeoGroup &h = G.g[geo_group(G, fn, &lfn)];
         const size_t at = (size_t)lfn * h.ncp + (lane ? h.ncp - 1 : 0);
-        tpf::prefetch_l1(h.cp + at);
-        tpf::prefetch_l1(h.dest + at);
+        prefetch_l1(h.cp + at);
+        prefetch_l1(h.dest + at);
       }
     }
     int dest = 0;
