@@ -171,38 +171,62 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks)
   }
 }
 
-// Sum of the slots of coordinate t = 3 i + k of the product.
-__device__ __forceinline__ double slot_sum(int t, int chunks, long long units, long long W,
-                                           const double *__restrict__ part, int slots) {
-  const int i = t / 3, k = t - 3 * i, g = i / kRows, q = 3 * (i - g * kRows) + k;
-  const int ns = (int)(warp_of((long long)(g + 1) * chunks - 1, units, W) - warp_of((long long)g * chunks, units, W)) + 1;
-  double s = 0;
-  for (int a = 0; a < ns; ++a) s += part[((size_t)g * slots + a) * kSums + q];
-  return s;
-}
+// The slots of coordinate t = 3 i + k of the product and their sum, in order. Where
+// they lie does not depend on the kernel before: found (by 64-bit divisions) before
+// the wait for it.
+struct Slots {
+  const double *first;
+  int n;
+  __device__ __forceinline__ Slots(int t, int chunks, long long units, long long W, const double *__restrict__ part,
+                                   int slots) {
+    const int i = t / 3, k = t - 3 * i, g = i / kRows;
+    n = (int)(warp_of((long long)(g + 1) * chunks - 1, units, W) - warp_of((long long)g * chunks, units, W)) + 1;
+    first = part + (size_t)g * slots * kSums + 3 * (i - g * kRows) + k;
+  }
+  __device__ __forceinline__ double sum() const {
+    double s = 0;
+    int a = 0;
+    for (; a + 4 <= n; a += 4) {
+      double x[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) x[j] = first[(size_t)(a + j) * kSums];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s += x[j];
+    }
+    for (; a < n; ++a) s += first[(size_t)a * kSums];
+    return s;
+  }
+};
 
 // out (+)= f_c (scalev ? scalev[c n + i] : 1) (A x), one thread per coordinate.
 __global__ void dense_finish32_kernel(int n, int chunks, long long units, long long W, const double *__restrict__ part,
                                       int slots, MassScale f, const double *__restrict__ scalev,
                                       double *__restrict__ out, int accumulate) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, i = t / 3, k = t - 3 * i;
+  const bool on = t < 3 * n;
+  const Slots mine(on ? t : 0, chunks, units, W, part, slots);
   grid_dependency_wait();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * n) return;
-  const int i = t / 3, k = t - 3 * i;
+  if (!on) return;
   double v = f.f[k];
   if (scalev) v *= scalev[(size_t)k * n + i];
-  v *= slot_sum(t, chunks, units, W, part, slots);
-  out[t] = accumulate ? out[t] + v : v;
+  const double before = accumulate ? out[t] : 0.0;
+  v *= mine.sum();
+  out[t] = accumulate ? before + v : v;
 }
 
 __global__ void dense_drift32_kernel(int n, int chunks, long long units, long long W, const double *__restrict__ part,
                                      int slots, StepArgs a, double *__restrict__ r, double *__restrict__ p,
                                      float *__restrict__ rhi, float *__restrict__ rlo, const double *__restrict__ r0,
                                      float *__restrict__ dsp, const int *__restrict__ status) {
-  grid_dependency_wait();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= 3 * n || *status) return;
-  drift(a, t, slot_sum(t, chunks, units, W, part, slots), r, p, rhi, rlo, r0, dsp);
+  const bool on = t < 3 * n;
+  const Slots mine(on ? t : 0, chunks, units, W, part, slots);
+  grid_dependency_wait();
+  if (!on) return;
+  const int stopped = *status;
+  const double q = mine.sum();  // its loads go out beside the status word's
+  if (stopped) return;
+  drift(a, t, q, r, p, rhi, rlo, r0, dsp);
 }
 
 }  // namespace dense32
