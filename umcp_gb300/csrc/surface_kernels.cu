@@ -1535,13 +1535,14 @@ __global__ void batch_pack_kernel(const BatchJob *__restrict__ jobs, const Batch
 // Precision. The restraint on V is stiff (K_V (V - V0) is a force per unit
 // volume), so V must be exact far below an FP32 ulp of V: on a 1000 A vesicle
 // a 1e-3 A^3 error already moves every vertex's restraint force by about
-// K_V 1e-3 A^3 x 300 A^2. The sums kernel therefore forms R, R_u, R_v and
-// R.(R_u x R_v) in FP64 from FP64 local coordinates (relative to the patch
-// corner, which is added back exactly). The area, whose restraint is soft, and
-// the box-scale derivatives come from FP32 copies in the precision form. The
-// gradient kernel needs only the relative accuracy of any other gradient term
-// and runs in the form's own arithmetic (FP32 local coordinates from the hi/lo
-// pairs, as the face pass forms them).
+// K_V 1e-3 A^3 x 300 A^2. The sums therefore form R, R_u, R_v and R.(R_u x R_v)
+// beyond FP32 from local coordinates (relative to the patch corner, which is
+// added back exactly): in FP64 here, in integers and pairs of FP32 in the
+// precision form (geo32.cu), whose area, with its soft restraint, and box-scale
+// derivatives come from the FP32 leading parts. The gradient needs only the
+// relative accuracy of any other gradient term and runs in the form's own
+// arithmetic (FP32 local coordinates from the hi/lo pairs, as the face pass forms
+// them).
 
 constexpr int kGeoHW = kGeoThreads / 16;  // faces in flight per block
 
