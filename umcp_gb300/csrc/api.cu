@@ -379,8 +379,8 @@ class MeshArena {
     if (e != cudaSuccess) return e;
     unsigned char *base = store.as<unsigned char>();
     for (Part &q : parts_) q.buf->view(base + q.at, q.n);
-    if (!host_.empty()) e = cudaMemcpy(base, host_.data(), host_.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && zero_end > off[1]) e = cudaMemset(base + off[1], 0, zero_end - off[1]);
+    if (!host_.empty()) e = umcp::fill_device(base, host_.data(), host_.size());
+    if (e == cudaSuccess && zero_end > off[1]) e = umcp::fill_device(base + off[1], nullptr, zero_end - off[1]);
     return e;
   }
 
@@ -1074,7 +1074,7 @@ extern "C" umcp_status umcp_restraints_set(umcp_mesh *m, const umcp_restraints *
     UMCP_CUDA(m->geo_block.alloc((size_t)nblk * kGeoWords * sizeof(double)));
     UMCP_CUDA(m->gterm.alloc(kGeoWords * sizeof(double)));
     UMCP_CUDA(m->geo_done.alloc(sizeof(unsigned)));
-    UMCP_CUDA(cudaMemset(m->geo_done.p, 0, sizeof(unsigned)));
+    UMCP_CUDA(cudaMemsetAsync(m->geo_done.p, 0, sizeof(unsigned), s));
   }
   umcp_mesh::Restraints R;
   R.on = true;

@@ -216,11 +216,23 @@ inline uint32_t pack_cp(int v, const int8_t img[3]) {
   return (uint32_t)v | ((uint32_t)code << dev::kVertexBits);
 }
 
+// Device memory filled outside of any run, complete when the call returns: src's n
+// bytes into dst, or (src NULL) zeros. Copy and memset go to the legacy stream, so
+// that they neither wait for nor stall what the context's stream is running; that
+// stream does not wait for the legacy one in turn, and neither call waits for the
+// device by itself (a memset is only queued, and a copy from pageable memory may
+// return once its source has been staged).
+inline cudaError_t fill_device(void *dst, const void *src, size_t n) {
+  cudaError_t e = src ? cudaMemcpy(dst, src, n, cudaMemcpyHostToDevice) : cudaMemset(dst, 0, n);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(0);
+  return e;
+}
+
 template <class T>
 inline cudaError_t upload(DevBuf &b, const std::vector<T> &h) {
   cudaError_t e = b.alloc(h.size() * sizeof(T));
   if (e != cudaSuccess || h.empty()) return e;
-  return cudaMemcpy(b.p, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+  return fill_device(b.p, h.data(), h.size() * sizeof(T));
 }
 
 }  // namespace umcp

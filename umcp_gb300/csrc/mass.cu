@@ -275,10 +275,11 @@ cudaError_t umcp::queue_mass_product(umcp_mesh *m, const double *scalev, const M
 }
 
 cudaError_t umcp::alloc_mass_input(umcp_mesh *m, int n) {
-  // float4 per row (CSR), or three padded vectors (dense); the padding stays zero
+  // float4 per row (CSR, the fourth is never used), or three padded vectors (dense): their padding is zeroed here,
+  // on the stream of the kernels that write and read them, and stays zero
   const size_t bytes = !m->mass_f32 ? 0 : m->mass_dense ? 3 * (size_t)dense32_ld(n) * sizeof(float) : n * sizeof(float4);
   cudaError_t e = m->min32.alloc(bytes);
-  if (e == cudaSuccess && bytes) e = cudaMemset(m->min32.p, 0, bytes);
+  if (e == cudaSuccess && bytes && m->mass_dense) e = cudaMemsetAsync(m->min32.p, 0, bytes, m->ctx->stream);
   if (e == cudaSuccess)
     e = m->mpart.alloc(m->mass_f32 && m->mass_dense ? dense32_scratch_doubles(n) * sizeof(double) : 0);
   return e;
