@@ -743,7 +743,7 @@ static cudaError_t queue_faces(umcp_mesh *m, const double *d_r, const FinishArgs
   GeoArgs GA{};
   if (geo) {
     GA = geo_args(m, d_r);
-    cudaError_t e = sizeof(T) == 8 ? launch_geo_sums(GA, s) : launch_geo_sums32(GA, fused, s);
+    cudaError_t e = sizeof(T) == 8 ? launch_geo_sums(GA, fin.host_status != nullptr, s) : launch_geo_sums32(GA, fused, s);
     if (e != cudaSuccess) return e;
     fin.gterm = m->gterm.as<double>();
   }
@@ -1090,7 +1090,7 @@ extern "C" umcp_status umcp_restraints_set(umcp_mesh *m, const umcp_restraints *
       UMCP_CUDA(launch_split_positions(3 * m->nv, m->r.as<double>(), m->f32pos(), s));
     m->split_valid = true;
     const GeoArgs GA = geo_args(m, m->r.as<double>());
-    UMCP_CUDA(m->precision == UMCP_FP64 ? launch_geo_sums(GA, s) : launch_geo_sums32(GA, true, s));
+    UMCP_CUDA(m->precision == UMCP_FP64 ? launch_geo_sums(GA, false, s) : launch_geo_sums32(GA, true, s));
     double gt[kGeoWords];
     UMCP_CUDA(cudaMemcpyAsync(gt, m->gterm.p, sizeof gt, cudaMemcpyDeviceToHost, s));
     UMCP_CUDA(cudaStreamSynchronize(s));

@@ -65,8 +65,8 @@ inline int geo_blocks(int nfaces) {
   return b < 152 * 8 ? b : 152 * 8;
 }
 // Sums A, V and their alpha derivatives; the last block writes gterm. The plain
-// path, in FP64 throughout.
-cudaError_t launch_geo_sums(const GeoArgs &G, cudaStream_t s);
+// path, in FP64 throughout. staged: launch_stage_in comes before (a host call).
+cudaError_t launch_geo_sums(const GeoArgs &G, bool staged, cudaStream_t s);
 // The precision form (geo32.cu). fused: the face launches form the restraints' gradient (and with it dE_r/dalpha, which gterm then
 // has as zero): its SIMT kernels.
 cudaError_t launch_geo_sums32(const GeoArgs &G, bool fused, cudaStream_t s);

@@ -1983,8 +1983,9 @@ cudaError_t launch_split_positions(int n, const double *r, const F32Pos &f, cuda
   return cudaGetLastError();
 }
 
+constexpr int kStageThreads = 128;
 cudaError_t launch_stage_in(int n, const double *host_r, double *r, const F32Pos &f, int *status, cudaStream_t s) {
-  return launch_after(dev::stage_in_kernel, grid_for(n, 128), 128, 0, s, n, host_r, r, f.hi, f.lo, f.r0, f.dsp, status);
+  return launch_after(dev::stage_in_kernel, grid_for(n, kStageThreads), kStageThreads, 0, s, n, host_r, r, f.hi, f.lo, f.r0, f.dsp, status);
 }
 
 cudaError_t launch_status_merge(const int *src, int *dst, cudaStream_t s) {
@@ -2121,10 +2122,24 @@ cudaError_t launch_batch_pack(const BatchJob *jobs, const BatchTile *vtiles, con
 
 namespace umcp {
 
-cudaError_t launch_geo_sums(const GeoArgs &G, cudaStream_t s) {
-  return launch_after(dev::geo_sums_kernel, geo_blocks(G.nfaces), kGeoThreads, 0, s, G);
+// The FP64 pipe bounds the plain path's sums, so their blocks have to lie evenly over
+// the SMs. Launched early beside a gather or a host call's stage-in that triggers
+// (they do up to kFewGatherBlocks blocks), the blocks gather on the few SMs which
+// that kernel leaves first. So above kChainedSums blocks they are a plain launch on
+// meshes for which it triggers: a restrained evaluation of a 42 x 42 membrane (111
+// blocks) 174 -> 150 us. Below, the early launch gains 3% (36 x 36, 81 blocks: 147 /
+// 152 us; 38 x 38, 91 blocks: 172 / 150 us).
+constexpr int kChainedSums = 84;
+cudaError_t launch_geo_sums(const GeoArgs &G, bool staged, cudaStream_t s) {
+  const int grid = geo_blocks(G.nfaces);
+  const int triggering = (int)dev::kFewGatherBlocks * (staged ? kStageThreads : kGatherThreads) / 3;  // vertices
+  if (grid <= kChainedSums || G.nv > triggering)
+    return launch_after(dev::geo_sums_kernel, grid, kGeoThreads, 0, s, G);
+  dev::geo_sums_kernel<<<grid, kGeoThreads, 0, s>>>(G);
+  return cudaGetLastError();
 }
 
+// (The FP64 face pass does not trigger where this launch follows it, see face64.cu.)
 template <typename T>
 cudaError_t launch_geo_grad(const GeoArgs &G, T *partial, cudaStream_t s) {
   if (G.nfaces <= 0) return cudaSuccess;
