@@ -1863,11 +1863,15 @@ constexpr int kSpmvUnroll = 4;
 // there (40,962-vertex M^-1, 415 M nonzeros: 546 -> about 475 us per apply).
 constexpr int kSpmvAhead = 32;
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+// kSpmvBlocks: the blocks a SM that its 40 registers allow, given to the compiler. Left
+// to itself it took 34 (as many blocks) and put loads of a round behind one another:
+// 488 us a call with that matrix, 461 with all of them in flight.
+constexpr int kSpmvThreads = 256, kSpmvBlocks = 6;
 template <typename C>  // column index type: int, or uint16_t for up to 65,536 columns
-__global__ void spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C *__restrict__ col,
-                              const float *__restrict__ val, const double *__restrict__ scalev, MassScale F,
-                              const float4 *__restrict__ in4,
-                              double *__restrict__ out, int accumulate) {
+__global__ void __launch_bounds__(kSpmvThreads, kSpmvBlocks)
+    spmv32_kernel(int nrow, const int *__restrict__ row_ptr, const C *__restrict__ col, const float *__restrict__ val,
+                  const double *__restrict__ scalev, MassScale F, const float4 *__restrict__ in4,
+                  double *__restrict__ out, int accumulate) {
   grid_dependency_wait();
   const int lane = threadIdx.x & 31;
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -2034,16 +2038,15 @@ cudaError_t launch_spmv32(int nrow, const int *row_ptr, const void *col, bool co
                           const double *scalev, const MassScale &f, const float4 *in, double *out, int accumulate,
                           cudaStream_t s) {
   if (nrow <= 0) return cudaSuccess;
-  int warps_per_block = 8;
-  int grid = grid_for(nrow, warps_per_block);
+  int grid = grid_for(nrow, dev::kSpmvThreads / 32);
   if (grid > 152 * 16) grid = 152 * 16;
   // consecutive lanes take consecutive nonzeros, so runs of consecutive columns
   // gather the input with coalesced loads (a form with four nonzeros per lane,
   // 16-byte value loads, was slower: 0.80 against 0.55 ms at 40,962 rows)
   if (col16)
-    return launch_after(dev::spmv32_kernel<uint16_t>, grid, 32 * warps_per_block, 0, s, nrow, row_ptr,
+    return launch_after(dev::spmv32_kernel<uint16_t>, grid, dev::kSpmvThreads, 0, s, nrow, row_ptr,
                         static_cast<const uint16_t *>(col), val, scalev, f, in, out, accumulate);
-  return launch_after(dev::spmv32_kernel<int>, grid, 32 * warps_per_block, 0, s, nrow, row_ptr,
+  return launch_after(dev::spmv32_kernel<int>, grid, dev::kSpmvThreads, 0, s, nrow, row_ptr,
                       static_cast<const int *>(col), val, scalev, f, in, out, accumulate);
 }
 
