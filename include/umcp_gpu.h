@@ -360,8 +360,9 @@ typedef struct umcp_batch umcp_batch;
  * multiples of the face kernel's faces per block pass, irregular tiles of 1 to
  * 8 faces per half-warp, and the occupancy limit or one block fewer. The
  * choice is keyed by (device, precision, patch types present, log2 of the
- * face count) and, with tune_cache set, read from and written to that JSON
- * file, so a later batch of the same kind takes it without timing. The
+ * face count, version of the face kernels) and, with tune_cache set, read from
+ * and written to that JSON file, so a later batch of the same kind takes it
+ * without timing; entries of other versions stay in the file, unused. The
  * choice changes how the energy sums are grouped (their last bits), never the
  * per-vertex gradient sums, so trajectories do not depend on it. */
 typedef struct {

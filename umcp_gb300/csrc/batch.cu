@@ -372,7 +372,14 @@ struct Layout {
   double face_ms = 0;
 };
 
-// Key of a batch's kind: device, precision, patch types present, log2 of faces.
+// The face kernels a timed layout holds for: raised whenever a batch's face kernels
+// change, so that layouts timed with others are timed anew. (1: until the kernels
+// took four blocks a SM; a layout of three from then runs 256 vesicles' face pass in
+// 579 us instead of 550.)
+constexpr int kFaceKernels = 2;
+
+// Key of a batch's kind: device, precision, patch types present, log2 of faces,
+// face kernels.
 std::string layout_key(const umcp_batch *b, long long faces) {
   cudaDeviceProp prop;
   std::string dev = cudaGetDeviceProperties(&prop, b->ctx->device) == cudaSuccess ? prop.name : "device";
@@ -380,7 +387,8 @@ std::string layout_key(const umcp_batch *b, long long faces) {
   for (int t = 0; t < kTypes; ++t)
     if (b->have_type[t]) types += (types.empty() ? "" : "+") + std::to_string(t == 0 ? 6 : t == 1 ? 5 : 7);
   const int bucket = faces > 0 ? (int)std::floor(std::log2((double)faces)) : 0;
-  return dev + "|" + (b->precision == UMCP_FP64 ? "fp64" : "fp32") + "|" + types + "|" + std::to_string(bucket);
+  return dev + "|" + (b->precision == UMCP_FP64 ? "fp64" : "fp32") + "|" + types + "|" + std::to_string(bucket) + "|k" +
+         std::to_string(kFaceKernels);
 }
 
 // The cache file holds one JSON object, {"<key>": {"tile_faces": n,
