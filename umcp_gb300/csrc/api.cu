@@ -328,10 +328,25 @@ extern "C" umcp_status umcp_ctx_synchronize(umcp_ctx *ctx) {
 
 static void fill_params(umcp_mesh *m, const umcp_params *p) {
   m->kT = (5.92186663194E-01 / 298.0) * p->temperature;
-  m->P.kc = p->kc;
+  m->P.kc = p->kc * m->area_unit;
   m->P.KA = p->KA;
   m->P.kg = p->kg;
   m->P.k_reg = p->k_reg;
+  // the coefficients as f32::point_coef forms them, over the same in FP32
+  for (int k = 0; k < 2; ++k) {
+    const double dudv = k == 0 ? 0.5 : 1.0;
+    double sum[3] = {0, 0, 0}, rounded[3] = {0, 0, 0};
+    auto add = [&](int q, double c) {
+      sum[q] += c;
+      rounded[q] += (float)c;
+    };
+    for (double w : m->point_weight[k]) {
+      add(0, dudv * w * m->P.KA);
+      add(1, 0.25 * m->P.kc * w);
+    }
+    add(2, m->P.k_reg);
+    for (int q = 0; q < 3; ++q) m->P.e_scale[k][q] = rounded[q] != 0.0 ? sum[q] / rounded[q] : 1.0;
+  }
 }
 
 namespace {
@@ -426,6 +441,13 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
       m->P.box_hi[d][c] = (float)ME.box[d][c];
       m->P.box_lo[d][c] = (float)(ME.box[d][c] - (double)m->P.box_hi[d][c]);
     }
+  // A face's lipid areas P2 and Pres (composition_coeffs) are whole lipids times their
+  // area, so with lipids of one area every face's P2 would carry the same rounding to
+  // FP32 (136.6 A^2 for two: 4.5e-8), which no sum over faces averages out. Counted
+  // in lipids they are exact, and the unit goes into the points' coefficients.
+  if (prm->precision == UMCP_FP32_CENTRED && !PL.lipids.empty() && PL.lipids[0].apl > 0) m->area_unit = PL.lipids[0].apl;
+  m->point_weight[0] = PL.regular.weight;
+  m->point_weight[1] = PL.irregular[5].weight;
   fill_params(m.get(), prm);
 
   // Face groups: regular, then irregular by valence (5, 7).
@@ -495,6 +517,8 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
     if (prm->precision == UMCP_FP32_CENTRED) {  // the precision form's kernels read only the FP32 copies
       arena.stage(G->g0f, std::vector<float>(g0.begin(), g0.end()));
       arena.stage(G->rr0f, std::vector<float>(rr0.begin(), rr0.end()));
+      for (size_t q = 0; q < comp.size(); ++q)
+        if (q % 3 != 1) comp[q] /= m->area_unit;  // P2 and Pres; Hbar is a curvature
       arena.stage(G->compf, std::vector<float>(comp.begin(), comp.end()));
     } else {
       arena.stage(G->g0, g0);

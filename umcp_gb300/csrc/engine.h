@@ -108,6 +108,10 @@ struct umcp_mesh {
   umcp::DevBuf r_eval;    // staging for host-pointer energy/gradient calls (keeps the resident state)
   umcp::DevBuf done;      // finished-block counter of the face pass
   bool split_valid = false;  // the FP32 positions hold the resident state r
+  // unit of the faces' lipid areas in compf: the precision form counts them in lipids
+  // (see umcp_mesh_create), and P.kc is per unit
+  double area_unit = 1.0;
+  std::vector<double> point_weight[2];  // of regular and irregular patches (P.e_scale)
   double kT = 0.592186663194;  // kcal/mol at the params' temperature (src/hd.C:142-143)
   umcp::DevBuf energies;
   size_t energies_cap = 0;

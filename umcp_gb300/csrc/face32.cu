@@ -41,9 +41,10 @@ __device__ __forceinline__ void faces(Smem<NCP, NPT> &sm, const FaceSrc &S, cons
   }
 }
 
-// Block sums of n per-lane sums in a fixed order into out[n].
-__device__ __forceinline__ void block_row(double (*red)[6], const KahanSums<6> &sums, const double *scale, int n,
-                                          double *out) {
+// Block sums of n per-lane sums in a fixed order into out[n]: energies times e_scale
+// (SurfaceParams), box-scale derivatives over alpha.
+__device__ __forceinline__ void block_row(double (*red)[6], const KahanSums<6> &sums, const double *e_scale,
+                                          const double *alpha, int n, double *out) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
   for (int q = 0; q < 6; ++q) {
@@ -56,7 +57,7 @@ __device__ __forceinline__ void block_row(double (*red)[6], const KahanSums<6> &
     double s = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) s += red[w][threadIdx.x];
-    out[threadIdx.x] = threadIdx.x < 3 ? s : s / scale[threadIdx.x - 3];
+    out[threadIdx.x] = threadIdx.x < 3 ? s * e_scale[threadIdx.x] : s / alpha[threadIdx.x - 3];
   }
 }
 
@@ -84,7 +85,7 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block
     if (kg_reg) faces<NCP, NPT, true, false>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
     else faces<NCP, NPT, false, false>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
   }
-  block_row(sm.red, sums, r + 3 * (size_t)P.nv, want_da ? 6 : 3, row);
+  block_row(sm.red, sums, P.e_scale[NCP != 12], r + 3 * (size_t)P.nv, want_da ? 6 : 3, row);
 }
 
 }  // namespace f32
@@ -144,7 +145,7 @@ __global__ void __launch_bounds__(f32::kThreads, f32::kMinBlocks)
       else
         faces<NCP, NPT, false, false>(sm, src, sj.P, tile.first, end, pair, kWarps, w, dudv, false, (float *)sj.partial, sums);
     }
-    block_row(sm.red, sums, nullptr, 3, tile_sums + 3 * (size_t)(tile_base + t));
+    block_row(sm.red, sums, sj.P.e_scale[1], nullptr, 3, tile_sums + 3 * (size_t)(tile_base + t));
   }
 }
 

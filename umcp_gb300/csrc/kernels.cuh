@@ -54,6 +54,11 @@ struct SurfaceParams {
   double kc, KA, kg, k_reg;
   double box[3][3];
   float box_hi[3][3], box_lo[3][3];  // box = hi + lo, for the precision form
+  // Precision form, [regular, irregular patches][area, curvature, angle]: the points'
+  // coefficients over the same rounded to FP32. One relative error of every face
+  // alike, which no sum over faces averages out (all 15 weights of the regular rule
+  // are 1/15), so each block's or tile's energy sums are scaled by it, in FP64.
+  double e_scale[2][3];
   int nv;
 };
 

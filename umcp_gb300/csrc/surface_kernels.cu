@@ -535,14 +535,14 @@ __device__ bool tile(Smem &sm, const FaceSrc &S, const SurfaceParams &P, const f
 
 // Fixed-order block sum of the six per-thread sums into out[6] (global). The
 // reduction buffer lies over the Kb operand, which no MMA reads any more.
-__device__ void block_sums(Smem &sm, const KahanSums<6> &acc, double *out) {
+__device__ void block_sums(Smem &sm, const KahanSums<6> &acc, const SurfaceParams &P, double *out) {
   double(*red)[6] = reinterpret_cast<double(*)[6]>(&sm.A2[0][0]);
   for (int q = 0; q < 6; ++q) red[threadIdx.x][q] = acc.get(q);
   __syncthreads();
   if (threadIdx.x < 6) {
     double s = 0;
     for (int t = 0; t < kThreads; ++t) s += red[t][threadIdx.x];
-    out[threadIdx.x] = s;
+    out[threadIdx.x] = threadIdx.x < 3 ? s * P.e_scale[0][threadIdx.x] : s;
   }
   __syncthreads();
 }
@@ -573,7 +573,7 @@ __global__ void __launch_bounds__(tc::kThreads, 2)
   }
   if (!ok && threadIdx.x == 0) atomicOr(status, kStatusTimeout);
   tc::teardown(sm, phase, !ok);
-  tc::block_sums(sm, acc, blockpart + 6 * (size_t)(L.block_base + blockIdx.x));
+  tc::block_sums(sm, acc, P, blockpart + 6 * (size_t)(L.block_base + blockIdx.x));
   count_and_finish<tc::kThreads>(fin, blockpart);
 }
 
@@ -1273,7 +1273,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kMinBlocks)
     double s = 0;
 #pragma unroll
     for (int w = 0; w < kWarps; ++w) s += sm.red[w][threadIdx.x];
-    blockpart[6 * (size_t)(L.block_base + blockIdx.x) + threadIdx.x] = s;
+    blockpart[6 * (size_t)(L.block_base + blockIdx.x) + threadIdx.x] = threadIdx.x < 3 ? s * P.e_scale[0][threadIdx.x] : s;
   }
   count_and_finish<kThreads>(fin, blockpart);
 }
@@ -1353,7 +1353,7 @@ __global__ void __launch_bounds__(tpf::kThreads, tpf::kBatchMinBlocks)
       double s = 0;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) s += sm.red[w][threadIdx.x];
-      tile_sums[3 * (size_t)(tile_base + t) + threadIdx.x] = s;
+      tile_sums[3 * (size_t)(tile_base + t) + threadIdx.x] = s * sj.P.e_scale[0][threadIdx.x];
     }
   }
   __threadfence();  // this block's last draw on counter[0] is ordered before its count on counter[1]
