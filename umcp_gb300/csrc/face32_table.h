@@ -5,6 +5,8 @@
 #pragma once
 #include <string.h>
 
+#include <algorithm>
+#include <cmath>
 #include <vector>
 
 namespace umcp {
@@ -29,6 +31,41 @@ struct TpfRows {
   float V[15][12];     // value rows (restraints)
 };
 
+// A regular patch's first-derivative row in FP32, its entries chosen so that the row
+// still gives the derivative of a linear field: over the control points' lattice
+// coordinates (relative to control point 0, the patch corner) the rounding errors sum
+// to nothing, to about 4e-9. A field that is linear over the patch is most of the
+// tangents Ru and Rv, and every face has the same rows, so what plain rounding leaves
+// of the two sums is one relative error of every tangent (2e-8 of the curvature
+// energy). Largest entry first, each rounded after the least change of the entries
+// still to be rounded that takes up the errors so far.
+inline void round_tangent_row(const double *b, float *f) {
+  static const int at[12][2] = {{0, 0},  {0, 1},  {1, 0}, {1, -1}, {0, -1}, {-1, 0},
+                                {-1, 1}, {-1, 2}, {0, 2}, {1, 1},  {2, 0},  {2, -1}};
+  int order[12];
+  for (int x = 0; x < 12; ++x) order[x] = x;
+  std::stable_sort(order, order + 12, [&](int x, int y) { return std::fabs(b[x]) > std::fabs(b[y]); });
+  double sum[2] = {0, 0};  // errors so far times the lattice coordinates
+  for (int k = 0; k < 12; ++k) {
+    double uu = 0, uv = 0, vv = 0;
+    for (int i = k; i < 12; ++i) {
+      const int *q = at[order[i]];
+      uu += q[0] * q[0];
+      uv += q[0] * q[1];
+      vv += q[1] * q[1];
+    }
+    const int x = order[k], *q = at[x];
+    const double det = uu * vv - uv * uv;
+    double change = 0;
+    if (det > 0.5)
+      change = -(q[0] * (vv * sum[0] - uv * sum[1]) + q[1] * (uu * sum[1] - uv * sum[0])) / det;
+    else if (uu + vv > 0)  // the entries left lie on one line
+      change = -(q[0] * sum[0] + q[1] * sum[1]) / (uu + vv);
+    f[x] = (float)(b[x] + change);
+    for (int d = 0; d < 2; ++d) sum[d] += ((double)f[x] - b[x]) * q[d];
+  }
+}
+
 // Floats of a patch type's table.
 inline int f32_table_floats(int ncp) {
   return ncp == 12 ? F32Table<12, 15>::kFloats : ncp == 11 ? F32Table<11, 16>::kFloats : F32Table<13, 16>::kFloats;
@@ -40,13 +77,13 @@ void fill_f32_table(const std::vector<double> &basis, const std::vector<double> 
   using L = F32Table<NCP, NPT>;
   t->assign(L::kFloats, 0.f);
   for (int p = 0; p < NPT; ++p) {
-    for (int k = 0; k < 5; ++k)
-      for (int x = 0; x < NCP; ++x) {
-        const float b = (float)basis[((size_t)p * 5 + k) * (4 * L::NC4) + x];
-        (*t)[(size_t)(p * L::ROW4 + k * L::NC4) * 4 + x] = b;
-        if (k < 4) (*t)[L::kPoint4 + (p * NCP + x) * 4 + k] = b;
-        else (*t)[L::kPoint1 + p * 16 + x] = b;
-      }
+    for (int k = 0; k < 5; ++k) {
+      const double *row = &basis[((size_t)p * 5 + k) * (4 * L::NC4)];
+      float *f = &(*t)[(size_t)(p * L::ROW4 + k * L::NC4) * 4];
+      if (NCP == 12 && k < 2) round_tangent_row(row, f);
+      else std::copy(row, row + NCP, f);
+      for (int x = 0; x < NCP; ++x) (k < 4 ? (*t)[L::kPoint4 + (p * NCP + x) * 4 + k] : (*t)[L::kPoint1 + p * 16 + x]) = f[x];
+    }
     for (int x = 0; x < NCP; ++x) (*t)[L::kValue + p * 4 * L::NC4 + x] = (float)value[(size_t)p * NCP + x];
   }
   memcpy(t->data() + L::kWeights, weight.data(), NPT * sizeof(double));
