@@ -67,6 +67,9 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block
                                       double *__restrict__ row, bool want_da, const double *__restrict__ gterm) {
   Smem<NCP, NPT> &sm = *reinterpret_cast<Smem<NCP, NPT> *>(raw);
   const double w = stage(sm, G.table);
+  if (gterm)  // restraints
+    for (int i = threadIdx.x; i < NCP * F32Table<NCP, NPT>::NC4; i += kThreads)
+      (&sm.M[0][0])[i] = __ldg(reinterpret_cast<const float4 *>(G.table + F32Table<NCP, NPT>::kCorner) + i);
   __syncthreads();
   grid_dependency_wait();  // the state comes from the kernels before
   grid_dependents(kFewFaceBlocks);
@@ -78,6 +81,7 @@ __device__ __forceinline__ void group(void *raw, const FaceGroup32 &G, int block
   const bool kg_reg = P.kg != 0.0 || P.k_reg != 0.0;
   if (gterm) {  // restraints: their coefficients come from the sums kernel
     if (threadIdx.x < NPT) sm.geo[threadIdx.x] = geo_coef(gterm, w, G.dudv);
+    if (threadIdx.x == 0) sm.cV = (float)gterm[kGeoCV];
     __syncthreads();
     if (kg_reg) faces<NCP, NPT, true, true>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);
     else faces<NCP, NPT, false, true>(sm, S, P, 0, G.nfaces, pair, stride, w, G.dudv, want_da, partial, sums);

@@ -123,10 +123,35 @@ __device__ __forceinline__ Coef point_coef(const SurfaceParams &P, double w, dou
 }
 
 // The global restraints at a point: dE_r/dA and dE_r/dV times the point's area
-// and volume weights (cA cw, cV cw / 3), and the limit point (GEO).
+// and volume weights (cA cw, cV cw / 3), and the limit point relative to the patch
+// corner (GEO). The corner's own part of the volume gradient is formed once per face
+// (GeoCorner; corner_entry in face32_table.h has the reason): with absolute limit points
+// in the points' sums, the gradient of a 40,962-vertex vesicle under a volume restraint
+// was off by 1.07e-6 of its norm, now 6.5e-7.
 struct GeoPoint {
   float kA, kV;
   Vec3<float> R;
+};
+// The patch corner, absolute and box-scaled (it carries no image): x = hi + lo, times dE_r/dV.
+struct GeoCorner {
+  float x[3], hi[3], lo[3];
+  __device__ __forceinline__ GeoCorner(const float alpha[3], const float ahi[3], const float alo[3], float cV) {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const float p = mul(alpha[c], ahi[c]), e = fma(alpha[c], alo[c], fma(alpha[c], ahi[c], -p));
+      x[c] = add(p, e);
+      hi[c] = mul(cV, p);
+      lo[c] = fma(cV, e, fma(cV, p, -hi[c]));
+    }
+  }
+  // its part of control point j's gradient, t x (hi + lo) with t = sum_i M[j][i] X_i
+  __device__ __forceinline__ void gradient(const float t[3], float d[3]) const {
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+      const int a = (c + 1) % 3, b = (c + 2) % 3;
+      d[c] = fma(t[a], hi[b], fma(-t[b], hi[a], fma(t[a], lo[b], -mul(t[b], lo[a]))));
+    }
+  }
 };
 __device__ __forceinline__ float2 geo_coef(const double *gterm, double w, double dudv) {
   return make_float2((float)(gterm[kGeoCA] * (dudv * w)), (float)(gterm[kGeoCV] * (dudv * w) / 3.0));
@@ -153,8 +178,8 @@ struct Point {
 // of the gradient.
 // KG_REG = false: kg and k_reg are zero and their terms are left out.
 // GEO: the restraints' gradient goes along, dE_r/dg = kA (g = |m|), dE_r/dm =
-// kV R and dE_r/dR = kV m (the last for the caller: one more coefficient of m
-// beside lb, kb, nb, on the value row).
+// kV R (R relative to the corner) and dE_r/dR = kV m (the last for the caller: one
+// more coefficient of m beside lb, kb, nb, on the value row).
 // Products and sums are rounded as written (no contraction is left to the
 // compiler), so every kernel that inlines this rounds alike: a batch's job
 // follows its single-mesh trajectory bit for bit whichever kernels run it.
@@ -232,9 +257,12 @@ __device__ __forceinline__ Vec3<float> scale_derivative(const Point &o, const Ve
           one(o.Ku.y, K[0].y, o.Kv.y, K[1].y, o.m.y, K[2].y, K[3].y, K[4].y, s.y),
           one(o.Ku.z, K[0].z, o.Kv.z, K[1].z, o.m.z, K[2].z, K[3].z, K[4].z, s.z)};
 }
-// The restraints' value-row part of it, kV m . R.
-__device__ __forceinline__ Vec3<float> geo_scale_derivative(const Point &o, const GeoPoint &geo, const Vec3<float> &s) {
-  return {fma(mul(geo.kV, o.m.x), geo.R.x, s.x), fma(mul(geo.kV, o.m.y), geo.R.y, s.y), fma(mul(geo.kV, o.m.z), geo.R.z, s.z)};
+// The restraints' value-row part of it, kV m . (X0 + R). (The corner's part of the
+// volume gradient adds its own, sum_j d_j . X_j over GeoCorner::gradient.)
+__device__ __forceinline__ Vec3<float> geo_scale_derivative(const Point &o, const GeoPoint &geo, const float X0[3],
+                                                            const Vec3<float> &s) {
+  return {fma(mul(geo.kV, o.m.x), add(X0[0], geo.R.x), s.x), fma(mul(geo.kV, o.m.y), add(X0[1], geo.R.y), s.y),
+          fma(mul(geo.kV, o.m.z), add(X0[2], geo.R.z), s.z)};
 }
 
 }  // namespace f32
@@ -273,6 +301,9 @@ struct Smem {
   float4 D[kHW][3][L::NC4];         // the same points' change from the reference state
   float4 A[kHW][NPT][3];            // {Ku, lb}, {Kv, kb}, {m, nb} of each point
   float2 geo[16];                   // restraints: each point's kA, kV
+  float4 M[NCP][L::NC4];            // the corner matrix
+  float cV;                         // and dE_r/dV
+  float corner[kHW][2][3];          // and each face's corner, hi and lo
   double red[kWarps][6];
 };
 
@@ -347,10 +378,12 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
       for (int c = 0; c < 3; ++c) {
         reinterpret_cast<float *>(sm.X[hw][c])[lane] = mul(alpha[c], l[c]);
         reinterpret_cast<float *>(sm.D[hw][c])[lane] = fma(am1[c], l[c], sub(cur.dsp[c], ad[c]));
+        if (GEO && lane == 0) {
+          sm.corner[hw][0][c] = ahi[c];
+          sm.corner[hw][1][c] = alo[c];
+        }
       }
     }
-    if constexpr (GEO)  // the corner, absolute (it carries no image)
-      geo.R = {mul(alpha[0], add(ahi[0], alo[0])), mul(alpha[1], add(ahi[1], alo[1])), mul(alpha[2], add(ahi[2], alo[2]))};
   }
   __syncwarp();
   // ---- lanes as quadrature points; K[k]_c as two partial sums (even and odd
@@ -400,7 +433,7 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
     for (int k = 0; k < 2; ++k)
       dR[k] = {add(Ad[k][0].x, Ad[k][0].y), add(Ad[k][1].x, Ad[k][1].y), add(Ad[k][2].x, Ad[k][2].y)};
     if constexpr (GEO) {
-      geo.R = {add(geo.R.x, add(Av[0].x, Av[0].y)), add(geo.R.y, add(Av[1].x, Av[1].y)), add(geo.R.z, add(Av[2].x, Av[2].y))};
+      geo.R = {add(Av[0].x, Av[0].y), add(Av[1].x, Av[1].y), add(Av[2].x, Av[2].y)};
       geo.kA = sm.geo[lane].x;
       geo.kV = sm.geo[lane].y;
     }
@@ -414,7 +447,7 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
       if constexpr (KG_REG) sums.add(2, o.er);
       if (want_da) {
         Vec3<float> d = scale_derivative(o, K, {0.f, 0.f, 0.f});
-        if constexpr (GEO) d = geo_scale_derivative(o, geo, d);
+        if constexpr (GEO) d = geo_scale_derivative(o, geo, GeoCorner(alpha, sm.corner[hw][0], sm.corner[hw][1], 0.f).x, d);
         if (KG_REG && reg_alpha) {
           // the angle term's extra box-scale part (src/grad.C:7414-7421):
           // sum_x (b_u Kreg_u + b_v Kreg_v) X = Kreg_u Ru + Kreg_v Rv, times alpha - 1
@@ -441,6 +474,25 @@ __device__ __forceinline__ void face(Smem<NCP, NPT> &sm, int hw, int lane, const
       g[0] = fma(s, m.x, fma(b.y, v.x, fma(b.x, u.x, g[0])));
       g[1] = fma(s, m.y, fma(b.y, v.y, fma(b.x, u.y, g[1])));
       g[2] = fma(s, m.z, fma(b.y, v.z, fma(b.x, u.z, g[2])));
+    }
+    if (GEO && sm.cV != 0.f) {  // a volume restraint acts
+      float t[3] = {0.f, 0.f, 0.f};
+#pragma unroll 1
+      for (int c4 = 0; c4 < NC4; ++c4) {
+        const float4 w = sm.M[lane][c4];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          const float4 x = sm.X[hw][c][c4];
+          t[c] = fma(w.w, x.w, fma(w.z, x.z, fma(w.y, x.y, fma(w.x, x.x, t[c]))));
+        }
+      }
+      float d[3];
+      GeoCorner(alpha, sm.corner[hw][0], sm.corner[hw][1], sm.cV).gradient(t, d);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        g[c] = add(g[c], d[c]);
+        if (want_da && cur.on) sums.add(3 + c, mul(d[c], reinterpret_cast<const float *>(sm.X[hw][c])[lane]));
+      }
     }
     if (cur.dest >= 0)
       reinterpret_cast<float4 *>(partial)[cur.dest] =

@@ -1,7 +1,7 @@
 // The precision form's staged table of a patch type: the image of the leading
 // part of the half-warp face kernel's shared memory (face32.cuh), then the
-// quadrature weights. Formed once per mesh on the host, so that no block
-// converts rows from FP64.
+// quadrature weights, then the restraints' corner matrix. Formed once per mesh on
+// the host, so that no block converts rows from FP64.
 #pragma once
 #include <string.h>
 
@@ -20,7 +20,8 @@ struct F32Table {
   static constexpr int kPoint1 = kPoint4 + NPT * NCP * 4;  // [NPT][16]: vv
   static constexpr int kValue = kPoint1 + NPT * 16;        // [NPT][4 NC4]: the value row (restraints)
   static constexpr int kWeights = kValue + NPT * 4 * NC4;  // [16] doubles
-  static constexpr int kFloats = kWeights + 32;
+  static constexpr int kCorner = kWeights + 32;            // [NCP][4 NC4]: corner_matrix
+  static constexpr int kFloats = kCorner + NCP * 4 * NC4;
 };
 
 // The regular patch's rows for the thread-per-face kernel, which takes them as a
@@ -29,7 +30,25 @@ struct F32Table {
 struct TpfRows {
   float B[15][5][12];  // rows u, v, uu, uv, vv of each point
   float V[15][12];     // value rows (restraints)
+  float M[12][12];     // corner matrix (restraints)
 };
+
+// What the patch corner's position X0 has to do with the volume's gradient. Of the
+// limit point R in the volume's sum c R.(Ru x Rv) the gradient's terms b_u (Rv x R) +
+// b_v (R x Ru) take the corner's part as (sum_i M[j][i] X_i) x X0 for control point j,
+//   M[j][i] = sum over the points of c (b_u[j] b_v[i] - b_v[j] b_u[i]),  c = dudv w / 3.
+// The corner is a vesicle's radius away and the patch some tenths of an edge wide: left
+// in the points' sums, X0 makes of every product a number that the others cancel to a
+// fiftieth.
+inline double corner_entry(const double *basis, const std::vector<double> &weight, double dudv, int npt, int ncpp, int j,
+                           int i) {
+  double s = 0;
+  for (int p = 0; p < npt; ++p) {
+    const double *u = basis + (size_t)p * 5 * ncpp, *v = u + ncpp;
+    s += dudv * weight[p] / 3.0 * (u[j] * v[i] - v[j] * u[i]);
+  }
+  return s;
+}
 
 // A regular patch's first-derivative row in FP32, its entries chosen so that the row
 // still gives the derivative of a linear field: over the control points' lattice
@@ -87,6 +106,10 @@ void fill_f32_table(const std::vector<double> &basis, const std::vector<double> 
     for (int x = 0; x < NCP; ++x) (*t)[L::kValue + p * 4 * L::NC4 + x] = (float)value[(size_t)p * NCP + x];
   }
   memcpy(t->data() + L::kWeights, weight.data(), NPT * sizeof(double));
+  for (int j = 0; j < NCP; ++j)
+    for (int i = 0; i < NCP; ++i)
+      (*t)[L::kCorner + j * 4 * L::NC4 + i] =
+          (float)corner_entry(basis.data(), weight, NCP == 12 ? 0.5 : 1.0, NPT, 4 * L::NC4, j, i);
 }
 
 // The table from rows basis[npt][5][ncp rounded up to 4], value rows [npt][ncp] and the weights.
@@ -107,6 +130,7 @@ inline TpfRows tpf_rows(const std::vector<float> &table) {
     memcpy(r.B[p], &table[(size_t)p * L::ROW4 * 4], sizeof r.B[p]);
     memcpy(r.V[p], &table[L::kValue + (size_t)p * 12], sizeof r.V[p]);
   }
+  memcpy(r.M, &table[L::kCorner], sizeof r.M);
   return r;
 }
 

@@ -969,6 +969,7 @@ struct Smem {
   float2 C[kNpt];  // each point's coefficients curv, area (f32::Coef)
   float Cg[kNpt];  // and gauss
   float2 geo[kNpt];  // and kA, kV (restraints)
+  float cV;          // and dE_r/dV
   double red[kWarps][6];
 };
 constexpr size_t kSumBytes = sizeof(float) * 12 * kThreads;  // per-thread Kahan totals (dynamic shared memory)
@@ -1000,6 +1001,7 @@ __device__ __forceinline__ void tpf_stage_geo(tpf::Smem &sm, const float *__rest
   using L = F32Table<tpf::kNcp, tpf::kNpt>;
   if ((int)threadIdx.x < tpf::kNpt)
     sm.geo[threadIdx.x] = f32::geo_coef(gterm, __ldg(reinterpret_cast<const double *>(table + L::kWeights) + threadIdx.x), dudv);
+  if (threadIdx.x == 0) sm.cV = (float)gterm[kGeoCV];
 }
 // The points' coefficients for a mesh's moduli, by the block's first threads.
 __device__ __forceinline__ void tpf_coefs(tpf::Smem &sm, const float *__restrict__ table, const SurfaceParams &P,
@@ -1139,10 +1141,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const TpfRows &rows, con
     if constexpr (GEO) {
       geo.kA = sm.geo[p].x;
       geo.kV = sm.geo[p].y;
-      // the corner's absolute position (it carries no image) plus the local limit point
-      geo.R = {f32::add(f32::mul(alpha[0], f32::add(ahi[0], alo[0])), f32::add(Av[0].x, Av[0].y)),
-               f32::add(f32::mul(alpha[1], f32::add(ahi[1], alo[1])), f32::add(Av[1].x, Av[1].y)),
-               f32::add(f32::mul(alpha[2], f32::add(ahi[2], alo[2])), f32::add(Av[2].x, Av[2].y))};
+      geo.R = {f32::add(Av[0].x, Av[0].y), f32::add(Av[1].x, Av[1].y), f32::add(Av[2].x, Av[2].y)};
     }
     const f32::Point o = f32::point<KG_REG, GEO>(K, dR, M, k_reg, g0, rr0, P2, Hbar, Pres, geo);
     ea += o.ea;
@@ -1150,7 +1149,7 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const TpfRows &rows, con
     er += o.er;
     if (want_da) {
       da3 = f32::scale_derivative(o, K, da3);
-      if constexpr (GEO) da3 = f32::geo_scale_derivative(o, geo, da3);
+      if constexpr (GEO) da3 = f32::geo_scale_derivative(o, geo, f32::GeoCorner(alpha, ahi, alo, 0.f).x, da3);
     }
     // G[j]_c += B[u][j] Kb[u]_c + B[v][j] Kb[v]_c + s[j] m_c in scalar multiply-adds: with the
     // forward contraction in paired ones, the mix keeps both FP32 multiply-add pipes busy
@@ -1170,6 +1169,30 @@ __device__ __forceinline__ void tpf_face(tpf::Smem &sm, const TpfRows &rows, con
           for (int cc = 0; cc < 3; ++cc) g[cc] = fmaf(sj, md[cc], fmaf(v[jj], kv[cc], fmaf(u[jj], ku[cc], g[cc])));
         }
       }
+    }
+  }
+  if (GEO && sm.cV != 0.f) {  // the corner's part of the volume gradient, where that restraint acts
+    float x[3][kNcp];
+#pragma unroll
+    for (int c = 0; c < 3; ++c)
+#pragma unroll
+      for (int c4 = 0; c4 < kNc4; ++c4) {
+        const float4 v = ld4(&xs[kNc4 * c + c4]);
+        x[c][4 * c4] = v.x; x[c][4 * c4 + 1] = v.y; x[c][4 * c4 + 2] = v.z; x[c][4 * c4 + 3] = v.w;
+      }
+    const f32::GeoCorner corner(alpha, ahi, alo, sm.cV);
+#pragma unroll
+    for (int j = 0; j < kNcp; ++j) {
+      float t[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+      for (int i = 0; i < kNcp; ++i)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) t[c] = fmaf(rows.M[j][i], x[c][i], t[c]);
+      float d[3];
+      corner.gradient(t, d);
+#pragma unroll
+      for (int c = 0; c < 3; ++c) G[j][c] = f32::add(G[j][c], d[c]);
+      if (want_da) da3 = {fmaf(d[0], x[0][j], da3.x), fmaf(d[1], x[1][j], da3.y), fmaf(d[2], x[2][j], da3.z)};
     }
   }
   // ---- dE/dalpha_c: K is linear in the alpha-scaled coordinates, so
