@@ -8,6 +8,7 @@
 #include <cstring>
 #include <fstream>
 #include <memory>
+#include <mutex>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -394,8 +395,9 @@ class MeshArena {
     if (e != cudaSuccess) return e;
     unsigned char *base = store.as<unsigned char>();
     for (Part &q : parts_) q.buf->view(base + q.at, q.n);
-    if (!host_.empty()) e = umcp::fill_device(base, host_.data(), host_.size());
-    if (e == cudaSuccess && zero_end > off[1]) e = umcp::fill_device(base + off[1], nullptr, zero_end - off[1]);
+    // zeros first, on the copy's stream: the wait is for both
+    if (zero_end > off[1]) e = cudaMemsetAsync(base + off[1], 0, zero_end - off[1], cudaStreamLegacy);
+    if (e == cudaSuccess) e = umcp::fill_device(base, host_.data(), host_.size());
     return e;
   }
 
@@ -419,6 +421,28 @@ static size_t slot_bytes(int precision) {
 // Whether a regular group of the precision form takes the thread-per-face
 // kernel instead of the half-warp one.
 static bool use_tpf(int ncp, int nfaces) { return ncp == 12 && nfaces >= kTpfFaces; }
+
+// A patch type's staged tables. They depend on its valence only, and a process forms
+// each once (making a 162-vertex FP64 mesh took 126 us with its tables, 109 without).
+namespace {
+struct PatchTables {
+  std::vector<int> fixed;
+  std::vector<float> f32;
+  TpfRows rows;  // regular patches
+};
+}  // namespace
+static const PatchTables &patch_tables(const PatchBasis &B, const std::vector<double> &basis,
+                                       const std::vector<double> &value, int ncpp) {
+  static std::once_flag once[8];
+  static PatchTables tables[8];
+  PatchTables &t = tables[B.valence];
+  std::call_once(once[B.valence], [&] {
+    t.fixed = fixed::basis_table(basis, B.ncp, B.npt, ncpp);
+    t.f32 = f32_table(basis, value, B.weight, B.ncp);
+    if (B.ncp == 12) t.rows = tpf_rows(t.f32);
+  });
+  return t;
+}
 
 extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, const umcp_params *prm, umcp_mesh **out) {
   if (!ctx || !plan || !out) return fail(UMCP_ERR_INVALID, "null argument");
@@ -513,7 +537,6 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
     block_rows += group_block_rows(prm->precision, G->ncp, G->nfaces);
     arena.stage(G->cp, cp);
     arena.stage(G->basis, basis);
-    if (prm->precision == UMCP_FP64) arena.stage(G->table, fixed::basis_table(basis, G->ncp, G->npt, ncpp));
     if (prm->precision == UMCP_FP32_CENTRED) {  // the precision form's kernels read only the FP32 copies
       arena.stage(G->g0f, std::vector<float>(g0.begin(), g0.end()));
       arena.stage(G->rr0f, std::vector<float>(rr0.begin(), rr0.end()));
@@ -531,10 +554,12 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
       for (int p = 0; p < G->npt; ++p)
         for (int x = 0; x < G->ncp; ++x) bw[(size_t)p * G->ncp + x] = B.at(0, p, x);
       arena.stage(G->basis_w, bw);
-      if (prm->precision == UMCP_FP32_CENTRED) {
-        const std::vector<float> table = f32_table(basis, bw, B.weight, G->ncp);
-        if (G->ncp == 12) G->rows = tpf_rows(table);
-        arena.stage(G->table, table);
+      const PatchTables &T = patch_tables(B, basis, bw, ncpp);
+      if (prm->precision == UMCP_FP64) {
+        arena.stage(G->table, T.fixed);
+      } else {
+        if (G->ncp == 12) G->rows = &T.rows;
+        arena.stage(G->table, T.f32);
       }
     }
     face_base += G->nfaces;
@@ -743,7 +768,7 @@ static cudaError_t queue_groups(umcp_mesh *m, const FaceBuffers &B, const Finish
   L.dudv = own->dudv;
   e = own->tc ? launch_faces_tc(L, own->dest.as<int>(), m->P, B.r, B.f32.hi, B.f32.lo, B.f32.dsp, partial, B.blockpart,
                                 B.status, own->nblocks, fin, s)
-              : launch_faces_tpf(own->rows, L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
+              : launch_faces_tpf(*own->rows, L, own->dest.as<int>(), m->P, B.r, B.f32, partial, B.blockpart, B.status, own->nblocks,
                                  fin, geo, s);
   if (e == cudaSuccess)
     e = launch_faces32(F, m->P, B.r, B.f32, partial, B.blockpart, fin, fork ? m->ctx->side : s, !fork);

@@ -609,7 +609,7 @@ extern "C" umcp_status umcp_batch_add(umcp_batch *b, umcp_mesh *m, const umcp_in
     UMCP_CUDA(b->weight[t].alloc(G.weight.bytes));
     UMCP_CUDA(cudaMemcpyAsync(b->table[t].p, G.table.p, G.table.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
     UMCP_CUDA(cudaMemcpyAsync(b->weight[t].p, G.weight.p, G.weight.bytes, cudaMemcpyDeviceToDevice, b->ctx->stream));
-    if (t == 0) b->rows = G.rows;
+    if (t == 0 && G.rows) b->rows = *G.rows;
     b->dudv[t] = G.dudv;
     b->have_type[t] = true;
     b->drop_graphs();  // the captured steps do not launch this type yet

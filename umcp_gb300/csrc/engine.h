@@ -56,7 +56,7 @@ struct Group {
   DevBuf cp, g0, rr0, comp, basis, weight, dest;
   DevBuf basis_w;           // value rows [npt][ncp] (area and volume terms)
   DevBuf table;             // staged rows: fixed point in the plain path (fixed64.h), else FP32 (face32_table.h)
-  TpfRows rows;             // regular patches of the precision form: the thread-per-face kernel's parameter
+  const TpfRows *rows = nullptr;  // regular patches of the precision form: the thread-per-face kernel's parameter
   DevBuf g0f, rr0f, compf;  // FP32 copies for the precision form
   DevBuf geo_tab;           // the precision form's restraint table (GeoGroup::tab), built when restraints are first set
 };
