@@ -500,7 +500,6 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
     G->npt = B.npt;
     G->nfaces = (int)s.idx.size();
     G->slot_base = slot_base;
-    G->irregular = s.irr;
     G->valence = B.valence;
     G->dudv = s.irr ? 1.0 : 0.5;
     for (int f : s.idx) G->face_index.push_back(s.irr ? (int)PL.reg_faces.size() + f : f);
@@ -591,7 +590,6 @@ extern "C" umcp_status umcp_mesh_create(umcp_ctx *ctx, const umcp_plan *plan, co
   std::copy(ME.r.begin(), ME.r.end(), r0.begin());
   r0[3 * ME.nv] = r0[3 * ME.nv + 1] = r0[3 * ME.nv + 2] = 1.0;
   arena.stage(m->r, r0);
-  arena.uninit(m->g, nst * sizeof(double));
   arena.zeroed(m->p, 3 * (size_t)ME.nv * sizeof(double));
   arena.uninit(m->qdot, 3 * (size_t)ME.nv * sizeof(double));
   arena.uninit(m->E, sizeof(double));
@@ -960,7 +958,7 @@ extern "C" umcp_status umcp_plan_device_bytes(const umcp_plan *plan, umcp_ctx *c
   b += 2 * nv * 4;                                    // slot locations
   b += (size_t)std::max(nblocks, 1) * 6 * 8;          // blockpart
   b += slots * slot_bytes(precision);                 // partial
-  b += 3 * nst * 8 + 2 * 3 * nv * 8;                  // r, g, r_eval; p, qdot
+  b += 2 * nst * 8 + 2 * 3 * nv * 8;                  // r, r_eval; p, qdot
   b += 8 + 3 * 8 + 4 + 2 * 8 + 4;                     // E, parts, status, cnt, done
   if (f32) b += dev::kPosStride * nv * 4 + 3 * nv * 8;  // hi, lo, dsp; r0
   b += (size_t)n_energies * 8;                        // energy record

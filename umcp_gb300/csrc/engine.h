@@ -46,7 +46,7 @@ struct DevBuf {
 };
 
 struct Group {
-  int ncp = 0, npt = 0, nfaces = 0, slot_base = 0, irregular = 0;
+  int ncp = 0, npt = 0, nfaces = 0, slot_base = 0;
   int valence = 6;                  // of the patch type's lowest corner
   std::vector<int> face_index;      // each face's index in the plan (regular faces, then irregular)
   bool tc = false;                  // regular faces of the precision form on the tensor cores
@@ -102,7 +102,7 @@ struct umcp_mesh {
   std::vector<std::unique_ptr<umcp::Group>> groups;
   umcp::DevBuf partial, off, blockpart;
   int nblocks = 0;
-  umcp::DevBuf r, g, p, qdot, E, parts, status, cnt;  // cnt: {first step of the run, run index}
+  umcp::DevBuf r, p, qdot, E, parts, status, cnt;  // cnt: {first step of the run, run index}
   umcp::DevBuf pos32;     // precision form: FP32 positions hi, lo (r = hi + lo) and r - r0 (dev::kPosStride floats a vertex)
   umcp::DevBuf r0;        // precision form: reference state (FP64)
   umcp::DevBuf r_eval;    // staging for host-pointer energy/gradient calls (keeps the resident state)
@@ -162,7 +162,7 @@ struct umcp_mesh {
       for (const umcp::DevBuf *x : {&G->cp, &G->g0, &G->rr0, &G->comp, &G->basis, &G->weight, &G->dest, &G->g0f,
                                     &G->rr0f, &G->compf, &G->basis_w, &G->table, &G->geo_tab})
         b += x->bytes;
-    for (const umcp::DevBuf *x : {&partial, &off, &blockpart, &r, &g, &p, &qdot, &E, &parts, &status, &cnt, &pos32,
+    for (const umcp::DevBuf *x : {&partial, &off, &blockpart, &r, &p, &qdot, &E, &parts, &status, &cnt, &pos32,
                                   &r0, &r_eval, &done, &energies, &mrow, &mcol, &mval, &mdense, &min32, &mpart, &geo_block, &gterm,
                                   &geo_done})
       b += x->bytes;

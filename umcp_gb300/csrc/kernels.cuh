@@ -90,14 +90,6 @@ template <typename T>
 struct Vec3 {
   T x, y, z;
 };
-template <typename T>
-__device__ __forceinline__ Vec3<T> cross(const Vec3<T> &a, const Vec3<T> &b) {
-  return {a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
-}
-template <typename T>
-__device__ __forceinline__ T dot(const Vec3<T> &a, const Vec3<T> &b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z;
-}
 
 }  // namespace dev
 }  // namespace umcp
