@@ -103,3 +103,36 @@ def test_mesh_and_restraints_made_beside_a_busy_legacy_stream(tmp_path, precisio
         assert np.array_equal(a, b)
     O = B.Oracle(plan, prm)
     assert rel_inf(outs[0][1][:-3], O.grad(r)[:-3]) <= (1e-10 if precision == U.FP64 else 1e-6)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [U.FP64, U.FP32_CENTRED])
+def test_runs_queued_behind_one_another_keep_their_steps(tmp_path, precision):
+    """Two runs queued while the context's stream is still busy draw the noise of
+    their own steps, as the same runs do one by one."""
+    torch = pytest.importorskip("torch")
+    path = tmp_path / "m.mesh"
+    U.generate_icosphere(path, 2, 75.0, 0.5, 3)
+    prm = U.params(precision=precision)
+    plan = U.Plan(path, prm)
+    it = U.integrator(U.OVERDAMPED_BD, time_step=1.0, D=1e-4, seed=5, stream=2)
+    states = []
+    for queued in (False, True):
+        ctx = U.Context(0)
+        m = U.Mesh(ctx, plan, prm)
+        m.run(it, 0, 16)  # the steps are captured
+        m.state_set(plan.positions())
+        x = torch.ones(1 << 28, device="cuda")
+        torch.cuda.synchronize()
+        if queued:
+            with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream())):
+                for _ in range(100):  # some 30 ms
+                    x.mul_(1.0)
+        for step0 in (40, 1000, 56):
+            m.run_async(it, step0, 16)
+            if not queued:
+                ctx.synchronize()
+        ctx.synchronize()
+        states.append(m.state_get()[0])
+        del x
+    assert np.array_equal(*states)

@@ -351,20 +351,19 @@ static void fill_params(umcp_mesh *m, const umcp_params *p) {
 }
 
 namespace {
-// The pinned host staging of the host-pointer calls (state in and out, run
-// counters), allocated at the first such call: meshes run only from the
+// The pinned host staging of the host-pointer calls (state in and out),
+// allocated at the first such call: meshes run only from the
 // device (batches, servers) never pay for page-locking.
 cudaError_t ensure_pinned(umcp_mesh *m) {
   if (m->h_pinned) return cudaSuccess;
   const size_t nst = 3 * (size_t)m->nv + 3;
   const size_t a = (nst * sizeof(double) + 63) & ~(size_t)63, b = (3 * (size_t)m->nv * sizeof(double) + 63) & ~(size_t)63;
-  cudaError_t e = cudaMallocHost(&m->h_pinned, a + b + 2 * sizeof(uint64_t) + (nst + 5) * sizeof(double));
+  cudaError_t e = cudaMallocHost(&m->h_pinned, a + b + (nst + 5) * sizeof(double));
   if (e != cudaSuccess) return e;
   unsigned char *h = (unsigned char *)m->h_pinned;
   m->h_stage = (double *)h;
   m->h_stage2 = (double *)(h + a);
-  m->h_cnt = (uint64_t *)(h + a + b);
-  m->h_eval = (double *)(m->h_cnt + 2);
+  m->h_eval = (double *)(h + a + b);
   return cudaSuccess;
 }
 
@@ -1271,10 +1270,10 @@ static umcp_status run_steps(umcp_mesh *m, const umcp_integrator *it, uint64_t s
   if (m->precision == UMCP_FP32_CENTRED && !m->split_valid)
     UMCP_CUDA(launch_split_positions(3 * m->nv, m->r.as<double>(), m->f32pos(), s));
   m->split_valid = true;  // every step rewrites the pairs of the new positions
-  UMCP_CUDA(ensure_pinned(m));
-  m->h_cnt[0] = step0;
-  m->h_cnt[1] = 0;
-  UMCP_CUDA(cudaMemcpyAsync(m->cnt.p, m->h_cnt, 2 * sizeof(uint64_t), cudaMemcpyHostToDevice, s));
+  // from pageable memory, which is read before the call returns: a run may be queued
+  // while one before it has yet to start
+  const uint64_t start[2] = {step0, 0};
+  UMCP_CUDA(cudaMemcpyAsync(m->cnt.p, start, sizeof start, cudaMemcpyHostToDevice, s));
   UMCP_CUDA(cudaMemsetAsync(m->status.p, 0, sizeof(int), s));
   const int use_mass = (it->kind != 0 && it->use_mass) ? 1 : 0;
   // kGraphChunk steps at a time, then the rest as one captured run per set bit

@@ -126,7 +126,6 @@ struct umcp_mesh {
   void *h_pinned = nullptr;   // one pinned block holding the three below
   double *h_stage = nullptr;  // pinned, 3*nv+3 doubles
   double *h_stage2 = nullptr; // pinned, 3*nv doubles
-  uint64_t *h_cnt = nullptr;  // pinned, 2 counters
   // pinned, written by the kernels of a host call: gradient (3*nv+3 doubles), energy, its three parts, the status word
   double *h_eval = nullptr;
   // effective inverse mass: CSR (mrow, mcol, mval) or dense row-major (mdense);
