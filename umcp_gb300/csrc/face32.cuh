@@ -113,8 +113,9 @@ __device__ __forceinline__ void local_position(const float hi[3], const float lo
 }
 
 // The moduli times a quadrature point's weight, formed in FP64 once per launch
-// or job and rounded once: kc w / 4, dudv w KA, dudv w kg. (Products of rounded
-// factors carry one rounding into every face alike, 1e-7 of the energy.)
+// or job and rounded once: kc w / 4, dudv w KA, dudv w kg. (The weights of a rule
+// being equal, all faces share that rounding; SurfaceParams::e_scale takes it out of
+// the energies.)
 struct Coef {
   float curv, area, gauss;
 };

@@ -162,8 +162,10 @@ __global__ void __launch_bounds__(f64::kThreads, f64::kMinBlocks)
 
 int face_blocks64(int nfaces) {
   if (nfaces <= 0) return 0;
-  // Persistent grid: as many blocks as fit on the device at once (a fixed
-  // number per device, so the face-to-block assignment and the sums' order are fixed).
+  // A group's persistent grid: at most as many blocks as fit on the device at once (a
+  // fixed number per device, so the face-to-block assignment and the sums' order are
+  // fixed). A launch takes the groups' grids together: on a mesh whose regular group
+  // fills the device, the irregular groups' few blocks make a second wave.
   static PerDevice pd;
   const int cached = per_device(pd, [] {
     int per_sm = 0;

@@ -13,9 +13,9 @@ namespace umcp {
 // Status bits written by kernels into the mesh's device status word.
 enum : int { kStatusNonFinite = 1, kStatusDiverged = 2, kStatusTimeout = 4 };
 
-// Where and how the block partials of a face pass are summed (see
-// launch_finish). done: device counter of finished blocks, zero between
-// launches; when non-null, the last block of that face launch does the sum.
+// Where and how the block partials of a face pass are summed (dev::count_and_finish).
+// done: device counter of finished blocks, zero between launches; when non-null,
+// the last block of the pass's face launches does the sum.
 struct FinishArgs {
   int nblk;            // block-partial rows to sum: every block of every face launch of the pass, each of
                        // which counts on `done`; the block that brings it to nblk sums the rows
@@ -30,8 +30,9 @@ struct FinishArgs {
   int store_galpha;    // galpha is overwritten instead of added to
 };
 
-// Global area and volume of the limit surface and their restraint (one
-// half-warp per face over every patch type; V in FP64, see geo_sums_kernel):
+// Global area and volume of the limit surface and their restraint, over every patch
+// type (the plain path in FP64, a half-warp per face: geo_sums_kernel; the precision
+// form with V beyond FP32, four warps per 32 faces: geo32.cu):
 //   A = sum dudv w |Ru x Rv|,  V = 1/3 sum dudv w R.(Ru x Rv)
 //   E_r = 1/2 K_A (A-A0)^2/A0 + 1/2 K_V (V-V0)^2
 // gterm receives {A, V, E_r, dE_r/dA, dE_r/dV, dE_r/dalpha_xyz}.
@@ -50,7 +51,7 @@ struct GeoArgs {
   GeoGroup g[3];
   int ngroups, nfaces, nv;
   const double *r;
-  const float *rhi, *rlo;  // r = hi + lo (precision form; read by the FP32 gradient pass)
+  const float *rhi, *rlo;  // r = hi + lo (precision form)
   double box[3][3];
   float box_hi[3][3], box_lo[3][3];
   double KA, A0, KV, V0;

@@ -1894,7 +1894,7 @@ constexpr int kSpmvUnroll = 4;
 // spmv32_kernel streams each row's values and columns, kSpmvUnroll windows of
 // 32 nonzeros per warp iteration; a warp also asks L2 for the lines
 // kSpmvAhead windows ahead of the ones it loads, so that its loads find them
-// there (40,962-vertex M^-1, 415 M nonzeros: 546 -> about 475 us per apply).
+// there (40,962-vertex M^-1, 415 M nonzeros: 546 -> 475 us per apply when it came in).
 constexpr int kSpmvAhead = 32;
 __device__ __forceinline__ void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 // kSpmvBlocks: the blocks a SM that its 40 registers allow, given to the compiler. Left
