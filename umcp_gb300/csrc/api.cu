@@ -982,6 +982,7 @@ extern "C" umcp_status umcp_mass_set(umcp_mesh *m, int nrow, const int *row_ptr,
   for (int k = 0; k < nnz; ++k)
     if (col[k] < 0 || col[k] >= m->nv) return fail(UMCP_ERR_INVALID, "column index out of range");
   UMCP_CUDA(cudaSetDevice(m->ctx->device));
+  m->mrows = 0;  // none installed until all of it is: an allocation may fail on the way
   UMCP_CUDA(upload(m->mrow, std::vector<int>(row_ptr, row_ptr + nrow + 1)));
   m->mass_f32 = m->precision == UMCP_FP32_CENTRED;  // the precision form applies M^-1 in FP32
   m->mcol16 = m->mass_f32 && nrow <= 65536;         // and stores its columns in 16 bits when they fit

@@ -377,6 +377,7 @@ extern "C" umcp_status umcp_mass_build(umcp_mesh *m, const umcp_plan *plan, cons
   // the precision form keeps M^-1 in FP32 (rounded once from the FP64 inverse)
   const bool f32 = m->precision == UMCP_FP32_CENTRED;
   if (fill >= 0.3) {
+    m->mrows = 0;  // none installed until all of it is: an allocation may fail on the way
     if (f32) {
       UMCP_CUDA(m->mdense.alloc((size_t)n * dense32_ld(n) * sizeof(float)));
       dense_to_f32_kernel<<<sms * 8, 256, 0, s>>>(n, dense32_ld(n), A.as<double>(), m->mdense.as<float>());
@@ -404,6 +405,7 @@ extern "C" umcp_status umcp_mass_build(umcp_mesh *m, const umcp_plan *plan, cons
     UMCP_CUDA(cudaStreamSynchronize(s));
     for (int i = 0; i < n; ++i) rp[(size_t)i + 1] = rp[i] + cnt[i];
     if ((unsigned long long)rp[n] != kept) return fail(UMCP_ERR_CUDA, "M^-1 nonzero count mismatch between the truncation and the CSR pass");
+    m->mrows = 0;
     UMCP_CUDA(upload(m->mrow, rp));
     m->mcol16 = f32 && n <= 65536;
     UMCP_CUDA(m->mcol.alloc(kept * (m->mcol16 ? sizeof(uint16_t) : sizeof(int))));
